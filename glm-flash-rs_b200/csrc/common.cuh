@@ -73,8 +73,16 @@ int launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaS
 
 // ---- codebook ------------------------------------------------------------------------------------------
 // The 32-bit codeword of a 16-bit trellis state: two fp16 halves whose sum is the weight
-// (upstream native/exl3.cu:21-25).
-__device__ __forceinline__ uint32_t codeword(uint32_t state) { return ((state * MCG_MUL) & MCG_AND) ^ MCG_XOR; }
+// (upstream native/exl3.cu:21-25).  Mask and flip are ONE three-input logic instruction, asked for by name: written as
+// (x & A) ^ X the compiler splits the constant into a part inside and a part outside the mask and issues two, and the
+// integer ALU they run on is what every decode loop of this library waits for (5.97 -> 4.99 instructions per weight,
+// 15.7 -> 19.1 weights per clock and SM in a loop that does nothing else).
+__device__ __forceinline__ uint32_t mcg_mask(uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(x), "r"(MCG_AND), "r"(MCG_XOR));   // 0x6a: (a & b) ^ c
+    return r;
+}
+__device__ __forceinline__ uint32_t codeword(uint32_t state) { return mcg_mask(state * MCG_MUL); }
 
 // The weight itself: half-precision sum of the two halves, round to nearest even (upstream :26-29).
 __device__ __forceinline__ __half codebook(uint32_t state) {
@@ -96,8 +104,8 @@ __device__ __forceinline__ void codeword_pair(uint32_t u, uint32_t &x_hi, uint32
     asm("mul.lo.u32 %0, %1, %2;" : "=r"(ph) : "r"(h), "r"(MCG_MUL));
     asm("mul.lo.u32 %0, %1, %2;" : "=r"(pu) : "r"(u), "r"(MCG_MUL));
     asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(pl) : "r"(ph), "r"(0xFFFF0000u), "r"(pu));
-    x_hi = (ph & MCG_AND) ^ MCG_XOR;
-    x_lo = (pl & MCG_AND) ^ MCG_XOR;
+    x_hi = mcg_mask(ph);
+    x_lo = mcg_mask(pl);
 #else
     x_hi = codeword(h);
     x_lo = codeword(u & 0xffffu);
