@@ -8,52 +8,23 @@
 
 namespace gf {
 
-// logits[r][e] = sum_k x[r][k] * wr[e][k]: one warp per (row, group of EPW experts); 16-byte loads, lane-strided
-// over K, fp32 accumulation, butterfly-reduced.  EPW = 8 re-uses a loaded piece of the row for eight experts (large
-// windows: the work is a small GEMM); EPW = 1 gives every (row, expert) its own warp, so that a window of a few rows
-// still spreads over many SMs and all of a warp's loads are in flight at once (one memory round trip).
-template <int EPW>
-__global__ void __launch_bounds__(256) router_logits_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride,
-                                                            const __nv_bfloat16 *__restrict__ wr, int rows, int H, int E,
-                                                            float *__restrict__ logits) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int groups = (E + EPW - 1) / EPW;
-    const long item = (long)blockIdx.x * 8 + warp;
-    if (item >= (long)rows * groups) return;
-    const int r = (int)(item / groups), e0 = (int)(item % groups) * EPW;
-    const uint4 *xr = reinterpret_cast<const uint4 *>(x + (size_t)r * x_stride);     // 8 bf16 per load
-    float acc[EPW];
-#pragma unroll
-    for (int j = 0; j < EPW; ++j) acc[j] = 0.f;
-#pragma unroll 8
-    for (int c = lane; c < H / 8; c += 32) {
-        const uint4 xv = __ldg(xr + c);
-        uint4 wv[EPW];
-#pragma unroll
-        for (int j = 0; j < EPW; ++j)
-            wv[j] = e0 + j < E ? __ldg(reinterpret_cast<const uint4 *>(wr + (size_t)(e0 + j) * H) + c) : make_uint4(0u, 0u, 0u, 0u);
-        const __nv_bfloat162 *xp = reinterpret_cast<const __nv_bfloat162 *>(&xv);
-        float xf[8];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { xf[2 * q] = __bfloat162float(xp[q].x); xf[2 * q + 1] = __bfloat162float(xp[q].y); }
-#pragma unroll
-        for (int j = 0; j < EPW; ++j) {
-            const __nv_bfloat162 *wp = reinterpret_cast<const __nv_bfloat162 *>(&wv[j]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                acc[j] = fmaf(xf[2 * q], __bfloat162float(wp[q].x), acc[j]);
-                acc[j] = fmaf(xf[2 * q + 1], __bfloat162float(wp[q].y), acc[j]);
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < EPW; ++j) {
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], m);
-        if (lane == 0 && e0 + j < E) logits[(size_t)r * E + e0 + j] = acc[j];
-    }
+// logits[r][e] = sum_k x[r][k] * wr[e][k] and, with picks, the top-k of every row, in one launch for any number of rows.
+//
+// CTA = 16 MT rows (of a cluster of CTAs that cut K between them when there are few rows); 8 warps cut the CTA's K; a warp runs
+// mma.m16n8k16 (bf16, fp32 accumulation) on 64 experts at a time.  The k slots of a fragment may be any eight k as long as both
+// operands agree, so a lane loads 16 contiguous bytes of a row (k = 8 t .. 8 t + 7 of a 32-k step) and uses them as the fragments
+// of two instructions: no shared memory, no shuffles in front of the tensor cores.  The warps' and CTAs' sums are added in a
+// fixed order.  Few rows are bound by latency: one memory round trip for the whole matrix (a cluster of 8 CTAs = 64 warps, one
+// 32-k step each at K = 2048), one exchange through distributed shared memory.  Many rows are bound by reading the router matrix
+// from L2 once per CTA (256 KB at 64 experts).  One warp per (row, expert) with scalar multiply-adds, and a CTA per row in the
+// small form, took 133 us at 4096 rows and 9 us at one.
+constexpr int RT_NE = 64, RT_ST = RT_NE + 4;                 // experts per round; floats per row of a partial
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // Top-k of one row by one warp: lane l holds the logits of experts l, l + 32, ...; k rounds of a warp arg-max (value
@@ -73,6 +44,7 @@ __device__ __forceinline__ void topk_row(const float *row, int E, int topk, int 
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             const int e = lane + 32 * j;
+            if (32 * j >= E) break;                                         // (uniform)
             if (e < E && (v[j] > best || (v[j] == best && e < bid))) { best = v[j]; bid = e; }
         }
 #pragma unroll
@@ -82,8 +54,10 @@ __device__ __forceinline__ void topk_row(const float *row, int E, int topk, int 
             if (ob > best || (ob == best && oi < bid)) { best = ob; bid = oi; }
         }
 #pragma unroll
-        for (int j = 0; j < PER; ++j)
+        for (int j = 0; j < PER; ++j) {
+            if (32 * j >= E) break;
             if (lane + 32 * j == bid) v[j] = -INFINITY;                     // struck out (its owner lane only)
+        }
         const float score = 1.f / (1.f + expf(-best));
         sum += score;
         if (lane == t) { mine = score; picks[t] = bid; }
@@ -102,38 +76,108 @@ __global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ log
     topk_row(logits + (size_t)r * E, E, topk, picks + (size_t)r * (topk + 1), weights + (size_t)r * (topk + 1), lane);
 }
 
-// Small windows: logits and top-k of a row in ONE launch.  CTA = row, 32 warps; warp w computes the logits of experts
-// w, w + 32, ... (whole-row dot products, all loads of a warp in flight at once, the summation order of
-// router_logits_kernel), leaves them in shared memory (and in `logits`), and warp 0 selects.
-__global__ void __launch_bounds__(1024) route_row_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride,
-                                                         const __nv_bfloat16 *__restrict__ wr, int H, int E, int topk,
-                                                         float *__restrict__ logits, int *__restrict__ picks,
-                                                         float *__restrict__ weights) {
-    __shared__ float row_sh[1024];
+template <int MT>
+__global__ void __launch_bounds__(256) route_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride,
+                                                    const __nv_bfloat16 *__restrict__ wr, int rows, int H, int E, int topk,
+                                                    float *__restrict__ logits, int *__restrict__ picks, float *__restrict__ weights) {
+    extern __shared__ __align__(16) float part[];                          // [8 warps][16 MT][RT_ST], then the CTA's sums [16 MT][RT_ST]
+    float *red = part + 8 * 16 * MT * RT_ST;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    uint32_t cr, cn;
+    asm("mov.u32 %0, %cluster_ctarank;" : "=r"(cr));
+    asm("mov.u32 %0, %cluster_nctarank;" : "=r"(cn));
+    const int r0 = (int)(blockIdx.x / cn) * 16 * MT, steps = (H + 31) >> 5, first = (int)cr * 8 + warp, stride = (int)cn * 8;
+    if (first < steps && first * 32 + 8 * t < H)                           // the router matrix is a constant: hint its first lines into L2
+        for (int n = 0; n < RT_NE / 8; ++n)
+            if (8 * n + g < E) asm volatile("prefetch.global.L2 [%0];" ::"l"(wr + (size_t)(8 * n + g) * H + first * 32 + 8 * t));
     pdl_wait();
     pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x;
-    const uint4 *xr = reinterpret_cast<const uint4 *>(x + (size_t)r * x_stride);
-    for (int e = warp; e < E; e += 32) {
-        const uint4 *wrow = reinterpret_cast<const uint4 *>(wr + (size_t)e * H);
-        float acc = 0.f;
-#pragma unroll 8
-        for (int c = lane; c < H / 8; c += 32) {
-            const uint4 xv = __ldg(xr + c), wv = __ldg(wrow + c);
-            const __nv_bfloat162 *xp = reinterpret_cast<const __nv_bfloat162 *>(&xv);
-            const __nv_bfloat162 *wp = reinterpret_cast<const __nv_bfloat162 *>(&wv);
+    for (int e0 = 0; e0 < E; e0 += RT_NE) {
+        float acc[MT][RT_NE / 8][4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                acc = fmaf(__bfloat162float(xp[q].x), __bfloat162float(wp[q].x), acc);
-                acc = fmaf(__bfloat162float(xp[q].y), __bfloat162float(wp[q].y), acc);
-            }
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < RT_NE / 8; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[m][n][c] = 0.f;
+        for (int s = first; s < steps; s += stride) {
+            const int k = s * 32 + 8 * t;
+            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+            uint4 av[MT][2], bv[RT_NE / 8];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int r = r0 + 16 * m + 8 * h + g;
+                    av[m][h] = r < rows && k < H ? __ldg(reinterpret_cast<const uint4 *>(x + (size_t)r * x_stride + k)) : zero;
+                }
+#pragma unroll
+            for (int n = 0; n < RT_NE / 8; ++n)
+                bv[n] = e0 + 8 * n + g < E && k < H ? __ldg(reinterpret_cast<const uint4 *>(wr + (size_t)(e0 + 8 * n + g) * H + k)) : zero;
+#pragma unroll
+            for (int n = 0; n < RT_NE / 8; ++n)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    mma_bf16(acc[m][n], av[m][0].x, av[m][1].x, av[m][0].y, av[m][1].y, bv[n].x, bv[n].y);
+                    mma_bf16(acc[m][n], av[m][0].z, av[m][1].z, av[m][0].w, av[m][1].w, bv[n].z, bv[n].w);
+                }
         }
 #pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-        if (lane == 0) { row_sh[e] = acc; logits[(size_t)r * E + e] = acc; }
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < RT_NE / 8; ++n) {
+                float *p = part + (size_t)(warp * 16 * MT + 16 * m + g) * RT_ST + 8 * n + 2 * t;
+                *reinterpret_cast<float2 *>(p) = make_float2(acc[m][n][0], acc[m][n][1]);
+                *reinterpret_cast<float2 *>(p + 8 * RT_ST) = make_float2(acc[m][n][2], acc[m][n][3]);
+            }
+        __syncthreads();
+        for (int i = tid; i < 16 * MT * RT_NE; i += 256) {
+            const int r = i / RT_NE, c = i % RT_NE;
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) v += part[(size_t)(w * 16 * MT + r) * RT_ST + c];
+            if (cn > 1) red[r * RT_ST + c] = v;
+            else if (r0 + r < rows && e0 + c < E) logits[(size_t)(r0 + r) * E + e0 + c] = v;
+        }
+        if (cn > 1) {                                                      // row r of the tile is finished by CTA r % cn
+            cluster_sync();
+            for (int i = tid; i < 16 * MT * RT_NE; i += 256) {
+                const int r = i / RT_NE, c = i % RT_NE;
+                if (r % (int)cn != (int)cr || r0 + r >= rows || e0 + c >= E) continue;
+                float v = 0.f;
+                for (uint32_t q = 0; q < cn; ++q) v += cluster_map(red, q)[r * RT_ST + c];
+                logits[(size_t)(r0 + r) * E + e0 + c] = v;
+            }
+            cluster_sync();                                                // peers may still be reading this CTA's sums
+        } else {
+            __syncthreads();
+        }
     }
+    if (!picks) return;
     __syncthreads();
-    if (warp == 0) topk_row(row_sh, E, topk, picks + (size_t)r * (topk + 1), weights + (size_t)r * (topk + 1), lane);
+    for (int r = (int)cr + (int)cn * warp; r < 16 * MT; r += (int)cn * 8)
+        if (r0 + r < rows)
+            topk_row(logits + (size_t)(r0 + r) * E, E, topk, picks + (size_t)(r0 + r) * (topk + 1), weights + (size_t)(r0 + r) * (topk + 1), lane);
+}
+
+static int launch_route(cudaStream_t s, const uint16_t *x, int x_stride, const uint16_t *wr, int rows, int H, int E, int topk, float *logits,
+                        int *picks, float *weights, bool pdl) {
+    // Rows per CTA: 32 once 16 would give more CTAs than the SMs hold side by side (the matrix is read once per CTA).  Clusters of
+    // 8 along K while the rows fill less than an eighth of the GPU.
+    const bool wide = rows > 2368;
+    const int tiles = wide ? (rows + 31) / 32 : (rows + 15) / 16, cn = tiles * 8 <= 148 && H >= 512 ? 8 : 1;
+    const size_t smem = (size_t)9 * (wide ? 32 : 16) * RT_ST * sizeof(float);
+    static bool configured[64] = {};
+    int dev = 0;
+    GF_CUDA(cudaGetDevice(&dev));
+    if (!configured[dev & 63]) {
+        GF_CUDA(cudaFuncSetAttribute(route_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * 32 * RT_ST * (int)sizeof(float)));
+        configured[dev & 63] = true;
+    }
+    const dim3 grid((unsigned)(tiles * cn)), block(256), cluster((unsigned)cn);
+    const __nv_bfloat16 *xb = (const __nv_bfloat16 *)x, *wb = (const __nv_bfloat16 *)wr;
+    return wide ? launch_kc(route_kernel<2>, grid, block, cluster, smem, s, pdl, xb, x_stride, wb, rows, H, E, topk, logits, picks, weights)
+                : launch_kc(route_kernel<1>, grid, block, cluster, smem, s, pdl, xb, x_stride, wb, rows, H, E, topk, logits, picks, weights);
 }
 }  // namespace gf
 
@@ -145,14 +189,7 @@ extern "C" int glmflash_router_logits(void *stream, const uint16_t *x, int x_str
     GF_REQUIRE(rows > 0 && hidden > 0 && hidden % 8 == 0 && experts > 0, "rows, experts positive; hidden a multiple of 8");
     GF_REQUIRE(x_stride >= hidden && x_stride % 8 == 0, "x_stride must be >= hidden and a multiple of 8");
     GF_REQUIRE(((uintptr_t)x | (uintptr_t)wr) % 16 == 0, "x and the router matrix must be 16-byte aligned");
-    if (rows >= 64) {
-        const long items = (long)rows * ((experts + 7) / 8);
-        return launch_k(router_logits_kernel<8>, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, pdl != 0,
-                        (const __nv_bfloat16 *)x, x_stride, (const __nv_bfloat16 *)wr, rows, hidden, experts, logits);
-    }
-    const long items = (long)rows * experts;
-    return launch_k(router_logits_kernel<1>, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, pdl != 0,
-                    (const __nv_bfloat16 *)x, x_stride, (const __nv_bfloat16 *)wr, rows, hidden, experts, logits);
+    return launch_route((cudaStream_t)stream, x, x_stride, wr, rows, hidden, experts, 0, logits, nullptr, nullptr, pdl != 0);
 }
 
 extern "C" int glmflash_topk(void *stream, const float *logits, int rows, int experts, int topk, int32_t *picks, float *weights,
@@ -172,10 +209,5 @@ extern "C" int glmflash_route(void *stream, const uint16_t *x, int x_stride, con
     GF_REQUIRE(topk >= 1 && topk <= 31 && topk <= experts, "topk must be in 1..31 and at most the number of experts");
     GF_REQUIRE(x_stride >= hidden && x_stride % 8 == 0, "x_stride must be >= hidden and a multiple of 8");
     GF_REQUIRE(((uintptr_t)x | (uintptr_t)wr) % 16 == 0, "x and the router matrix must be 16-byte aligned");
-    if (rows <= 16)
-        return launch_k(route_row_kernel, dim3((unsigned)rows), dim3(1024), 0, (cudaStream_t)stream, pdl != 0,
-                        (const __nv_bfloat16 *)x, x_stride, (const __nv_bfloat16 *)wr, hidden, experts, topk, logits, picks,
-                        weights);
-    if (glmflash_router_logits(stream, x, x_stride, wr, rows, hidden, experts, logits, pdl)) return -1;
-    return glmflash_topk(stream, logits, rows, experts, topk, picks, weights, pdl);
+    return launch_route((cudaStream_t)stream, x, x_stride, wr, rows, hidden, experts, topk, logits, picks, weights, pdl != 0);
 }
