@@ -414,7 +414,7 @@ class Bench:
             gu_bytes = distinct * GATEUP_BYTES_E + rows * H * 2 * 2
             gbs = gu_bytes / (ms_pass / L * 1e-3) / 1e9
             lgbs = layer_bytes / (ms_step / L * 1e-3) / 1e9
-            res["roofline"] = {"bound": "hbm", "kernel": "gemv_kernel<2,*> (gate/up grouped GEMV + grouping + input rotation + SwiGLU epilogue)",
+            res["roofline"] = {"bound": "hbm", "kernel": "stream_kernel, gate/up units alone (grouping + input rotation + grouped GEMV + SwiGLU epilogue)",
                                "achieved": gbs, "peak": self.peaks["hbm_gbs"], "peak_source": self.peaks["source"] + " hbm_gbs", "unit": "GB/s",
                                "frac": gbs / self.peaks["hbm_gbs"], "us_per_launch": ms_pass / L * 1e3, "algorithmic_bytes_per_launch": gu_bytes,
                                "distinct_experts_per_layer": distinct, "traffic": recorded_traffic(f"gemv_gateup_rows{rows}"),
@@ -664,7 +664,7 @@ def main():
     else:
         head = b.decode(args.rows, args.steps, args.warmup, headline=True, cpu=True)
         config = decode_config(args.rows, args.layers, world)
-        per_layer = (1 if args.layer_kernels == 1 else 3) + (1 if args.router else 0)
+        per_layer = 1 + (1 if world > 1 and args.layer_kernels != 1 else 0) + (1 if args.router else 0)      # layer kernel, exchange, router
         launches = per_layer * args.layers * args.steps
         if args.workload == "all":
             for r in ((4, 8, 16) if world == 1 else (16,)):

@@ -33,6 +33,28 @@ int fail_cuda(cudaError_t e, const char *what);
         if (!(cond)) return gf::fail(msg);   \
     } while (0)
 
+// The buffers of an owner as one zeroed allocation (an allocator call costs as much as a layer's kernels, and hosts build an
+// owner per layer): take() names the buffers, alloc() makes them.
+class Pool {
+  public:
+    template <typename T>
+    void take(T **p, size_t bytes) {
+        slots_[n_++] = {reinterpret_cast<void **>(p), total_};
+        total_ += (bytes + 255) / 256 * 256;
+    }
+    int alloc(void **base) {
+        GF_CUDA(cudaMalloc(base, total_ ? total_ : 1));
+        GF_CUDA(cudaMemset(*base, 0, total_));
+        for (int i = 0; i < n_; ++i) *slots_[i].p = (unsigned char *)*base + slots_[i].at;
+        return 0;
+    }
+
+  private:
+    struct Slot { void **p; size_t at; } slots_[24];
+    int n_ = 0;
+    size_t total_ = 0;
+};
+
 // Launch with or without the programmatic-dependent-launch attribute (the kernel's griddepcontrol instructions
 // are no-ops without it).
 template <typename... KArgs, typename... Args>

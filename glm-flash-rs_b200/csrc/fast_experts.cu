@@ -739,6 +739,7 @@ int make_map(CUtensorMap *map, void *base, uint64_t rows, uint64_t K) {
 
 struct glmflash_fast_experts {
     glmflash_config cfg;
+    void *pool = nullptr;                                   // the one allocation behind the buffers below
     __half *xg = nullptr, *xu = nullptr, *xd = nullptr;     // grouped rows
     float *out = nullptr;                                   // pair rows
     int *plan = nullptr, *src_pair = nullptr, *row_expert = nullptr, *status = nullptr;
@@ -756,11 +757,6 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
     GF_REQUIRE(f != nullptr, "out of host memory");
     f->cfg = *cfg;
     const size_t H = cfg->hidden, I = cfg->inter, P = (size_t)cfg->max_rows * cfg->slots;
-    auto alloc = [&](void **p, size_t bytes) -> int {
-        GF_CUDA(cudaMalloc(p, bytes));
-        GF_CUDA(cudaMemset(*p, 0, bytes));
-        return 0;
-    };
     int dev = 0;
     cudaDeviceProp prop;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaGetDeviceProperties(&prop, dev) != cudaSuccess) {
@@ -772,9 +768,16 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
         delete f;
         return fail("the prefill path needs an sm_100 GPU (tcgen05 / tensor memory)");
     }
-    if (alloc((void **)&f->xg, P * H * 2) || alloc((void **)&f->xu, P * H * 2) || alloc((void **)&f->xd, P * I * 2) ||
-        alloc((void **)&f->out, P * H * 4) || alloc((void **)&f->plan, PLAN_INTS * 4) || alloc((void **)&f->src_pair, P * 4) ||
-        alloc((void **)&f->row_expert, P * 4) || alloc((void **)&f->status, 16) || make_map(&f->map_xg, f->xg, P, H) ||
+    Pool pool;
+    pool.take(&f->xg, P * H * 2);
+    pool.take(&f->xu, P * H * 2);
+    pool.take(&f->xd, P * I * 2);
+    pool.take(&f->out, P * H * 4);
+    pool.take(&f->plan, PLAN_INTS * 4);
+    pool.take(&f->src_pair, P * 4);
+    pool.take(&f->row_expert, P * 4);
+    pool.take(&f->status, 16);
+    if (pool.alloc(&f->pool) || make_map(&f->map_xg, f->xg, P, H) ||
         make_map(&f->map_xu, f->xu, P, H) || make_map(&f->map_xd, f->xd, P, I) ||
         fail_if(cudaFuncSetAttribute(fast_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<2>::SMEM)) ||
         fail_if(cudaFuncSetAttribute(fast_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<1>::SMEM))) {
@@ -787,8 +790,7 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
 
 extern "C" void glmflash_fast_experts_free(glmflash_fast_experts *f) {
     if (!f) return;
-    cudaFree(f->xg); cudaFree(f->xu); cudaFree(f->xd); cudaFree(f->out); cudaFree(f->plan); cudaFree(f->src_pair);
-    cudaFree(f->row_expert); cudaFree(f->status);
+    cudaFree(f->pool);
     delete f;
 }
 

@@ -97,6 +97,7 @@ using namespace gf;
 
 struct glmflash_grouping {
     glmflash_config cfg;
+    void *pool = nullptr;                                    // the one allocation behind the tables
     int *ids = nullptr, *count = nullptr, *members = nullptr;
 };
 
@@ -108,14 +109,15 @@ extern "C" int glmflash_grouping_new(const glmflash_config *cfg, size_t cfg_byte
     GF_REQUIRE(g != nullptr, "out of host memory");
     g->cfg = *cfg;
     const size_t E1 = cfg->experts + 1;
-    cudaError_t e1 = cudaMalloc((void **)&g->ids, E1 * 4), e2 = cudaMalloc((void **)&g->count, 4),
-                e3 = cudaMalloc((void **)&g->members, E1 * cfg->max_rows * 4);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
+    Pool pool;
+    pool.take(&g->ids, E1 * 4);
+    pool.take(&g->count, 4);
+    pool.take(&g->members, E1 * cfg->max_rows * 4);
+    if (pool.alloc(&g->pool)) {
         glmflash_grouping_free(g);
-        return fail_cuda(e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3), "cudaMalloc(grouping)");
+        return -1;
     }
     cudaMemset(g->ids, 0xff, E1 * 4);
-    cudaMemset(g->count, 0, 4);
     cudaMemset(g->members, 0xff, E1 * cfg->max_rows * 4);
     *out = g;
     return 0;
@@ -123,7 +125,7 @@ extern "C" int glmflash_grouping_new(const glmflash_config *cfg, size_t cfg_byte
 
 extern "C" void glmflash_grouping_free(glmflash_grouping *g) {
     if (!g) return;
-    cudaFree(g->ids); cudaFree(g->count); cudaFree(g->members);
+    cudaFree(g->pool);
     delete g;
 }
 

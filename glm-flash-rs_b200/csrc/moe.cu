@@ -11,7 +11,7 @@
 
 namespace gf {
 int experts_run_fused(glmflash_experts *e, cudaStream_t s, const glmflash_weights *w, const void *input, int x_stride,
-                      const int32_t *picks, int rows);
+                      const int32_t *picks, const float *route_w, float *out, float *out2, int rows);
 
 // out[r][d] = sum_{s < slots-1, expert computed here} w[r][s] * Y[r*slots+s][d]  (+ Y[shared pair] if computed here)
 // fp32, ascending slot order, shared last: the order of the oracle's combine.
@@ -81,11 +81,17 @@ int launch_combine(cudaStream_t s, const float *Y, const int *picks, const float
 
 using namespace gf;
 
+bool gf::one_launch_selected() {
+    const char *env = getenv("GLMFLASH_LAYER_KERNELS");
+    return env && env[0] == '1';
+}
+
 struct glmflash_moe {
     glmflash_config cfg;
     glmflash_grouping *grouping = nullptr;
     glmflash_experts *experts = nullptr;            // windows of <= 16 rows
     glmflash_fast_experts *fast = nullptr;          // chunks of > 16 rows
+    void *pool = nullptr;                           // the one allocation behind the buffers below
     float *out = nullptr;
     void *in_dev = nullptr;                         // staging for run_host
     int *picks_dev = nullptr;
@@ -101,23 +107,20 @@ extern "C" int glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, gl
     glmflash_moe *m = new (std::nothrow) glmflash_moe();
     GF_REQUIRE(m != nullptr, "out of host memory");
     m->cfg = *cfg;
-    int rc = glmflash_grouping_new(cfg, cfg_bytes, &m->grouping);
-    if (!rc) rc = cfg->max_rows <= 16 ? glmflash_experts_new(cfg, cfg_bytes, &m->experts)
-                                      : glmflash_fast_experts_new(cfg, cfg_bytes, &m->fast);
+    int rc;                                         // (the window kernel groups its rows itself)
+    if (cfg->max_rows <= 16) rc = glmflash_experts_new(cfg, cfg_bytes, &m->experts);
+    else if (!(rc = glmflash_grouping_new(cfg, cfg_bytes, &m->grouping))) rc = glmflash_fast_experts_new(cfg, cfg_bytes, &m->fast);
     const size_t rows = cfg->max_rows;
-    if (!rc && cudaMalloc((void **)&m->out, rows * cfg->hidden * 4) != cudaSuccess) rc = fail("cudaMalloc(moe out)");
-    if (!rc && cudaMalloc(&m->in_dev, rows * cfg->hidden * 2) != cudaSuccess) rc = fail("cudaMalloc(moe staging)");
-    if (!rc && cudaMalloc((void **)&m->picks_dev, rows * cfg->slots * 4) != cudaSuccess) rc = fail("cudaMalloc(moe staging)");
-    if (!rc && cudaMalloc((void **)&m->w_dev, rows * cfg->slots * 4) != cudaSuccess) rc = fail("cudaMalloc(moe staging)");
-    if (rc) {
+    Pool pool;
+    pool.take(&m->out, rows * cfg->hidden * 4);
+    pool.take(&m->in_dev, rows * cfg->hidden * 2);
+    pool.take(&m->picks_dev, rows * cfg->slots * 4);
+    pool.take(&m->w_dev, rows * cfg->slots * 4);
+    if (rc || pool.alloc(&m->pool)) {
         glmflash_moe_free(m);
         return -1;
     }
-    cudaMemset(m->out, 0, rows * cfg->hidden * 4);
-    // Windows of <= 16 rows: three launches per layer (gate/up, down, combine) by default; GLMFLASH_LAYER_KERNELS=1
-    // selects the one-launch layer kernel (window.cu), which measured slower on one GPU (43 vs 28 us per one-token layer)
-    const char *env = getenv("GLMFLASH_LAYER_KERNELS");
-    m->one_launch = env && env[0] == '1';
+    m->one_launch = one_launch_selected();
     *out = m;
     return 0;
 }
@@ -127,7 +130,7 @@ extern "C" void glmflash_moe_free(glmflash_moe *m) {
     glmflash_grouping_free(m->grouping);
     glmflash_experts_free(m->experts);
     glmflash_fast_experts_free(m->fast);
-    cudaFree(m->out); cudaFree(m->in_dev); cudaFree(m->picks_dev); cudaFree(m->w_dev);
+    cudaFree(m->pool);
     delete m;
 }
 
@@ -140,9 +143,8 @@ extern "C" int glmflash_moe_run(glmflash_moe *m, void *stream, const glmflash_we
         // windows of <= 16 rows: grouping, rotation, both projections, epilogues and the combine in one launch
         return experts_run_window(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, rows, m->out, nullptr, -1);
     if (m->experts) {
-        // the same as three launches: grouping and input rotation happen inside the expert kernels
-        if (experts_run_fused(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, rows)) return -1;
-        Y = glmflash_experts_y(m->experts);
+        // one streamed launch: grouping, input rotation, both projections, epilogues and the combine
+        return experts_run_fused(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows);
     } else {
         if ((m->phases & 1) && glmflash_grouping_run(m->grouping, stream, picks, rows)) return -1;
         const int32_t *ids = glmflash_grouping_ids(m->grouping), *count = glmflash_grouping_count(m->grouping),

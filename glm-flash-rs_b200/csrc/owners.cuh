@@ -5,7 +5,11 @@
 
 struct glmflash_experts {
     glmflash_config cfg;
-    __half *xg = nullptr, *xu = nullptr, *xd = nullptr;   // rotated inputs [P][H], down-projection inputs [P][I]
+    void *pool = nullptr;                                 // the one allocation behind every buffer below
+    __half *xd = nullptr;                                 // down-projection inputs [P][I] (public)
+    // streamed layer kernel (stream.cu): {value, epoch} words of the partial sums and of the finished rows, its counters
+    unsigned long long *ll_z1 = nullptr, *ll_z2 = nullptr, *ll_xd = nullptr, *ll_xr = nullptr;
+    unsigned *ctrl = nullptr;
     float *y = nullptr;                                   // pair results [P][H] (public)
     int *status = nullptr;
     int phases = 7;                                       // profiling aid: 1 = input rotation, 2 = gate/up, 4 = down
@@ -13,11 +17,12 @@ struct glmflash_experts {
     float *z1 = nullptr, *z2 = nullptr;                   // split partials [2][H/128][P][I], [I/128][P][H]
     unsigned *sync = nullptr;
     size_t sync_words = 0;
-    float *out = nullptr;                                 // [max_rows][H] combined rows of the last window run
     int sm_count = 0;
 };
 
 namespace gf {
+// GLMFLASH_LAYER_KERNELS=1 (read when an owner is created) selects the alternative layer kernel (window.cu).
+bool one_launch_selected();
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 
 // Peer-mapped receive areas of the expert-parallel exchange fused into the layer kernel's last step.

@@ -1,0 +1,682 @@
+// The MoE layer for windows of 1..16 rows (decode and speculative verify) as ONE launch: a persistent, warp-specialised
+// kernel that streams the packed words of the chosen experts through shared memory and never lets the decode warps wait
+// for a phase of the layer.
+//
+// Replaces upstream's rot_in / exl3_grouped_8_4 / gateup_epilogue / down_epilogue / combine sequence (native/exl3.cu:59-321,
+// native/expert_loads.cu:130-285, src/moe.rs:101-181).  Same operands, member and pair conventions and rounding points.
+//
+// Work is cut into units of up to 32 KB of packed words: (distinct expert, matrix, 512-k split, 128-column block), one or two
+// stages of 16 k-tiles x 8 n-tiles, the gate / up units of all experts first, the down units after them.  A CTA (512 threads)
+// has four roles:
+//   warps 0-7   decode: warp = n-tile.  A lane reads 16 bytes (4 words of one tile: all 16 k of columns G and G + 8) with
+//               one LDS.128, cuts the states in pairs with funnel shifts, forms the weights exactly as upstream does (fp16
+//               sum of the codeword halves) and packs them into A operands of mma.m16n8k16; members are the N dimension
+//               (8 per set, two sets for 9..16 rows), fp32 accumulation over the unit.
+//   warps 8-10  X: put the members' activations of a unit's k range into shared memory as soon as they are there: rotated layer
+//               inputs (gate / up) or the finished rows of the gate / up phase (down).
+//   warp 11     feeds a four-stage ring, ONE tensor copy per unit (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
+//               bulk copies of the 1-KB rows held the issuing warp for 2,900 clocks per unit, longer than its decode takes.
+//   warps 12-15 finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of an output block in a fixed order and run the epilogue (Hadamard, scales, limited
+//               SwiGLU, down-input rotation; for the down phase Hadamard, output scale and the weighted sum over the row's
+//               slots, ascending, shared expert last).
+// Partial sums and finished rows travel through L2 as 8-byte words {value, launch epoch}: the reader polls the data itself
+// until it carries the epoch, so a hand-over costs one L2 round trip instead of fence + counter + load, and nothing has
+// to be cleared between launches.
+//
+// Units and finish jobs are drawn from two counters, in order, by CTAs that are running.  A gate / up unit waits for nothing,
+// and everything that a later unit or job waits for has been drawn by a CTA that runs: the launch makes progress with any
+// number of resident CTAs, next to any other kernel (no co-residency is assumed).  Sums have a fixed order (k-tiles of a
+// split, then splits ascending) that does not depend on the window: a row has the bits of its 1-row call.
+//
+// What bounds it: the decode instructions.  A unit is 32,768 weights at about 5 instructions; a loop that does nothing else
+// sustains 17.6 weights per clock and SM with 8 warps (two chunks in flight per warp) and 18.7 with 16, so 8 decode warps
+// per CTA and one or two CTAs per SM (launch_stream) are enough.  The earlier form (clusters of short-lived CTAs, three
+// launches per layer) spent half of its time on the phases around the decode.
+#include <algorithm>
+
+#include "gemv.cuh"
+#include "owners.cuh"
+#include "stream.cuh"
+
+namespace gf {
+
+constexpr int ST_THREADS = 512, ST_STAGES = 4, ST_XSTAGES = 2;
+constexpr int ST_DEC = 8, ST_XW = 3;                         // decode and X warps, then the producer, then four finish warps
+constexpr int ST_PROD = ST_DEC + ST_XW, ST_FIN = ST_PROD + 1;
+constexpr uint32_t ST_POLLS = 1u << 21;                      // polls of a global word before a wait gives up (about a second)
+
+enum : int { UNIT_G = 0, UNIT_D = 1, UNIT_END = 2 };       // low byte of a descriptor, matrix in bit 8
+constexpr int DESC_TWO = 1 << 16;                            // the unit has two stages
+
+// ---- {value, epoch} words -------------------------------------------------------------------------------------------
+__device__ __forceinline__ void ll_store(unsigned long long *p, uint32_t v, uint32_t epoch) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)epoch << 32) | v) : "memory");
+}
+__device__ __forceinline__ void ll_store2(unsigned long long *p, uint32_t v0, uint32_t v1, uint32_t epoch) {
+    const unsigned long long e = (unsigned long long)epoch << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(e | v0), "l"(e | v1) : "memory");
+}
+__device__ __forceinline__ void ll_load4(const unsigned long long *p, unsigned long long (&w)[4]) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w[0]), "=l"(w[1]) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w[2]), "=l"(w[3]) : "l"(p + 2) : "memory");
+}
+__device__ __forceinline__ bool ll_ready(const unsigned long long (&w)[4], uint32_t epoch) {
+    return (uint32_t)(w[0] >> 32) == epoch && (uint32_t)(w[1] >> 32) == epoch && (uint32_t)(w[2] >> 32) == epoch &&
+           (uint32_t)(w[3] >> 32) == epoch;
+}
+
+// t / d for 0 <= t < 2^21 with inv = 1 / d (approximate): the half keeps the product away from the integers.  An integer
+// division costs about 130 clocks of latency, and drawing a unit takes six of them.
+__device__ __forceinline__ float fast_inv(int d) { return __fdividef(1.f, (float)d); }
+__device__ __forceinline__ int fast_div(int t, float inv) { return (int)(((float)t + 0.5f) * inv); }
+
+// Shared state of a CTA: give-ups are sticky, every wait of the CTA then ends at once.
+struct StCta {
+    volatile int *abort_flag;
+    int *status;
+    __device__ __forceinline__ void give_up(int code) const {
+        *abort_flag = 1;
+        atomicExch(status, code);
+    }
+    // Poll bookkeeping of a wait on global memory: false when it has to end.
+    __device__ __forceinline__ bool again(uint32_t &n) const {
+        if (*abort_flag) return false;
+        if ((++n & 255u) == 0u) {
+            if (*reinterpret_cast<volatile int *>(status) != 0) { *abort_flag = 1; return false; }
+            if (n >= ST_POLLS) { give_up(GF_STATUS_TMA_TIMEOUT); return false; }
+        }
+        return true;
+    }
+    __device__ __forceinline__ bool wait(uint64_t *bar, uint32_t parity) const {
+        if (mbar_try_wait(bar, parity)) return true;
+        for (uint32_t i = 0; i < 4000000u; ++i) {
+            if (mbar_try_wait_hint(bar, parity, 1000u)) return true;
+            if (*abort_flag) return false;
+            if ((i & 255u) == 255u && *reinterpret_cast<volatile int *>(status) != 0) { *abort_flag = 1; return false; }
+        }
+        give_up(GF_STATUS_TMA_TIMEOUT);
+        return false;
+    }
+};
+
+// Four words of this lane, polled until they carry the epoch (uniform result for the warp).
+__device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long long *p, uint32_t epoch, unsigned long long (&w)[4]) {
+    ll_load4(p, w);
+    uint32_t n = 0;
+    while (!__all_sync(0xffffffffu, ll_ready(w, epoch))) {
+        if (!__all_sync(0xffffffffu, c.again(n))) return false;
+        __nanosleep(20);
+        ll_load4(p, w);
+    }
+    return true;
+}
+
+// Sum of the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the
+// epoch.
+__device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
+                                           float (&v)[4]) {
+    z += (size_t)lo * split_stride;
+#pragma unroll 1
+    for (; lo < hi; lo += 4, z += 4 * split_stride) {
+        unsigned long long w[4][4];
+        uint32_t n = 0;
+#pragma unroll 1
+        for (;;) {
+            // (past the end the last split is read again: no branches between the loads)
+            bool ok = true;
+            const unsigned long long *zi = z;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                ll_load4(zi, w[i]);
+                if (lo + i + 1 < hi) zi += split_stride;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ok = ok && ll_ready(w[i], epoch);
+            if (__all_sync(0xffffffffu, ok)) break;
+            if (!__all_sync(0xffffffffu, c.again(n))) return false;
+            __nanosleep(20);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (lo + i < hi)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] += __uint_as_float((uint32_t)w[i][j]);
+    }
+    return true;
+}
+
+
+// ---- shared memory of a CTA ------------------------------------------------------------------------------------------
+// [stages] words | [X stages] activations | barriers, descriptors | tables of the window
+struct StTables {
+    int *e, *mask, *pref;                // [umax] expert id, row mask (bit = row of the window); [umax + 1] finish-job prefix
+    uint16_t *pair;                      // [umax][16] pair index of member m
+    short *state;                        // [P] expert of a pair computed here, -1 not computed, -2 a repeated pick of its row
+};
+constexpr int ST_META = 1024;            // barriers and descriptors
+inline size_t st_smem_bytes(int sets, int umax, int P) {
+    const size_t tables = (size_t)(3 * umax + 1) * 4 + (size_t)umax * 32 + (size_t)P * 2 + 64;
+    return (size_t)ST_STAGES * ST_WBYTES + (size_t)ST_XSTAGES * sets * 8 * ST_XROW + ST_META + (tables + 127) / 128 * 128 +
+           1024 /*align*/;
+}
+
+// Distinct experts of the window that this GPU computes (ascending), their members (ascending rows) and the prefix of
+// their members (one finish job per member and column block).  All threads of the CTA; the caller's barrier publishes the
+// tables.  This is the head of every layer's critical path.  `used` (32 words) and tb.mask are zero on entry; row, slot: of
+// pick number threadIdx.x.  Returns the number of experts.
+__device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTables &tb, uint32_t *used, int row, int slot) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (a.picks && a.rows == 1 && a.shared != 2) {
+        // one row: every warp finds the order of the picks itself and writes the same tables (no block barrier)
+        constexpr int NONE = 0x7fffffff;
+        const int e = lane < a.slots ? __ldcg(a.picks + lane) : NONE;
+        int key = e == NONE || expert_skipped(e, a.E, a.shared, a.e_lo, a.e_hi) ? NONE : e;
+        int less = 0;
+        bool dup = false;
+        for (int j = 0; j < a.slots; ++j) {
+            const int v = __shfl_sync(0xffffffffu, key, j);
+            less += v < key;
+            dup |= v == key && j < lane && key != NONE;
+        }
+        if (__any_sync(0xffffffffu, dup)) {                      // a repeated pick counts once: rank among the first ones
+            const int first = dup ? NONE : key;
+            less = 0;
+            for (int j = 0; j < a.slots; ++j) less += __shfl_sync(0xffffffffu, first, j) < key;
+        }
+        const bool here = key != NONE && !dup;
+        if (here) {
+            tb.e[less] = e;
+            tb.mask[less] = 1;
+            tb.pair[less * 16] = (uint16_t)lane;
+        }
+        if (lane < a.slots) tb.state[lane] = here ? (short)e : key == NONE ? (short)-1 : (short)-2;
+        const int U = __popc(__ballot_sync(0xffffffffu, here));
+        if (lane < U) tb.pref[lane] = lane;
+        if (lane == 0) tb.pref[U] = U;
+        __syncwarp();
+        return U;
+    }
+    const int P = a.rows * a.slots;                              // <= 512 = one per thread
+    // key: the expert id (routing table) or the place in ids (grouping tables)
+    int key = -1, e = -1, n_ids = 0;
+    if (a.picks) {
+        if (tid < P) {
+            e = __ldcg(a.picks + tid);
+            tb.state[tid] = (short)e;
+            if (e >= 0 && e <= a.E) {                            // ids above E name nothing
+                key = e;
+                atomicOr(&used[key >> 5], 1u << (key & 31));
+            }
+        }
+    } else {
+        n_ids = min(__ldcg(a.count), a.umax);
+        if (tid < P) tb.state[tid] = -1;
+        if (tid < n_ids) {
+            e = __ldcg(a.ids + tid);
+            if (!expert_skipped(e, a.E, a.shared, a.e_lo, a.e_hi)) {
+                key = tid;
+                atomicOr(&used[key >> 5], 1u << (key & 31));
+            }
+        }
+    }
+    __syncthreads();
+    // experts that another GPU computes do not count: the expert window, and the shared expert by the config's switch or,
+    // when its owner is decided per window, by shared_owner_rank
+    int sh = a.shared;
+    if (a.picks && sh == 2) sh = shared_owner_rank(used, a.E, a.e_hi - a.e_lo, lane) == a.e_lo / (a.e_hi - a.e_lo);
+    if (a.picks && key >= 0 && expert_skipped(key, a.E, sh, a.e_lo, a.e_hi)) key = -1;
+    const int words = a.picks ? (a.E >> 5) + 1 : (n_ids + 31) >> 5;
+    int U = 0, u = 0;
+    const bool all = !a.picks || (sh && a.e_lo == 0 && a.e_hi == a.E);   // every id of the bitmap is computed here
+#pragma unroll 4
+    for (int w = 0; w < words; ++w) {
+        uint32_t bits = used[w];
+        if (!all) {
+            const int lo = min(max(a.e_lo - 32 * w, 0), 32), hi = min(max(a.e_hi - 32 * w, 0), 32);
+            uint32_t keep = hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
+            if (sh && (a.E >> 5) == w) keep |= 1u << (a.E & 31);
+            bits &= keep;
+        }
+        U += __popc(bits);
+        if (w < (key >> 5)) u += __popc(bits);
+        else if (w == (key >> 5)) u += __popc(bits & ((1u << (key & 31)) - 1u));
+    }
+    U = min(U, a.umax);
+    if (key < 0 || u >= U) u = -1;
+    bool dup = false;
+    if (u >= 0) tb.e[u] = e;
+    if (a.picks) {
+        if (u >= 0) {                                            // a pick that repeats an earlier slot of its row does not count
+            for (int q = 1; q <= slot; ++q) dup |= tb.state[tid - q] == (short)e;
+            if (!dup) atomicOr(&tb.mask[u], 1 << row);
+        }
+    } else if (u >= 0) {                                         // members come first; a member is row * 32 + slot
+        uint32_t bits = 0u;
+        for (int m = 0; m < min(a.maxm, 16); ++m) {
+            const int code = __ldcg(a.members + (size_t)tid * a.maxm + m);
+            if (code < 0) break;
+            const int p = (code >> 5) * a.slots + (code & 31);
+            tb.pair[u * 16 + m] = (uint16_t)p;
+            tb.state[p] = (short)e;
+            bits |= 1u << m;
+        }
+        tb.mask[u] = (int)bits;
+    }
+    __syncthreads();
+    if (a.picks) {
+        if (u >= 0 && !dup) tb.pair[u * 16 + __popc(tb.mask[u] & ((1u << row) - 1u))] = (uint16_t)tid;
+        if (tid < P) tb.state[tid] = u < 0 ? (short)-1 : dup ? (short)-2 : (short)e;
+    }
+    if (warp == ST_FIN) {
+        int run = 0;
+        for (int u0 = 0; u0 < U; u0 += 32) {
+            const int c = u0 + lane < U ? __popc(tb.mask[u0 + lane]) : 0;
+            int incl = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            if (u0 + lane < U) tb.pref[u0 + lane] = run + incl - c;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) tb.pref[U] = run;
+    }
+    return U;
+}
+
+// Register split over the warpgroups (decode, decode, X + producer, finish): 4 x 128 threads at 64 registers in all.
+template <bool INC, int N>
+__device__ __forceinline__ void st_regs() {
+    if (INC) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+template <int SETS>
+__global__ void __launch_bounds__(ST_THREADS, 2)
+stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_d,
+              const __grid_constant__ StreamArgs a) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);          // the swizzle atom is 1024 bytes
+    constexpr int XBYTES = SETS * 8 * ST_XROW;
+    unsigned char *words = smem, *xbuf = smem + ST_STAGES * ST_WBYTES;
+    unsigned char *meta = xbuf + ST_XSTAGES * XBYTES;
+    uint64_t *wfull = reinterpret_cast<uint64_t *>(meta);             // words of the stage landed (and its descriptor written)
+    uint64_t *empty = wfull + ST_STAGES;                              // stage consumed
+    uint64_t *xready = empty + ST_STAGES;                             // unit described
+    uint64_t *xfull = xready + ST_XSTAGES;                            // activations of the unit staged
+    uint64_t *xempty = xfull + ST_XSTAGES;                            // unit consumed
+    int4 *desc = reinterpret_cast<int4 *>(meta + 256);                // {kind | matrix << 8 | flags, expert number, split, block}
+    int4 *xdesc = desc + ST_STAGES;                                   // {kind | matrix << 8, expert number, split, -}
+    int *job_sh = reinterpret_cast<int *>(xdesc + ST_XSTAGES);        // [2]
+    StTables tb;
+    tb.e = reinterpret_cast<int *>(meta + ST_META);
+    tb.mask = tb.e + a.umax;
+    tb.pref = tb.mask + a.umax;
+    tb.pair = reinterpret_cast<uint16_t *>(tb.pref + a.umax + 1);
+    tb.state = reinterpret_cast<short *>(tb.pair + a.umax * 16);
+    __shared__ int abort_sh;
+    __shared__ uint32_t used_sh[32];
+    __shared__ __align__(16) float fin_sh[8][128];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int H = a.H, I = a.I, P = a.rows * a.slots;
+    const int SK1 = (H + 511) >> 9, SK2 = (I + 511) >> 9, NB1 = I >> 7, NB2 = H >> 7;
+    const StCta cta{&abort_sh, a.status};
+    if (tid == 0) {
+        for (int s = 0; s < ST_STAGES; ++s) {
+            mbar_init(wfull + s, 1);
+            mbar_init(empty + s, ST_DEC);
+        }
+        for (int s = 0; s < ST_XSTAGES; ++s) {
+            mbar_init(xready + s, 1);
+            mbar_init(xfull + s, ST_XW);
+            mbar_init(xempty + s, ST_DEC);
+        }
+        abort_sh = 0;
+        mbar_fence_init();
+    }
+    if (tid < 32) used_sh[tid] = 0u;
+    for (int i = tid; i < a.umax; i += ST_THREADS) tb.mask[i] = 0;
+    __syncthreads();
+    // The arguments of a launch and the tables' inputs are cold everywhere: touch the argument lines (constant-cache misses cost a
+    // thousand clocks each where they are met one after another) and hint the inputs into L2 while the kernel before drains.
+    // (a plain indexed read of the parameter: a volatile one would not be a parameter-space access)
+    if (tid < (int)(sizeof(StreamArgs) / 4)) asm volatile("" ::"r"(reinterpret_cast<const int *>(&a)[tid]));
+    if (tid >= 256 && tid < 259) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(tid == 256 ? &map_g : tid == 257 ? &map_u : &map_d)) : "memory");
+    if (tid < P && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
+    const int row = tid / a.slots, slot = tid - row * a.slots;        // of routing-table entry number tid
+    pdl_launch_dependents();                        // the next kernel waits for all of this one before it touches memory
+    pdl_wait();
+    // the first draws of the producer and the finish group travel while the tables are built
+    int drawn = 0;
+    if (tid == ST_PROD * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
+    if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
+    const uint32_t epoch = __ldcg(a.ctrl + CTRL_EPOCH) + 1u;          // words of earlier launches carry smaller ones
+    const int U = st_build_tables(a, tb, used_sh, row, slot);
+    if (tid == ST_FIN * 32) job_sh[0] = drawn;
+    __syncthreads();
+    const int units_g = a.do_g ? U * 2 * SK1 * NB1 : 0, units = units_g + (a.do_d ? U * SK2 * NB2 : 0);
+
+    // ---- rotated layer inputs, once per (member, matrix, 128-block): fp16(H(x * suh) / sqrt 128) (upstream rot_in_kernel,
+    //      native/exl3.cu:224-241).  They are the first jobs of the finish queue, cut so that every CTA gets about one, and the
+    //      first job of a CTA is done by all of its warps but the producer: nothing else can start before.
+    const int HB = H >> 7, rots = a.do_g ? tb.pref[U] * 2 * HB : 0;
+    const int rot_job = max(1, fast_div(rots + (int)gridDim.x - 1, fast_inv((int)gridDim.x))), jobs_r = fast_div(rots + rot_job - 1, fast_inv(rot_job));
+    const float inv_hb = fast_inv(HB), inv_slots = fast_inv(a.slots);
+    auto member_expert = [&](int q) {                                 // expert number of member q of all experts' lists
+        int lo = 0, hi = U;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (tb.pref[mid] <= q) lo = mid; else hi = mid;
+        }
+        return lo;
+    };
+    auto rotate = [&](int r) {                                        // one warp
+        const int rq = fast_div(r, inv_hb), k = (r - rq * HB) * 128 + 4 * lane, q = rq >> 1, mat = rq & 1;
+        const int u = member_expert(q), p = tb.pair[u * 16 + q - tb.pref[u]];
+        const uint2 sv = ldg_half4((mat ? a.suh_u : a.suh_g) + (size_t)tb.e[u] * H + k, a.vec);
+        const uint2 xv = __ldcg(reinterpret_cast<const uint2 *>(a.x + (size_t)fast_div(p, inv_slots) * a.x_stride + k));
+        const __nv_bfloat162 x01 = *reinterpret_cast<const __nv_bfloat162 *>(&xv.x), x23 = *reinterpret_cast<const __nv_bfloat162 *>(&xv.y);
+        const __half2 s01 = *reinterpret_cast<const __half2 *>(&sv.x), s23 = *reinterpret_cast<const __half2 *>(&sv.y);
+        float v[4] = {__bfloat162float(x01.x) * __low2float(s01), __bfloat162float(x01.y) * __high2float(s01),
+                      __bfloat162float(x23.x) * __low2float(s23), __bfloat162float(x23.y) * __high2float(s23)};
+        fwht128(v, lane);
+        ll_store2(a.xr + ((size_t)(mat * P + p) * H + k) / 2, pack_half2(v[0] * HAD_SCALE, v[1] * HAD_SCALE), pack_half2(v[2] * HAD_SCALE, v[3] * HAD_SCALE), epoch);
+    };
+    if (warp != ST_PROD) {
+        const int first = job_sh[0], w = warp - (warp > ST_PROD);
+        if (first < jobs_r)
+            for (int r = first * rot_job + w; r < min(rots, (first + 1) * rot_job); r += ST_THREADS / 32 - 1) rotate(r);
+    }
+
+    if (warp < ST_DEC) {
+        if (SETS == 1) st_regs<false, 56>();
+        // ---------------------------------------------------------------------------------------------- decode
+        const int G = lane >> 2, T = lane & 3;
+        uint32_t it = 0;
+        for (uint32_t c = 0;; ++c) {
+            const int xs = c % ST_XSTAGES;
+            if (!cta.wait(wfull + it % ST_STAGES, (it / ST_STAGES) & 1)) break;
+            const int4 d = desc[it % ST_STAGES];
+            const int kind = d.x & 0xff;
+            if (kind == UNIT_END) break;
+            const int nmem = __popc(tb.mask[d.y]);
+            const uint32_t p01 = *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 2 * T);
+            const uint32_t p23 = SETS == 2 ? *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 8 + 2 * T) : 0u;
+            if (!cta.wait(xfull + xs, (c / ST_XSTAGES) & 1)) break;
+            float acc[SETS][4];
+#pragma unroll
+            for (int q = 0; q < SETS; ++q)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[q][j] = 0.f;
+            const int halves = d.x & DESC_TWO ? 2 : 1;
+            bool ok = true;
+            for (int half = 0; half < halves; ++half, ++it) {
+                const int s = it % ST_STAGES;
+                if (half) ok = cta.wait(wfull + s, (it / ST_STAGES) & 1);
+                if (!ok) break;
+                st_decode<SETS>(words + s * ST_WBYTES, xbuf + xs * XBYTES + half * 512, warp, lane, SETS == 2 && nmem > 8, acc);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty + s);
+            }
+            if (!ok) break;
+            if (lane == 0) mbar_arrive(xempty + xs);
+            const int N = kind == UNIT_G ? I : H;
+            unsigned long long *z = kind == UNIT_G ? a.z1 + (size_t)(((d.x >> 8) & 1) * SK1 + d.z) * P * I : a.z2 + (size_t)d.z * P * H;
+            z += d.w * 128 + warp * 16 + G;
+#pragma unroll
+            for (int q = 0; q < SETS; ++q) {
+                const uint32_t pp = q ? p23 : p01;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (q * 8 + 2 * T + j < nmem) {
+                        unsigned long long *zp = z + (size_t)(j ? pp >> 16 : pp & 0xffffu) * N;
+                        ll_store(zp, __float_as_uint(acc[q][j]), epoch);
+                        ll_store(zp + 8, __float_as_uint(acc[q][2 + j]), epoch);
+                    }
+            }
+        }
+    } else if (warp < ST_PROD) {
+        st_regs<false, SETS == 1 ? 56 : 48>();
+        // ---------------------------------------------------------------------------------------------- activations
+        const int xw = warp - ST_DEC;
+        for (uint32_t it = 0;; ++it) {
+            const int s = it % ST_XSTAGES;
+            if (!cta.wait(xready + s, (it / ST_XSTAGES) & 1)) break;
+            const int4 d = xdesc[s];
+            const int kind = d.x & 0xff;
+            if (kind == UNIT_END) break;
+            const int nmem = __popc(tb.mask[d.y]), K = kind == UNIT_G ? H : I, halves = min(2, (K >> 8) - 2 * d.z);
+            const uint16_t *pair = tb.pair + d.y * 16;
+            const unsigned long long *src = (kind == UNIT_G ? a.xr + (size_t)((d.x >> 8) & 1) * P * (H / 2) : a.xdl) + d.z * 256 + 4 * lane;
+            unsigned char *xs = xbuf + s * XBYTES + 16 * lane;
+            const bool poll = kind == UNIT_G || a.do_g;               // (the down phase alone takes what the last run left)
+            bool ok = true;
+            // a warp per (member, 256 k), the loads of two in flight
+            for (int t0 = xw; t0 < nmem * halves; t0 += 2 * ST_XW) {
+                unsigned long long w[2][4];
+                int m[2], h[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int q = min(t0 + i * ST_XW, nmem * halves - 1);       // past the end: the last one again
+                    m[i] = halves == 2 ? q >> 1 : q;
+                    h[i] = halves == 2 ? q & 1 : 0;
+                    ll_load4(src + (size_t)pair[m[i]] * (K / 2) + h[i] * 128, w[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (poll && !__all_sync(0xffffffffu, ll_ready(w[i], epoch)))
+                        ok = ok && ll_wait4(cta, src + (size_t)pair[m[i]] * (K / 2) + h[i] * 128, epoch, w[i]);
+                    *reinterpret_cast<uint4 *>(xs + m[i] * ST_XROW + h[i] * 512) =
+                        make_uint4((uint32_t)w[i][0], (uint32_t)w[i][1], (uint32_t)w[i][2], (uint32_t)w[i][3]);
+                }
+            }
+            __syncwarp();
+            if (!ok) break;
+            if (lane == 0) mbar_arrive(xfull + s);
+        }
+    } else if (warp >= ST_FIN) {
+        st_regs<true, SETS == 1 ? 88 : 80>();
+        // ---------------------------------------------------------------------------------------------- finish
+        const int fw = warp - ST_FIN, ft = tid - ST_FIN * 32;
+        const int jobs_g = jobs_r + (a.do_g ? tb.pref[U] * NB1 : 0), jobs = jobs_g + (a.do_d ? a.rows * NB2 : 0);
+        const float inv_nb1 = fast_inv(NB1), inv_nb2 = fast_inv(NB2);
+        if (ft == 0 && drawn < jobs_r) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);      // the first job was a rotation: done above
+        for (uint32_t it = 0;; ++it) {
+            // one thread publishes the group's job and draws the next; a group that has given up ends together here
+            if (ft == 0) {
+                job_sh[it & 1] = abort_sh ? 0x7fffffff : drawn;
+                if (drawn < jobs) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
+            }
+            asm volatile("bar.sync 5, 128;" ::: "memory");
+            const int j = job_sh[it & 1];
+            if (j >= jobs) break;
+            if (j < jobs_r) {
+                for (int r = j * rot_job + fw; r < min(rots, (j + 1) * rot_job); r += 4) rotate(r);
+            } else if (j < jobs_g) {
+                // gate / up of one member: warp = (matrix, half of the splits).  The halves of a matrix meet in shared memory; warp 2
+                // transforms the up matrix and hands the clamped values over, warp 0 does the same for gate, applies SwiGLU, rotates
+                // and stores.
+                const int q = fast_div(j - jobs_r, inv_nb1), nb = j - jobs_r - q * NB1, lo = member_expert(q);
+                const int role = fw >> 1, half = fw & 1, mid = (SK1 + 1) >> 1;
+                const int p = tb.pair[lo * 16 + q - tb.pref[lo]], col = nb * 128 + 4 * lane;
+                const size_t so = (size_t)tb.e[lo] * I + col;
+                const uint2 sv = ldg_half4((role ? a.svh_u : a.svh_g) + so, a.vec);
+                const uint2 sd = ldg_half4(a.suh_d + so, a.vec);
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                sum_splits(cta, a.z1 + ((size_t)role * SK1 * P + p) * I + col, (size_t)P * I, half ? mid : 0, half ? SK1 : mid, epoch, v);
+                if (half) *reinterpret_cast<float4 *>(&fin_sh[fw][4 * lane]) = make_float4(v[0], v[1], v[2], v[3]);
+                pair_barrier(role);
+                if (!half) {
+                    const float4 o = *reinterpret_cast<const float4 *>(&fin_sh[fw + 1][4 * lane]);
+                    v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
+                    fwht128(v, lane);
+                    const float2 c01 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.x)), c23 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.y));
+                    const float r[4] = {bf16r(v[0] * HAD_SCALE * c01.x), bf16r(v[1] * HAD_SCALE * c01.y), bf16r(v[2] * HAD_SCALE * c23.x),
+                                        bf16r(v[3] * HAD_SCALE * c23.y)};
+                    if (role == 1) {
+                        *reinterpret_cast<float4 *>(&fin_sh[2][4 * lane]) =
+                            make_float4(fminf(fmaxf(r[0], -a.limit), a.limit), fminf(fmaxf(r[1], -a.limit), a.limit),
+                                        fminf(fmaxf(r[2], -a.limit), a.limit), fminf(fmaxf(r[3], -a.limit), a.limit));
+                        pair_barrier(2);
+                    } else {
+                        float sg[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float g = fminf(r[i], a.limit);
+                            sg[i] = bf16r(g / (1.f + expf(-g)));
+                        }
+                        pair_barrier(2);
+                        const float4 uu = *reinterpret_cast<const float4 *>(&fin_sh[2][4 * lane]);
+                        const float2 d01 = __half22float2(*reinterpret_cast<const __half2 *>(&sd.x)), d23 = __half22float2(*reinterpret_cast<const __half2 *>(&sd.y));
+                        float o4[4] = {bf16r(sg[0] * uu.x) * d01.x, bf16r(sg[1] * uu.y) * d01.y, bf16r(sg[2] * uu.z) * d23.x, bf16r(sg[3] * uu.w) * d23.y};
+                        fwht128(o4, lane);
+                        const uint32_t w0 = pack_half2(o4[0] * HAD_SCALE, o4[1] * HAD_SCALE), w1 = pack_half2(o4[2] * HAD_SCALE, o4[3] * HAD_SCALE);
+                        if (!abort_sh) {
+                            ll_store2(a.xdl + ((size_t)p * I + col) / 2, w0, w1, epoch);
+                            *reinterpret_cast<uint2 *>(a.xd + (size_t)p * I + col) = make_uint2(w0, w1);
+                        }
+                    }
+                }
+                // (the group's barrier at the top of the loop separates the uses of fin_sh of one job from the next: a warp
+                // writes its row of the next job only after every warp of the group has passed it)
+            } else {
+                // down: the slots of a row eight at a time, two per warp, then the weighted sum, ascending slots
+                const int row = fast_div(j - jobs_g, inv_nb2), nb = j - jobs_g - row * NB2, col = nb * 128 + 4 * lane;
+                float acc = 0.f;
+                for (int s0 = 0; s0 < a.slots; s0 += 8) {
+                    int e[2];
+                    float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                    uint2 sv[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int s = s0 + 4 * i + fw, p = row * a.slots + s;
+                        e[i] = s < a.slots ? tb.state[p] : -1;
+                        if (e[i] >= 0) sv[i] = ldg_half4(a.svh_d + (size_t)e[i] * H + col, a.vec);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        if (e[i] >= 0)
+                            sum_splits(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col, (size_t)P * H, 0, SK2, epoch, v[i]);
+                    if (e[0] >= 0) fwht128(v[0], lane);
+                    if (e[1] >= 0) fwht128(v[1], lane);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float *y = a.y + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col;
+                        if (e[i] >= 0) {
+                            const float2 c01 = __half22float2(*reinterpret_cast<const __half2 *>(&sv[i].x)), c23 = __half22float2(*reinterpret_cast<const __half2 *>(&sv[i].y));
+                            const float4 o = make_float4(v[i][0] * HAD_SCALE * c01.x, v[i][1] * HAD_SCALE * c01.y, v[i][2] * HAD_SCALE * c23.x,
+                                                         v[i][3] * HAD_SCALE * c23.y);
+                            *reinterpret_cast<float4 *>(y) = o;
+                            *reinterpret_cast<float4 *>(&fin_sh[4 * i + fw][4 * lane]) = o;
+                        } else if (e[i] == -2) {                  // a repeated pick: its pair row is not computed here
+                            *reinterpret_cast<float4 *>(&fin_sh[4 * i + fw][4 * lane]) = *reinterpret_cast<const float4 *>(y);
+                        }
+                    }
+                    if (a.out) {
+                        asm volatile("bar.sync 5, 128;" ::: "memory");
+                        for (int i = 0; i < min(8, a.slots - s0); ++i)
+                            if (tb.state[row * a.slots + s0 + i] != -1) {
+                                const float y = fin_sh[i][ft];
+                                acc = s0 + i == a.slots - 1 ? acc + y : acc + __ldcg(a.route_w + row * a.slots + s0 + i) * y;
+                            }
+                        asm volatile("bar.sync 5, 128;" ::: "memory");
+                    }
+                }
+                if (a.out) a.out[(size_t)row * H + nb * 128 + ft] = acc;
+                if (a.out2) a.out2[(size_t)row * H + nb * 128 + ft] = acc;
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------------------------------------- producer
+        st_regs<false, SETS == 1 ? 56 : 48>();
+        uint32_t it = 0;
+        bool ok = true;
+        const float inv_nb1 = fast_inv(NB1), inv_nb2 = fast_inv(NB2), inv_sk1 = fast_inv(SK1), inv_sk2 = fast_inv(SK2);
+        for (uint32_t c = 0; ok; ++c) {
+            const int xs = c % ST_XSTAGES;
+            // A unit is drawn only when there is room for it (the draw and the copy take 3,000 clocks, the stages in front of it
+            // 6,000 and more): units drawn earlier would only arrive late at whoever waits for their sums.
+            ok = __all_sync(0xffffffffu, cta.wait(xempty + xs, ((c / ST_XSTAGES) & 1) ^ 1) &&
+                                             cta.wait(empty + it % ST_STAGES, ((it / ST_STAGES) & 1) ^ 1));
+            if (!ok) break;
+            if (c && lane == 0) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
+            int t = __shfl_sync(0xffffffffu, drawn, 0);
+            if (t >= units) {
+                const int s = it % ST_STAGES;
+                if (lane == 0) {
+                    desc[s] = xdesc[xs] = make_int4(UNIT_END, 0, 0, 0);
+                    mbar_arrive(xready + xs);
+                    mbar_arrive(wfull + s);
+                }
+                break;
+            }
+            const bool g = t < units_g;
+            if (!g) t -= units_g;
+            const int SK = g ? SK1 : SK2, q = fast_div(t, g ? inv_nb1 : inv_nb2), nb = t - q * (g ? NB1 : NB2);
+            t = fast_div(q, g ? inv_sk1 : inv_sk2);
+            const int split = q - t * SK;
+            const int mat = g ? t & 1 : 0, u = g ? t >> 1 : t, kind = g ? UNIT_G : UNIT_D;
+            if (lane == 0) {
+                xdesc[xs] = make_int4(kind | mat << 8, u, split, 0);
+                mbar_arrive(xready + xs);
+            }
+            const CUtensorMap *map = g ? (mat ? &map_u : &map_g) : &map_d;
+            const int K = g ? H : I, kt = tb.e[u] * (K >> 4) + split * 32, halves = min(2, (K >> 8) - 2 * split);
+            for (int half = 0; half < halves; ++half, ++it) {
+                const int s = it % ST_STAGES;
+                ok = __all_sync(0xffffffffu, cta.wait(empty + s, ((it / ST_STAGES) & 1) ^ 1));
+                if (!ok) break;
+                if (lane == 0) {
+                    desc[s] = make_int4(kind | mat << 8 | (halves == 2 ? DESC_TWO : 0), u, split, nb);
+                    mbar_expect_tx(wfull + s, ST_WBYTES);
+                    tma_load_3d(words + s * ST_WBYTES, map, 0, kt + half * 16, nb * 8, wfull + s);
+                }
+            }
+        }
+        // after a give-up copies may be in flight: they have landed before the CTA leaves (bounded)
+        if (abort_sh && lane == 0)
+            for (uint32_t k = it > ST_STAGES ? it - ST_STAGES : 0; k < it; ++k) mbar_wait(wfull + k % ST_STAGES, (k / ST_STAGES) & 1);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        // the last CTA of the launch puts the counters back and advances the epoch; a later launch of the stream reads them
+        if (atomicAdd(a.ctrl + CTRL_DONE, 1u) == gridDim.x - 1) {
+            a.ctrl[CTRL_UNIT] = 0u;
+            a.ctrl[CTRL_FIN] = 0u;
+            a.ctrl[CTRL_DONE] = 0u;
+            a.ctrl[CTRL_EPOCH] = epoch;
+        }
+    }
+}
+
+int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
+    static int sms[64] = {};
+    static size_t configured[64][2] = {};
+    int dev = 0;
+    GF_CUDA(cudaGetDevice(&dev));
+    GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
+    if (!sms[dev]) GF_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
+    const int sets = a.rows > 8 ? 2 : 1;
+    const size_t smem = st_smem_bytes(sets, a.umax, a.rows * a.slots);
+    GF_REQUIRE(smem <= 227 * 1024, "routing table too large for the window kernel");
+    size_t &have = configured[dev][sets - 1];
+    if (have < smem) {
+        GF_CUDA(cudaFuncSetAttribute(sets == 2 ? stream_kernel<2> : stream_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        have = smem;
+    }
+    // CTAs per SM.  One leaves room for the next layer's CTAs, which then set up while this layer drains (one token: 24.4 us a
+    // layer against 28.6 with two); two fill the decode pipes (16 rows: 85 against 95 us).  The lines cross at about 16 units per
+    // SM, counted with one expert per pick of this GPU's window (2,160 units: 37.8 | 38.7 us, 2,880: 44.5 | 43.6).
+    const long pairs = (long)a.rows * (((long)(a.slots - 1) * (a.e_hi - a.e_lo) + a.E - 1) / a.E + (a.shared ? 1 : 0));
+    const long units = std::min<long>(pairs, a.umax) * (2L * ((a.H + 511) / 512) * (a.I / 128) + (long)((a.I + 511) / 512) * (a.H / 128));
+    const int per_sm = units >= 16L * sms[dev] ? 2 : 1;
+    const dim3 grid((unsigned)(sms[dev] * per_sm)), block(ST_THREADS);
+    CUtensorMap mg, mu, md;
+    if (bank_map(&mg, a.gt, a.E + 1, a.H, a.I) || bank_map(&mu, a.ut, a.E + 1, a.H, a.I) || bank_map(&md, a.dt, a.E + 1, a.I, a.H)) return -1;
+    return sets == 2 ? launch_k(stream_kernel<2>, grid, block, smem, s, pdl, mg, mu, md, a)
+                     : launch_k(stream_kernel<1>, grid, block, smem, s, pdl, mg, mu, md, a);
+}
+
+}  // namespace gf

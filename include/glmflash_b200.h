@@ -88,21 +88,16 @@ const char *glmflash_error(void);                 /* last error of this thread (
 int glmflash_exl3_decode(void *stream, const uint32_t *words, int64_t tiles, uint16_t *out);
 
 /* y[rows][N] fp16 = H(fp16(H(x*suh)/sqrt128) @ W_q)/sqrt128 * svh for fp16 x[rows][K], rows <= 16
- * (one matrix of src/experts.rs:100-135).  scratch: at least glmflash_exl3_linear_scratch_bytes(K,N). */
+ * (one matrix of src/experts.rs:100-135), in one launch.  scratch: a 256-byte aligned device address; nothing is kept in it
+ * (glmflash_exl3_linear_scratch_bytes(K,N) still names the size that callers used to provide, 0 for an unsupported shape). */
 size_t glmflash_exl3_linear_scratch_bytes(int K, int N);
 int glmflash_exl3_linear(void *stream, const uint16_t *x, int rows, const uint32_t *words, const uint16_t *suh,
                          const uint16_t *svh, int K, int N, uint16_t *y, void *scratch);
 
-/* The same linear for callers that cannot allocate device memory.  This entry point has no counterpart in the
- * reference.  It exists for hosts that took over the whole device heap at start-up (so a later cudaMalloc by a
- * library would fail or fragment their pool) and for serving loops where an allocator call would stall every
- * stream of the device.  The scratch is a fixed array inside the library (glmflash_exl3_linear_static_max_bytes(),
- * 132 KiB, held by every GPU that loads the library until the process exits), so shapes are limited to
- * K <= 4096; larger shapes are rejected with an error.  The call itself allocates nothing.
- * The first call on a device looks up the array's device address (a one-time, per-device set-up step): make that
- * first call outside any stream capture.  All calls share the one array and it keeps the previous call's
- * contents; the call clears what has to start at zero, but two calls that overlap on the GPU (different streams
- * without ordering, or different host threads) race on it: order them. */
+/* The same linear without the scratch argument.  This entry point has no counterpart in the reference.  It exists for hosts that
+ * took over the whole device heap at start-up (so a later cudaMalloc by a library would fail or fragment their pool) and for
+ * serving loops where an allocator call would stall every stream of the device.  It once ran on a fixed array inside the library;
+ * K <= 4096 and the size below remain from that.  Nothing is shared between calls: they may overlap on the GPU. */
 size_t glmflash_exl3_linear_static_max_bytes(void);
 int glmflash_exl3_linear_static(void *stream, const uint16_t *x, int rows, const uint32_t *words, const uint16_t *suh,
                                 const uint16_t *svh, int K, int N, uint16_t *y);
@@ -140,8 +135,9 @@ const int32_t *glmflash_experts_status(const glmflash_experts *e);
  * src/roce.rs:275-282). */
 int  glmflash_experts_clear_status(glmflash_experts *e, void *stream);
 /* Profiling aid in the spirit of upstream's PROBE modes (native/expert_loads.cu:46-47): run only the selected
- * kernels of the pipeline (1 = input rotation, 2 = gate/up GEMV + SwiGLU epilogue, 4 = down GEMV + epilogue;
- * default 7).  Skipped phases leave the scratch of the previous run in place; results are then meaningless. */
+ * phases of the kernel (2 = input rotation, gate/up GEMV and SwiGLU epilogue, 4 = down GEMV + epilogue; default 7; bit 1, once
+ * a rotation kernel of its own, selects nothing).  Skipped phases leave the scratch of the previous run in place; results
+ * are then meaningless. */
 int  glmflash_experts_set_phases(glmflash_experts *e, int mask);
 
 /* ---- FastExperts: prefill chunks of up to 8192 rows  (src/fast_experts.rs:27-208) ------------------- */
@@ -171,10 +167,10 @@ int  glmflash_fast_experts_set_phases(glmflash_fast_experts *f, int mask);
 /* ---- Moe: the whole layer after routing  (src/moe.rs:11-182, src/batch.rs:1160-1210) ---------------- */
 typedef struct glmflash_moe glmflash_moe;
 /* max_rows <= 16 builds the decode / verify pipeline, larger the prefill pipeline.
- * Windows of <= 16 rows run as three launches per layer (gate/up with grouping and input rotation inside, down,
- * combine: upstream's router-to-combine sequence src/moe.rs:101-181 in three kernels instead of eight).  With the
- * environment variable GLMFLASH_LAYER_KERNELS=1 (read at construction) they run as ONE kernel per layer, which also
- * carries the cross-GPU exchange of glmflash_moe_run_ep; on one GPU it measured slower than the three launches. */
+ * Windows of <= 16 rows run as ONE launch per layer: a persistent kernel that streams the chosen experts' words (upstream's
+ * router-to-combine sequence src/moe.rs:101-181 takes eight kernels).  The environment variable GLMFLASH_LAYER_KERNELS=1
+ * (read when an owner is created) selects an alternative one-launch kernel, which also carries the cross-GPU exchange of
+ * glmflash_moe_run_ep; on one GPU it is slower. */
 int  glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_moe **out);
 void glmflash_moe_free(glmflash_moe *m);
 /* group -> routed and shared experts -> combine:
@@ -191,7 +187,7 @@ const float *glmflash_moe_pairs(const glmflash_moe *m);
 const int32_t *glmflash_moe_status(const glmflash_moe *m);
 int  glmflash_moe_clear_status(glmflash_moe *m, void *stream);
 /* Profiling aid: 1 = grouping, 2 / 4 / 8 = the three ExpertGpu phases above, 16 = combine (default 31).  For
- * windows of <= 16 rows grouping and input rotation are fused into the gate/up kernel (bits 1 and 2 select nothing). */
+ * windows of <= 16 rows everything is one kernel (bits 1 and 2 select nothing). */
 int  glmflash_moe_set_phases(glmflash_moe *m, int mask);
 /* Host-buffer convenience used by the end-to-end measurement: copies input / picks / route_w from host
  * memory, runs, copies out[rows][H] back, and synchronises the stream. */

@@ -1,0 +1,52 @@
+"""GPU parity of the streamed window kernel (Moe for windows of <= 16 rows) at the edges of its cuts: k ranges of one stage
+(256) and of an odd number of them, one block of columns' worth of experts, one and two member sets, repeated picks, windows
+without an expert of this GPU, and both launch widths."""
+import numpy as np
+import pytest
+
+from conftest import TOL, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def run(pkg, cuda, bank, x, picks, rw, H, I, E, S, rows, synth, **kw):
+    import torch
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=rows, **kw))
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd = t(x.view(np.int16)).view(torch.bfloat16)
+    for _ in range(2):                                   # the second launch runs on the first one's counters and words
+        moe.run(bank, xd, t(picks), t(rw), rows)
+    torch.cuda.synchronize()
+    assert int(moe.status.cpu()[0]) == 0
+    return moe.output[:rows].cpu().numpy()
+
+
+@pytest.mark.parametrize("H,I,E,S,rows", [(256, 256, 3, 2, 1), (768, 256, 5, 3, 7), (512, 1280, 9, 4, 16), (2304, 768, 8, 5, 9),
+                                          (1024, 512, 40, 32, 16), (256, 768, 1, 2, 8)])
+def test_edges_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows):
+    bank = synth.expert_bank(31 + H + I, H, I, E, svh_scale=True)
+    x, (picks, rw) = synth.activations_bf16(32, rows, H), synth.route(33, rows, E, S - 1, shared_bias=rows > 1)
+    got = run(pkg, cuda, synth.to_device(bank, cuda), x, picks, rw, H, I, E, S, rows, synth)
+    want = oracle.combine(oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1), rw, rows, S, H)
+    emax, erms = rel_err(got, want)
+    assert np.isfinite(got).all() and emax < TOL and erms < TOL, (emax, erms)
+
+
+@pytest.mark.parametrize("rows", [1, 5])
+def test_window_without_experts_and_repeated_picks(pkg, oracle, synth, cuda, rows):
+    H, I, E, S = 512, 256, 8, 4
+    bank = synth.expert_bank(41, H, I, E, svh_scale=True)
+    dbank = synth.to_device(bank, cuda)
+    x, (picks, rw) = synth.activations_bf16(42, rows, H), synth.route(43, rows, E, S - 1)
+    # nothing of the window is computed here: the partial rows are zero
+    lo = next(e for e in range(E) if e not in picks)
+    none = run(pkg, cuda, dbank, x, picks, rw, H, I, E, S, rows, synth, shared_exl3=0, expert_lo=lo, expert_hi=lo + 1)
+    assert (none == 0).all()
+    # a pick that repeats an earlier slot of its row is not computed again: with weight 0 it must not change the row
+    again, rw2 = picks.copy(), rw.copy()
+    again[:, 1] = again[:, 0]
+    rw2[:, 1] = 0
+    got = run(pkg, cuda, dbank, x, again, rw2, H, I, E, S, rows, synth)
+    Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, again, mode=1)
+    want = oracle.combine(Y, rw2, rows, S, H)
+    assert rel_err(got, want)[0] < TOL
