@@ -291,17 +291,25 @@ def make_config(hidden=2048, inter=1536, experts=64, slots=5, max_rows=1, shared
                   experts if expert_hi is None else expert_hi, limit, pdl, shared_rows[0], shared_rows[1])
 
 
+_cuda_torch = None
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise GlmFlashError("no CUDA device: this library has no CPU path")
-    return torch
+    global _cuda_torch
+    if _cuda_torch is None:                          # asked once: the answer costs more than a launch
+        import torch
+        if not torch.cuda.is_available():
+            raise GlmFlashError("no CUDA device: this library has no CPU path")
+        torch.cuda.init()
+        _cuda_torch = torch
+    return _cuda_torch
 
 
 def _stream_ptr(stream=None):
-    torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    cuda = _torch()._C
+    return cuda._cuda_getCurrentRawStream(cuda._cuda_getDevice())
 
 
 def weights_struct(w):
@@ -337,14 +345,14 @@ def exl3_linear(x, words, suh, svh, K, N, stream=None):
     """x fp16 [rows][K] (rows <= 16) -> fp16 [rows][N]."""
     torch = _torch()
     rows = x.shape[0]
-    nbytes = lib().glmflash_exl3_linear_scratch_bytes(K, N)
-    if nbytes == 0:
+    if K <= 0 or N <= 0 or K % 256 or N % 128:
         raise GlmFlashError("unsupported linear shape")
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     y = torch.empty((rows, N), dtype=torch.float16, device=x.device)
+    # the kernel keeps nothing in the scratch argument: any 256-byte aligned device address serves, and y outlives the call
     _check(lib().glmflash_exl3_linear(_stream_ptr(stream), x.data_ptr(), rows, words.data_ptr(), suh.data_ptr(),
-                                      svh.data_ptr(), K, N, y.data_ptr(), scratch.data_ptr()))
-    torch.cuda.current_stream().synchronize()      # scratch is freed on return
+                                      svh.data_ptr(), K, N, y.data_ptr(), y.data_ptr()))
+    if stream is not None:
+        y.record_stream(stream)
     return y
 
 

@@ -2,6 +2,7 @@
 // src/model_verifier.rs:1291-1305 and src/batch.rs:1160-1210 for windows and chunks), plus the rank-ordered
 // sum that follows the cross-GPU all-gather (upstream src/model.rs:485-496).
 #include <algorithm>
+#include <initializer_list>
 #include <new>
 
 #include <stdlib.h>
@@ -57,6 +58,18 @@ __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ 
         }
     }
     *reinterpret_cast<float4 *>(out + (size_t)r * H + d) = acc;
+}
+
+// Inputs of a window from pinned host memory to the owner's buffers: the input rows in 16-byte words, then the routing table
+// and its weights.
+__global__ void __launch_bounds__(256) stage_in_kernel(const uint4 *x_host, uint4 *x, int nx, const int *picks_host, int *picks,
+                                                       const float *w_host, float *w, int np) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < nx) x[i] = x_host[i];
+    else if (i < nx + np) picks[i - nx] = picks_host[i - nx];
+    else if (i < nx + 2 * np) w[i - nx - np] = w_host[i - nx - np];
 }
 
 __global__ void __launch_bounds__(256) rank_sum_kernel(const float *__restrict__ gathered, int world, size_t n,
@@ -205,6 +218,20 @@ extern "C" const float *glmflash_moe_pairs(const glmflash_moe *m) {
     return m->experts ? glmflash_experts_y(m->experts) : glmflash_fast_experts_output(m->fast);
 }
 
+// Whether kernels of the current device can read and write these host buffers where they are (pinned memory under unified
+// addressing).
+static bool device_reads(std::initializer_list<const void *> ptrs) {
+    for (const void *p : ptrs) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeHost || at.devicePointer != p) return false;
+    }
+    return true;
+}
+
 extern "C" int glmflash_moe_run_host(glmflash_moe *m, void *stream, const glmflash_weights *w, const void *input_host,
                                      int x_stride, const int32_t *picks_host, const float *route_w_host, int rows,
                                      float *out_host) {
@@ -213,6 +240,19 @@ extern "C" int glmflash_moe_run_host(glmflash_moe *m, void *stream, const glmfla
     GF_REQUIRE(x_stride == m->cfg.hidden, "run_host takes densely packed rows (x_stride == hidden)");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t H = m->cfg.hidden, S = m->cfg.slots;
+    if (m->experts && !m->one_launch && m->phases == 31 && device_reads({input_host, picks_host, route_w_host, out_host}) &&
+        ((uintptr_t)input_host | (uintptr_t)out_host) % 16 == 0) {
+        // Windows of <= 16 rows in pinned memory: one kernel fetches all three inputs over the bus and the layer kernel stores the
+        // finished rows to host memory beside the owner's.  Three copies in and one out are four trips through a copy engine,
+        // each longer than its few KB take (8 rows: 112 us a call, of which the layer is half).
+        const int nx = (int)((size_t)rows * H * 2 / 16), np = (int)(rows * S);
+        if (launch_k(stage_in_kernel, dim3((unsigned)((nx + 2 * np + 255) / 256)), dim3(256), 0, s, m->cfg.pdl != 0, (const uint4 *)input_host,
+                     (uint4 *)m->in_dev, nx, (const int *)picks_host, m->picks_dev, route_w_host, m->w_dev, np))
+            return -1;
+        if (experts_run_fused(m->experts, s, w, m->in_dev, x_stride, m->picks_dev, m->w_dev, m->out, out_host, rows)) return -1;
+        GF_CUDA(cudaStreamSynchronize(s));
+        return 0;
+    }
     GF_CUDA(cudaMemcpyAsync(m->in_dev, input_host, (size_t)rows * H * 2, cudaMemcpyHostToDevice, s));
     GF_CUDA(cudaMemcpyAsync(m->picks_dev, picks_host, (size_t)rows * S * 4, cudaMemcpyHostToDevice, s));
     GF_CUDA(cudaMemcpyAsync(m->w_dev, route_w_host, (size_t)rows * S * 4, cudaMemcpyHostToDevice, s));
