@@ -5,30 +5,32 @@
 // fast_down_large (native/exl3_prefill.cu:402-430,657-889), which decode each 16x16 trellis tile into mma.sync
 // fragments in registers.  Here:
 //
-//   plan      one block: members per distinct expert, 128-row M tiles per expert, and the GROUPED row order
-//             (rows of an expert contiguous): src_pair[j] = pair index of grouped row j.  Work items are
-//             (expert, PAIR of M tiles, 128-column block); an expert with an odd tile count ends with a single.
-//             Pairs come first in the item list, so that the static round-robin over CTAs is balanced.
-//   rot       the input rotation writes Xs[j] = fp16(H(x[row] * suh[e]) / sqrt 128) in grouped order, so the A
-//             operand of every M tile is a contiguous 128 x K slab that one TMA tensor load brings into shared
-//             memory in the 128-byte-swizzled K-major layout the tensor core reads.
-//   gemm      persistent CTAs, one per SM, 28 warps:
-//               warp 0       TMA producer of the A stages (two M tiles of 128 rows x 64 k)
-//               warp 1       issues tcgen05.mma (M 128 x N 128 x K 16, fp16 -> fp32), commits stages and passes
+//   plan      members per distinct expert, chunks of at most 256 rows (as even as an expert's rows go, long ones first) and the
+//             GROUPED row order (rows of an expert contiguous): src_pair[j] = pair index of grouped row j.
+//   rot       the input rotation writes Xs[j] = fp16(H(x[row] * suh[e]) / sqrt 128) in grouped order, so the A operand of a chunk is
+//             a contiguous slab that TMA tensor loads bring into shared memory in the 128-byte-swizzled K-major layout the tensor
+//             core reads.
+//   gemm      persistent PAIRS of CTAs (74 clusters of two), one CTA per SM, 28 warps.  A work item is (chunk, pair of 128-column
+//             blocks): tcgen05.mma.cta_group::2, M 256 x N 256 x K 16 -- each CTA brings half of the rows and decodes ONE of the two
+//             column blocks, and keeps its rows' accumulators for both.  Roles:
+//               warp 0       TMA producer of the row tiles (128 rows x 64 k per stage)
+//               warp 1       first CTA: issues the MMAs of the pair, commits stages and passes to both CTAs; second CTA: relays
+//                            "my half of the stage is there" to the first
 //               warp 2       allocates / frees tensor memory (512 columns)
-//               warps 4-11   epilogue, one accumulator row per thread (tile 0: warps 4-7, tile 1: warps 8-11):
-//                            tcgen05.ld 128 fp32, the 128-point Hadamard transform in the thread's registers,
-//                            scales, limited SwiGLU, down-input rotation; fp16 Xd rows (gate/up) or fp32 Y rows (down)
-//               warps 12-27  decode the trellis tiles of B (the weights) to fp16 straight into the swizzled K-major
-//                            shared-memory tile (bit-exact codebook; conflict-free 32-bit stores); the packed words
-//                            of the next stage are already in registers while a stage is decoded
-//             A decoded B stage serves BOTH M tiles of the item (256 rows), which halves the decode work per
-//             flop.  The gate and the up projection of an item are two PASSES over K with their own accumulators
-//             (2 x 128 columns each): while the up pass runs, the epilogue warps turn the gate accumulators into
-//             silu(gate) (kept as bf16 in shared memory), and the up pass's epilogue overlaps the next item's gate
-//             pass, so tensor memory is double-buffered by construction.  Down is one pass per item, alternating
-//             the two accumulator halves.  setmaxnreg moves registers from the producer and decode warpgroups to
-//             the epilogue warpgroups.
+//               warp 3       TMA producer of the packed words, a ring of its own
+//               warps 4-11   epilogue, one accumulator row per thread (column block 0: warps 4-7, block 1: warps 8-11):
+//                            tcgen05.ld 128 fp32, the 128-point Hadamard transform in the thread's registers, scales, limited
+//                            SwiGLU, down-input rotation; fp16 Xd rows (gate/up) or fp32 Y rows (down)
+//               warps 12-27  decode the trellis tiles (bit-exact codebook) in registers and, when the slot is free, store them to
+//                            the swizzled K-major tile
+//             The gate and the up projection of an item are two PASSES over K with their own accumulators (256 columns each):
+//             while the up pass runs, the epilogue warps turn the gate accumulators into silu(gate) (kept as bf16 in shared
+//             memory), and the up pass's epilogue overlaps the next item's gate pass, so tensor memory is double-buffered by
+//             construction.  Down is one pass per item, alternating the two accumulator halves.
+//             What bounds it: with one CTA per tile pair (M 128 x N 128 instructions) the operand reads of the MMAs alone filled
+//             shared memory (128 bytes a clock); the pair halves them.  What is left is the loop from a stage's release to its
+//             next use (decode store, relay, issue, commit) and the decode itself: 4096 tokens, gate/up 407 -> 350 us, of which
+//             256 us remain without decode and epilogue arithmetic.
 // Arithmetic: one full-K fp32 accumulation chain per output (as upstream's prefill path, which is likewise not
 // bit-equal to its decode path: native/exl3_prefill.cu:20-23), the same transforms and rounding points as
 // upstream's epilogue (native/exl3_prefill.cu:596-622 == native/exl3.cu:260-321) with exp / divide in their fast
@@ -45,44 +47,24 @@
 namespace gf {
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 
-// FG_PROBE (timing experiments only, wrong results): 1 = decode warps store the raw words instead of decoding,
-// 2 = epilogue warps skip their arithmetic, 4 = no packed-word loads (decode a constant).
-#ifndef FG_PROBE
-#define FG_PROBE 0
-#endif
-// FG_DEC_WARPS: trellis-decode warps per CTA (8 or 16).  With 16 (the default: the decode is what the kernel waits for,
-// and four instead of two decode warps per scheduler raise its issue rate; measured 0.90 -> 0.80 ms per layer) every
-// warp owns two n-tiles of a k-tile instead of four, the CTA has 896 threads, and the register pool (896 x 72) is
-// split 24 / 152 / 40 per thread over the producer, epilogue and decode warpgroups (8 warps: 40 / 152 / 64 of 640 x 96).
-#ifndef FG_DEC_WARPS
-#define FG_DEC_WARPS 16
-#endif
-#ifndef FG_EPI_REGS
-#define FG_EPI_REGS 152
-#endif
-#ifndef FG_DEC_REGS
-#define FG_DEC_REGS 40
-#endif
-#define FG_STR2(x) #x
-#define FG_STR(x) FG_STR2(x)
-constexpr int FG_THREADS = (12 + FG_DEC_WARPS) * 32;
-constexpr int FG_BM = 128, FG_BN = 128, FG_BK = 64;
+constexpr int FG_DEC = 16;                                 // trellis-decode warps: n-tile by n-tile, round robin
+constexpr int FG_THREADS = (12 + FG_DEC) * 32;
+constexpr int FG_BM = 128, FG_BN = 128, FG_BK = 64;        // rows and columns of a CTA's operand tiles, k of a stage
 constexpr int FG_TILE_BYTES = FG_BM * FG_BK * 2;           // 16 KB: one 128 x 64 fp16 operand tile
+constexpr int FG_WORD_BYTES = 4096;                        // packed words of a stage: 4 k-tiles x 8 n-tiles
+constexpr int FG_CHUNK = 2 * FG_BM;                        // rows of a work item: 128 per CTA of the pair
 constexpr int FG_MAXU = 1024;
 
-// plan layout (int32): [0] total M tiles, [1] total grouped rows, [2] pair items, [3] single items,
-// then three prefix arrays of FG_MAXU + 1 entries: pair_base, single_base, row_base
-constexpr int PLAN_PAIR_BASE = 4, PLAN_SINGLE_BASE = PLAN_PAIR_BASE + FG_MAXU + 1,
-              PLAN_ROW_BASE = PLAN_SINGLE_BASE + FG_MAXU + 1, PLAN_INTS = PLAN_ROW_BASE + FG_MAXU + 1;
-
+// plan layout (int32): [0] total 128-row tiles, [1] total grouped rows, [2] chunks
+constexpr int PLAN_INTS = 4;
 // ---------------------------------------------------------------------------------------------- plan
 // Launched with one block per bank entry: every block recomputes the (tiny) scans, block 0 publishes the plan,
 // block b writes the grouped rows of distinct expert b.
 __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restrict__ ids, const int *__restrict__ count,
                                                           const int *__restrict__ members, int maxm, int slots, int E,
                                                           int shared_exl3, int e_lo, int e_hi, int srow_lo, int srow_hi,
-                                                          int *__restrict__ plan, int *__restrict__ src_pair,
-                                                          int *__restrict__ row_expert) {
+                                                          int *__restrict__ plan, int4 *__restrict__ chunks,
+                                                          int *__restrict__ src_pair, int *__restrict__ row_expert) {
     __shared__ int cnt_sh[FG_MAXU], row_sh[FG_MAXU], e_sh[FG_MAXU], first_sh[FG_MAXU];
     __shared__ int wsum[4][32];
     const int u = threadIdx.x, lane = u & 31, warp = u >> 5;
@@ -114,9 +96,11 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
             }
         }
     }
-    const int tiles = (cnt + FG_BM - 1) / FG_BM;
-    const int pairs = tiles >> 1, single = tiles & 1;
-    // block-wide exclusive scans of pairs, singles, rows (and the tile total)
+    // chunks of at most 256 rows, as even as they go; those of more than 128 rows come first in the list, so that the static
+    // round robin over the CTA pairs ends with the short ones
+    const int tiles = (cnt + FG_BM - 1) / FG_BM, nch = (cnt + FG_CHUNK - 1) / FG_CHUNK, size = nch ? (cnt + nch - 1) / nch : 0;
+    const int pairs = size > FG_BM ? nch : 0, single = nch - pairs;
+    // block-wide exclusive scans of long chunks, short chunks, rows (and the tile total)
     int p_inc = pairs, s_inc = single, r_inc = cnt, t_inc = tiles;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -133,17 +117,10 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
     }
     const int p_ex = p_off + p_inc - pairs, s_ex = s_off + s_inc - single, r_ex = r_off + r_inc - cnt;
     cnt_sh[u] = cnt; row_sh[u] = r_ex; e_sh[u] = e; first_sh[u] = first;
-    if (blockIdx.x == 0) {
-        plan[PLAN_PAIR_BASE + u] = p_ex;
-        plan[PLAN_SINGLE_BASE + u] = s_ex;
-        plan[PLAN_ROW_BASE + u] = r_ex;
-    }
-    if (u == 0 && blockIdx.x == 0) {
-        plan[0] = t_all; plan[1] = r_all; plan[2] = p_all; plan[3] = s_all;
-        plan[PLAN_PAIR_BASE + FG_MAXU] = p_all;
-        plan[PLAN_SINGLE_BASE + FG_MAXU] = s_all;
-        plan[PLAN_ROW_BASE + FG_MAXU] = r_all;
-    }
+    if (u == 0 && blockIdx.x == 0) { plan[0] = t_all; plan[1] = r_all; plan[2] = p_all + s_all; }
+    if (u < n && u % (int)gridDim.x == (int)blockIdx.x)
+        for (int c = 0; c < nch; ++c)
+            chunks[(pairs ? p_ex : p_all + s_ex) + c] = make_int4(e, r_ex + c * size, min(size, cnt - c * size), 0);
     __syncthreads();
     for (int uu = blockIdx.x; uu < n; uu += gridDim.x) {
         const int c = cnt_sh[uu], rb = row_sh[uu], ee = e_sh[uu], f0 = first_sh[uu];
@@ -156,50 +133,82 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
 }
 
 // ---------------------------------------------------------------------------------------------- rotation
-// One CTA (8 warps) per grouped row: the row's expert and source row are looked up once, every warp rotates
-// K/128/8 blocks, for one (shared_x) or both input scale vectors.
+// A warp takes 512 values of a grouped row: 8 lanes per 128-block, 16 values per lane, so that four of the seven butterflies run in
+// registers (from stride 2 on as packed fp32) and three across lanes.  The butterflies keep their order (stride 1..64), so the
+// sums are those of a warp per block.  With four values per lane and five butterflies across lanes the kernel issued 29
+// instructions a value and took 83 us at 4096 rows x 2048 x 5 pairs x 2 matrices (168 MB written).
 __global__ void __launch_bounds__(256) fast_rot_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride,
                                                        const int *__restrict__ plan, const int *__restrict__ src_pair,
                                                        const int *__restrict__ row_expert, const __half *__restrict__ suh0,
                                                        const __half *__restrict__ suh1, __half *__restrict__ out0,
-                                                       __half *__restrict__ out1, int K, int slots, int mats) {
+                                                       __half *__restrict__ out1, int K, int slots, int mats, bool vec) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int KB = K >> 7, rows = plan[1];
-    for (int j = blockIdx.x; j < rows; j += gridDim.x) {
-        const int p = src_pair[j], e = row_expert[j], row = p / slots;
-        // two 128-blocks of the warp per round: all their loads are issued before the first transform
-        for (int blk0 = warp; blk0 < KB; blk0 += 16) {
-            const int n2 = blk0 + 8 < KB ? 2 : 1;
-            uint2 xv[2], sv[2][2];
+    const int KB = K >> 7, parts = (KB + 3) >> 2;
+    const long items = (long)plan[1] * parts;
+    const float2 neg1 = make_float2(-1.f, -1.f);
+    for (long it = (long)blockIdx.x * 8 + warp; it < items; it += (long)gridDim.x * 8) {
+        const int j = (int)(it / parts), blk = (int)(it % parts) * 4 + (lane >> 3);
+        if (blk >= KB) continue;                                           // (whole groups of eight lanes)
+        const unsigned group = 0xffu << (lane & 24);
+        const int e = row_expert[j], row = src_pair[j] / slots, k = blk * 128 + (lane & 7) * 16;
+        const __nv_bfloat16 *xp = x + (size_t)row * x_stride + k;
+        uint32_t xw[8];
+        if (vec) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(xp), b = *reinterpret_cast<const uint4 *>(xp + 8);
+            xw[0] = a.x; xw[1] = a.y; xw[2] = a.z; xw[3] = a.w; xw[4] = b.x; xw[5] = b.y; xw[6] = b.z; xw[7] = b.w;
+        } else {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i >= n2) break;
-                const int k = (blk0 + 8 * i) * 128 + 4 * lane;
-                xv[i] = *reinterpret_cast<const uint2 *>(x + (size_t)row * x_stride + k);
-#pragma unroll
-                for (int mat = 0; mat < 2; ++mat)
-                    if (mat < mats) sv[i][mat] = __ldg(reinterpret_cast<const uint2 *>((mat ? suh1 : suh0) + (size_t)e * K + k));
+            for (int i = 0; i < 4; ++i) {
+                const uint2 a = *reinterpret_cast<const uint2 *>(xp + 4 * i);
+                xw[2 * i] = a.x; xw[2 * i + 1] = a.y;
             }
+        }
+#pragma unroll 1
+        for (int mat = 0; mat < mats; ++mat) {
+            const __half *sp = (mat ? suh1 : suh0) + (size_t)e * K + k;
+            uint32_t sw[8];
+            if (vec) {
+                const uint4 a = __ldg(reinterpret_cast<const uint4 *>(sp)), b = __ldg(reinterpret_cast<const uint4 *>(sp + 8));
+                sw[0] = a.x; sw[1] = a.y; sw[2] = a.z; sw[3] = a.w; sw[4] = b.x; sw[5] = b.y; sw[6] = b.z; sw[7] = b.w;
+            } else {
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i >= n2) break;
-                const int k = (blk0 + 8 * i) * 128 + 4 * lane;
-                const __nv_bfloat162 x01 = *reinterpret_cast<const __nv_bfloat162 *>(&xv[i].x),
-                                     x23 = *reinterpret_cast<const __nv_bfloat162 *>(&xv[i].y);
-                const float xf[4] = {__bfloat162float(x01.x), __bfloat162float(x01.y), __bfloat162float(x23.x), __bfloat162float(x23.y)};
-#pragma unroll
-                for (int mat = 0; mat < 2; ++mat) {
-                    if (mat >= mats) break;
-                    const __half2 s01 = *reinterpret_cast<const __half2 *>(&sv[i][mat].x),
-                                  s23 = *reinterpret_cast<const __half2 *>(&sv[i][mat].y);
-                    float v[4] = {xf[0] * __low2float(s01), xf[1] * __high2float(s01), xf[2] * __low2float(s23), xf[3] * __high2float(s23)};
-                    fwht128(v, lane);
-                    __half2 h01 = __halves2half2(__float2half_rn(v[0] * HAD_SCALE), __float2half_rn(v[1] * HAD_SCALE));
-                    __half2 h23 = __halves2half2(__float2half_rn(v[2] * HAD_SCALE), __float2half_rn(v[3] * HAD_SCALE));
-                    *reinterpret_cast<uint2 *>((mat ? out1 : out0) + (size_t)j * K + k) =
-                        make_uint2(*reinterpret_cast<uint32_t *>(&h01), *reinterpret_cast<uint32_t *>(&h23));
+                for (int i = 0; i < 4; ++i) {
+                    const uint2 a = __ldg(reinterpret_cast<const uint2 *>(sp + 4 * i));
+                    sw[2 * i] = a.x; sw[2 * i + 1] = a.y;
                 }
             }
+            float2 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {                                   // times the sign / scale vector, stride 1
+                const float2 s = __half22float2(*reinterpret_cast<const __half2 *>(&sw[i]));
+                const float a = __uint_as_float(xw[i] << 16) * s.x, b = __uint_as_float(xw[i] & 0xffff0000u) * s.y;
+                v[i] = make_float2(a + b, a - b);
+            }
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1)                                // strides 2, 4, 8
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (!(i & d)) {
+                        const float2 a = v[i], b = v[i | d];
+                        v[i] = __fadd2_rn(a, b);
+                        v[i | d] = __ffma2_rn(b, neg1, a);
+                    }
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) {                              // strides 16, 32, 64: lower + upper | lower - upper
+                const float sg = lane & d ? -1.f : 1.f;
+                const float2 s2 = make_float2(sg, sg);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 o = make_float2(__shfl_xor_sync(group, v[i].x, d), __shfl_xor_sync(group, v[i].y, d));
+                    v[i] = __ffma2_rn(v[i], s2, o);
+                }
+            }
+            uint32_t w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = pack_half2(v[i].x * HAD_SCALE, v[i].y * HAD_SCALE);
+            uint4 *dst = reinterpret_cast<uint4 *>((mat ? out1 : out0) + (size_t)j * K + k);
+            dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
     }
 }
@@ -210,24 +219,47 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_smem)), "r"(cols)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_smem)), "r"(cols)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T, M 128 x N 128 x K 16, fp16 operands, fp32 accumulate
+// D[tmem] (+)= A[smem desc] * B[smem desc]^T over a pair of CTAs, M 256 x N 256 x K 16, fp16 operands, fp32 accumulate: each CTA
+// brings 128 rows of A and 128 rows (columns of D) of B at the same shared-memory offsets and keeps its 128 rows of D
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// arrive on an mbarrier when every tcgen05.mma issued so far by this thread has completed
+// arrive on the mbarrier of both CTAs of the pair when every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+// arrive on the mbarrier at the same offset in CTA `cta` of the cluster
+__device__ __forceinline__ void mbar_arrive_cluster(uint64_t *bar, uint32_t cta) {
+    asm volatile(
+        "{\n\t.reg .b32 r;\n\t"
+        "mapa.shared::cluster.u32 r, %0, %1;\n\t"
+        "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}"
+        ::"r"(smem_u32(bar)), "r"(cta)
+        : "memory");
+}
+// one thread of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
 }
 // 32 consecutive fp32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
@@ -257,8 +289,8 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                               // SWIZZLE_128B
     return d;
 }
-// kind::f16: D fp32, A and B fp16, both K-major, N 128, M 128
-constexpr uint32_t UMMA_IDESC = (1u << 4) | ((uint32_t)(FG_BN >> 3) << 17) | ((uint32_t)(FG_BM >> 4) << 24);
+// kind::f16: D fp32, A and B fp16, both K-major, N 256, M 256 (the pair's)
+constexpr uint32_t UMMA_IDESC = (1u << 4) | ((uint32_t)(2 * FG_BN >> 3) << 17) | ((uint32_t)(2 * FG_BM >> 4) << 24);
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
     asm volatile(
@@ -267,11 +299,14 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// Wait on an mbarrier phase, giving up when the abort flag is up or after a bounded number of polls.
+// Wait on an mbarrier phase, giving up when the abort flag is up or after a bounded number of polls.  SLEEP: nanoseconds a poll may
+// sleep; every role but the two on the critical path (MMA issue, relay) sleeps, because two dozen polling warps delay those two
+// by some 200 clocks per wait.
+template <uint32_t SLEEP>
 __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
     if (mbar_try_wait(bar, parity)) return true;
-    for (uint32_t i = 0; i < 400000u; ++i) {                  // each poll may sleep up to 10 us: at most about 4 s
-        if (mbar_try_wait_hint(bar, parity, 10000u)) return true;
+    for (uint32_t i = 0; i < 4000000u; ++i) {
+        if (SLEEP ? mbar_try_wait_hint(bar, parity, SLEEP) : mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
         // another CTA of this launch has already given up: leave as well instead of sitting out the limit here too
         if ((i & 15u) == 15u && *reinterpret_cast<volatile int *>(status) != 0) { *abort_flag = 1; return false; }
@@ -313,8 +348,8 @@ __device__ __forceinline__ void fwht128_regs(float (&v)[128]) {
 }
 
 struct FastGemmArgs {
-    const uint32_t *T0, *T1;       // trellis banks of pass 0 / pass 1 (gate, up;  down: T0 only)
-    const int *ids, *plan, *src_pair;
+    const int *plan, *src_pair;
+    const int4 *chunks;            // {expert, first grouped row, rows, -}
     const __half *sv0, *sv1, *sd;  // gate/up: svh_g, svh_u, suh_d;  down: svh_d
     __half *xd;                    // gate/up out, grouped rows [rows][N]
     float *y;                      // down out, pair rows [P][N]
@@ -323,215 +358,206 @@ struct FastGemmArgs {
     float limit;
 };
 
-// One work item: expert u (id e), its M tiles tile0 (and tile0 + 1 when ntiles == 2) starting at grouped row row0,
-// cnt0 / cnt1 valid rows in them, column block nb.
+// One work item of a CTA pair: a chunk of an expert's rows and a pair of 128-column blocks.  This CTA brings `cnt` of the rows
+// (starting at grouped row `row`) and decodes column block 2 * nbp + its rank.
 struct ItemInfo {
-    int e, row0, cnt0, cnt1, ntiles, nb;
+    int e, row, cnt, nbp;
 };
-__device__ __forceinline__ int last_le(const int *base, int n, int v) {     // largest i < n with base[i] <= v
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (base[mid] <= v) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-__device__ __forceinline__ ItemInfo item_info(int item, int NB, int pairs_all, const int *pair_base, const int *single_base,
-                                              const int *row_base, const int *ids) {
-    ItemInfo t;
-    const int q = item / NB;
-    t.nb = item % NB;
-    int u, tile0;
-    if (q < pairs_all) {
-        u = last_le(pair_base, FG_MAXU, q);
-        tile0 = 2 * (q - pair_base[u]);
-        t.ntiles = 2;
-    } else {
-        u = last_le(single_base, FG_MAXU, q - pairs_all);
-        const int cnt = row_base[u + 1] - row_base[u];
-        tile0 = (cnt + FG_BM - 1) / FG_BM - 1;
-        t.ntiles = 1;
-    }
-    const int cnt = row_base[u + 1] - row_base[u];
-    t.e = ids[u];
-    t.row0 = row_base[u] + tile0 * FG_BM;
-    t.cnt0 = min(FG_BM, cnt - tile0 * FG_BM);
-    t.cnt1 = t.ntiles == 2 ? min(FG_BM, cnt - (tile0 + 1) * FG_BM) : 0;
-    return t;
+__device__ __forceinline__ ItemInfo item_info(int item, int NBP, const int4 *chunks, int rank) {
+    const int4 c = __ldg(chunks + item / NBP);
+    const int h = (c.z + 1) >> 1;                            // rows of the first CTA; both take about half
+    return ItemInfo{c.x, c.y + (rank ? h : 0), rank ? c.z - h : h, item % NBP};
 }
 
 template <int MATS>
 struct FgCfg {
-    static constexpr int STAGES = MATS == 2 ? 3 : 4;
-    static constexpr int STAGE_BYTES = 3 * FG_TILE_BYTES;                                    // A tile 0, A tile 1, B
+    static constexpr int ASTAGES = MATS == 2 ? 4 : 6;        // rows
+    static constexpr int BSTAGES = 4;                        // decoded weights: written from registers as soon as the slot is free
+    static constexpr int WSTAGES = MATS == 2 ? 5 : 6;        // packed words
+    static constexpr int DONE = 8;                           // ring of stage-completed barriers (more than any ring above)
     static constexpr int GBUF_BYTES = MATS == 2 ? 64 * 256 * 4 : 0;                          // silu(gate) as bf16 pairs
-    static constexpr int TABLE_BYTES = (256 + 3 * 128 * 4 + 2 * (FG_MAXU + 1) * 4 + 64 + 127) / 128 * 128;   // keeps tbuf 128-byte aligned
+    static constexpr int TABLE_BYTES = 512 + 2 * 3 * 128 * 4;                                // barriers, scale vectors
     static constexpr int TBUF_BYTES = MATS == 1 ? 8 * 32 * 16 * 4 : 0;        // down: per epilogue warp 32 rows x 16 floats
-    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)STAGES * STAGE_BYTES + GBUF_BYTES + TABLE_BYTES + TBUF_BYTES;
+    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)(ASTAGES + BSTAGES) * FG_TILE_BYTES + (size_t)WSTAGES * FG_WORD_BYTES +
+                                   GBUF_BYTES + TABLE_BYTES + TBUF_BYTES;
 };
 
+// Registers per thread: launched with 72 x 896; the producer warpgroup and the decode warpgroups give theirs to the two epilogue
+// warpgroups (24 + 2 x 152 + 4 x 40 = 488 of 504).
+constexpr uint32_t FG_SLEEP = 500;
+constexpr int FG_REGS_MMA = 24, FG_REGS_EPI = 152, FG_REGS_DEC = 40;
+
 template <int MATS>
-__global__ void __launch_bounds__(FG_THREADS, 1)
-fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1, const FastGemmArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FG_THREADS, 1)
+fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1, const __grid_constant__ CUtensorMap mapT0,
+                 const __grid_constant__ CUtensorMap mapT1, const FastGemmArgs a) {
     using C = FgCfg<MATS>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // 1024-aligned operand tiles
-    unsigned char *stages = smem;
-    uint32_t *gbuf = reinterpret_cast<uint32_t *>(smem + (size_t)C::STAGES * C::STAGE_BYTES); // [64][256]
-    unsigned char *tables = smem + (size_t)C::STAGES * C::STAGE_BYTES + C::GBUF_BYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(tables);                 // [STAGES] A landed (tx) + the decode warps
-    uint64_t *empty = full + C::STAGES;                                    // [STAGES] MMAs of the stage completed
-    uint64_t *tmem_full = empty + C::STAGES;                               // [2] accumulators of a pass complete
-    uint64_t *tmem_empty = tmem_full + 2;                                  // [2] accumulators drained (8 epilogue warps)
+    unsigned char *aring = smem, *bring = aring + (size_t)C::ASTAGES * FG_TILE_BYTES;
+    unsigned char *wring = bring + (size_t)C::BSTAGES * FG_TILE_BYTES;     // [WSTAGES] packed words, 128-byte swizzle
+    uint32_t *gbuf = reinterpret_cast<uint32_t *>(wring + (size_t)C::WSTAGES * FG_WORD_BYTES);       // [64][256]
+    unsigned char *tables = wring + (size_t)C::WSTAGES * FG_WORD_BYTES + C::GBUF_BYTES;
+    uint64_t *afull = reinterpret_cast<uint64_t *>(tables);                // [ASTAGES] rows landed
+    uint64_t *bfull = afull + C::ASTAGES;                                  // [BSTAGES] decoded (+ in the first CTA: the second CTA's half)
+    uint64_t *done = bfull + C::BSTAGES;                                   // [DONE] MMAs of stage i completed: done[i % DONE]
+    uint64_t *wfull = done + C::DONE;                                   // [WSTAGES] packed words landed
+    uint64_t *wempty = wfull + C::WSTAGES;                                 // [WSTAGES] read by the stage's decode warps
+    uint64_t *tmem_full = wempty + C::WSTAGES;                             // [2] accumulators of a pass complete
+    uint64_t *tmem_empty = tmem_full + 2;                                  // [2] (first CTA) accumulators drained, both CTAs' warps
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    float *scales = reinterpret_cast<float *>(tables + 256);               // [3][128]
-    int *pair_base = reinterpret_cast<int *>(tables + 256 + 3 * 128 * 4);  // [FG_MAXU + 1]
-    int *single_base = pair_base + FG_MAXU + 1;                            // [FG_MAXU + 1]
+    float *scales = reinterpret_cast<float *>(tables + 512);               // [2 column blocks][3][128]
     float *tbuf = reinterpret_cast<float *>(tables + C::TABLE_BYTES);      // [8 warps][32 rows][16] (down only)
-    const int *row_base = a.plan + PLAN_ROW_BASE;                          // global (L1 / L2 hits)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int KT = a.K >> 4, NTILES = a.N >> 4, NB = a.N >> 7, KS = a.K / FG_BK;
-    const int pairs_all = a.plan[2];
-    const int total = (pairs_all + a.plan[3]) * NB;
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int KT = a.K >> 4, NBP = a.N >> 8, KS = a.K / FG_BK;
+    const int total = a.plan[2] * NBP, items = total > pair ? (total - pair + pairs - 1) / pairs : 0;
 
     if (tid == 0) {
-        for (int s = 0; s < C::STAGES; ++s) { mbar_init(full + s, 1 + FG_DEC_WARPS); mbar_init(empty + s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + b, 1); mbar_init(tmem_empty + b, 8); }
+        for (int s = 0; s < C::ASTAGES; ++s) mbar_init(afull + s, 1);
+        for (int s = 0; s < C::BSTAGES; ++s) mbar_init(bfull + s, 8 + (rank == 0));
+        for (int s = 0; s < C::DONE; ++s) mbar_init(done + s, 1);
+        for (int s = 0; s < C::WSTAGES; ++s) { mbar_init(wfull + s, 1); mbar_init(wempty + s, 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + b, 1); mbar_init(tmem_empty + b, 16); }
         *abort_flag = 0;
         mbar_fence_init();
     }
-    for (int i = tid; i <= FG_MAXU; i += FG_THREADS) {
-        pair_base[i] = a.plan[PLAN_PAIR_BASE + i];
-        single_base[i] = a.plan[PLAN_SINGLE_BASE + i];
-    }
     if (warp == 2) tmem_alloc(tmem_slot, 512);
     tc_fence_before();
-    __syncthreads();
+    cluster_sync();                                                        // the peer's barriers are initialised as well
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // the slot that stage `it` of a ring of `depth` stages takes is free: stage it - depth has been consumed
+    auto slot_free = [&](uint32_t it, uint32_t depth) {
+        if (it < depth) return true;
+        const uint32_t j = it - depth;
+        return wait_or_abort<FG_SLEEP>(done + j % C::DONE, (j / C::DONE) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT);
+    };
 
     if (warp < 4) {
-        // ------------------------------------------------------------------ warpgroup 0: TMA, MMA issue
-#if FG_DEC_WARPS == 16
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
-#else
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-#endif
+        // ------------------------------------------------------------------ warpgroup 0: TMA, MMA issue, relay
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_MMA));
         if (warp == 0 && lane == 0) {
             uint32_t it = 0;
-            for (int item = blockIdx.x; item < total && !*abort_flag; item += gridDim.x) {
-                const ItemInfo t = item_info(item, NB, pairs_all, pair_base, single_base, row_base, a.ids);
-                bool ok = true;
+            bool ok = true;
+            for (int item = pair; item < total && ok && !*abort_flag; item += pairs) {
+                const ItemInfo t = item_info(item, NBP, a.chunks, rank);
                 for (int pm = 0; pm < MATS && ok; ++pm) {
                     const CUtensorMap *map = (pm == 1 && !a.shared_x) ? &mapA1 : &mapA0;
                     for (int s = 0; s < KS; ++s, ++it) {
-                        const int slot = it % C::STAGES;
-                        const uint32_t n = it / C::STAGES;
-                        if (!wait_or_abort(empty + slot, (n & 1) ^ 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT)) { ok = false; break; }
-                        unsigned char *st = stages + (size_t)slot * C::STAGE_BYTES;
-                        if (FG_PROBE & 16) { mbar_arrive(full + slot); continue; }   // no A loads
-                        mbar_expect_tx(full + slot, t.ntiles * FG_TILE_BYTES);
-                        tma_load_2d(st, map, s * FG_BK, t.row0, full + slot);
-                        if (t.ntiles == 2) tma_load_2d(st + FG_TILE_BYTES, map, s * FG_BK, t.row0 + FG_BM, full + slot);
+                        const uint32_t slot = it % C::ASTAGES;
+                        if (!slot_free(it, C::ASTAGES)) { ok = false; break; }
+                        if (t.cnt == 0) { mbar_arrive(afull + slot); continue; }       // (a chunk of one row: the peer has it)
+                        mbar_expect_tx(afull + slot, FG_TILE_BYTES);
+                        tma_load_2d(aring + (size_t)slot * FG_TILE_BYTES, map, s * FG_BK, t.row, afull + slot);
                     }
                 }
-                if (!ok) break;
             }
-        } else if (warp == 1 && lane == 0) {
-            // One thread issues every MMA.  Its own instruction stream is the critical path of the tensor pipe, so the
+        } else if (warp == 1 && rank == 0) {
+            // One elected thread of this warp issues every MMA of the pair; the warp runs the loop together, so that the descriptors
+            // stay in uniform registers.  Its instruction stream is the critical path of the tensor pipe, so the
             // shared-memory descriptors are built once (stage 0) and advanced by adding constants: the address field
-            // counts 16-byte units, a stage is STAGE_BYTES apart, a K step of 16 halves is 32 bytes.
-            const uint64_t desc_a0 = umma_desc_sw128(smem_u32(stages));
-            const uint64_t desc_b0 = umma_desc_sw128(smem_u32(stages) + 2 * FG_TILE_BYTES);
+            // counts 16-byte units, a stage is a tile apart, a K step of 16 halves is 32 bytes.
+            const uint64_t desc_a0 = umma_desc_sw128(smem_u32(aring)), desc_b0 = umma_desc_sw128(smem_u32(bring));
             uint32_t it = 0, pc = 0;
-            for (int item = blockIdx.x; item < total && !*abort_flag; item += gridDim.x) {
-                const ItemInfo t = item_info(item, NB, pairs_all, pair_base, single_base, row_base, a.ids);
-                const bool two = t.ntiles == 2;
-                bool ok = true;
+            bool ok = true;
+            for (int item = pair; item < total && ok; item += pairs) {
                 for (int pm = 0; pm < MATS && ok; ++pm, ++pc) {
                     const uint32_t pb = pc & 1;
-                    if (!wait_or_abort(tmem_empty + pb, ((pc >> 1) & 1) ^ 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, wait_or_abort<0>(tmem_empty + pb, ((pc >> 1) & 1) ^ 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
+                    if (!ok) break;
                     tc_fence_after();
                     const uint32_t d0 = tmem_base + pb * 256;
                     for (int s = 0; s < KS; ++s, ++it) {
-                        const uint32_t slot = it % C::STAGES;
-                        const uint32_t n = it / C::STAGES;
-                        if (!wait_or_abort(full + slot, n & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)) { ok = false; break; }
+                        const uint32_t sa = it % C::ASTAGES, sb = it % C::BSTAGES;
+                        ok = __all_sync(0xffffffffu, wait_or_abort<0>(afull + sa, (it / C::ASTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
+                                                         wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
+                        if (!ok) break;
                         tc_fence_after();
-                        const uint64_t da = desc_a0 + (uint64_t)(slot * (C::STAGE_BYTES >> 4));
-                        const uint64_t db = desc_b0 + (uint64_t)(slot * (C::STAGE_BYTES >> 4));
-                        const uint32_t acc0 = s > 0 ? 1u : 0u;
-                        if (two) {
+                        const uint64_t da = desc_a0 + (uint64_t)(sa * (FG_TILE_BYTES >> 4)), db = desc_b0 + (uint64_t)(sb * (FG_TILE_BYTES >> 4));
+                        if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < FG_BK / 16; ++kk) {
-                                umma_f16(d0, da + 2 * kk, db + 2 * kk, UMMA_IDESC, kk > 0 ? 1u : acc0);
-                                umma_f16(d0 + FG_BN, da + (FG_TILE_BYTES >> 4) + 2 * kk, db + 2 * kk, UMMA_IDESC, kk > 0 ? 1u : acc0);
-                            }
-                        } else {
-#pragma unroll
-                            for (int kk = 0; kk < FG_BK / 16; ++kk)
-                                umma_f16(d0, da + 2 * kk, db + 2 * kk, UMMA_IDESC, kk > 0 ? 1u : acc0);
+                            for (int kk = 0; kk < FG_BK / 16; ++kk) umma_f16(d0, da + 2 * kk, db + 2 * kk, UMMA_IDESC, kk > 0 || s > 0 ? 1u : 0u);
+                            umma_commit(done + it % C::DONE);       // both CTAs may overwrite the stage once these MMAs have read it
+                            if (s == KS - 1) umma_commit(tmem_full + pb);      // the accumulators of this pass are complete
                         }
-                        umma_commit(empty + slot);          // the stage may be overwritten once these MMAs have read it
+                        __syncwarp();
                     }
-                    if (ok) umma_commit(tmem_full + pb);    // the accumulators of this pass are complete
                 }
-                if (!ok) break;
             }
+        } else if (warp == 3 && lane == 0) {
+            // packed words of this CTA's column block, a ring of their own a few stages ahead of the decode
+            uint32_t it = 0;
+            bool ok = true;
+            for (int item = pair; item < total && ok && !*abort_flag; item += pairs) {
+                const ItemInfo t = item_info(item, NBP, a.chunks, rank);
+                for (int pm = 0; pm < MATS && ok; ++pm)
+                    for (int s = 0; s < KS; ++s, ++it) {
+                        const uint32_t ws = it % C::WSTAGES;
+                        if (!wait_or_abort<FG_SLEEP>(wempty + ws, ((it / C::WSTAGES) & 1) ^ 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT)) { ok = false; break; }
+                        mbar_expect_tx(wfull + ws, FG_WORD_BYTES);
+                        tma_load_3d(wring + ws * FG_WORD_BYTES, pm ? &mapT1 : &mapT0, 0, t.e * KT + 4 * s, (2 * t.nbp + rank) * 8, wfull + ws);
+                    }
+            }
+        } else if (warp == 1 && lane == 0) {
+            // second CTA: tell the issuing thread that this CTA's half of a stage is there
+            uint32_t it = 0;
+            bool ok = true;
+            for (int item = pair; item < total && ok && !*abort_flag; item += pairs)
+                for (int s = 0; s < MATS * KS && ok; ++s, ++it) {
+                    const uint32_t sa = it % C::ASTAGES, sb = it % C::BSTAGES;
+                    ok = wait_or_abort<0>(afull + sa, (it / C::ASTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
+                         wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
+                    if (ok) mbar_arrive_cluster(bfull + sb, 0);
+                }
         }
     } else if (warp < 12) {
-        // ------------------------------------------------------------------ warpgroups 1-2: epilogue (tile 0 | tile 1)
-#if FG_DEC_WARPS == 16
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 " FG_STR(FG_EPI_REGS) ";");
-#else
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-#endif
-        const int q = warp & 3, tl = (warp - 4) >> 2;        // TMEM lane quadrant, M tile of the item
-        const int m = q * 32 + lane, em = tl * 128 + m;      // row of the tile, row of the item (0..255)
+        // ------------------------------------------------------------------ warpgroups 1-2: epilogue (column block 0 | 1)
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FG_REGS_EPI));
+        const int q = warp & 3, cb = (warp - 4) >> 2;        // TMEM lane quadrant, column block of the item
+        const int m = q * 32 + lane, em = cb * 128 + m;      // row of this CTA, thread of the epilogue (0..255)
+        const float *sc = scales + cb * 384;
         uint32_t pc = 0;
         bool ok = true;
         // A warp whose wait gave up (or that sees the abort flag) does not leave this loop: it walks the remaining items
         // arriving at the two barriers only, so that a sibling which passed the same wait at the last moment never
         // stands alone at a barrier of eight warps.
-        for (int item = blockIdx.x; item < total; item += gridDim.x) {
-            const ItemInfo t = item_info(item, NB, pairs_all, pair_base, single_base, row_base, a.ids);
-            const bool has = tl < t.ntiles;
-            const int cnt = tl == 0 ? t.cnt0 : t.cnt1;
-            // scale vectors of (expert, column block): written by the first 128 epilogue threads, read by all 256
+        for (int item = pair; item < total; item += pairs) {
+            const ItemInfo t = item_info(item, NBP, a.chunks, rank);
+            const int nb = 2 * t.nbp + cb;
+            // scale vectors of (expert, column block): written by the block's 128 threads, read by them
             asm volatile("bar.sync 1, 256;");
             if (ok && *abort_flag) ok = false;
-            if (ok && em < 128) {
-                const size_t o = (size_t)t.e * a.N + t.nb * 128 + em;
+            if (ok) {
+                const size_t o = (size_t)t.e * a.N + nb * 128 + m;
                 // the 1 / sqrt(128) of every Hadamard transform is folded into the scale vectors here (the transform is
                 // linear), which takes one multiply per element out of each epilogue step
-                scales[em] = __half2float(a.sv0[o]) * HAD_SCALE;
-                if (MATS == 2) { scales[128 + em] = __half2float(a.sv1[o]) * HAD_SCALE; scales[256 + em] = __half2float(a.sd[o]) * HAD_SCALE; }
+                float *w = scales + cb * 384 + m;
+                w[0] = __half2float(a.sv0[o]) * HAD_SCALE;
+                if (MATS == 2) { w[128] = __half2float(a.sv1[o]) * HAD_SCALE; w[256] = __half2float(a.sd[o]) * HAD_SCALE; }
             }
             asm volatile("bar.sync 1, 256;");
             if (!ok) continue;
             float v[128];
             for (int pm = 0; pm < MATS; ++pm, ++pc) {
                 const uint32_t pb = pc & 1;
-                if (!wait_or_abort(tmem_full + pb, (pc >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)) { ok = false; break; }
+                if (!wait_or_abort<FG_SLEEP>(tmem_full + pb, (pc >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)) { ok = false; break; }
                 tc_fence_after();
+                const bool has = t.cnt > q * 32;             // (uniform: rows of this warp)
                 if (has) {
-                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + pb * 256 + tl * FG_BN;
+                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + pb * 256 + cb * FG_BN;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) tmem_ld32(taddr + c * 32, v + c * 32);
                     tmem_ld_wait();
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(tmem_empty + pb);             // this warp's rows are in registers
+                if (lane == 0) mbar_arrive_cluster(tmem_empty + pb, 0);  // this warp's rows are in registers
                 if (!has) continue;
-                if (FG_PROBE & 2) {
-                    if (v[5] == 1.2345f && m < cnt) a.status[1] = 1;
-                    continue;
-                }
                 fwht128_regs(v);
-                const float2 *sc2 = reinterpret_cast<const float2 *>(scales);       // (8-byte aligned: the tables are 128-byte aligned)
+                const float2 *sc2 = reinterpret_cast<const float2 *>(sc);
                 if (MATS == 2 && pm == 0) {
                     // gate: scale, bf16 rounding, clamp, silu (rounded) -> two bf16 per word, this thread's column of gbuf
 #pragma unroll
@@ -556,8 +582,8 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                         v[2 * i + 1] = pr.y * sd2.y;
                     }
                     fwht128_regs(v);
-                    if (m < cnt) {
-                        uint4 *o = reinterpret_cast<uint4 *>(a.xd + (size_t)(t.row0 + em) * a.N + t.nb * 128);
+                    if (m < t.cnt) {
+                        uint4 *o = reinterpret_cast<uint4 *>(a.xd + (size_t)(t.row + m) * a.N + nb * 128);
 #pragma unroll
                         for (int c = 0; c < 16; ++c) {
                             __half2 h[4];
@@ -573,14 +599,14 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                     // put 32 rows x 16 bytes into every store instruction (half-filled sectors).  The rows go through a
                     // per-warp shared-memory tile, 16 columns at a time, and leave as 8 rows x 64 contiguous bytes per
                     // instruction.  Chunk c of row r sits at chunk c ^ ((r >> 1) & 3): conflict-free both ways.
-                    const int p = m < cnt ? a.src_pair[t.row0 + em] : -1;
+                    const int p = m < t.cnt ? a.src_pair[t.row + m] : -1;
                     float *wbuf = tbuf + (warp - 4) * 512;
 #pragma unroll
                     for (int ch = 0; ch < 8; ++ch) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
                             const int col = ch * 16 + 4 * c;
-                            const float4 s4 = *reinterpret_cast<const float4 *>(scales + col);
+                            const float4 s4 = *reinterpret_cast<const float4 *>(sc + col);
                             *reinterpret_cast<float4 *>(wbuf + lane * 16 + ((c ^ ((lane >> 1) & 3)) << 2)) =
                                 make_float4(v[col] * s4.x, v[col + 1] * s4.y, v[col + 2] * s4.z, v[col + 3] * s4.w);
                         }
@@ -591,7 +617,7 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
                             const float4 val = *reinterpret_cast<const float4 *>(wbuf + rr * 16 + ((c ^ ((rr >> 1) & 3)) << 2));
                             const int pr = __shfl_sync(0xffffffffu, p, rr);              // pair row of warp row rr
                             if (pr >= 0)
-                                *reinterpret_cast<float4 *>(a.y + (size_t)pr * a.N + t.nb * 128 + ch * 16 + 4 * c) = val;
+                                *reinterpret_cast<float4 *>(a.y + (size_t)pr * a.N + nb * 128 + ch * 16 + 4 * c) = val;
                         }
                         __syncwarp();
                     }
@@ -599,108 +625,58 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             }
         }
     } else {
-        // ------------------------------------------------------------------ warpgroups 3-4: trellis decode of B
-#if FG_DEC_WARPS == 16
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 " FG_STR(FG_DEC_REGS) ";");
-#else
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-#endif
-        const int dw = warp - 12;
-        constexpr int NTL = 32 / FG_DEC_WARPS;               // n tiles of this warp per stage (4 k-tiles x 8 n-tiles in all)
-        const int ktl = dw & 3, nt_begin = (dw >> 2) * NTL;
-        const int g = lane >> 2, tq = lane & 3;
-        // byte offsets inside the B tile of this lane's four 32-bit stores (before the n-tile offset)
-        const int c0 = 2 * ktl, c1 = 2 * ktl + 1;
-        const int off_lo0 = nt_begin * 2048 + g * 128 + ((c0 ^ g) << 4) + 4 * tq;     // n = g,     k = 2t
-        const int off_lo1 = nt_begin * 2048 + g * 128 + ((c1 ^ g) << 4) + 4 * tq;     // n = g,     k = 2t + 8
-        uint32_t it = 0;
-        bool ok = true;
-        int item = blockIdx.x, pm = 0;
-        ItemInfo t{};
-        auto src_of = [&](const ItemInfo &ti, int pmat, int s) {
-            return (pmat ? a.T1 : a.T0) + (((size_t)ti.e * KT + 4 * s + ktl) * NTILES + (size_t)ti.nb * 8 + nt_begin) * 32 + lane;
-        };
-        auto load_words = [&](const uint32_t *src, uint32_t (&w)[NTL]) {
+        // ------------------------------------------------------------------ warpgroups 3-6: trellis decode of B
+        // An n-tile of a stage at a time, round robin over the warps.  A lane reads 16 bytes (four words: all 16 k of columns G and
+        // G + 8) of k-tile T of the stage, decodes them in registers and, once the slot is free, stores them as four 16-byte pieces
+        // of the K-major tile, conflict-free under its swizzle: the decode is not part of the loop from a slot's release to the
+        // next MMA.
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_DEC));
+        const int G = lane >> 2, T = lane & 3;
+        // byte offsets in the n-tile of the B tile: rows G and + 8; 16-byte pieces 2 T and 2 T + 1, piece c of row r at c ^ (r & 7)
+        const uint32_t off0 = G * 128 + ((2 * T) ^ G) * 16, off1 = G * 128 + ((2 * T + 1) ^ G) * 16;
+        const uint32_t tiles_all = (uint32_t)(items * MATS * KS) * 8;
+        for (uint32_t c = warp - 12; c < tiles_all; c += FG_DEC) {
+            const uint32_t it = c >> 3, nt = c & 7, sb = it % C::BSTAGES, ws = it % C::WSTAGES;
+            // (the vote also brings the lanes together again: they may have left the wait apart)
+            if (!__all_sync(0xffffffffu, wait_or_abort<FG_SLEEP>(wfull + ws, (it / C::WSTAGES) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT))) break;
+            // the lane's four words and the word in front of them (circular): row (n-tile, k-tile) of 128 bytes, piece c of row r at
+            // c ^ (r & 7)
+            const uint32_t row = nt * 4 + T;
+            const unsigned char *wp = wring + ws * FG_WORD_BYTES + row * 128;
+            const uint4 wv = *reinterpret_cast<const uint4 *>(wp + ((G ^ (row & 7)) << 4));
+            const uint32_t before = *reinterpret_cast<const uint32_t *>(wp + ((((G + 7) & 7) ^ (row & 7)) << 4) + 12);
+            const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
+            uint32_t o[4][4];
 #pragma unroll
-            for (int i = 0; i < NTL; ++i) w[i] = (FG_PROBE & 4) ? (uint32_t)(size_t)src : __ldg(src + i * 32);
-        };
-        auto do_stage = [&](const uint32_t (&wr)[NTL]) {
-            const int slot = it % C::STAGES;
-            const uint32_t n = it / C::STAGES;
-            if (!wait_or_abort(empty + slot, (n & 1) ^ 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT)) { ok = false; return; }
-            unsigned char *bt = stages + (size_t)slot * C::STAGE_BYTES + 2 * FG_TILE_BYTES;
-#pragma unroll
-            for (int i = 0; i < NTL; ++i) {
-                const uint32_t w = wr[i];
-                if (FG_PROBE & 8) continue;                    // no stores at all
-                if (FG_PROBE & 1) {
-                    unsigned char *tbp = bt + i * 2048;
-                    *reinterpret_cast<uint32_t *>(tbp + off_lo0) = w;
-                    *reinterpret_cast<uint32_t *>(tbp + off_lo1) = w;
-                    *reinterpret_cast<uint32_t *>(tbp + off_lo0 + 1024) = w;
-                    *reinterpret_cast<uint32_t *>(tbp + off_lo1 + 1024) = w;
-                    continue;
-                }
-                const uint32_t pw = __shfl_sync(0xffffffffu, w, (lane + 31) & 31);
-                uint32_t x0, x1, x2, x3, x4, x5, x6, x7;
-                codeword_pair(__funnelshift_r(w, pw, 12), x0, x4);     // j = 0 | 4
-                codeword_pair(__funnelshift_r(w, pw, 8), x1, x5);      // j = 1 | 5
-                codeword_pair(__funnelshift_r(w, pw, 4), x2, x6);      // j = 2 | 6
-                codeword_pair(w, x3, x7);                              // j = 3 | 7
-                const uint32_t p01 = __byte_perm(weight_dup(x0), weight_dup(x1), 0x5410);
-                const uint32_t p23 = __byte_perm(weight_dup(x2), weight_dup(x3), 0x5410);
-                const uint32_t p45 = __byte_perm(weight_dup(x4), weight_dup(x5), 0x5410);
-                const uint32_t p67 = __byte_perm(weight_dup(x6), weight_dup(x7), 0x5410);
-                unsigned char *tb = bt + i * 2048;
-                *reinterpret_cast<uint32_t *>(tb + off_lo0) = p01;
-                *reinterpret_cast<uint32_t *>(tb + off_lo1) = p23;
-                *reinterpret_cast<uint32_t *>(tb + off_lo0 + 1024) = p45;           // n = g + 8
-                *reinterpret_cast<uint32_t *>(tb + off_lo1 + 1024) = p67;
+            for (int t = 0; t < 4; ++t) {
+                const uint32_t pw = t == 0 ? before : w[t - 1];
+                uint32_t hi[4], lo[4];
+                codeword_pair(__funnelshift_r(w[t], pw, 12), hi[0], lo[0]);                  // k = 2t:     columns G, G + 8
+                codeword_pair(__funnelshift_r(w[t], pw, 8), hi[1], lo[1]);                   // k = 2t + 1
+                codeword_pair(__funnelshift_r(w[t], pw, 4), hi[2], lo[2]);                   // k = 2t + 8
+                codeword_pair(w[t], hi[3], lo[3]);                                           // k = 2t + 9
+                o[0][t] = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410);
+                o[1][t] = __byte_perm(weight_dup(hi[2]), weight_dup(hi[3]), 0x5410);
+                o[2][t] = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
+                o[3][t] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(wempty + ws);
+            if (!__all_sync(0xffffffffu, slot_free(it, C::BSTAGES))) break;
+            unsigned char *bt = bring + (size_t)sb * FG_TILE_BYTES + nt * 2048;
+            *reinterpret_cast<uint4 *>(bt + off0) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+            *reinterpret_cast<uint4 *>(bt + off1) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+            *reinterpret_cast<uint4 *>(bt + off0 + 1024) = make_uint4(o[2][0], o[2][1], o[2][2], o[2][3]);
+            *reinterpret_cast<uint4 *>(bt + off1 + 1024) = make_uint4(o[3][0], o[3][1], o[3][2], o[3][3]);
             fence_async_smem();                              // generic-proxy stores -> visible to the tensor core
             __syncwarp();
-            if (lane == 0) mbar_arrive(full + slot);
-            ++it;
-        };
-        // Packed words are fetched three stages ahead into four register buffers; KS is a multiple of 4, so the
-        // buffer of a stage is s & 3 at compile time.  (pass, stage) + d stages ahead, across pass / item boundaries:
-        uint32_t w0[NTL], w1[NTL], w2[NTL], w3[NTL];
-        bool valid = item < total;
-        int n_item = item, n_pm = 0;
-        ItemInfo tn{};
-        bool n_valid = false;
-        auto fetch = [&](int s, uint32_t (&w)[NTL]) {          // stage s of the current pass; s >= KS: the next pass
-            if (s < KS) load_words(src_of(t, pm, s), w);
-            else if (n_valid) load_words(src_of(tn, n_pm, s - KS), w);
-        };
-        auto advance = [&]() {                                 // describe the pass after (item, pm)
-            n_item = item; n_pm = pm + 1; tn = t; n_valid = true;
-            if (n_pm == MATS) {
-                n_pm = 0;
-                n_item = item + gridDim.x;
-                n_valid = n_item < total;
-                if (n_valid) tn = item_info(n_item, NB, pairs_all, pair_base, single_base, row_base, a.ids);
-            }
-        };
-        if (valid) {
-            t = item_info(item, NB, pairs_all, pair_base, single_base, row_base, a.ids);
-            advance();
-            fetch(0, w0); fetch(1, w1); fetch(2, w2);
-        }
-        while (valid && ok && !*abort_flag) {
-            for (int s = 0; s < KS && ok; s += 4) {
-                fetch(s + 3, w3); do_stage(w0); if (!ok) break;
-                fetch(s + 4, w0); do_stage(w1); if (!ok) break;
-                fetch(s + 5, w1); do_stage(w2); if (!ok) break;
-                fetch(s + 6, w2); do_stage(w3);
-            }
-            item = n_item; pm = n_pm; t = tn; valid = n_valid;
-            if (valid) advance();
+            if (lane == 0) mbar_arrive(bfull + sb);
         }
     }
 
     tc_fence_before();
-    __syncthreads();
+    // the pair ends together: no arrival or operand read is outstanding (not the aligned form: one lane of warps 0 and 1 worked alone)
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     tc_fence_after();
     if (warp == 2) tmem_dealloc(tmem_base, 512);
 }
@@ -712,28 +688,12 @@ using namespace gf;
 // ---------------------------------------------------------------------------------------------- host side
 namespace {
 int fail_if(cudaError_t e) { return e == cudaSuccess ? 0 : gf::fail_cuda(e, "cudaFuncSetAttribute"); }
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 // fp16 matrix [rows][K] row-major; box = 128 rows x 64 halves (128 bytes), 128-byte swizzle
 int make_map(CUtensorMap *map, void *base, uint64_t rows, uint64_t K) {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        GF_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
-        GF_REQUIRE(p != nullptr && q == cudaDriverEntryPointSuccess, "cuTensorMapEncodeTiled is not available in this driver");
-        fn = (EncodeTiledFn)p;
-    }
-    const cuuint64_t dims[2] = {K, rows};
-    const cuuint64_t strides[1] = {K * 2};
-    const cuuint32_t box[2] = {FG_BK, FG_BM};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    GF_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
-    return 0;
+    const uint64_t dims[2] = {K, rows}, strides[1] = {K * 2};
+    const uint32_t box[2] = {FG_BK, FG_BM};
+    return gf::encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, "grouped rows");
 }
 }  // namespace
 
@@ -742,6 +702,7 @@ struct glmflash_fast_experts {
     void *pool = nullptr;                                   // the one allocation behind the buffers below
     __half *xg = nullptr, *xu = nullptr, *xd = nullptr;     // grouped rows
     float *out = nullptr;                                   // pair rows
+    int4 *chunks = nullptr;
     int *plan = nullptr, *src_pair = nullptr, *row_expert = nullptr, *status = nullptr;
     CUtensorMap map_xg, map_xu, map_xd;
     int sms = 0;
@@ -774,6 +735,7 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
     pool.take(&f->xd, P * I * 2);
     pool.take(&f->out, P * H * 4);
     pool.take(&f->plan, PLAN_INTS * 4);
+    pool.take(&f->chunks, (P / FG_CHUNK + cfg->experts + 1) * sizeof(int4));
     pool.take(&f->src_pair, P * 4);
     pool.take(&f->row_expert, P * 4);
     pool.take(&f->status, 16);
@@ -808,23 +770,26 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
     const long P = (long)rows * c.slots;
     if (f->phases & 1)
         fast_plan_kernel<<<c.experts + 1, FG_MAXU, 0, s>>>(ids, count, members, maxm, c.slots, c.experts, c.shared_exl3, c.expert_lo,
-                                              c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->src_pair, f->row_expert);
+                                              c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->chunks, f->src_pair, f->row_expert);
     GF_CUDA(cudaGetLastError());
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)
-        fast_rot_kernel<<<(unsigned)std::min<long>(P, 148L * 32), 256, 0, s>>>((const __nv_bfloat16 *)input, x_stride, f->plan, f->src_pair,
-                                                              f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u,
-                                                              f->xg, f->xu, H, c.slots, mats);
+        fast_rot_kernel<<<(unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 148L * 32), 256, 0, s>>>(
+            (const __nv_bfloat16 *)input, x_stride, f->plan, f->src_pair, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg,
+            f->xu, H, c.slots, mats, (((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 16 == 0 && x_stride % 8 == 0));
     GF_CUDA(cudaGetLastError());
     FastGemmArgs a{};
-    a.ids = ids; a.plan = f->plan; a.src_pair = f->src_pair; a.status = f->status; a.limit = c.limit;
-    a.T0 = w->gt; a.T1 = w->ut; a.sv0 = (const __half *)w->svh_g; a.sv1 = (const __half *)w->svh_u; a.sd = (const __half *)w->suh_d;
+    a.plan = f->plan; a.chunks = f->chunks; a.src_pair = f->src_pair; a.status = f->status; a.limit = c.limit;
+    CUtensorMap mg, mu, md;
+    if (bank_map(&mg, w->gt, c.experts + 1, H, I, 4) || bank_map(&mu, w->ut, c.experts + 1, H, I, 4) || bank_map(&md, w->dt, c.experts + 1, I, H, 4))
+        return -1;
+    a.sv0 = (const __half *)w->svh_g; a.sv1 = (const __half *)w->svh_u; a.sd = (const __half *)w->suh_d;
     a.xd = f->xd; a.y = nullptr; a.K = H; a.N = I; a.shared_x = shared_x ? 1 : 0;
-    if (f->phases & 4) fast_gemm_kernel<2><<<f->sms, FG_THREADS, FgCfg<2>::SMEM, s>>>(f->map_xg, f->map_xu, a);
+    if (f->phases & 4) fast_gemm_kernel<2><<<f->sms & ~1, FG_THREADS, FgCfg<2>::SMEM, s>>>(f->map_xg, f->map_xu, mg, mu, a);
     GF_CUDA(cudaGetLastError());
-    a.T0 = w->dt; a.T1 = w->dt; a.sv0 = (const __half *)w->svh_d; a.sv1 = nullptr; a.sd = nullptr;
+    a.sv0 = (const __half *)w->svh_d; a.sv1 = nullptr; a.sd = nullptr;
     a.xd = nullptr; a.y = f->out; a.K = I; a.N = H; a.shared_x = 1;
-    if (f->phases & 8) fast_gemm_kernel<1><<<f->sms, FG_THREADS, FgCfg<1>::SMEM, s>>>(f->map_xd, f->map_xd, a);
+    if (f->phases & 8) fast_gemm_kernel<1><<<f->sms & ~1, FG_THREADS, FgCfg<1>::SMEM, s>>>(f->map_xd, f->map_xd, md, md, a);
     GF_CUDA(cudaGetLastError());
     return 0;
 }
