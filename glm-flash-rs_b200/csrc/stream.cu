@@ -315,7 +315,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     tb.pref = tb.mask + a.umax;
     tb.pair = reinterpret_cast<uint16_t *>(tb.pref + a.umax + 1);
     tb.state = reinterpret_cast<short *>(tb.pair + a.umax * 16);
-    __shared__ int abort_sh;
+    __shared__ int abort_sh, first_sh;
     __shared__ uint32_t used_sh[32];
     __shared__ __align__(16) float fin_sh[8][128];
 
@@ -354,7 +354,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
     const uint32_t epoch = __ldcg(a.ctrl + CTRL_EPOCH) + 1u;          // words of earlier launches carry smaller ones
     const int U = st_build_tables(a, tb, used_sh, row, slot);
-    if (tid == ST_FIN * 32) job_sh[0] = drawn;
+    if (tid == ST_FIN * 32) first_sh = drawn;
     __syncthreads();
     const int units_g = a.do_g ? U * 2 * SK1 * NB1 : 0, units = units_g + (a.do_d ? U * SK2 * NB2 : 0);
 
@@ -385,7 +385,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         ll_store2(a.xr + ((size_t)(mat * P + p) * H + k) / 2, pack_half2(v[0] * HAD_SCALE, v[1] * HAD_SCALE), pack_half2(v[2] * HAD_SCALE, v[3] * HAD_SCALE), epoch);
     };
     if (warp != ST_PROD) {
-        const int first = job_sh[0], w = warp - (warp > ST_PROD);
+        const int first = first_sh, w = warp - (warp > ST_PROD);
         if (first < jobs_r)
             for (int r = first * rot_job + w; r < min(rots, (first + 1) * rot_job); r += ST_THREADS / 32 - 1) rotate(r);
     }
@@ -397,14 +397,14 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         uint32_t it = 0;
         for (uint32_t c = 0;; ++c) {
             const int xs = c % ST_XSTAGES;
-            if (!cta.wait(wfull + it % ST_STAGES, (it / ST_STAGES) & 1)) break;
+            if (!__all_sync(0xffffffffu, cta.wait(wfull + it % ST_STAGES, (it / ST_STAGES) & 1))) break;
             const int4 d = desc[it % ST_STAGES];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
             const int nmem = __popc(tb.mask[d.y]);
             const uint32_t p01 = *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 2 * T);
             const uint32_t p23 = SETS == 2 ? *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 8 + 2 * T) : 0u;
-            if (!cta.wait(xfull + xs, (c / ST_XSTAGES) & 1)) break;
+            if (!__all_sync(0xffffffffu, cta.wait(xfull + xs, (c / ST_XSTAGES) & 1))) break;
             float acc[SETS][4];
 #pragma unroll
             for (int q = 0; q < SETS; ++q)
@@ -414,7 +414,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             bool ok = true;
             for (int half = 0; half < halves; ++half, ++it) {
                 const int s = it % ST_STAGES;
-                if (half) ok = cta.wait(wfull + s, (it / ST_STAGES) & 1);
+                if (half) ok = __all_sync(0xffffffffu, cta.wait(wfull + s, (it / ST_STAGES) & 1));
                 if (!ok) break;
                 st_decode<SETS>(words + s * ST_WBYTES, xbuf + xs * XBYTES + half * 512, warp, lane, SETS == 2 && nmem > 8, acc);
                 __syncwarp();
@@ -443,7 +443,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         const int xw = warp - ST_DEC;
         for (uint32_t it = 0;; ++it) {
             const int s = it % ST_XSTAGES;
-            if (!cta.wait(xready + s, (it / ST_XSTAGES) & 1)) break;
+            if (!__all_sync(0xffffffffu, cta.wait(xready + s, (it / ST_XSTAGES) & 1))) break;
             const int4 d = xdesc[s];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
