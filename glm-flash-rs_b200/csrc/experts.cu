@@ -38,10 +38,11 @@ int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limi
 
 using namespace gf;
 
-extern "C" int glmflash_experts_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_experts **out) {
+// max_rows_limit: 16 for the public owner; chunk owners keep one for their short chunks.
+int gf::experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit, glmflash_experts **out) {
     GF_REQUIRE(out != nullptr, "out is null");
     *out = nullptr;
-    if (check_config(cfg, cfg_bytes, 16)) return -1;      // upstream: 1..=MAX_ROWS (16), src/experts.rs:391-394
+    if (check_config(cfg, cfg_bytes, max_rows_limit)) return -1;
     glmflash_experts *e = new (std::nothrow) glmflash_experts();
     GF_REQUIRE(e != nullptr, "out of host memory");
     e->cfg = *cfg;
@@ -55,7 +56,7 @@ extern "C" int glmflash_experts_new(const glmflash_config *cfg, size_t cfg_bytes
     pool.take(&e->ll_xr, stream_xr_words(*cfg) * 8);
     pool.take(&e->ll_xd, stream_xdl_words(*cfg) * 8);
     pool.take(&e->ctrl, CTRL_WORDS * 4);
-    if (one_launch_selected()) {                          // scratch of the alternative layer kernel (window.cu)
+    if (cfg->max_rows <= 16 && one_launch_selected()) {                          // scratch of the alternative layer kernel (window.cu)
         e->sync_words = experts_window_sync_words(*cfg);
         pool.take(&e->z1, (size_t)2 * (H / 128) * P * I * 4);
         pool.take(&e->z2, (size_t)(I / 128) * P * H * 4);
@@ -69,6 +70,10 @@ extern "C" int glmflash_experts_new(const glmflash_config *cfg, size_t cfg_bytes
     return 0;
 }
 
+extern "C" int glmflash_experts_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_experts **out) {
+    return experts_new(cfg, cfg_bytes, 16, out);              // upstream: 1..=MAX_ROWS (16), src/experts.rs:391-394
+}
+
 extern "C" void glmflash_experts_free(glmflash_experts *e) {
     if (!e) return;
     cudaFree(e->pool);
@@ -76,7 +81,7 @@ extern "C" void glmflash_experts_free(glmflash_experts *e) {
 }
 
 // Fills in what both forms of a window share and launches it.
-static int run_stream(glmflash_experts *e, cudaStream_t s, StreamArgs a, const glmflash_weights *w, const void *input, int x_stride, int rows) {
+static int run_stream(const glmflash_experts *e, cudaStream_t s, StreamArgs a, const glmflash_weights *w, const void *input, int x_stride, int rows) {
     const glmflash_config &c = e->cfg;
     GF_REQUIRE(((uintptr_t)w->gt | (uintptr_t)w->ut | (uintptr_t)w->dt) % 16 == 0, "trellis tensors must be 16-byte aligned");
     GF_REQUIRE(((uintptr_t)input) % 8 == 0, "input must be 8-byte aligned");
@@ -85,13 +90,17 @@ static int run_stream(glmflash_experts *e, cudaStream_t s, StreamArgs a, const g
     a.suh_g = (const __half *)w->suh_g; a.suh_u = (const __half *)w->suh_u; a.suh_d = (const __half *)w->suh_d;
     a.svh_g = (const __half *)w->svh_g; a.svh_u = (const __half *)w->svh_u; a.svh_d = (const __half *)w->svh_d;
     a.x = (const __nv_bfloat16 *)input; a.x_stride = x_stride;
-    a.z1 = e->ll_z1; a.z2 = e->ll_z2; a.xr = e->ll_xr; a.xdl = e->ll_xd; a.xd = e->xd; a.y = e->y;
-    a.ctrl = e->ctrl; a.status = e->status;
+    a.z1 = e->ll_z1; a.z2 = e->ll_z2; a.xr = e->ll_xr; a.xdl = e->ll_xd; a.xd = e->xd;
+    if (!a.y) a.y = e->y;
+    a.ctrl = e->ctrl;
+    if (!a.status) a.status = e->status;
     a.H = c.hidden; a.I = c.inter; a.rows = rows; a.slots = c.slots; a.E = c.experts;
     a.e_lo = c.expert_lo; a.e_hi = c.expert_hi; a.shared = c.shared_exl3; a.limit = c.limit;
     // distinct experts that THIS GPU computes: at most one per pick, and at most its expert window (+ the shared expert)
+    a.srow_lo = c.shared_row_lo; a.srow_hi = c.shared_row_hi;
     a.umax = std::max(1, std::min(rows * c.slots, (c.expert_hi - c.expert_lo) + (c.shared_exl3 ? 1 : 0)));
     if (!a.picks) a.umax = std::max(1, std::min(rows * c.slots, c.experts + 1));   // (places in ids, skipped experts included)
+    if (rows > 16) a.umax += rows * c.slots / 16;                  // (an entry for every 16 members)
     a.do_g = (e->phases & 2) != 0;
     a.do_d = (e->phases & 4) != 0;
     return launch_stream(s, a, c.pdl != 0);
@@ -114,12 +123,12 @@ extern "C" int glmflash_experts_run_rows(glmflash_experts *e, void *stream, cons
 // `out` the rows are combined in the same launch.
 namespace gf {
 int experts_run_fused(glmflash_experts *e, cudaStream_t s, const glmflash_weights *w, const void *input, int x_stride,
-                      const int32_t *picks, const float *route_w, float *out, float *out2, int rows) {
+                      const int32_t *picks, const float *route_w, float *out, float *out2, int rows, float *y, int *status) {
     const glmflash_config &c = e->cfg;
     GF_REQUIRE(rows > 0 && rows <= c.max_rows, "expert verifier row/member bounds");
     GF_REQUIRE(x_stride >= c.hidden && x_stride % 4 == 0, "x_stride must be >= hidden and a multiple of 4");
     StreamArgs a{};
-    a.picks = picks; a.route_w = route_w; a.out = out; a.out2 = out2;
+    a.picks = picks; a.route_w = route_w; a.out = out; a.out2 = out2; a.y = y; a.status = status;
     return run_stream(e, s, a, w, input, x_stride, rows);
 }
 }  // namespace gf

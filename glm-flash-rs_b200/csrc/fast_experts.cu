@@ -46,6 +46,7 @@
 
 namespace gf {
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
+int *fast_experts_status_word(glmflash_fast_experts *f);
 
 constexpr int FG_DEC = 16;                                 // trellis-decode warps: n-tile by n-tile, round robin
 constexpr int FG_THREADS = (12 + FG_DEC) * 32;
@@ -793,6 +794,8 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
     GF_CUDA(cudaGetLastError());
     return 0;
 }
+
+int *gf::fast_experts_status_word(glmflash_fast_experts *f) { return f->status; }
 
 extern "C" int glmflash_fast_experts_set_phases(glmflash_fast_experts *f, int mask) {
     GF_REQUIRE(f != nullptr, "null argument");

@@ -9,10 +9,12 @@
 
 #include "common.cuh"
 #include "owners.cuh"
+#include "stream.cuh"
 
 namespace gf {
 int experts_run_fused(glmflash_experts *e, cudaStream_t s, const glmflash_weights *w, const void *input, int x_stride,
-                      const int32_t *picks, const float *route_w, float *out, float *out2, int rows);
+                      const int32_t *picks, const float *route_w, float *out, float *out2, int rows, float *y, int *status);
+int *fast_experts_status_word(glmflash_fast_experts *f);
 
 // out[r][d] = sum_{s < slots-1, expert computed here} w[r][s] * Y[r*slots+s][d]  (+ Y[shared pair] if computed here)
 // fp32, ascending slot order, shared last: the order of the oracle's combine.
@@ -99,11 +101,27 @@ bool gf::one_launch_selected() {
     return env && env[0] == '1';
 }
 
+// Chunks up to this many rows go to the streamed kernel, which decodes an expert's weights once per 16 of its rows (the GEMMs:
+// once per 256).  It wins while the decoding bounds both: us a layer, streamed | GEMMs, 2048 x 1536, 64 experts, top-4: 17 rows
+// 144 | 221, 40: 195 | 289, 128: 263 | 323, 192: 321 | 323, 256: 577 | 327; 4096 x 512, 288 experts, top-8: 17: 230 | 380, 128:
+// 814 | 974, 256: 1153 | 1009; eight experts of 64: 17: 45 | 83, 128: 83 | 94, 192: 110 | 96.  Hence 128 rows, fewer where the
+// routed experts have more than 16 rows on average (1024 x 2048, 24 experts, top-3, 128 rows: 141 | 145), and none where the
+// exchange areas, which grow with the rows, would pass 256 MB.
+static int short_chunk_rows(const glmflash_config &c) {
+    glmflash_config one = c;
+    one.max_rows = 1;
+    const size_t row = 8 * (stream_z1_words(one) + stream_z2_words(one) + stream_xr_words(one) + stream_xdl_words(one));
+    const size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)16 * c.experts / (c.slots - 1), ((size_t)256 << 20) / row});
+    return rows > 16 ? (int)rows : 0;
+}
+
 struct glmflash_moe {
     glmflash_config cfg;
     glmflash_grouping *grouping = nullptr;
     glmflash_experts *experts = nullptr;            // windows of <= 16 rows
     glmflash_fast_experts *fast = nullptr;          // chunks of > 16 rows
+    glmflash_experts *chunk = nullptr;              // the streamed kernel's buffers for chunks of up to chunk_rows rows
+    int chunk_rows = 0;
     void *pool = nullptr;                           // the one allocation behind the buffers below
     float *out = nullptr;
     void *in_dev = nullptr;                         // staging for run_host
@@ -122,7 +140,17 @@ extern "C" int glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, gl
     m->cfg = *cfg;
     int rc;                                         // (the window kernel groups its rows itself)
     if (cfg->max_rows <= 16) rc = glmflash_experts_new(cfg, cfg_bytes, &m->experts);
-    else if (!(rc = glmflash_grouping_new(cfg, cfg_bytes, &m->grouping))) rc = glmflash_fast_experts_new(cfg, cfg_bytes, &m->fast);
+    else if (!(rc = glmflash_grouping_new(cfg, cfg_bytes, &m->grouping)) && !(rc = glmflash_fast_experts_new(cfg, cfg_bytes, &m->fast))) {
+        m->chunk_rows = short_chunk_rows(*cfg);
+        if (m->chunk_rows > 0) {
+            glmflash_config cc = *cfg;
+            cc.max_rows = m->chunk_rows;
+            cc.shared_row_lo = cc.shared_row_hi = 0;
+            rc = experts_new(&cc, sizeof(cc), ST_MAX_ROWS, &m->chunk);
+            if (!rc)                                // (the row window counts rows of the chunk, whatever the owner holds)
+                m->chunk->cfg.shared_row_lo = cfg->shared_row_lo, m->chunk->cfg.shared_row_hi = cfg->shared_row_hi;
+        }
+    }
     const size_t rows = cfg->max_rows;
     Pool pool;
     pool.take(&m->out, rows * cfg->hidden * 4);
@@ -143,6 +171,7 @@ extern "C" void glmflash_moe_free(glmflash_moe *m) {
     glmflash_grouping_free(m->grouping);
     glmflash_experts_free(m->experts);
     glmflash_fast_experts_free(m->fast);
+    glmflash_experts_free(m->chunk);
     cudaFree(m->pool);
     delete m;
 }
@@ -157,7 +186,12 @@ extern "C" int glmflash_moe_run(glmflash_moe *m, void *stream, const glmflash_we
         return experts_run_window(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, rows, m->out, nullptr, -1);
     if (m->experts) {
         // one streamed launch: grouping, input rotation, both projections, epilogues and the combine
-        return experts_run_fused(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows);
+        return experts_run_fused(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows,
+                                 nullptr, nullptr);
+    } else if (m->chunk && rows <= m->chunk_rows && (m->phases | 16) == 31) {
+        // a short chunk: the streamed kernel as well, its pair rows and status word those of the chunk owner
+        return experts_run_fused(m->chunk, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows,
+                                 glmflash_fast_experts_output(m->fast), fast_experts_status_word(m->fast));
     } else {
         if ((m->phases & 1) && glmflash_grouping_run(m->grouping, stream, picks, rows)) return -1;
         const int32_t *ids = glmflash_grouping_ids(m->grouping), *count = glmflash_grouping_count(m->grouping),
@@ -249,7 +283,7 @@ extern "C" int glmflash_moe_run_host(glmflash_moe *m, void *stream, const glmfla
         if (launch_k(stage_in_kernel, dim3((unsigned)((nx + 2 * np + 255) / 256)), dim3(256), 0, s, m->cfg.pdl != 0, (const uint4 *)input_host,
                      (uint4 *)m->in_dev, nx, (const int *)picks_host, m->picks_dev, route_w_host, m->w_dev, np))
             return -1;
-        if (experts_run_fused(m->experts, s, w, m->in_dev, x_stride, m->picks_dev, m->w_dev, m->out, out_host, rows)) return -1;
+        if (experts_run_fused(m->experts, s, w, m->in_dev, x_stride, m->picks_dev, m->w_dev, m->out, out_host, rows, nullptr, nullptr)) return -1;
         GF_CUDA(cudaStreamSynchronize(s));
         return 0;
     }

@@ -23,6 +23,7 @@ struct glmflash_experts {
 namespace gf {
 // GLMFLASH_LAYER_KERNELS=1 (read when an owner is created) selects the alternative layer kernel (window.cu).
 bool one_launch_selected();
+int experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit, glmflash_experts **out);
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 
 // Peer-mapped receive areas of the expert-parallel exchange fused into the layer kernel's last step.

@@ -1,6 +1,6 @@
-// The MoE layer for windows of 1..16 rows (decode and speculative verify) as ONE launch: a persistent, warp-specialised
-// kernel that streams the packed words of the chosen experts through shared memory and never lets the decode warps wait
-// for a phase of the layer.
+// The MoE layer for windows of 1..16 rows (decode and speculative verify) and for chunks of up to 128 as ONE launch: a
+// persistent, warp-specialised kernel that streams the packed words of the chosen experts through shared memory and never
+// lets the decode warps wait for a phase of the layer.
 //
 // Replaces upstream's rot_in / exl3_grouped_8_4 / gateup_epilogue / down_epilogue / combine sequence (native/exl3.cu:59-321,
 // native/expert_loads.cu:130-285, src/moe.rs:101-181).  Same operands, member and pair conventions and rounding points.
@@ -16,9 +16,10 @@
 //               inputs (gate / up) or the finished rows of the gate / up phase (down).
 //   warp 11     feeds a four-stage ring, ONE tensor copy per unit (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
 //               bulk copies of the 1-KB rows held the issuing warp for 2,900 clocks per unit, longer than its decode takes.
-//   warps 12-15 finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of an output block in a fixed order and run the epilogue (Hadamard, scales, limited
-//               SwiGLU, down-input rotation; for the down phase Hadamard, output scale and the weighted sum over the row's
-//               slots, ascending, shared expert last).
+//   warps 12-15 finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of
+//               an output block in a fixed order and run the epilogue (Hadamard, scales, limited SwiGLU, down-input
+//               rotation; for the down phase Hadamard, output scale and the weighted sum over the row's slots,
+//               ascending, shared expert last).
 // Partial sums and finished rows travel through L2 as 8-byte words {value, launch epoch}: the reader polls the data itself
 // until it carries the epoch, so a hand-over costs one L2 round trip instead of fence + counter + load, and nothing has
 // to be cleared between launches.
@@ -152,10 +153,15 @@ struct StTables {
     int *e, *mask, *pref;                // [umax] expert id, row mask (bit = row of the window); [umax + 1] finish-job prefix
     uint16_t *pair;                      // [umax][16] pair index of member m
     short *state;                        // [P] expert of a pair computed here, -1 not computed, -2 a repeated pick of its row
+    // more than 16 rows only
+    int *base;                           // [E + 1] number of an expert's first entry above
+    uint32_t *rows_of;                   // [E + 1][words] rows that picked the expert, a bit each
+    int words;
 };
 constexpr int ST_META = 1024;            // barriers and descriptors
-inline size_t st_smem_bytes(int sets, int umax, int P) {
-    const size_t tables = (size_t)(3 * umax + 1) * 4 + (size_t)umax * 32 + (size_t)P * 2 + 64;
+inline size_t st_smem_bytes(int sets, int umax, int rows, int P, int E) {
+    const size_t tables = (size_t)(3 * umax + 1) * 4 + (size_t)umax * 32 + (size_t)P * 2 + 64 +
+                          (rows > 16 ? (size_t)(E + 1) * 4 * (1 + (rows + 31) / 32) : 0);
     return (size_t)ST_STAGES * ST_WBYTES + (size_t)ST_XSTAGES * sets * 8 * ST_XROW + ST_META + (tables + 127) / 128 * 128 +
            1024 /*align*/;
 }
@@ -285,6 +291,86 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
     return U;
 }
 
+// The same for chunks of more than 16 rows (routing table only): an expert with more than 16 members gets an entry for every 16
+// of them, for which its weights are decoded again.  Every CTA has to come to the same tables.  tb.rows_of is zero on entry.
+__device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const StTables &tb) {
+    __shared__ int total;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, P = a.rows * a.slots, W = tb.words;
+    const float inv_slots = fast_inv(a.slots);
+    auto members = [&](int e) {
+        int n = 0;
+        for (int w = 0; w < W; ++w) n += __popc(tb.rows_of[e * W + w]);
+        return n;
+    };
+    for (int i = tid; i < P; i += ST_THREADS) {
+        const int e = __ldcg(a.picks + i);
+        tb.state[i] = e < 0 || e > a.E ? (short)-1 : (short)e;
+    }
+    __syncthreads();
+    auto first_of_row = [&](int i, int row, int e) {             // a pick that repeats an earlier slot of its row does not count
+        bool dup = false;
+        for (int q = row * a.slots; q < i; ++q) dup |= tb.state[q] == (short)e;
+        return !dup;
+    };
+    auto skipped = [&](int row, int e) {
+        return expert_skipped(e, a.E, a.shared, a.e_lo, a.e_hi) ||
+               (e == a.E && a.srow_hi > a.srow_lo && (row < a.srow_lo || row >= a.srow_hi));     // shared expert: row window
+    };
+    for (int i = tid; i < P; i += ST_THREADS) {
+        const int e = tb.state[i], row = fast_div(i, inv_slots);
+        if (!skipped(row, e) && first_of_row(i, row, e)) atomicOr(&tb.rows_of[e * W + (row >> 5)], 1u << (row & 31));
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int run = 0;
+        for (int e0 = 0; e0 <= a.E; e0 += 32) {
+            const int g = e0 + lane <= a.E ? (members(e0 + lane) + 15) >> 4 : 0;
+            int incl = g;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            if (e0 + lane <= a.E) tb.base[e0 + lane] = run + incl - g;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) total = run;
+    }
+    __syncthreads();
+    for (int i = tid; i < P; i += ST_THREADS) {
+        const int e = tb.state[i], row = fast_div(i, inv_slots);
+        // (marking a pick changes nothing for the row's others: the first one of an expert keeps its id)
+        if (skipped(row, e)) { tb.state[i] = -1; continue; }
+        if (!first_of_row(i, row, e)) { tb.state[i] = -2; continue; }
+        int pos = __popc(tb.rows_of[e * W + (row >> 5)] & ((1u << (row & 31)) - 1u));
+        for (int w = 0; w < (row >> 5); ++w) pos += __popc(tb.rows_of[e * W + w]);
+        const int v = tb.base[e] + (pos >> 4);
+        tb.pair[v * 16 + (pos & 15)] = (uint16_t)i;
+        if ((pos & 15) == 0) {
+            tb.e[v] = e;
+            tb.mask[v] = (1 << min(16, members(e) - pos)) - 1;
+        }
+    }
+    __syncthreads();
+    const int U = total;
+    if (warp == ST_FIN) {
+        int run = 0;
+        for (int u0 = 0; u0 < U; u0 += 32) {
+            const int c = u0 + lane < U ? __popc(tb.mask[u0 + lane]) : 0;
+            int incl = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += up;
+            }
+            if (u0 + lane < U) tb.pref[u0 + lane] = run + incl - c;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) tb.pref[U] = run;
+    }
+    return U;
+}
+
 // Register split over the warpgroups (decode, decode, X + producer, finish): 4 x 128 threads at 64 registers in all.
 template <bool INC, int N>
 __device__ __forceinline__ void st_regs() {
@@ -315,6 +401,10 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     tb.pref = tb.mask + a.umax;
     tb.pair = reinterpret_cast<uint16_t *>(tb.pref + a.umax + 1);
     tb.state = reinterpret_cast<short *>(tb.pair + a.umax * 16);
+    const bool many = a.rows > 16;
+    tb.base = reinterpret_cast<int *>(tb.state + ((a.rows * a.slots + 1) & ~1));
+    tb.rows_of = reinterpret_cast<uint32_t *>(tb.base + a.E + 1);
+    tb.words = (a.rows + 31) >> 5;
     __shared__ int abort_sh, first_sh;
     __shared__ uint32_t used_sh[32];
     __shared__ __align__(16) float fin_sh[8][128];
@@ -338,13 +428,15 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     }
     if (tid < 32) used_sh[tid] = 0u;
     for (int i = tid; i < a.umax; i += ST_THREADS) tb.mask[i] = 0;
+    if (many)
+        for (int i = tid; i < (a.E + 1) * tb.words; i += ST_THREADS) tb.rows_of[i] = 0u;
     __syncthreads();
     // The arguments of a launch and the tables' inputs are cold everywhere: touch the argument lines (constant-cache misses cost a
     // thousand clocks each where they are met one after another) and hint the inputs into L2 while the kernel before drains.
     // (a plain indexed read of the parameter: a volatile one would not be a parameter-space access)
     if (tid < (int)(sizeof(StreamArgs) / 4)) asm volatile("" ::"r"(reinterpret_cast<const int *>(&a)[tid]));
     if (tid >= 256 && tid < 259) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(tid == 256 ? &map_g : tid == 257 ? &map_u : &map_d)) : "memory");
-    if (tid < P && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
+    if (tid < min(P, ST_THREADS) && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
     const int row = tid / a.slots, slot = tid - row * a.slots;        // of routing-table entry number tid
     pdl_launch_dependents();                        // the next kernel waits for all of this one before it touches memory
     pdl_wait();
@@ -353,7 +445,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     if (tid == ST_PROD * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
     if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
     const uint32_t epoch = __ldcg(a.ctrl + CTRL_EPOCH) + 1u;          // words of earlier launches carry smaller ones
-    const int U = st_build_tables(a, tb, used_sh, row, slot);
+    const int U = many ? st_build_tables_many(a, tb) : st_build_tables(a, tb, used_sh, row, slot);
     if (tid == ST_FIN * 32) first_sh = drawn;
     __syncthreads();
     const int units_g = a.do_g ? U * 2 * SK1 * NB1 : 0, units = units_g + (a.do_d ? U * SK2 * NB2 : 0);
@@ -659,7 +751,7 @@ int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
     if (!sms[dev]) GF_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
     const int sets = a.rows > 8 ? 2 : 1;
-    const size_t smem = st_smem_bytes(sets, a.umax, a.rows * a.slots);
+    const size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
     GF_REQUIRE(smem <= 227 * 1024, "routing table too large for the window kernel");
     size_t &have = configured[dev][sets - 1];
     if (have < smem) {

@@ -1,4 +1,4 @@
-// Launch interface of the streamed layer kernel (stream.cu) for windows of <= 16 rows.
+// Launch interface of the streamed layer kernel (stream.cu).
 #pragma once
 #include "common.cuh"
 
@@ -20,7 +20,7 @@ struct StreamArgs {
     float *y, *out, *out2;                                   // pair results [P][H]; combined rows [rows][H] (out2: a second copy) or nullptr
     unsigned *ctrl;                                          // CTRL_WORDS
     int *status;
-    int H, I, rows, x_stride, slots, maxm, E, e_lo, e_hi, shared, umax;
+    int H, I, rows, x_stride, slots, maxm, E, e_lo, e_hi, shared, srow_lo, srow_hi, umax;
     float limit;
     int vec;                                                 // the scale vectors are 8-byte aligned
     int do_g, do_d;                                          // profiling aid: the phases to run
@@ -34,6 +34,8 @@ inline size_t stream_z2_words(const glmflash_config &c) { return (size_t)((c.int
 inline size_t stream_xr_words(const glmflash_config &c) { return (size_t)c.max_rows * c.slots * c.hidden; }
 inline size_t stream_xdl_words(const glmflash_config &c) { return (size_t)c.max_rows * c.slots * c.inter / 2; }
 
+// Most rows of a chunk that the kernel takes (its tables live in shared memory and its exchange areas grow with the rows).
+constexpr int ST_MAX_ROWS = 128;
 int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl);
 
 }  // namespace gf

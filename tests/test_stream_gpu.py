@@ -32,6 +32,25 @@ def test_edges_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows):
     assert np.isfinite(got).all() and emax < TOL and erms < TOL, (emax, erms)
 
 
+@pytest.mark.parametrize("H,I,E,S,rows,kw", [(256, 512, 3, 3, 17, {}), (512, 512, 40, 9, 40, {}), (768, 512, 8, 2, 128, {}),
+                                             (512, 512, 12, 4, 64, dict(expert_lo=1, expert_hi=9, shared_rows=(10, 50)))])
+def test_short_chunks_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows, kw):
+    # more than 16 rows: experts with one member, with a whole number of sixteens and with a remainder; a rank's share
+    bank = synth.expert_bank(51 + H + rows, H, I, E, svh_scale=True)
+    x, (picks, rw) = synth.activations_bf16(52, rows, H), synth.route(53, rows, E, S - 1)
+    if S > 2:
+        picks[3, 1] = picks[3, 0]                        # a repeated pick is not computed again
+        rw[3, 1] = 0
+    got = run(pkg, cuda, synth.to_device(bank, cuda), x, picks, rw, H, I, E, S, rows, synth, **kw)
+    Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1).reshape(rows, S, H)
+    lo, hi = kw.get("expert_lo", 0), kw.get("expert_hi", E)
+    r0, r1 = kw.get("shared_rows", (0, rows))
+    here = (picks >= lo) & (picks < hi) | (picks == E) & (np.arange(rows)[:, None] >= r0) & (np.arange(rows)[:, None] < r1)
+    want = np.where(here[..., None], np.where((np.arange(S) == S - 1)[None, :, None], 1, rw[..., None]) * Y, 0).sum(1)
+    emax, erms = rel_err(got, want)
+    assert emax < TOL and erms < TOL, (emax, erms)
+
+
 @pytest.mark.parametrize("rows", [1, 5])
 def test_window_without_experts_and_repeated_picks(pkg, oracle, synth, cuda, rows):
     H, I, E, S = 512, 256, 8, 4
