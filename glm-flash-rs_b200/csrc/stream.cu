@@ -378,7 +378,7 @@ __device__ __forceinline__ void st_regs() {
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-template <int SETS>
+template <int SETS, bool MANY>
 __global__ void __launch_bounds__(ST_THREADS, 2)
 stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_d,
               const __grid_constant__ StreamArgs a) {
@@ -401,7 +401,6 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     tb.pref = tb.mask + a.umax;
     tb.pair = reinterpret_cast<uint16_t *>(tb.pref + a.umax + 1);
     tb.state = reinterpret_cast<short *>(tb.pair + a.umax * 16);
-    const bool many = a.rows > 16;
     tb.base = reinterpret_cast<int *>(tb.state + ((a.rows * a.slots + 1) & ~1));
     tb.rows_of = reinterpret_cast<uint32_t *>(tb.base + a.E + 1);
     tb.words = (a.rows + 31) >> 5;
@@ -428,7 +427,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     }
     if (tid < 32) used_sh[tid] = 0u;
     for (int i = tid; i < a.umax; i += ST_THREADS) tb.mask[i] = 0;
-    if (many)
+    if (MANY)
         for (int i = tid; i < (a.E + 1) * tb.words; i += ST_THREADS) tb.rows_of[i] = 0u;
     __syncthreads();
     // The arguments of a launch and the tables' inputs are cold everywhere: touch the argument lines (constant-cache misses cost a
@@ -436,7 +435,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     // (a plain indexed read of the parameter: a volatile one would not be a parameter-space access)
     if (tid < (int)(sizeof(StreamArgs) / 4)) asm volatile("" ::"r"(reinterpret_cast<const int *>(&a)[tid]));
     if (tid >= 256 && tid < 259) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(tid == 256 ? &map_g : tid == 257 ? &map_u : &map_d)) : "memory");
-    if (tid < min(P, ST_THREADS) && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
+    if (tid < P && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
     const int row = tid / a.slots, slot = tid - row * a.slots;        // of routing-table entry number tid
     pdl_launch_dependents();                        // the next kernel waits for all of this one before it touches memory
     pdl_wait();
@@ -445,7 +444,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     if (tid == ST_PROD * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
     if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
     const uint32_t epoch = __ldcg(a.ctrl + CTRL_EPOCH) + 1u;          // words of earlier launches carry smaller ones
-    const int U = many ? st_build_tables_many(a, tb) : st_build_tables(a, tb, used_sh, row, slot);
+    const int U = MANY ? st_build_tables_many(a, tb) : st_build_tables(a, tb, used_sh, row, slot);
     if (tid == ST_FIN * 32) first_sh = drawn;
     __syncthreads();
     const int units_g = a.do_g ? U * 2 * SK1 * NB1 : 0, units = units_g + (a.do_d ? U * SK2 * NB2 : 0);
@@ -745,17 +744,19 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
 int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     static int sms[64] = {};
-    static size_t configured[64][2] = {};
+    static size_t configured[64][3] = {};
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
     GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
     if (!sms[dev]) GF_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
-    const int sets = a.rows > 8 ? 2 : 1;
+    const int sets = a.rows > 8 ? 2 : 1, which = a.rows > 16 ? 2 : sets - 1;
+    // (chunks have a kernel of their own: with their tables as a branch, windows of 11 rows were 1 % slower)
+    const auto kernel = which == 2 ? stream_kernel<2, true> : which ? stream_kernel<2, false> : stream_kernel<1, false>;
     const size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
     GF_REQUIRE(smem <= 227 * 1024, "routing table too large for the window kernel");
-    size_t &have = configured[dev][sets - 1];
+    size_t &have = configured[dev][which];
     if (have < smem) {
-        GF_CUDA(cudaFuncSetAttribute(sets == 2 ? stream_kernel<2> : stream_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         have = smem;
     }
     // CTAs per SM.  One leaves room for the next layer's CTAs, which then set up while this layer drains (one token: 24.4 us a
@@ -767,8 +768,7 @@ int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     const dim3 grid((unsigned)(sms[dev] * per_sm)), block(ST_THREADS);
     CUtensorMap mg, mu, md;
     if (bank_map(&mg, a.gt, a.E + 1, a.H, a.I) || bank_map(&mu, a.ut, a.E + 1, a.H, a.I) || bank_map(&md, a.dt, a.E + 1, a.I, a.H)) return -1;
-    return sets == 2 ? launch_k(stream_kernel<2>, grid, block, smem, s, pdl, mg, mu, md, a)
-                     : launch_k(stream_kernel<1>, grid, block, smem, s, pdl, mg, mu, md, a);
+    return launch_k(kernel, grid, block, smem, s, pdl, mg, mu, md, a);
 }
 
 }  // namespace gf
