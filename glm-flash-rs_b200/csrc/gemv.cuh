@@ -73,8 +73,7 @@ inline int bank_map(CUtensorMap *map, const uint32_t *bank, int experts, int K, 
 // ---- decode: one stage (256 k of one matrix and 128 columns) by eight warps ------------------------------------------
 // words: the stage; x: the members' activations of its 256 k; warp = n-tile.  acc[s] += columns G, G + 8 of members 8 s + 2 T, + 1.
 template <int SETS>
-__device__ __forceinline__ void st_decode(const unsigned char *words, const unsigned char *x, int warp, int lane, bool two,
-                                          float (&acc)[SETS][4]) {
+__device__ __forceinline__ void st_decode(const unsigned char *words, const unsigned char *x, int warp, int lane, float (&acc)[SETS][4]) {
     const int G = lane >> 2, T = lane & 3;
     // row (n-tile, k-tile) of 128 bytes; its 16-byte chunk c sits at c ^ (k-tile & 7): k-tiles T and 4 + T of a pair of groups
     const unsigned char *wrow = words + warp * 2048 + T * 128;
@@ -114,7 +113,7 @@ __device__ __forceinline__ void st_decode(const unsigned char *words, const unsi
                 af[2] = __byte_perm(weight_dup(hi[2]), weight_dup(hi[3]), 0x5410);
                 af[3] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
                 mma16816(acc[0], af, b0[0][t], b1[0][t]);
-                if (SETS == 2 && two) mma16816(acc[SETS - 1], af, b0[SETS - 1][t], b1[SETS - 1][t]);
+                if (SETS == 2) mma16816(acc[SETS - 1], af, b0[SETS - 1][t], b1[SETS - 1][t]);
             }
         }
     }

@@ -507,7 +507,11 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                 const int s = it % ST_STAGES;
                 if (half) ok = __all_sync(0xffffffffu, cta.wait(wfull + s, (it / ST_STAGES) & 1));
                 if (!ok) break;
-                st_decode<SETS>(words + s * ST_WBYTES, xbuf + xs * XBYTES + half * 512, warp, lane, SETS == 2 && nmem > 8, acc);
+                const unsigned char *ws = words + s * ST_WBYTES, *xh = xbuf + xs * XBYTES + half * 512;
+                // (few experts of a window or chunk have more than eight members; with the second set's operand loads in every
+                // unit, eleven rows took 459 us over 6 layers instead of 428 and a chunk of 40 192 instead of 180)
+                if (SETS == 1 || nmem <= 8) st_decode<1>(ws, xh, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
+                else st_decode<SETS>(ws, xh, warp, lane, acc);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty + s);
             }
