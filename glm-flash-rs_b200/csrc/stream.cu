@@ -113,7 +113,11 @@ __device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long lon
 }
 
 // Sum of the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the
-// epoch.
+// epoch.  LAST: between the attempts only the last of the four is polled; it is mostly the last to come.  With more than 8 rows up to
+// eight finish warps an SM are always waiting, and their polls of all four cost the decode warps issue slots and L2 a tenth of its
+// rate (11 rows, 6 layers 428 -> 414 us, 16 rows 8 layers 672 -> 640); for fewer rows the extra round trip costs more (1137 ->
+// 1152 us for 47 layers of one token).
+template <bool LAST>
 __device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
                                            float (&v)[4]) {
     z += (size_t)lo * split_stride;
@@ -136,6 +140,8 @@ __device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long l
             if (__all_sync(0xffffffffu, ok)) break;
             if (!__all_sync(0xffffffffu, c.again(n))) return false;
             __nanosleep(20);
+            unsigned long long last[4];
+            if (LAST && !ll_wait4(c, z + (size_t)(min(hi - lo, 4) - 1) * split_stride, epoch, last)) return false;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -600,7 +606,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                 const uint2 sv = ldg_half4((role ? a.svh_u : a.svh_g) + so, a.vec);
                 const uint2 sd = ldg_half4(a.suh_d + so, a.vec);
                 float v[4] = {0.f, 0.f, 0.f, 0.f};
-                sum_splits(cta, a.z1 + ((size_t)role * SK1 * P + p) * I + col, (size_t)P * I, half ? mid : 0, half ? SK1 : mid, epoch, v);
+                sum_splits<SETS == 2>(cta, a.z1 + ((size_t)role * SK1 * P + p) * I + col, (size_t)P * I, half ? mid : 0, half ? SK1 : mid, epoch, v);
                 if (half) *reinterpret_cast<float4 *>(&fin_sh[fw][4 * lane]) = make_float4(v[0], v[1], v[2], v[3]);
                 pair_barrier(role);
                 if (!half) {
@@ -653,7 +659,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0)
-                            sum_splits(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col, (size_t)P * H, 0, SK2, epoch, v[i]);
+                            sum_splits<SETS == 2>(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col, (size_t)P * H, 0, SK2, epoch, v[i]);
                     if (e[0] >= 0) fwht128(v[0], lane);
                     if (e[1] >= 0) fwht128(v[1], lane);
 #pragma unroll
