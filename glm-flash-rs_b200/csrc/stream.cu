@@ -44,6 +44,8 @@ namespace gf {
 constexpr int ST_THREADS = 512, ST_STAGES = 4, ST_XSTAGES = 2;
 constexpr int ST_DEC = 8, ST_XW = 3;                         // decode and X warps, then the producer, then four finish warps
 constexpr int ST_PROD = ST_DEC + ST_XW, ST_FIN = ST_PROD + 1;
+constexpr size_t ST_MAX_SMEM = 227 * 1024 - 4352;            // dynamic part (4,240 bytes are static)
+constexpr size_t ST_HALF_SM = 116 * 1024;                    // two such CTAs do not fit an SM
 constexpr uint32_t ST_POLLS = 1u << 21;                      // polls of a global word before a wait gives up (about a second)
 
 enum : int { UNIT_G = 0, UNIT_D = 1, UNIT_END = 2 };       // low byte of a descriptor, matrix in bit 8
@@ -754,7 +756,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
 int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     static int sms[64] = {};
-    static size_t configured[64][3] = {};
+    static bool configured[64][3] = {};
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
     GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
@@ -762,20 +764,23 @@ int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     const int sets = a.rows > 8 ? 2 : 1, which = a.rows > 16 ? 2 : sets - 1;
     // (chunks have a kernel of their own: with their tables as a branch, windows of 11 rows were 1 % slower)
     const auto kernel = which == 2 ? stream_kernel<2, true> : which ? stream_kernel<2, false> : stream_kernel<1, false>;
-    const size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
-    GF_REQUIRE(smem <= 227 * 1024, "routing table too large for the window kernel");
-    size_t &have = configured[dev][which];
-    if (have < smem) {
-        GF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        have = smem;
-    }
-    // CTAs per SM.  One leaves room for the next layer's CTAs, which then set up while this layer drains (one token: 24.4 us a
-    // layer against 28.6 with two); two fill the decode pipes (16 rows: 85 against 95 us).  The lines cross at about 16 units per
-    // SM, counted with one expert per pick of this GPU's window (2,160 units: 37.8 | 38.7 us, 2,880: 44.5 | 43.6).
+    size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
+    GF_REQUIRE(smem <= ST_MAX_SMEM, "routing table too large for the window kernel");
+    // CTAs per SM.  One has shorter chains for few units (one token: 24.4 us a layer against 28.6 with two); two fill the decode
+    // pipes (16 rows: 85 against 95 us).  The lines cross at about 16 units per SM, counted with one expert per pick of this GPU's
+    // window (2,160 units: 37.8 | 38.7 us, 2,880: 44.5 | 43.6).
     const long pairs = (long)a.rows * (((long)(a.slots - 1) * (a.e_hi - a.e_lo) + a.E - 1) / a.E + (a.shared ? 1 : 0));
     const long units = std::min<long>(pairs, a.umax) * (2L * ((a.H + 511) / 512) * (a.I / 128) + (long)((a.I + 511) / 512) * (a.H / 128));
     const int per_sm = units >= 16L * sms[dev] ? 2 : 1;
     const dim3 grid((unsigned)(sms[dev] * per_sm)), block(ST_THREADS);
+    // One CTA per SM asks for more than half of the shared memory: next to a few CTAs of another kernel (the router of the next
+    // layer) the second CTA of an emptier SM was placed before the first of a busier one (8 layers of one token with their
+    // router 293 -> 266 us; 47 without 1140 -> 1144, whose next layer now sets up after this one).
+    if (per_sm == 1) smem = std::max<size_t>(smem, ST_HALF_SM);
+    if (!configured[dev][which]) {                 // (a bound, not a request; threads that come here together set the same)
+        GF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST_MAX_SMEM));
+        configured[dev][which] = true;
+    }
     CUtensorMap mg, mu, md;
     if (bank_map(&mg, a.gt, a.E + 1, a.H, a.I) || bank_map(&mu, a.ut, a.E + 1, a.H, a.I) || bank_map(&md, a.dt, a.E + 1, a.I, a.H)) return -1;
     return launch_k(kernel, grid, block, smem, s, pdl, mg, mu, md, a);
