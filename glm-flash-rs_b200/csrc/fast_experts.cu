@@ -69,6 +69,8 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
     __shared__ int cnt_sh[FG_MAXU], row_sh[FG_MAXU], e_sh[FG_MAXU], first_sh[FG_MAXU];
     __shared__ int wsum[4][32];
     const int u = threadIdx.x, lane = u & 31, warp = u >> 5;
+    pdl_wait();                                             // (every kernel of the chain: nothing is read or written before)
+    pdl_launch_dependents();
     const int n = min(count[0], FG_MAXU);
     int cnt = 0, e = -1, first = 0;
     if (u < n) {
@@ -145,6 +147,8 @@ __global__ void __launch_bounds__(256) fast_rot_kernel(const __nv_bfloat16 *__re
                                                        __half *__restrict__ out1, int K, int slots, int mats, bool vec) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KB = K >> 7, parts = (KB + 3) >> 2;
+    pdl_wait();
+    pdl_launch_dependents();
     const long items = (long)plan[1] * parts;
     const float2 neg1 = make_float2(-1.f, -1.f);
     for (long it = (long)blockIdx.x * 8 + warp; it < items; it += (long)gridDim.x * 8) {
@@ -414,7 +418,6 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int KT = a.K >> 4, NBP = a.N >> 8, KS = a.K / FG_BK;
-    const int total = a.plan[2] * NBP, items = total > pair ? (total - pair + pairs - 1) / pairs : 0;
 
     if (tid == 0) {
         for (int s = 0; s < C::ASTAGES; ++s) mbar_init(afull + s, 1);
@@ -430,6 +433,9 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
     cluster_sync();                                                        // the peer's barriers are initialised as well
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
+    const int total = a.plan[2] * NBP, items = total > pair ? (total - pair + pairs - 1) / pairs : 0;
     // the slot that stage `it` of a ring of `depth` stages takes is free: stage it - depth has been consumed
     auto slot_free = [&](uint32_t it, uint32_t depth) {
         if (it < depth) return true;
@@ -780,16 +786,17 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
     cudaStream_t s = (cudaStream_t)stream;
     const int H = c.hidden, I = c.inter;
     const long P = (long)rows * c.slots;
+    const bool pdl = c.pdl != 0;                            // a kernel's launch and set-up overlap the tail of the one in front
     if (f->phases & 1)
-        fast_plan_kernel<<<c.experts + 1, FG_MAXU, 0, s>>>(ids, count, members, maxm, c.slots, c.experts, c.shared_exl3, c.expert_lo,
-                                              c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->chunks, f->src_pair, f->row_expert);
-    GF_CUDA(cudaGetLastError());
+        if (launch_k(fast_plan_kernel, dim3((unsigned)c.experts + 1), dim3(FG_MAXU), 0, s, pdl, ids, count, members, maxm, c.slots, c.experts,
+                     c.shared_exl3, c.expert_lo, c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->chunks, f->src_pair, f->row_expert))
+            return -1;
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)
-        fast_rot_kernel<<<(unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 148L * 32), 256, 0, s>>>(
+        if (launch_k(fast_rot_kernel, dim3((unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 148L * 32)), dim3(256), 0, s, pdl,
             (const __nv_bfloat16 *)input, x_stride, f->plan, f->src_pair, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg,
-            f->xu, H, c.slots, mats, (((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 16 == 0 && x_stride % 8 == 0));
-    GF_CUDA(cudaGetLastError());
+            f->xu, H, c.slots, mats, (((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 16 == 0 && x_stride % 8 == 0)))
+            return -1;
     FastGemmArgs a{};
     a.plan = f->plan; a.chunks = f->chunks; a.src_pair = f->src_pair; a.status = f->status; a.limit = c.limit;
     CUtensorMap mg, mu, md;
@@ -797,12 +804,12 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
         return -1;
     a.sv0 = (const __half *)w->svh_g; a.sv1 = (const __half *)w->svh_u; a.sd = (const __half *)w->suh_d;
     a.xd = f->xd; a.y = nullptr; a.K = H; a.N = I; a.shared_x = shared_x ? 1 : 0;
-    if (f->phases & 4) fast_gemm_kernel<2><<<f->sms & ~1, FG_THREADS, FgCfg<2>::SMEM, s>>>(f->map_xg, f->map_xu, mg, mu, a);
-    GF_CUDA(cudaGetLastError());
+    if ((f->phases & 4) && launch_k(fast_gemm_kernel<2>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<2>::SMEM, s, pdl, f->map_xg, f->map_xu, mg, mu, a))
+        return -1;
     a.sv0 = (const __half *)w->svh_d; a.sv1 = nullptr; a.sd = nullptr;
     a.xd = nullptr; a.y = f->out; a.K = I; a.N = H; a.shared_x = 1;
-    if (f->phases & 8) fast_gemm_kernel<1><<<f->sms & ~1, FG_THREADS, FgCfg<1>::SMEM, s>>>(f->map_xd, f->map_xd, md, md, a);
-    GF_CUDA(cudaGetLastError());
+    if ((f->phases & 8) && launch_k(fast_gemm_kernel<1>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<1>::SMEM, s, pdl, f->map_xd, f->map_xd, md, md, a))
+        return -1;
     return 0;
 }
 
