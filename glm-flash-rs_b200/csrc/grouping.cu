@@ -5,11 +5,13 @@
 //   members[u]  row * 32 + slot of every row that picked ids[u], ascending rows, then -1 up to maxm;
 //               rows u >= count are all -1
 // One launch for any window size (upstream: one block for <= 32 rows, five launches up to 8192 rows): CTA e
-// owns expert e.  It first builds the bitmap of used experts from the picks itself (so it knows its place
-// among the used experts without a second kernel or a global scan), then walks the rows in order, 1024 at a
-// time, and compacts the rows that picked e with a block scan.  Nothing is ordered by atomics: the shared-
-// memory atomicOr only sets bits.  A row that names an expert twice counts once, with its first slot, as in
+// owns expert e.  It first marks the used experts from the picks itself (so it knows its place among them without
+// a second kernel or a global scan), then compacts the rows that picked e in row order with one block scan per 8192
+// rows.  Nothing is ordered by atomics.  A row that names an expert twice counts once, with its first slot, as in
 // upstream's row-bitmap.
+// A launch is bound by the latency of its steps.  Marking by atomicOr on a bitmap queued a whole window on a few words of
+// shared memory, and a scan per 1024 rows was a chain of barriers: 4096 rows x 5 of 65 experts 14.1 -> 6.4 us, 8192 rows 25.0 ->
+// 9.0, 17 rows 4.5 -> 4.1, 8192 x 9 of 289 45.8 -> 26.5 (launches back to back).
 #include <algorithm>
 #include <new>
 
@@ -18,68 +20,69 @@
 namespace gf {
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 
-constexpr int GROUP_THREADS = 1024;
+constexpr int GROUP_THREADS = 1024, GROUP_STEPS = 8;
 
 __global__ void __launch_bounds__(GROUP_THREADS) grouping_kernel(const int *__restrict__ picks, int rows, int slots, int E1,
                                                                 int maxm, int *__restrict__ ids, int *__restrict__ count,
                                                                 int *__restrict__ members) {
-    __shared__ uint32_t used[32];                 // E1 <= 1024
-    __shared__ int warp_sums[32];
-    __shared__ int base_sh;
+    __shared__ int used[GROUP_THREADS];           // E1 <= 1024
+    __shared__ int sums[GROUP_STEPS * 32], totals[GROUP_STEPS];
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    used[tid] = 0;
     pdl_wait();                                   // picks may be the previous kernel's output; ids / members its input
     pdl_launch_dependents();
-    if (tid < 32) used[tid] = 0u;
-    if (tid == 0) base_sh = 0;
     __syncthreads();
     const int total = rows * slots;
+#pragma unroll 4
     for (int i = tid; i < total; i += GROUP_THREADS) {
         const int p = picks[i];
-        if (p >= 0 && p < E1) atomicOr(&used[p >> 5], 1u << (p & 31));
+        if (p >= 0 && p < E1) used[p] = 1;        // (every writer stores the same)
     }
     __syncthreads();
-    int place = 0, n_used = 0;
-    for (int wd = 0; wd < 32; ++wd) {
-        const uint32_t b = used[wd];
-        n_used += __popc(b);
-        if (wd < (e >> 5)) place += __popc(b);
-        else if (wd == (e >> 5)) place += __popc(b & ((1u << (e & 31)) - 1u));
-    }
-    const bool mine = (used[e >> 5] >> (e & 31)) & 1u;
+    const bool mine = used[e] != 0;
+    const int place = __syncthreads_count(used[tid] && tid < e), n_used = __syncthreads_count(used[tid]);
     if (e == 0 && tid == 0) *count = n_used;
     if (mine && tid == 0) ids[place] = e;
     if (!mine && e >= n_used && tid == 0) ids[e] = -1;       // tail of ids: not read by consumers, kept tidy
 
     if (mine) {
         int *out = members + (size_t)place * maxm;
-        for (int r0 = 0; r0 < rows; r0 += GROUP_THREADS) {
-            const int r = r0 + tid;
-            int slot = -1;
-            if (r < rows)
-                for (int s = slots - 1; s >= 0; --s)
-                    if (picks[r * slots + s] == e) slot = s;     // first matching slot wins
-            const int flag = slot >= 0;
-            // block exclusive scan of flag
-            const uint32_t ball = __ballot_sync(0xffffffffu, flag);
-            const int in_warp = __popc(ball & ((1u << lane) - 1u));
-            if (lane == 0) warp_sums[warp] = __popc(ball);
-            __syncthreads();
-            int before = 0, chunk = 0;
-            for (int w2 = 0; w2 < GROUP_THREADS / 32; ++w2) {
-                const int v = warp_sums[w2];
-                if (w2 < warp) before += v;
-                chunk += v;
-            }
-            const int base = base_sh;
-            if (flag) {
-                const int off = base + before + in_warp;
-                if (off < maxm) out[off] = r * 32 + slot;
+        int base = 0;
+        for (int r0 = 0; r0 < rows; r0 += GROUP_STEPS * GROUP_THREADS) {
+            int slot[GROUP_STEPS], before[GROUP_STEPS];
+#pragma unroll
+            for (int i = 0; i < GROUP_STEPS; ++i) {
+                const int r = r0 + i * GROUP_THREADS + tid;
+                slot[i] = -1;
+                if (r < rows)
+                    for (int s = slots - 1; s >= 0; --s)
+                        if (picks[r * slots + s] == e) slot[i] = s;     // first matching slot wins
+                const uint32_t ball = __ballot_sync(0xffffffffu, slot[i] >= 0);
+                before[i] = __popc(ball & ((1u << lane) - 1u));
+                if (lane == 0) sums[i * 32 + warp] = __popc(ball);
             }
             __syncthreads();
-            if (tid == 0) base_sh = base + chunk;
+            if (warp < GROUP_STEPS) {             // a warp scans the 32 sums of one step
+                const int v = sums[tid];
+                int incl = v;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+                    if (lane >= d) incl += up;
+                }
+                sums[tid] = incl - v;
+                if (lane == 31) totals[warp] = incl;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < GROUP_STEPS; ++i) {
+                const int off = base + sums[i * 32 + warp] + before[i];
+                if (slot[i] >= 0 && off < maxm) out[off] = (r0 + i * GROUP_THREADS + tid) * 32 + slot[i];
+                base += totals[i];
+            }
             __syncthreads();
         }
-        for (int j = min(base_sh, maxm) + tid; j < maxm; j += GROUP_THREADS) out[j] = -1;
+        for (int j = min(base, maxm) + tid; j < maxm; j += GROUP_THREADS) out[j] = -1;
     }
     // rows of `members` beyond the used ones: row e is unused exactly when e >= n_used
     if (e >= n_used)
