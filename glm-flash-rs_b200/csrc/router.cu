@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(256) route_kernel(const __nv_bfloat16 *__restr
             float v = 0.f;
 #pragma unroll
             for (int w = 0; w < 8; ++w) v += part[(size_t)(w * 16 * MT + r) * RT_ST + c];
-            if (cn > 1) red[r * RT_ST + c] = v;
-            else if (r0 + r < rows && e0 + c < E) logits[(size_t)(r0 + r) * E + e0 + c] = v;
+            red[r * RT_ST + c] = v;
+            if (cn == 1 && r0 + r < rows && e0 + c < E) logits[(size_t)(r0 + r) * E + e0 + c] = v;
         }
         if (cn > 1) {                                                      // row r of the tile is finished by CTA r % cn
             cluster_sync();
@@ -147,17 +147,25 @@ __global__ void __launch_bounds__(256) route_kernel(const __nv_bfloat16 *__restr
                 float v = 0.f;
                 for (uint32_t q = 0; q < cn; ++q) v += cluster_map(red, q)[r * RT_ST + c];
                 logits[(size_t)(r0 + r) * E + e0 + c] = v;
+                part[r * RT_ST + c] = v;                                   // (this CTA has read its warps' sums)
             }
-            cluster_sync();                                                // peers may still be reading this CTA's sums
+            // peers may still be reading this CTA's sums
+            if (e0 + RT_NE < E) cluster_sync();
+            else asm volatile("barrier.cluster.arrive.release;" ::: "memory");
         } else {
             __syncthreads();
         }
     }
-    if (!picks) return;
-    __syncthreads();
-    for (int r = (int)cr + (int)cn * warp; r < 16 * MT; r += (int)cn * 8)
-        if (r0 + r < rows)
-            topk_row(logits + (size_t)(r0 + r) * E, E, topk, picks + (size_t)(r0 + r) * (topk + 1), weights + (size_t)(r0 + r) * (topk + 1), lane);
+    if (picks) {
+        __syncthreads();
+        // the logits of up to 64 experts are still in shared memory: one trip to L2 less in front of the selection
+        const float *row = E > RT_NE ? logits + (size_t)r0 * E : cn > 1 ? part : red;
+        const int row_stride = E > RT_NE ? E : RT_ST;
+        for (int r = (int)cr + (int)cn * warp; r < 16 * MT; r += (int)cn * 8)
+            if (r0 + r < rows)
+                topk_row(row + (size_t)r * row_stride, E, topk, picks + (size_t)(r0 + r) * (topk + 1), weights + (size_t)(r0 + r) * (topk + 1), lane);
+    }
+    if (cn > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 static int launch_route(cudaStream_t s, const uint16_t *x, int x_stride, const uint16_t *wr, int rows, int H, int E, int topk, float *logits,
