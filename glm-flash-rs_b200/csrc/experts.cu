@@ -98,6 +98,8 @@ static int run_stream(const glmflash_experts *e, cudaStream_t s, StreamArgs a, c
     a.e_lo = c.expert_lo; a.e_hi = c.expert_hi; a.shared = c.shared_exl3; a.limit = c.limit;
     // distinct experts that THIS GPU computes: at most one per pick, and at most its expert window (+ the shared expert)
     a.srow_lo = c.shared_row_lo; a.srow_hi = c.shared_row_hi;
+    a.cut1 = stream_cut(c.hidden, rows > 16);
+    a.cut2 = stream_cut(c.inter, rows > 16);
     a.umax = std::max(1, std::min(rows * c.slots, (c.expert_hi - c.expert_lo) + (c.shared_exl3 ? 1 : 0)));
     if (!a.picks) a.umax = std::max(1, std::min(rows * c.slots, c.experts + 1));   // (places in ids, skipped experts included)
     if (rows > 16) a.umax += rows * c.slots / 16;                  // (an entry for every 16 members)

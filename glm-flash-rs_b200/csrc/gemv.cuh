@@ -8,11 +8,13 @@
 //     16-byte slot of four consecutive k-tiles.
 //   * states are cut with funnel shifts in pairs (state_j << 16 | state_{j+4}), multiplied by the codebook constant, masked, and the
 //     two fp16 halves of a codeword are added by one HADD2: exactly upstream's fp16 weight (bit-exact decode).
-//   * pairs of weights are packed into the A operand of mma.m16n8k16 (rows = 16 output columns); the k slots of the instruction
+//   * pairs of weights are packed into the A operand of mma.m16n8k8 (rows = 16 output columns); the k slots of the instruction
 //     are whatever k the lane holds, and the B operand (members, eight per set) is read to match.  fp32 accumulation; a member's
-//     column depends on its own activations only.
-// A loop of nothing else runs 19.1 weights per clock and SM with packed operands against 17.4 with every weight duplicated over a
-// doubled K (which also costs twice the tensor instructions: with two member sets 17.1 against 14.4).
+//     column depends on its own activations only.  An instruction adds eight products to the accumulator and rounds, which fixes the
+//     bits of a sum: m16n8k16 over every weight duplicated (a doubled K whose other half is zero) has the same ones, m16n8k16 over
+//     sixteen packed weights has not.
+// A loop of nothing else runs 19.1 weights per clock and SM with sixteen packed products an instruction, against 17.4 with every
+// weight duplicated over a doubled K; eight packed products cost the layer kernels up to 2 % of the former.
 #pragma once
 #include "common.cuh"
 #include "tensor_map.cuh"
@@ -42,7 +44,7 @@ __device__ __forceinline__ uint32_t weight_dup(uint32_t x) {
 }
 
 constexpr int ST_WBYTES = 16 * 1024;                         // [8 n-tiles][16 k-tiles][128 bytes], 128-byte swizzle
-constexpr int ST_XROW = 1024 + 16;                           // bytes per staged activation row (512 fp16): conflict-free LDS.128
+constexpr int ST_XROW = 512 + 16;                            // bytes per staged activation row (256 fp16): conflict-free LDS.128
 
 // Four fp16 constants; vec: the vector is 8-byte aligned (uniform over a launch; views of larger tensors may not be).
 __device__ __forceinline__ uint2 ldg_half4(const __half *p, bool vec) {
@@ -72,16 +74,17 @@ inline int bank_map(CUtensorMap *map, const uint32_t *bank, int experts, int K, 
 
 // ---- decode: one stage (256 k of one matrix and 128 columns) by eight warps ------------------------------------------
 // words: the stage; x: the members' activations of its 256 k; warp = n-tile.  acc[s] += columns G, G + 8 of members 8 s + 2 T, + 1.
-template <int SETS>
+// ROUNDS: 2, or 1 for a stage of 128 k.
+template <int SETS, int ROUNDS = 2>
 __device__ __forceinline__ void st_decode(const unsigned char *words, const unsigned char *x, int warp, int lane, float (&acc)[SETS][4]) {
     const int G = lane >> 2, T = lane & 3;
     // row (n-tile, k-tile) of 128 bytes; its 16-byte chunk c sits at c ^ (k-tile & 7): k-tiles T and 4 + T of a pair of groups
-    const unsigned char *wrow = words + warp * 2048 + T * 128;
+    const unsigned char *wrow = words + warp * (ROUNDS * 1024) + T * 128;
     const int sw[2] = {(G ^ T) * 16, (4 * 128) + (G ^ (4 + T)) * 16};
     const unsigned char *xrow = x + G * ST_XROW + T * 32;
     // two groups of four k-tiles per round: the decode chains of two words are in flight side by side
 #pragma unroll 1
-    for (int r = 0; r < 2; ++r, wrow += 8 * 128, xrow += 256) {
+    for (int r = 0; r < ROUNDS; ++r, wrow += 8 * 128, xrow += 256) {
         uint4 wv[2];
         uint32_t before[2];
 #pragma unroll
@@ -103,17 +106,16 @@ __device__ __forceinline__ void st_decode(const unsigned char *words, const unsi
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const uint32_t pw = t == 0 ? before[q] : w[t - 1];
-                uint32_t hi[4], lo[4], af[4];
-                codeword_pair(__funnelshift_r(w[t], pw, 12), hi[0], lo[0]);       // k = 2t:     columns G, G + 8
-                codeword_pair(__funnelshift_r(w[t], pw, 8), hi[1], lo[1]);        // k = 2t + 1
-                codeword_pair(__funnelshift_r(w[t], pw, 4), hi[2], lo[2]);        // k = 2t + 8
-                codeword_pair(w[t], hi[3], lo[3]);                                // k = 2t + 9
-                af[0] = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410);
-                af[1] = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
-                af[2] = __byte_perm(weight_dup(hi[2]), weight_dup(hi[3]), 0x5410);
-                af[3] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
-                mma16816(acc[0], af, b0[0][t], b1[0][t]);
-                if (SETS == 2) mma16816(acc[SETS - 1], af, b0[SETS - 1][t], b1[SETS - 1][t]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t hi[2], lo[2];
+                    codeword_pair(__funnelshift_r(w[t], pw, h ? 4 : 12), hi[0], lo[0]);         // k = 2t + 8h:     columns G, G + 8
+                    codeword_pair(h ? w[t] : __funnelshift_r(w[t], pw, 8), hi[1], lo[1]);       // k = 2t + 8h + 1
+                    const uint32_t a0 = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410),
+                                   a1 = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
+#pragma unroll
+                    for (int s = 0; s < SETS; ++s) mma1688(acc[s], a0, a1, h ? b1[s][t] : b0[s][t]);
+                }
             }
         }
     }

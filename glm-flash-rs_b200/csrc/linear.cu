@@ -14,7 +14,7 @@ namespace gf {
 
 constexpr int LIN_THREADS = 256, LIN_PST = 132;
 inline size_t lin_smem_bytes(int sets, int stages) {
-    return 1024 + (size_t)stages * ST_WBYTES + (size_t)((stages + 1) / 2) * sets * 8 * ST_XROW + (size_t)sets * 8 * LIN_PST * 4 + 256;
+    return 1024 + (size_t)stages * ST_WBYTES + (size_t)stages * sets * 8 * ST_XROW + (size_t)sets * 8 * LIN_PST * 4 + 256;
 }
 
 template <int SETS>
@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_kernel(const __grid_consta
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     constexpr int XBYTES = SETS * 8 * ST_XROW;
     unsigned char *words = smem, *xbuf = words + (size_t)max_stages * ST_WBYTES;
-    float *part = reinterpret_cast<float *>(xbuf + (size_t)((max_stages + 1) / 2) * XBYTES);       // [SETS * 8][LIN_PST]
+    float *part = reinterpret_cast<float *>(xbuf + (size_t)max_stages * XBYTES);       // [SETS * 8][LIN_PST]
     uint64_t *bars = reinterpret_cast<uint64_t *>(part + SETS * 8 * LIN_PST);                      // one per stage
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nb = blockIdx.x, cn = gridDim.y, cr = blockIdx.y;
     const int all = K >> 8, stages = (all - cr + cn - 1) / cn;                                     // stage i of this CTA: cr + i * cn
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_kernel(const __grid_consta
         const float2 s01 = __half22float2(*reinterpret_cast<const __half2 *>(&hv.x)), s23 = __half22float2(*reinterpret_cast<const __half2 *>(&hv.y));
         float v[4] = {x01.x * s01.x, x01.y * s01.y, x23.x * s23.x, x23.y * s23.y};
         fwht128(v, lane);
-        *reinterpret_cast<uint2 *>(xbuf + (size_t)(i >> 1) * XBYTES + r * ST_XROW + (i & 1) * 512 + blk * 256 + 8 * lane) =
+        *reinterpret_cast<uint2 *>(xbuf + (size_t)i * XBYTES + r * ST_XROW + blk * 256 + 8 * lane) =
             make_uint2(pack_half2(v[0] * HAD_SCALE, v[1] * HAD_SCALE), pack_half2(v[2] * HAD_SCALE, v[3] * HAD_SCALE));
     }
     __syncthreads();
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_kernel(const __grid_consta
         for (int c = 0; c < 4; ++c) acc[s][c] = 0.f;
     for (int i = 0; i < stages; ++i)
         if (__all_sync(0xffffffffu, mbar_wait(bars + i, 0)))                                 // (bounded; a copy that never lands leaves the sum short)
-            st_decode<SETS>(words + (size_t)i * ST_WBYTES, xbuf + (size_t)(i >> 1) * XBYTES + (i & 1) * 512, warp, lane, acc);
+            st_decode<SETS>(words + (size_t)i * ST_WBYTES, xbuf + (size_t)i * XBYTES, warp, lane, acc);
     const int G = lane >> 2, T = lane & 3;
 #pragma unroll
     for (int s = 0; s < SETS; ++s) {

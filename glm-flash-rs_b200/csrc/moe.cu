@@ -108,10 +108,7 @@ bool gf::one_launch_selected() {
 // routed experts have more than 16 rows on average (1024 x 2048, 24 experts, top-3, 128 rows: 141 | 145), and none where the
 // exchange areas, which grow with the rows, would pass 256 MB.
 static int short_chunk_rows(const glmflash_config &c) {
-    glmflash_config one = c;
-    one.max_rows = 1;
-    const size_t row = 8 * (stream_z1_words(one) + stream_z2_words(one) + stream_xr_words(one) + stream_xdl_words(one));
-    const size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)16 * c.experts / (c.slots - 1), ((size_t)256 << 20) / row});
+    const size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)16 * c.experts / (c.slots - 1), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
     return rows > 16 ? (int)rows : 0;
 }
 

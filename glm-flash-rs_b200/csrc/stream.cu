@@ -5,19 +5,19 @@
 // Replaces upstream's rot_in / exl3_grouped_8_4 / gateup_epilogue / down_epilogue / combine sequence (native/exl3.cu:59-321,
 // native/expert_loads.cu:130-285, src/moe.rs:101-181).  Same operands, member and pair conventions and rounding points.
 //
-// Work is cut into units of up to 32 KB of packed words: (distinct expert, matrix, 512-k split, 128-column block), one or two
-// stages of 16 k-tiles x 8 n-tiles, the gate / up units of all experts first, the down units after them.  A CTA (512 threads)
-// has four roles:
+// Work is cut into units of one partial sum: (distinct expert, matrix, split of k, 128-column block), the gate / up units of all experts
+// first, the down units after them.  A split is 256 k at K <= 2048 (stream_cut), one or more stages of 16 k-tiles x 8 n-tiles
+// (16 KB, 32,768 weights).  A CTA (512 threads) has four roles:
 //   warps 0-7   decode: warp = n-tile.  A lane reads 16 bytes (4 words of one tile: all 16 k of columns G and G + 8) with
 //               one LDS.128, cuts the states in pairs with funnel shifts, forms the weights exactly as upstream does (fp16
-//               sum of the codeword halves) and packs them into A operands of mma.m16n8k16; members are the N dimension
-//               (8 per set, two sets for 9..16 rows), fp32 accumulation over the unit.
-//   warps 8-10  X: put the members' activations of a unit's k range into shared memory as soon as they are there: rotated layer
+//               sum of the codeword halves) and packs them into A operands of mma.m16n8k8; members are the N dimension
+//               (8 per set, two sets for 9..16 rows), fp32 accumulation over the split.
+//   warps 8-10  X: put the members' activations of a stage's k range into shared memory as soon as they are there: rotated layer
 //               inputs (gate / up) or the finished rows of the gate / up phase (down).
-//   warp 11     feeds a four-stage ring, ONE tensor copy per unit (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
-//               bulk copies of the 1-KB rows held the issuing warp for 2,900 clocks per unit, longer than its decode takes.
+//   warp 11     feeds a four-stage ring, ONE tensor copy per stage (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
+//               bulk copies of the 1-KB rows held the issuing warp for 2,900 clocks a stage, longer than its decode takes.
 //   warps 12-15 finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of
-//               an output block in a fixed order and run the epilogue (Hadamard, scales, limited SwiGLU, down-input
+//               an output block, ascending, and run the epilogue (Hadamard, scales, limited SwiGLU, down-input
 //               rotation; for the down phase Hadamard, output scale and the weighted sum over the row's slots,
 //               ascending, shared expert last).
 // Partial sums and finished rows travel through L2 as 8-byte words {value, launch epoch}: the reader polls the data itself
@@ -26,13 +26,18 @@
 //
 // Units and finish jobs are drawn from two counters, in order, by CTAs that are running.  A gate / up unit waits for nothing,
 // and everything that a later unit or job waits for has been drawn by a CTA that runs: the launch makes progress with any
-// number of resident CTAs, next to any other kernel (no co-residency is assumed).  Sums have a fixed order (k-tiles of a
-// split, then splits ascending) that does not depend on the window: a row has the bits of its 1-row call.
+// number of resident CTAs, next to any other kernel (no co-residency is assumed).
 //
-// What bounds it: the decode instructions.  A unit is 32,768 weights at about 5 instructions; a loop that does nothing else
-// sustains 17.6 weights per clock and SM with 8 warps (two chunks in flight per warp) and 18.7 with 16, so 8 decode warps
-// per CTA and one or two CTAs per SM (launch_stream) are enough.  The earlier form (clusters of short-lived CTAs, three
-// launches per layer) spent half of its time on the phases around the decode.
+// Sums have a fixed order that does not depend on the window: eight products an instruction, the k-tiles of a split in order, the
+// splits ascending.  A row has the bits of its 1-row call, and of the cluster kernels that this one replaced.  With sixteen products
+// an instruction, 512 k a split and half as many partials, the sums were as far from 64-bit ones (6.3e-7 against 6.2e-7 of a down
+// row at K = 1536; 47 layers of one token 1142 us against 1101 now), but other bits: now and then a bf16 rounding behind them fell the
+// other way, and a one-row layer moved by up to 1e-3.
+//
+// What bounds it: the decode instructions, about 5 a weight; a loop that does nothing else sustains 17.6 weights per clock and SM with 8
+// warps (two chunks in flight per warp) and 18.7 with 16, so 8 decode warps per CTA and one or two CTAs per SM
+// (launch_stream) are enough.  The earlier form (clusters of short-lived CTAs, three launches per layer) spent half of its time on the
+// phases around the decode.  Units of 512 k leave some SMs with twice the work of others at one row: 24.4 us a layer, 23.4 with 256 k.
 #include <algorithm>
 
 #include "gemv.cuh"
@@ -41,7 +46,7 @@
 
 namespace gf {
 
-constexpr int ST_THREADS = 512, ST_STAGES = 4, ST_XSTAGES = 2;
+constexpr int ST_THREADS = 512, ST_STAGES = 4;
 constexpr int ST_DEC = 8, ST_XW = 3;                         // decode and X warps, then the producer, then four finish warps
 constexpr int ST_PROD = ST_DEC + ST_XW, ST_FIN = ST_PROD + 1;
 constexpr size_t ST_MAX_SMEM = 227 * 1024 - 4352;            // dynamic part (4,240 bytes are static)
@@ -49,12 +54,9 @@ constexpr size_t ST_HALF_SM = 116 * 1024;                    // two such CTAs do
 constexpr uint32_t ST_POLLS = 1u << 21;                      // polls of a global word before a wait gives up (about a second)
 
 enum : int { UNIT_G = 0, UNIT_D = 1, UNIT_END = 2 };       // low byte of a descriptor, matrix in bit 8
-constexpr int DESC_TWO = 1 << 16;                            // the unit has two stages
+enum : int { DESC_LAST = 1 << 9, DESC_CONT = 1 << 10, DESC_K = 12 };   // the stage ends its split; goes on with one; its first 128 k (from bit 12 on)
 
 // ---- {value, epoch} words -------------------------------------------------------------------------------------------
-__device__ __forceinline__ void ll_store(unsigned long long *p, uint32_t v, uint32_t epoch) {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)epoch << 32) | v) : "memory");
-}
 __device__ __forceinline__ void ll_store2(unsigned long long *p, uint32_t v0, uint32_t v1, uint32_t epoch) {
     const unsigned long long e = (unsigned long long)epoch << 32;
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(e | v0), "l"(e | v1) : "memory");
@@ -114,11 +116,9 @@ __device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long lon
     return true;
 }
 
-// Sum of the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the
-// epoch.  LAST: between the attempts only the last of the four is polled; it is mostly the last to come.  With more than 8 rows up to
-// eight finish warps an SM are always waiting, and their polls of all four cost the decode warps issue slots and L2 a tenth of its
-// rate (11 rows, 6 layers 428 -> 414 us, 16 rows 8 layers 672 -> 640); for fewer rows the extra round trip costs more (1137 ->
-// 1152 us for 47 layers of one token).
+// v += the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the epoch.  LAST:
+// between the attempts only the last of the four is polled; it is mostly the last to come (9 and more rows: polls of all four cost
+// the decode warps issue slots; for fewer rows the extra round trip costs more, 47 layers of one token 1113 -> 1144 us).
 template <bool LAST>
 __device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
                                            float (&v)[4]) {
@@ -154,9 +154,19 @@ __device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long l
     return true;
 }
 
+// A decode lane holds columns G and G + 8 of an n-tile and stores them side by side, so that one instruction takes both: word 2 G + h of
+// a tile is column G + 8 h.  A reading lane takes four consecutive words (z_word) and swaps two of them with its partner, which
+// leaves it columns 4 lane .. 4 lane + 3.
+__device__ __forceinline__ int z_word(int lane) { return (lane >> 2) * 16 + (lane & 1) * 8 + (lane & 2) * 2; }
+__device__ __forceinline__ void z_columns(float (&v)[4], int lane) {
+    const bool up = lane & 2;
+    const float a = __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], 2), b = __shfl_xor_sync(0xffffffffu, up ? v[2] : v[3], 2);
+    const float c = up ? v[1] : v[0], d = up ? v[3] : v[2];
+    v[0] = up ? a : c; v[1] = up ? b : d; v[2] = up ? c : a; v[3] = up ? d : b;
+}
 
 // ---- shared memory of a CTA ------------------------------------------------------------------------------------------
-// [stages] words | [X stages] activations | barriers, descriptors | tables of the window
+// [stages] words | [stages] activations | barriers, descriptors | tables of the window
 struct StTables {
     int *e, *mask, *pref;                // [umax] expert id, row mask (bit = row of the window); [umax + 1] finish-job prefix
     uint16_t *pair;                      // [umax][16] pair index of member m
@@ -170,7 +180,7 @@ constexpr int ST_META = 1024;            // barriers and descriptors
 inline size_t st_smem_bytes(int sets, int umax, int rows, int P, int E) {
     const size_t tables = (size_t)(3 * umax + 1) * 4 + (size_t)umax * 32 + (size_t)P * 2 + 64 +
                           (rows > 16 ? (size_t)(E + 1) * 4 * (1 + (rows + 31) / 32) : 0);
-    return (size_t)ST_STAGES * ST_WBYTES + (size_t)ST_XSTAGES * sets * 8 * ST_XROW + ST_META + (tables + 127) / 128 * 128 +
+    return (size_t)ST_STAGES * (ST_WBYTES + sets * 8 * ST_XROW) + ST_META + (tables + 127) / 128 * 128 +
            1024 /*align*/;
 }
 
@@ -379,30 +389,29 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
     return U;
 }
 
-// Register split over the warpgroups (decode, decode, X + producer, finish): 4 x 128 threads at 64 registers in all.
+// Register split over the warpgroups: decode and decode keep the 64 of the launch, X + producer give 16 to finish (64 + 64 + 48 + 80).
+// Decode at 56 registers took 60.5 us instead of 58.1 at 8 rows.
 template <bool INC, int N>
 __device__ __forceinline__ void st_regs() {
     if (INC) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-template <int SETS, bool MANY>
+template <int SETS, bool MANY, int ROUNDS>
 __global__ void __launch_bounds__(ST_THREADS, 2)
 stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_d,
               const __grid_constant__ StreamArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);          // the swizzle atom is 1024 bytes
-    constexpr int XBYTES = SETS * 8 * ST_XROW;
+    constexpr int XBYTES = SETS * 8 * ST_XROW, SKT = 8 * ROUNDS, SBYTES = SKT * 1024;          // k-tiles and bytes of a stage
     unsigned char *words = smem, *xbuf = smem + ST_STAGES * ST_WBYTES;
-    unsigned char *meta = xbuf + ST_XSTAGES * XBYTES;
-    uint64_t *wfull = reinterpret_cast<uint64_t *>(meta);             // words of the stage landed (and its descriptor written)
-    uint64_t *empty = wfull + ST_STAGES;                              // stage consumed
-    uint64_t *xready = empty + ST_STAGES;                             // unit described
-    uint64_t *xfull = xready + ST_XSTAGES;                            // activations of the unit staged
-    uint64_t *xempty = xfull + ST_XSTAGES;                            // unit consumed
-    int4 *desc = reinterpret_cast<int4 *>(meta + 256);                // {kind | matrix << 8 | flags, expert number, split, block}
-    int4 *xdesc = desc + ST_STAGES;                                   // {kind | matrix << 8, expert number, split, -}
-    int *job_sh = reinterpret_cast<int *>(xdesc + ST_XSTAGES);        // [2]
+    unsigned char *meta = xbuf + ST_STAGES * XBYTES;
+    uint64_t *ready = reinterpret_cast<uint64_t *>(meta);             // stage described
+    uint64_t *wfull = ready + ST_STAGES;                              // its words landed
+    uint64_t *xfull = wfull + ST_STAGES;                              // its activations staged
+    uint64_t *empty = xfull + ST_STAGES;                              // consumed
+    int4 *desc = reinterpret_cast<int4 *>(meta + 256);                // {kind | matrix << 8 | flags | k, expert number, first word of the partials, -}
+    int *job_sh = reinterpret_cast<int *>(desc + ST_STAGES);          // [2]
     StTables tb;
     tb.e = reinterpret_cast<int *>(meta + ST_META);
     tb.mask = tb.e + a.umax;
@@ -418,17 +427,14 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int H = a.H, I = a.I, P = a.rows * a.slots;
-    const int SK1 = (H + 511) >> 9, SK2 = (I + 511) >> 9, NB1 = I >> 7, NB2 = H >> 7;
+    const int SK1 = a.cut1.splits, SK2 = a.cut2.splits, NB1 = I >> 7, NB2 = H >> 7;
     const StCta cta{&abort_sh, a.status};
     if (tid == 0) {
         for (int s = 0; s < ST_STAGES; ++s) {
+            mbar_init(ready + s, 1);
             mbar_init(wfull + s, 1);
-            mbar_init(empty + s, ST_DEC);
-        }
-        for (int s = 0; s < ST_XSTAGES; ++s) {
-            mbar_init(xready + s, 1);
             mbar_init(xfull + s, ST_XW);
-            mbar_init(xempty + s, ST_DEC);
+            mbar_init(empty + s, ST_DEC);
         }
         abort_sh = 0;
         mbar_fence_init();
@@ -490,89 +496,73 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     }
 
     if (warp < ST_DEC) {
-        if (SETS == 1) st_regs<false, 56>();
         // ---------------------------------------------------------------------------------------------- decode
         const int G = lane >> 2, T = lane & 3;
-        uint32_t it = 0;
-        for (uint32_t c = 0;; ++c) {
-            const int xs = c % ST_XSTAGES;
-            if (!__all_sync(0xffffffffu, cta.wait(wfull + it % ST_STAGES, (it / ST_STAGES) & 1))) break;
-            const int4 d = desc[it % ST_STAGES];
+        float acc[SETS][4];                                           // over a split
+        for (uint32_t it = 0;; ++it) {
+            const int s = it % ST_STAGES, phase = (it / ST_STAGES) & 1;
+            if (!__all_sync(0xffffffffu, cta.wait(wfull + s, phase))) break;
+            const int4 d = desc[s];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
             const int nmem = __popc(tb.mask[d.y]);
             const uint32_t p01 = *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 2 * T);
             const uint32_t p23 = SETS == 2 ? *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 8 + 2 * T) : 0u;
-            if (!__all_sync(0xffffffffu, cta.wait(xfull + xs, (c / ST_XSTAGES) & 1))) break;
-            float acc[SETS][4];
+            if (!__all_sync(0xffffffffu, cta.wait(xfull + s, phase))) break;
+            if (!(d.x & DESC_CONT))
 #pragma unroll
-            for (int q = 0; q < SETS; ++q)
+                for (int q = 0; q < SETS; ++q)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[q][j] = 0.f;
-            const int halves = d.x & DESC_TWO ? 2 : 1;
-            bool ok = true;
-            for (int half = 0; half < halves; ++half, ++it) {
-                const int s = it % ST_STAGES;
-                if (half) ok = __all_sync(0xffffffffu, cta.wait(wfull + s, (it / ST_STAGES) & 1));
-                if (!ok) break;
-                const unsigned char *ws = words + s * ST_WBYTES, *xh = xbuf + xs * XBYTES + half * 512;
-                // (few experts of a window or chunk have more than eight members; with the second set's operand loads in every
-                // unit, eleven rows took 459 us over 6 layers instead of 428 and a chunk of 40 192 instead of 180)
-                if (SETS == 1 || nmem <= 8) st_decode<1>(ws, xh, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
-                else st_decode<SETS>(ws, xh, warp, lane, acc);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty + s);
-            }
-            if (!ok) break;
-            if (lane == 0) mbar_arrive(xempty + xs);
+                    for (int j = 0; j < 4; ++j) acc[q][j] = 0.f;
+            const unsigned char *ws = words + s * SBYTES, *xs = xbuf + s * XBYTES;
+            // (few experts of a window or chunk have more than eight members; with the second set's operand loads in every
+            // unit, eleven rows of the 4096 x 512 layer took 115 us instead of 107 and a chunk of 40 192 instead of 180)
+            if (SETS == 1 || nmem <= 8) st_decode<1, ROUNDS>(ws, xs, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
+            else st_decode<SETS, ROUNDS>(ws, xs, warp, lane, acc);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + s);
+            if (!(d.x & DESC_LAST)) continue;
             const int N = kind == UNIT_G ? I : H;
-            unsigned long long *z = kind == UNIT_G ? a.z1 + (size_t)(((d.x >> 8) & 1) * SK1 + d.z) * P * I : a.z2 + (size_t)d.z * P * H;
-            z += d.w * 128 + warp * 16 + G;
+            unsigned long long *z = (kind == UNIT_G ? a.z1 : a.z2) + (unsigned)d.z + warp * 16 + 2 * G;
 #pragma unroll
             for (int q = 0; q < SETS; ++q) {
                 const uint32_t pp = q ? p23 : p01;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    if (q * 8 + 2 * T + j < nmem) {
-                        unsigned long long *zp = z + (size_t)(j ? pp >> 16 : pp & 0xffffu) * N;
-                        ll_store(zp, __float_as_uint(acc[q][j]), epoch);
-                        ll_store(zp + 8, __float_as_uint(acc[q][2 + j]), epoch);
-                    }
+                    if (q * 8 + 2 * T + j < nmem)
+                        ll_store2(z + (size_t)(j ? pp >> 16 : pp & 0xffffu) * N, __float_as_uint(acc[q][j]), __float_as_uint(acc[q][2 + j]), epoch);
             }
         }
     } else if (warp < ST_PROD) {
-        st_regs<false, SETS == 1 ? 56 : 48>();
+        st_regs<false, 48>();
         // ---------------------------------------------------------------------------------------------- activations
         const int xw = warp - ST_DEC;
         for (uint32_t it = 0;; ++it) {
-            const int s = it % ST_XSTAGES;
-            if (!__all_sync(0xffffffffu, cta.wait(xready + s, (it / ST_XSTAGES) & 1))) break;
-            const int4 d = xdesc[s];
+            const int s = it % ST_STAGES;
+            if (!__all_sync(0xffffffffu, cta.wait(ready + s, (it / ST_STAGES) & 1))) break;
+            const int4 d = desc[s];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
-            const int nmem = __popc(tb.mask[d.y]), K = kind == UNIT_G ? H : I, halves = min(2, (K >> 8) - 2 * d.z);
+            const int nmem = __popc(tb.mask[d.y]), K = kind == UNIT_G ? H : I;
             const uint16_t *pair = tb.pair + d.y * 16;
-            const unsigned long long *src = (kind == UNIT_G ? a.xr + (size_t)((d.x >> 8) & 1) * P * (H / 2) : a.xdl) + d.z * 256 + 4 * lane;
-            unsigned char *xs = xbuf + s * XBYTES + 16 * lane;
+            // a warp per member, the loads of two in flight; 128 k are half a warp's, whose other half reads and writes the same again
+            const int part = ROUNDS == 2 ? lane : lane & 15;
+            const unsigned long long *src = (kind == UNIT_G ? a.xr + (size_t)((d.x >> 8) & 1) * P * (H / 2) : a.xdl) + (d.x >> DESC_K) * 64 + 4 * part;
+            unsigned char *xs = xbuf + s * XBYTES + 16 * part;
             const bool poll = kind == UNIT_G || a.do_g;               // (the down phase alone takes what the last run left)
             bool ok = true;
-            // a warp per (member, 256 k), the loads of two in flight
-            for (int t0 = xw; t0 < nmem * halves; t0 += 2 * ST_XW) {
+            for (int t0 = xw; t0 < nmem; t0 += 2 * ST_XW) {
                 unsigned long long w[2][4];
-                int m[2], h[2];
+                int m[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    const int q = min(t0 + i * ST_XW, nmem * halves - 1);       // past the end: the last one again
-                    m[i] = halves == 2 ? q >> 1 : q;
-                    h[i] = halves == 2 ? q & 1 : 0;
-                    ll_load4(src + (size_t)pair[m[i]] * (K / 2) + h[i] * 128, w[i]);
+                    m[i] = min(t0 + i * ST_XW, nmem - 1);             // past the end: the last one again
+                    ll_load4(src + (size_t)pair[m[i]] * (K / 2), w[i]);
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    if (poll && !__all_sync(0xffffffffu, ll_ready(w[i], epoch)))
-                        ok = ok && ll_wait4(cta, src + (size_t)pair[m[i]] * (K / 2) + h[i] * 128, epoch, w[i]);
-                    *reinterpret_cast<uint4 *>(xs + m[i] * ST_XROW + h[i] * 512) =
-                        make_uint4((uint32_t)w[i][0], (uint32_t)w[i][1], (uint32_t)w[i][2], (uint32_t)w[i][3]);
+                    if (poll && !__all_sync(0xffffffffu, ll_ready(w[i], epoch))) ok = ok && ll_wait4(cta, src + (size_t)pair[m[i]] * (K / 2), epoch, w[i]);
+                    *reinterpret_cast<uint4 *>(xs + m[i] * ST_XROW) = make_uint4((uint32_t)w[i][0], (uint32_t)w[i][1], (uint32_t)w[i][2], (uint32_t)w[i][3]);
                 }
             }
             __syncwarp();
@@ -580,7 +570,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             if (lane == 0) mbar_arrive(xfull + s);
         }
     } else if (warp >= ST_FIN) {
-        st_regs<true, SETS == 1 ? 88 : 80>();
+        st_regs<true, 80>();
         // ---------------------------------------------------------------------------------------------- finish
         const int fw = warp - ST_FIN, ft = tid - ST_FIN * 32;
         const int jobs_g = jobs_r + (a.do_g ? tb.pref[U] * NB1 : 0), jobs = jobs_g + (a.do_d ? a.rows * NB2 : 0);
@@ -598,22 +588,27 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             if (j < jobs_r) {
                 for (int r = j * rot_job + fw; r < min(rots, (j + 1) * rot_job); r += 4) rotate(r);
             } else if (j < jobs_g) {
-                // gate / up of one member: warp = (matrix, half of the splits).  The halves of a matrix meet in shared memory; warp 2
-                // transforms the up matrix and hands the clamped values over, warp 0 does the same for gate, applies SwiGLU, rotates
-                // and stores.
+                // gate / up of one member: warp 2 adds the up matrix's partials, transforms them and hands the clamped values over; warp
+                // 0 does the same for gate, applies SwiGLU, rotates and stores.
                 const int q = fast_div(j - jobs_r, inv_nb1), nb = j - jobs_r - q * NB1, lo = member_expert(q);
-                const int role = fw >> 1, half = fw & 1, mid = (SK1 + 1) >> 1;
+                const int role = fw >> 1, half = fw & 1;
                 const int p = tb.pair[lo * 16 + q - tb.pref[lo]], col = nb * 128 + 4 * lane;
                 const size_t so = (size_t)tb.e[lo] * I + col;
                 const uint2 sv = ldg_half4((role ? a.svh_u : a.svh_g) + so, a.vec);
                 const uint2 sd = ldg_half4(a.suh_d + so, a.vec);
                 float v[4] = {0.f, 0.f, 0.f, 0.f};
-                sum_splits<SETS == 2>(cta, a.z1 + ((size_t)role * SK1 * P + p) * I + col, (size_t)P * I, half ? mid : 0, half ? SK1 : mid, epoch, v);
-                if (half) *reinterpret_cast<float4 *>(&fin_sh[fw][4 * lane]) = make_float4(v[0], v[1], v[2], v[3]);
-                pair_barrier(role);
+                const unsigned long long *z = a.z1 + ((size_t)role * SK1 * P + p) * I + nb * 128 + z_word(lane);
+                if (SETS == 2) {
+                    // With more than 8 rows up to eight finish warps an SM are always waiting, and their polls cost the decode warps issue
+                    // slots: only warp 3 polls, for the partial that is drawn last (16 rows: 695 -> 671 us over 8 layers; for one row the
+                    // extra round trip costs more, 47 layers 1128 -> 1141 us).
+                    unsigned long long last[4];
+                    if (fw == 3) ll_wait4(cta, z + (size_t)(SK1 - 1) * P * I, epoch, last);
+                    asm volatile("bar.sync 5, 128;" ::: "memory");
+                }
                 if (!half) {
-                    const float4 o = *reinterpret_cast<const float4 *>(&fin_sh[fw + 1][4 * lane]);
-                    v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
+                    sum_splits<SETS == 2>(cta, z, (size_t)P * I, 0, SK1, epoch, v);
+                    z_columns(v, lane);
                     fwht128(v, lane);
                     const float2 c01 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.x)), c23 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.y));
                     const float r[4] = {bf16r(v[0] * HAD_SCALE * c01.x), bf16r(v[1] * HAD_SCALE * c01.y), bf16r(v[2] * HAD_SCALE * c23.x),
@@ -661,9 +656,13 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0)
-                            sum_splits<SETS == 2>(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col, (size_t)P * H, 0, SK2, epoch, v[i]);
-                    if (e[0] >= 0) fwht128(v[0], lane);
-                    if (e[1] >= 0) fwht128(v[1], lane);
+                            sum_splits<SETS == 2>(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + nb * 128 + z_word(lane), (size_t)P * H, 0, SK2, epoch, v[i]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        if (e[i] >= 0) {
+                            z_columns(v[i], lane);
+                            fwht128(v[i], lane);
+                        }
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         float *y = a.y + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + col;
@@ -693,49 +692,49 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         }
     } else {
         // ---------------------------------------------------------------------------------------------- producer
-        st_regs<false, SETS == 1 ? 56 : 48>();
+        st_regs<false, 48>();
         uint32_t it = 0;
         bool ok = true;
         const float inv_nb1 = fast_inv(NB1), inv_nb2 = fast_inv(NB2), inv_sk1 = fast_inv(SK1), inv_sk2 = fast_inv(SK2);
-        for (uint32_t c = 0; ok; ++c) {
-            const int xs = c % ST_XSTAGES;
+        const int split1 = a.cut1.split, split2 = a.cut2.split;
+        while (ok) {
             // A unit is drawn only when there is room for it (the draw and the copy take 3,000 clocks, the stages in front of it
             // 6,000 and more): units drawn earlier would only arrive late at whoever waits for their sums.
-            ok = __all_sync(0xffffffffu, cta.wait(xempty + xs, ((c / ST_XSTAGES) & 1) ^ 1) &&
-                                             cta.wait(empty + it % ST_STAGES, ((it / ST_STAGES) & 1) ^ 1));
+            int s = it % ST_STAGES;
+            ok = __all_sync(0xffffffffu, cta.wait(empty + s, ((it / ST_STAGES) & 1) ^ 1));
             if (!ok) break;
-            if (c && lane == 0) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
+            if (it && lane == 0) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
             int t = __shfl_sync(0xffffffffu, drawn, 0);
             if (t >= units) {
-                const int s = it % ST_STAGES;
                 if (lane == 0) {
-                    desc[s] = xdesc[xs] = make_int4(UNIT_END, 0, 0, 0);
-                    mbar_arrive(xready + xs);
+                    desc[s] = make_int4(UNIT_END, 0, 0, 0);
+                    mbar_arrive(ready + s);
                     mbar_arrive(wfull + s);
                 }
                 break;
             }
             const bool g = t < units_g;
             if (!g) t -= units_g;
-            const int SK = g ? SK1 : SK2, q = fast_div(t, g ? inv_nb1 : inv_nb2), nb = t - q * (g ? NB1 : NB2);
+            const int q = fast_div(t, g ? inv_nb1 : inv_nb2), nb = t - q * (g ? NB1 : NB2);
             t = fast_div(q, g ? inv_sk1 : inv_sk2);
-            const int split = q - t * SK;
-            const int mat = g ? t & 1 : 0, u = g ? t >> 1 : t, kind = g ? UNIT_G : UNIT_D;
-            if (lane == 0) {
-                xdesc[xs] = make_int4(kind | mat << 8, u, split, 0);
-                mbar_arrive(xready + xs);
-            }
+            const int split = q - t * (g ? SK1 : SK2), mat = g ? t & 1 : 0, u = g ? t >> 1 : t, head = (g ? UNIT_G : UNIT_D) | mat << 8;
             const CUtensorMap *map = g ? (mat ? &map_u : &map_g) : &map_d;
-            const int K = g ? H : I, kt = tb.e[u] * (K >> 4) + split * 32, halves = min(2, (K >> 8) - 2 * split);
-            for (int half = 0; half < halves; ++half, ++it) {
-                const int s = it % ST_STAGES;
+            const int KT = (g ? H : I) >> 4, len = g ? split1 : split2, row = tb.e[u] * KT, first = split * len, last = min(KT, first + len);
+            const unsigned z = (unsigned)(mat * SK1 + split) * (unsigned)(P * (g ? I : H)) + (unsigned)(nb * 128);
+            for (int kt = first;;) {
+                const bool end = kt + SKT == last;
+                if (lane == 0) {
+                    desc[s] = make_int4(head | (kt != first ? DESC_CONT : 0) | (end ? DESC_LAST : 0) | (kt >> 3) << DESC_K, u, (int)z, 0);
+                    mbar_arrive(ready + s);
+                    mbar_expect_tx(wfull + s, SBYTES);
+                    tma_load_3d(words + s * SBYTES, map, 0, row + kt, nb * 8, wfull + s);
+                }
+                ++it;
+                kt += SKT;
+                if (end) break;
+                s = it % ST_STAGES;
                 ok = __all_sync(0xffffffffu, cta.wait(empty + s, ((it / ST_STAGES) & 1) ^ 1));
                 if (!ok) break;
-                if (lane == 0) {
-                    desc[s] = make_int4(kind | mat << 8 | (halves == 2 ? DESC_TWO : 0), u, split, nb);
-                    mbar_expect_tx(wfull + s, ST_WBYTES);
-                    tma_load_3d(words + s * ST_WBYTES, map, 0, kt + half * 16, nb * 8, wfull + s);
-                }
             }
         }
         // after a give-up copies may be in flight: they have landed before the CTA leaves (bounded)
@@ -756,14 +755,20 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
 int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
     static int sms[64] = {};
-    static bool configured[64][3] = {};
+    static bool configured[64][5] = {};
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
     GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
     if (!sms[dev]) GF_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
-    const int sets = a.rows > 8 ? 2 : 1, which = a.rows > 16 ? 2 : sets - 1;
+    // Stages of 128 k where a split is not a whole number of 256 k (K = 2304): the stage is a constant of the kernel.
+    const bool fine = a.cut1.split % 16 || a.cut2.split % 16;
+    const int sets = a.rows > 8 ? 2 : 1, which = a.rows > 16 ? 4 : sets - 1 + 2 * fine;
     // (chunks have a kernel of their own: with their tables as a branch, windows of 11 rows were 1 % slower)
-    const auto kernel = which == 2 ? stream_kernel<2, true> : which ? stream_kernel<2, false> : stream_kernel<1, false>;
+    const auto kernel = which == 4   ? stream_kernel<2, true, 2>
+                        : which == 3 ? stream_kernel<2, false, 1>
+                        : which == 2 ? stream_kernel<1, false, 1>
+                        : which      ? stream_kernel<2, false, 2>
+                                     : stream_kernel<1, false, 2>;
     size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
     GF_REQUIRE(smem <= ST_MAX_SMEM, "routing table too large for the window kernel");
     // CTAs per SM.  One has shorter chains for few units (one token: 24.4 us a layer against 28.6 with two); two fill the decode
@@ -782,7 +787,8 @@ int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
         configured[dev][which] = true;
     }
     CUtensorMap mg, mu, md;
-    if (bank_map(&mg, a.gt, a.E + 1, a.H, a.I) || bank_map(&mu, a.ut, a.E + 1, a.H, a.I) || bank_map(&md, a.dt, a.E + 1, a.I, a.H)) return -1;
+    const uint32_t kt = fine ? 8 : 16;
+    if (bank_map(&mg, a.gt, a.E + 1, a.H, a.I, kt) || bank_map(&mu, a.ut, a.E + 1, a.H, a.I, kt) || bank_map(&md, a.dt, a.E + 1, a.I, a.H, kt)) return -1;
     return launch_k(kernel, grid, block, smem, s, pdl, mg, mu, md, a);
 }
 
