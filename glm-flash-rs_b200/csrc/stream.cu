@@ -184,6 +184,11 @@ inline size_t st_smem_bytes(int sets, int umax, int rows, int P, int E) {
            1024 /*align*/;
 }
 
+// Whether pair (row, expert e) is another GPU's: expert window, shared expert's switch (sh) and its row window.
+__device__ __forceinline__ bool st_skipped(const StreamArgs &a, int row, int e, int sh) {
+    return expert_skipped(e, a.E, sh, a.e_lo, a.e_hi) || (e == a.E && a.srow_hi > a.srow_lo && (row < a.srow_lo || row >= a.srow_hi));
+}
+
 // Distinct experts of the window that this GPU computes (ascending), their members (ascending rows) and the prefix of
 // their members (one finish job per member and column block).  All threads of the CTA; the caller's barrier publishes the
 // tables.  This is the head of every layer's critical path.  `used` (32 words) and tb.mask are zero on entry; row, slot: of
@@ -194,7 +199,7 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
         // one row: every warp finds the order of the picks itself and writes the same tables (no block barrier)
         constexpr int NONE = 0x7fffffff;
         const int e = lane < a.slots ? __ldcg(a.picks + lane) : NONE;
-        int key = e == NONE || expert_skipped(e, a.E, a.shared, a.e_lo, a.e_hi) ? NONE : e;
+        int key = e == NONE || st_skipped(a, 0, e, a.shared) ? NONE : e;
         int less = 0;
         bool dup = false;
         for (int j = 0; j < a.slots; ++j) {
@@ -227,7 +232,8 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
         if (tid < P) {
             e = __ldcg(a.picks + tid);
             tb.state[tid] = (short)e;
-            if (e >= 0 && e <= a.E) {                            // ids above E name nothing
+            // ids above E name nothing; the shared expert counts for the rows of its window only (no row: it is not in the bitmap)
+            if (e >= 0 && e <= a.E && !(e == a.E && st_skipped(a, row, e, 1))) {
                 key = e;
                 atomicOr(&used[key >> 5], 1u << (key & 31));
             }
@@ -330,10 +336,7 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
         for (int q = row * a.slots; q < i; ++q) dup |= tb.state[q] == (short)e;
         return !dup;
     };
-    auto skipped = [&](int row, int e) {
-        return expert_skipped(e, a.E, a.shared, a.e_lo, a.e_hi) ||
-               (e == a.E && a.srow_hi > a.srow_lo && (row < a.srow_lo || row >= a.srow_hi));     // shared expert: row window
-    };
+    auto skipped = [&](int row, int e) { return st_skipped(a, row, e, a.shared); };
     for (int i = tid; i < P; i += ST_THREADS) {
         const int e = tb.state[i], row = fast_div(i, inv_slots);
         if (!skipped(row, e) && first_of_row(i, row, e)) atomicOr(&tb.rows_of[e * W + (row >> 5)], 1u << (row & 31));

@@ -9,9 +9,9 @@ from conftest import TOL, rel_err
 pytestmark = pytest.mark.gpu
 
 
-def run(pkg, cuda, bank, x, picks, rw, H, I, E, S, rows, synth, **kw):
+def run(pkg, cuda, bank, x, picks, rw, H, I, E, S, rows, synth, max_rows=None, **kw):
     import torch
-    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=rows, **kw))
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=max_rows or rows, **kw))
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
     xd = t(x.view(np.int16)).view(torch.bfloat16)
     for _ in range(2):                                   # the second launch runs on the first one's counters and words
@@ -49,6 +49,24 @@ def test_short_chunks_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows, kw):
     want = np.where(here[..., None], np.where((np.arange(S) == S - 1)[None, :, None], 1, rw[..., None]) * Y, 0).sum(1)
     emax, erms = rel_err(got, want)
     assert emax < TOL and erms < TOL, (emax, erms)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 16])
+@pytest.mark.parametrize("shared_rows", [(512, 1024), (3, 6), (0, 1), (5, 64), (0, 64)])
+@pytest.mark.parametrize("share", [{}, dict(expert_lo=2, expert_hi=7)])
+def test_shared_row_window_of_a_short_call(pkg, oracle, synth, cuda, rows, shared_rows, share):
+    # a handle for large chunks whose shared expert is split by rows over the ranks, given a tail of 16 rows or fewer: none, some and
+    # all of its rows are in the window
+    H, I, E, S = 512, 512, 12, 4
+    bank = synth.expert_bank(57, H, I, E, svh_scale=True)
+    x, (picks, rw) = synth.activations_bf16(58, rows, H), synth.route(59, rows, E, S - 1)
+    got = run(pkg, cuda, synth.to_device(bank, cuda), x, picks, rw, H, I, E, S, rows, synth, max_rows=64, shared_rows=shared_rows, **share)
+    Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1).reshape(rows, S, H)
+    lo, hi, at = share.get("expert_lo", 0), share.get("expert_hi", E), np.arange(rows)[:, None]
+    here = (picks >= lo) & (picks < hi) | (picks == E) & (at >= shared_rows[0]) & (at < shared_rows[1])
+    want = np.where(here[..., None], np.where((np.arange(S) == S - 1)[None, :, None], 1, rw[..., None]) * Y, 0).sum(1)
+    scale = np.abs(Y).max()                              # (a share may leave a row, or all of a one-row call, without an expert)
+    assert np.abs(got - want).max() < TOL * scale
 
 
 @pytest.mark.parametrize("rows", [1, 5])
