@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(EP_THREADS) ep_combine_kernel(const float *__r
                                                                 int max_ctas, int slots, int H, int E, int shared_exl3,
                                                                 int e_lo, int e_hi, int srow_lo, int srow_hi,
                                                                 unsigned wait_polls) {
-    // (the routing table was complete before the expert kernels in front ran: it may be read ahead of the dependency wait)
-    __shared__ uint32_t used_sh[32];
-    if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
+    // (wait first: the layer kernel in front lets this one start before its own wait, so the router may still be writing the picks)
     pdl_wait();
     pdl_launch_dependents();
+    __shared__ uint32_t used_sh[32];
+    if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
     __shared__ int ok_sh;
     const int r = blockIdx.y;
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
@@ -162,11 +162,11 @@ __global__ void __launch_bounds__(EP_THREADS) ep_combine_ll_kernel(const float *
                                                                    int *status, int rank, int world, int rows, int max_rows,
                                                                    int slots, int H, int E, int shared_exl3, int e_lo, int e_hi,
                                                                    unsigned wait_polls) {
-    // (the routing table was complete before the expert kernels in front ran: it may be read ahead of the dependency wait)
-    __shared__ uint32_t used_sh[32];
-    if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
+    // (wait first: the layer kernel in front lets this one start before its own wait, so the router may still be writing the picks)
     pdl_wait();
     pdl_launch_dependents();
+    __shared__ uint32_t used_sh[32];
+    if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
     const int r = blockIdx.y;
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const unsigned epoch = *epoch_ptr + 1u;                   // every CTA reads it before the last one advances it

@@ -22,8 +22,9 @@ __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ 
                                                       const float *__restrict__ route_w, float *__restrict__ out, int rows,
                                                       int slots, int H, int E, int shared_exl3, int e_lo, int e_hi,
                                                       int srow_lo, int srow_hi) {
-    // The routing table and the weights were complete before the expert kernels ran (those read them), so they are
-    // fetched ahead of the dependency wait; only the pair results Y belong to the kernel in front.
+    // Launched behind the down GEMM only.  That kernel, like the grouping, plan, rotation and gate / up kernels in front of it, runs
+    // its own pdl_wait before it triggers, so when this one starts, everything in front of the down GEMM has completed, the
+    // router's table and weights among it: they are read ahead of the wait.  Only the pair results Y belong to the kernel in front.
     const int r = blockIdx.y;
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     __shared__ float wgt_sh[32];

@@ -454,7 +454,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     if (tid >= 256 && tid < 259) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)(tid == 256 ? &map_g : tid == 257 ? &map_u : &map_d)) : "memory");
     if (tid < P && tid % 32 == 0 && a.picks) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.picks + tid));
     const int row = tid / a.slots, slot = tid - row * a.slots;        // of routing-table entry number tid
-    pdl_launch_dependents();                        // the next kernel waits for all of this one before it touches memory
+    pdl_launch_dependents();                        // before the wait: the next kernel may start while the one in front of this still runs
     pdl_wait();
     // the first draws of the producer and the finish group travel while the tables are built
     int drawn = 0;

@@ -196,21 +196,25 @@ int  glmflash_moe_run_host(glmflash_moe *m, void *stream, const glmflash_weights
                            float *out_host);
 
 /* PDL contract (config.pdl = 1): how a host kernel joins the chain at either edge of a layer, as upstream chains its own
- * kernels around the expert loads (native/expert_loads.cu:38-44, src/experts.rs:350-354).  The kernels of a window of
- * <= 16 rows, and the grouping, router, combine and exchange kernels of every window, are launched with the
- * programmatic-stream-serialization attribute and execute griddepcontrol.wait in every CTA that does work, so "the
- * kernel before has completed" is transitive along the stream; the plan / rotation / GEMM kernels in the middle of a
- * prefill layer are plain launches (fully ordered).
+ * kernels around the expert loads (native/expert_loads.cu:38-44, src/experts.rs:350-354).  All kernels of a layer (layer
+ * kernel, grouping, plan, rotation, GEMMs, combine, exchange) and of the router are launched with the
+ * programmatic-stream-serialization attribute and execute griddepcontrol.wait in every CTA, so that what a kernel sees
+ * after its wait is everything in front of it in the stream, not its predecessor alone.  Before the wait nothing but
+ * constants (weights, scales, the router matrix) is read, with one exception that its comment explains (the combine of a
+ * chunk reads the routing table behind kernels that trigger after their own wait).
  *   In front of a layer (the producer of `input`, `picks`, `route_w`): nothing is required.  The first kernel of
  *     glmflash_moe_run / glmflash_moe_run_ep / glmflash_route touches no global memory before its griddepcontrol.wait, so
  *     the producer may be a plain kernel, or call griddepcontrol.launch_dependents as early as it likes (the layer's CTAs
  *     then become resident and set up their barriers while the producer drains).
  *   Behind a layer (a consumer of glmflash_moe_output / glmflash_ep_output), when the consumer is itself launched with the
  *     attribute: the layer's last kernel calls griddepcontrol.launch_dependents at its start, so the consumer's CTAs may
- *     start while the layer's last kernel (with GLMFLASH_LAYER_KERNELS=1: the whole layer) is still running.  Before its own
- *     griddepcontrol.wait the consumer may read its own weights and any buffer the layer does not write (a prefetch);
- *     it must not read the layer's output, pair buffer or status word, and must not write `input`, `picks`, `route_w`
- *     or the weights.  After the wait everything the layer wrote is visible.
+ *     start while the layer's last kernel is still running; for windows of <= 16 rows and short chunks that is the whole
+ *     layer, and since the layer kernel triggers before its own wait, the kernel in front of the layer (the router, the
+ *     producer of `input`) may still be running as well.  Before its own griddepcontrol.wait the consumer may therefore read
+ *     only what no kernel in front of it in the stream writes: its own weights and other constants (a prefetch).  It must
+ *     not read the layer's output, pair buffer or status word, nor `input`, `picks`, `route_w` or any other product of an
+ *     earlier kernel, and must write nothing that an earlier kernel reads or writes.  After the wait everything in front of
+ *     it is visible.
  *   A consumer launched without the attribute is ordered after the whole layer, as any kernel in the stream. */
 
 /* ---- expert-parallel combine over NVLink ------------------------------------------------------------ */
