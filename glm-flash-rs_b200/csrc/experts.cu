@@ -38,7 +38,8 @@ int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limi
 
 using namespace gf;
 
-// max_rows_limit: 16 for the public owner; chunk owners keep one for their short chunks.
+// max_rows_limit: 16 for the public owner.  Chunk owners keep one for their short chunks, whose pair rows are the chunk owner's and
+// whose down inputs nobody reads afterwards.
 int gf::experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit, glmflash_experts **out) {
     GF_REQUIRE(out != nullptr, "out is null");
     *out = nullptr;
@@ -48,8 +49,10 @@ int gf::experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_l
     e->cfg = *cfg;
     const size_t H = cfg->hidden, I = cfg->inter, P = (size_t)cfg->max_rows * cfg->slots;
     Pool pool;
-    pool.take(&e->xd, P * I * 2);
-    pool.take(&e->y, P * H * 4);
+    if (max_rows_limit <= 16) {
+        pool.take(&e->xd, P * I * 2);
+        pool.take(&e->y, P * H * 4);
+    }
     pool.take(&e->status, 4);
     pool.take(&e->ll_z1, stream_z1_words(*cfg) * 8);
     pool.take(&e->ll_z2, stream_z2_words(*cfg) * 8);

@@ -6,11 +6,11 @@
 struct glmflash_experts {
     glmflash_config cfg;
     void *pool = nullptr;                                 // the one allocation behind every buffer below
-    __half *xd = nullptr;                                 // down-projection inputs [P][I] (public)
+    __half *xd = nullptr;                                 // down-projection inputs [P][I] (public; not of a chunk owner)
     // streamed layer kernel (stream.cu): {value, epoch} words of the partial sums and of the finished rows, its counters
     unsigned long long *ll_z1 = nullptr, *ll_z2 = nullptr, *ll_xd = nullptr, *ll_xr = nullptr;
     unsigned *ctrl = nullptr;
-    float *y = nullptr;                                   // pair results [P][H] (public)
+    float *y = nullptr;                                   // pair results [P][H] (public; not of a chunk owner)
     int *status = nullptr;
     int phases = 7;                                       // profiling aid: 1 = input rotation, 2 = gate/up, 4 = down
     // one-launch layer kernel (window.cu): split partials, arrival counters / ready words, layer output

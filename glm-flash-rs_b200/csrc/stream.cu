@@ -636,7 +636,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                         const uint32_t w0 = pack_half2(o4[0] * HAD_SCALE, o4[1] * HAD_SCALE), w1 = pack_half2(o4[2] * HAD_SCALE, o4[3] * HAD_SCALE);
                         if (!abort_sh) {
                             ll_store2(a.xdl + ((size_t)p * I + col) / 2, w0, w1, epoch);
-                            *reinterpret_cast<uint2 *>(a.xd + (size_t)p * I + col) = make_uint2(w0, w1);
+                            if (a.xd) *reinterpret_cast<uint2 *>(a.xd + (size_t)p * I + col) = make_uint2(w0, w1);
                         }
                     }
                 }

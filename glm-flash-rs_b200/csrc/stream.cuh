@@ -35,7 +35,7 @@ struct StreamArgs {
     const int *ids, *count, *members;                        // (used when picks == nullptr; members [.][maxm])
     const float *route_w;                                    // [rows][slots] for the combine
     unsigned long long *z1, *z2, *xr, *xdl;                  // {value, epoch} words: gate / up and down partials, their inputs
-    __half *xd;                                              // plain down inputs [P][I]
+    __half *xd;                                              // plain down inputs [P][I], or nullptr
     float *y, *out, *out2;                                   // pair results [P][H]; combined rows [rows][H] (out2: a second copy) or nullptr
     unsigned *ctrl;                                          // CTRL_WORDS
     int *status;

@@ -170,7 +170,12 @@ typedef struct glmflash_moe glmflash_moe;
  * Windows of <= 16 rows run as ONE launch per layer: a persistent kernel that streams the chosen experts' words (upstream's
  * router-to-combine sequence src/moe.rs:101-181 takes eight kernels).  The environment variable GLMFLASH_LAYER_KERNELS=1
  * (read when an owner is created) selects an alternative one-launch kernel, which also carries the cross-GPU exchange of
- * glmflash_moe_run_ep; on one GPU it is slower. */
+ * glmflash_moe_run_ep; on one GPU it is slower.
+ * Calls of up to min(max_rows, 128, 16 experts / (slots - 1)) rows take that launch on a handle for more rows as well.  For them such
+ * a handle holds, beside the prefill scratch, exchange words of
+ *   8 slots (2 ceil(hidden / 512) inter + ceil(inter / 512) hidden + hidden + inter / 2) bytes
+ * for each of these rows (and never less than sixteen rows of a window take), at most about 256 MB: 850 KB a row, 109 MB a handle
+ * at hidden 2048, inter 1536, slots 5. */
 int  glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_moe **out);
 void glmflash_moe_free(glmflash_moe *m);
 /* group -> routed and shared experts -> combine:
