@@ -269,6 +269,10 @@ __device__ __forceinline__ void mma1688(float (&d)[4], uint32_t a0, uint32_t a1,
         : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// The launch counter that words and flags in global memory carry, one up.  They start zeroed, so after 2^32 launches 0 is left out: it
+// would pass for a word that was never written.  2 follows, which keeps the turns of buffers that alternate with the counter's parity.
+__device__ __forceinline__ unsigned next_epoch(unsigned e) { return e == 0xffffffffu ? 2u : e + 1u; }
+
 // Device status word shared by kernels with bounded waits: 0 = fine, otherwise the first failure code.
 enum : int { GF_STATUS_OK = 0, GF_STATUS_TMA_TIMEOUT = 1, GF_STATUS_TMEM = 2, GF_STATUS_MMA_TIMEOUT = 3, GF_STATUS_PEER_TIMEOUT = 4 };
 

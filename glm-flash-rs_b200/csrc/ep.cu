@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(EP_THREADS) ep_combine_kernel(const float *__r
     const int r = blockIdx.y;
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    const unsigned epoch = *epoch_ptr + 1u;                   // every CTA reads it before the last one advances it
+    const unsigned epoch = next_epoch(*epoch_ptr);                   // every CTA reads it before the last one advances it
     const unsigned par = epoch & 1u;
     const size_t slot_elems = (size_t)max_rows * H;
     if (d < H) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(EP_THREADS) ep_combine_ll_kernel(const float *
     if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
     const int r = blockIdx.y;
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    const unsigned epoch = *epoch_ptr + 1u;                   // every CTA reads it before the last one advances it
+    const unsigned epoch = next_epoch(*epoch_ptr);                   // every CTA reads it before the last one advances it
     const unsigned par = epoch & 1u;
     const size_t slot_words = (size_t)max_rows * H;
     if (d < H) {
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(EP_THREADS, 4) ep_exchange_rows_kernel(const f
     pdl_launch_dependents();
     __shared__ int ok_sh;
     const int chunk = blockIdx.x, r0 = chunk * EP_RB, r1 = min(r0 + EP_RB, rows);
-    const unsigned epoch = *epoch_ptr + 1u;
+    const unsigned epoch = next_epoch(*epoch_ptr);
     const unsigned par = epoch & 1u;
     const size_t slot_elems = (size_t)max_rows * H;
     const int chunks = (rows + EP_RB - 1) / EP_RB, per = (chunks + world - 1) / world;

@@ -460,7 +460,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     int drawn = 0;
     if (tid == ST_PROD * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
     if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
-    const uint32_t epoch = __ldcg(a.ctrl + CTRL_EPOCH) + 1u;          // words of earlier launches carry smaller ones
+    const uint32_t epoch = next_epoch(__ldcg(a.ctrl + CTRL_EPOCH));   // words of earlier launches carry others
     const int U = MANY ? st_build_tables_many(a, tb) : st_build_tables(a, tb, used_sh, row, slot);
     if (tid == ST_FIN * 32) first_sh = drawn;
     __syncthreads();

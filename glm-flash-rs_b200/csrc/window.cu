@@ -876,9 +876,9 @@ __global__ void __launch_bounds__(WIN_THREADS, 1) window_kernel(const __grid_con
     pdl_launch_dependents();
     pdl_wait();                                   // the routing table and the layer input may belong to the kernel before
     WIN_STAMP(1);
-    const unsigned epoch = __ldcg(a.sync) + 1u;
+    const unsigned epoch = next_epoch(__ldcg(a.sync));
     // the exchange counts on its own: every rank advances it once per exchange, whichever owners computed the layers
-    const unsigned xepoch = a.peers.world > 1 ? __ldcg(a.peers.epoch) + 1u : 0u;
+    const unsigned xepoch = a.peers.world > 1 ? next_epoch(__ldcg(a.peers.epoch)) : 0u;
 
     // ---- grouping (native/grouping.cu:67-100 semantics): distinct experts computed here in ascending id order, their
     //      members in ascending row order.  A pick that repeats an earlier slot of its row names nothing.

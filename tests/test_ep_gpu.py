@@ -188,6 +188,24 @@ def test_two_step_exchange_of_a_large_window_on_one_gpu(pkg, synth, cuda, bf16):
             assert not torch.allclose(got[:32], plain[:32], rtol=0, atol=1e-4)       # the rounding really happened
 
 
+def test_exchange_counter_wraps(pkg, synth, cuda):
+    """The counter that the exchange words and flags carry leaves out 0, which zeroed words have, and keeps alternating."""
+    import torch
+    from glmflash_b200 import _view
+    for rows in (4, 32):
+        ep = pkg.EpCombine(pkg.make_config(H, I, E, S, max_rows=rows), 0, 1, None)
+        picks, rw = synth.route(25, rows, E, S - 1)
+        pd, wd = torch.from_numpy(picks).to(cuda), torch.from_numpy(rw).to(cuda)
+        Y = torch.randn((rows * S, H), dtype=torch.float32, device=cuda)
+        counter = _view(ep.status.data_ptr() - 8, (1,), torch.int32)
+        counter.fill_(-2)
+        for epoch in (-1, 2, 3):
+            got = ep.combine(C_void(Y), pd, wd, rows, True)
+            torch.cuda.synchronize()
+            assert int(ep.status.cpu()[0]) == 0 and int(counter.cpu()[0]) == epoch
+            assert torch.allclose(got, (wd[:, :, None] * Y.view(rows, S, H)).sum(1), rtol=1e-5, atol=1e-5)
+
+
 def C_void(t):
     import ctypes
     return ctypes.c_void_p(t.data_ptr())

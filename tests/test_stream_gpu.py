@@ -87,3 +87,33 @@ def test_window_without_experts_and_repeated_picks(pkg, oracle, synth, cuda, row
     Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, again, mode=1)
     want = oracle.combine(Y, rw2, rows, S, H)
     assert rel_err(got, want)[0] < TOL
+
+
+def test_launch_counter_wraps(pkg, oracle, synth, cuda):
+    # The counter that the exchange words carry starts at 0 like the words themselves: 0 must never come round.  Rows 1..3 are first used
+    # in the launch after 2^32 - 1, on words that were never written.
+    import torch
+    from glmflash_b200 import _view
+    H, I, E, S, rows = 256, 256, 5, 3, 4
+    bank = synth.expert_bank(71, H, I, E, svh_scale=True)
+    dbank = synth.to_device(bank, cuda)
+    x, (picks, rw) = synth.activations_bf16(72, rows, H), synth.route(73, rows, E, S - 1)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd, pd, wd = t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw)
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=rows))
+    for _ in range(3):
+        moe.run(dbank, xd[:1], pd[:1], wd[:1], 1)
+    # the owner's allocation: status (256 bytes), the four areas of 8-byte words (one split of k each here), the counters
+    up = lambda n: (n + 255) // 256 * 256
+    at = 256 + sum(up(8 * rows * S * n) for n in (2 * I, H, H, I // 2)) + 384 * 4
+    torch.cuda.synchronize()
+    counter = _view(moe.status.data_ptr() + at, (1,), torch.int32)
+    assert int(counter.cpu()[0]) == 3
+    counter.fill_(-2)                                        # 2^32 - 2 launches
+    want = oracle.combine(oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1), rw, rows, S, H)
+    for n, epoch in ((1, -1), (rows, 2), (rows, 3), (2, 4)):
+        moe.output.fill_(0)
+        moe.run(dbank, xd[:n], pd[:n], wd[:n], n)
+        torch.cuda.synchronize()
+        assert int(moe.status.cpu()[0]) == 0 and int(counter.cpu()[0]) == epoch
+        assert rel_err(moe.output[:n].cpu().numpy(), want[:n])[0] < TOL
