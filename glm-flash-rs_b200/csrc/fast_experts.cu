@@ -793,7 +793,7 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
             return -1;
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)
-        if (launch_k(fast_rot_kernel, dim3((unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 148L * 32)), dim3(256), 0, s, pdl,
+        if (launch_k(fast_rot_kernel, dim3((unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 32L * f->sms)), dim3(256), 0, s, pdl,
             (const __nv_bfloat16 *)input, x_stride, f->plan, f->src_pair, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg,
             f->xu, H, c.slots, mats, (((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 16 == 0 && x_stride % 8 == 0)))
             return -1;

@@ -170,18 +170,21 @@ __global__ void __launch_bounds__(256) route_kernel(const __nv_bfloat16 *__restr
 
 static int launch_route(cudaStream_t s, const uint16_t *x, int x_stride, const uint16_t *wr, int rows, int H, int E, int topk, float *logits,
                         int *picks, float *weights, bool pdl) {
-    // Rows per CTA: 32 once 16 would give more CTAs than the SMs hold side by side (the matrix is read once per CTA).  Clusters of
-    // 8 along K while the rows fill less than an eighth of the GPU.
-    const bool wide = rows > 2368;
-    const int tiles = wide ? (rows + 31) / 32 : (rows + 15) / 16, cn = tiles * 8 <= 148 && H >= 512 ? 8 : 1;
-    const size_t smem = (size_t)9 * (wide ? 32 : 16) * RT_ST * sizeof(float);
-    static bool configured[64] = {};
+    static int sms[64] = {};                       // (threads that come here together set the same)
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
-    if (!configured[dev & 63]) {
+    GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
+    if (!sms[dev]) {
+        int n = 0;
+        GF_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         GF_CUDA(cudaFuncSetAttribute(route_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * 32 * RT_ST * (int)sizeof(float)));
-        configured[dev & 63] = true;
+        sms[dev] = n;
     }
+    // Rows per CTA: 32 once 16 would give more CTAs than there are SMs (the matrix is read once per CTA).  Clusters of 8 along K
+    // while the rows fill less than an eighth of the GPU.
+    const bool wide = rows > 16 * sms[dev];
+    const int tiles = wide ? (rows + 31) / 32 : (rows + 15) / 16, cn = tiles * 8 <= sms[dev] && H >= 512 ? 8 : 1;
+    const size_t smem = (size_t)9 * (wide ? 32 : 16) * RT_ST * sizeof(float);
     const dim3 grid((unsigned)(tiles * cn)), block(256), cluster((unsigned)cn);
     const __nv_bfloat16 *xb = (const __nv_bfloat16 *)x, *wb = (const __nv_bfloat16 *)wr;
     return wide ? launch_kc(route_kernel<2>, grid, block, cluster, smem, s, pdl, xb, x_stride, wb, rows, H, E, topk, logits, picks, weights)
