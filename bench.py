@@ -49,7 +49,8 @@ H, I, E, S = 2048, 1536, 64, 5
 MAT_BYTES = H * I // 2                                     # packed bytes of one matrix
 W_E = 3 * MAT_BYTES + (2 * H + 2 * I + I + H) * 2          # 4,740,096 B: one expert's matrices + its six scale vectors
 GATEUP_BYTES_E = 2 * MAT_BYTES + (2 * H + 3 * I) * 2       # what the gate/up kernel reads per expert (algorithmic)
-INSTRUCTION_CEILING_GBS = 3800.0                           # packed bytes/s at one decode instruction per cycle and scheduler
+INSTRUCTION_CEILING_GBS = 3800.0                           # packed bytes/s at one decode instruction per cycle and scheduler; the pipes
+                                                           # sustain 2,500 in a loop of nothing else (profiles/trellis_decode_cost.md)
 
 
 def peaks():
@@ -85,7 +86,7 @@ def recorded_traffic(key, path=None):
     return float(rec["traffic_bytes"])
 
 
-TRAFFIC_SOURCES = {"gemv": "glm-flash-rs_b200/csrc/gemv.cuh", "window": "glm-flash-rs_b200/csrc/window.cu",
+TRAFFIC_SOURCES = {"stream": "glm-flash-rs_b200/csrc/stream.cu", "gemv": "glm-flash-rs_b200/csrc/gemv.cuh", "window": "glm-flash-rs_b200/csrc/window.cu",
                    "fast": "glm-flash-rs_b200/csrc/fast_experts.cu"}
 
 
@@ -417,9 +418,10 @@ class Bench:
             res["roofline"] = {"bound": "hbm", "kernel": "stream_kernel, gate/up units alone (grouping + input rotation + grouped GEMV + SwiGLU epilogue)",
                                "achieved": gbs, "peak": self.peaks["hbm_gbs"], "peak_source": self.peaks["source"] + " hbm_gbs", "unit": "GB/s",
                                "frac": gbs / self.peaks["hbm_gbs"], "us_per_launch": ms_pass / L * 1e3, "algorithmic_bytes_per_launch": gu_bytes,
-                               "distinct_experts_per_layer": distinct, "traffic": recorded_traffic(f"gemv_gateup_rows{rows}"),
+                               "distinct_experts_per_layer": distinct, "traffic": recorded_traffic(f"stream_gateup_rows{rows}"),
                                "instruction_ceiling_gbs": INSTRUCTION_CEILING_GBS, "frac_of_instruction_ceiling": gbs / INSTRUCTION_CEILING_GBS,
                                "layer": {"algorithmic_bytes": layer_bytes, "us": ms_step / L * 1e3, "gbs": lgbs, "frac": lgbs / self.peaks["hbm_gbs"],
+                                         "traffic": recorded_traffic(f"stream_layer_rows{rows}"),
                                          "frac_of_instruction_ceiling": lgbs / INSTRUCTION_CEILING_GBS}}
         else:
             res["distinct_experts_per_layer"] = distinct

@@ -543,7 +543,7 @@ def topk(logits, picks, weights, stream=None, pdl=1):
 
 
 def route(x, wr, logits, picks, weights, stream=None, pdl=1):
-    """router_logits + topk; one launch for windows of <= 16 rows."""
+    """router_logits + topk in one launch, for any number of rows."""
     rows, E = logits.shape
     _check(lib().glmflash_route(_stream_ptr(stream), x.data_ptr(), x.stride(0), wr.data_ptr(), rows, wr.shape[1], E,
                                 picks.shape[1] - 1, logits.data_ptr(), picks.data_ptr(), weights.data_ptr(), pdl))

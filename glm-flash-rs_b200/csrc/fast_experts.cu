@@ -29,8 +29,8 @@
 //             construction.  Down is one pass per item, alternating the two accumulator halves.
 //             What bounds it: with one CTA per tile pair (M 128 x N 128 instructions) the operand reads of the MMAs alone filled
 //             shared memory (128 bytes a clock); the pair halves them.  What is left is the loop from a stage's release to its
-//             next use (decode store, relay, issue, commit) and the decode itself: 4096 tokens, gate/up 407 -> 350 us, of which
-//             256 us remain without decode and epilogue arithmetic.
+//             next use (decode store, relay, issue, commit) and the decode itself: 4096 tokens, gate/up 407 -> 358 us, of which
+//             249 us remain without decode and epilogue arithmetic.
 // Arithmetic: one full-K fp32 accumulation chain per output (as upstream's prefill path, which is likewise not
 // bit-equal to its decode path: native/exl3_prefill.cu:20-23), the same transforms and rounding points as
 // upstream's epilogue (native/exl3_prefill.cu:596-622 == native/exl3.cu:260-321) with exp / divide in their fast

@@ -19,9 +19,9 @@ int *fast_experts_status_word(glmflash_fast_experts *f);
 // out[r][d] = sum_{s < slots-1, expert computed here} w[r][s] * Y[r*slots+s][d]  (+ Y[shared pair] if computed here)
 // fp32, ascending slot order, shared last: the order of the oracle's combine.
 __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ Y, const int *__restrict__ picks,
-                                                      const float *__restrict__ route_w, float *__restrict__ out, int rows,
-                                                      int slots, int H, int E, int shared_exl3, int e_lo, int e_hi,
-                                                      int srow_lo, int srow_hi) {
+                                                      const float *__restrict__ route_w, float *__restrict__ out, int slots,
+                                                      int H, int E, int shared_exl3, int e_lo, int e_hi, int srow_lo,
+                                                      int srow_hi) {
     // Launched behind the down GEMM only.  That kernel, like the grouping, plan, rotation and gate / up kernels in front of it, runs
     // its own pdl_wait before it triggers, so when this one starts, everything in front of the down GEMM has completed, the
     // router's table and weights among it: they are read ahead of the wait.  Only the pair results Y belong to the kernel in front.
@@ -29,8 +29,6 @@ __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ 
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     __shared__ float wgt_sh[32];
     __shared__ uint32_t live_sh;
-    __shared__ uint32_t used_sh[32];
-    if (shared_exl3 == 2) shared_exl3 = shared_owner_of_window(picks, rows * slots, E, e_hi - e_lo, used_sh) == e_lo / (e_hi - e_lo);
     if (threadIdx.x < 32) {
         const int s = threadIdx.x;
         bool keep = false;
@@ -90,8 +88,8 @@ __global__ void __launch_bounds__(256) rank_sum_kernel(const float *__restrict__
 int launch_combine(cudaStream_t s, const float *Y, const int *picks, const float *route_w, float *out, int rows,
                    const glmflash_config &c) {
     const dim3 grid((unsigned)((c.hidden / 4 + 255) / 256), (unsigned)rows);
-    return launch_k(combine_kernel, grid, dim3(256), 0, s, c.pdl != 0, Y, picks, route_w, out, rows, c.slots, c.hidden,
-                    c.experts, c.shared_exl3, c.expert_lo, c.expert_hi, c.shared_row_lo, c.shared_row_hi);
+    return launch_k(combine_kernel, grid, dim3(256), 0, s, c.pdl != 0, Y, picks, route_w, out, c.slots, c.hidden, c.experts,
+                     c.shared_exl3, c.expert_lo, c.expert_hi, c.shared_row_lo, c.shared_row_hi);
 }
 }  // namespace gf
 

@@ -12,7 +12,7 @@ struct glmflash_experts {
     unsigned *ctrl = nullptr;
     float *y = nullptr;                                   // pair results [P][H] (public; not of a chunk owner)
     int *status = nullptr;
-    int phases = 7;                                       // profiling aid: 1 = input rotation, 2 = gate/up, 4 = down
+    int phases = 7;                                       // profiling aid: 2 = rotation and gate/up, 4 = down (1 selects nothing)
     // one-launch layer kernel (window.cu): split partials, arrival counters / ready words, layer output
     float *z1 = nullptr, *z2 = nullptr;                   // split partials [2][H/128][P][I], [I/128][P][H]
     unsigned *sync = nullptr;

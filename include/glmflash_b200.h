@@ -288,8 +288,7 @@ int glmflash_router_logits(void *stream, const uint16_t *x, int x_stride, const 
  * weight 1.  picks int32 [rows][topk + 1], weights fp32 [rows][topk + 1]: the routing table glmflash_moe_run takes. */
 int glmflash_topk(void *stream, const float *logits, int rows, int experts, int topk, int32_t *picks, float *weights,
                   int pdl);
-/* Both steps: windows of <= 16 rows take ONE launch (a CTA per row computes the row's logits and selects), larger
- * windows the two kernels above.  logits (fp32 [rows][experts], caller's) receives the logits in both cases. */
+/* Both steps in ONE launch, for any number of rows.  logits (fp32 [rows][experts], caller's) receives the logits. */
 int glmflash_route(void *stream, const uint16_t *x, int x_stride, const uint16_t *wr, int rows, int hidden, int experts,
                    int topk, float *logits, int32_t *picks, float *weights, int pdl);
 

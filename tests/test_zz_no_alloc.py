@@ -2,9 +2,8 @@
 
 Collected last on purpose: a run that stops at the first failure has then already run every other test.  Some
 hosts cannot let a library allocate device memory (they own the whole heap, or an allocator call would stall their
-serving streams); for them the library carries its scratch as a built-in array.  The two entry points run the same
-kernels, so their outputs must be identical bit for bit -- on the first call, and on a second call with other
-inputs that finds the previous call's leftovers in the shared array."""
+serving streams).  Both entry points run the same kernel, which needs no scratch, so their outputs must be identical
+bit for bit -- on the first call, and on a second call with other inputs."""
 import ctypes as C
 
 import numpy as np
