@@ -116,11 +116,11 @@ __device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long lon
     return true;
 }
 
-// v += the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the epoch.  LAST:
-// between the attempts only the last of the four is polled; it is mostly the last to come (9 and more rows: polls of all four cost
-// the decode warps issue slots; for fewer rows the extra round trip costs more, 47 layers of one token 1113 -> 1144 us).
-template <bool LAST>
-__device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
+// v += the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the epoch.
+// last_only: between the attempts only the last of the four is polled; it is mostly the last to come.  With two CTAs an SM polls of all
+// four cost the decode warps issue slots (8 rows 60.3 -> 59.5 us a layer); with one the extra round trip costs more (47 layers of
+// one token 1113 -> 1144 us).
+__device__ __forceinline__ bool sum_splits(bool last_only, const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
                                            float (&v)[4]) {
     z += (size_t)lo * split_stride;
 #pragma unroll 1
@@ -143,7 +143,7 @@ __device__ __forceinline__ bool sum_splits(const StCta &c, const unsigned long l
             if (!__all_sync(0xffffffffu, c.again(n))) return false;
             __nanosleep(20);
             unsigned long long last[4];
-            if (LAST && !ll_wait4(c, z + (size_t)(min(hi - lo, 4) - 1) * split_stride, epoch, last)) return false;
+            if (last_only && !ll_wait4(c, z + (size_t)(min(hi - lo, 4) - 1) * split_stride, epoch, last)) return false;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -554,7 +554,8 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             unsigned char *xs = xbuf + s * XBYTES + 16 * part;
             const bool poll = kind == UNIT_G || a.do_g;               // (the down phase alone takes what the last run left)
             bool ok = true;
-            for (int t0 = xw; t0 < nmem; t0 += 2 * ST_XW) {
+            // (the warps start in turn: most experts have a member or two; 8 rows 59.5 -> 59.1 us a layer with the polls above)
+            for (int t0 = (xw + ST_XW - (int)(it % ST_XW)) % ST_XW; t0 < nmem; t0 += 2 * ST_XW) {
                 unsigned long long w[2][4];
                 int m[2];
 #pragma unroll
@@ -601,16 +602,16 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                 const uint2 sd = ldg_half4(a.suh_d + so, a.vec);
                 float v[4] = {0.f, 0.f, 0.f, 0.f};
                 const unsigned long long *z = a.z1 + ((size_t)role * SK1 * P + p) * I + nb * 128 + z_word(lane);
-                if (SETS == 2) {
-                    // With more than 8 rows up to eight finish warps an SM are always waiting, and their polls cost the decode warps issue
-                    // slots: only warp 3 polls, for the partial that is drawn last (16 rows: 695 -> 671 us over 8 layers; for one row the
-                    // extra round trip costs more, 47 layers 1128 -> 1141 us).
+                if (a.two) {
+                    // With two CTAs an SM eight finish warps are always waiting, and their polls cost the decode warps issue slots: only
+                    // warp 3 polls, for the partial that is drawn last (16 rows: 695 -> 671 us over 8 layers; with one CTA the extra
+                    // round trip costs more, 47 layers of one row 1128 -> 1141 us).
                     unsigned long long last[4];
                     if (fw == 3) ll_wait4(cta, z + (size_t)(SK1 - 1) * P * I, epoch, last);
                     asm volatile("bar.sync 5, 128;" ::: "memory");
                 }
                 if (!half) {
-                    sum_splits<SETS == 2>(cta, z, (size_t)P * I, 0, SK1, epoch, v);
+                    sum_splits(a.two, cta, z, (size_t)P * I, 0, SK1, epoch, v);
                     z_columns(v, lane);
                     fwht128(v, lane);
                     const float2 c01 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.x)), c23 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.y));
@@ -659,7 +660,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0)
-                            sum_splits<SETS == 2>(cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + nb * 128 + z_word(lane), (size_t)P * H, 0, SK2, epoch, v[i]);
+                            sum_splits(a.two, cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + nb * 128 + z_word(lane), (size_t)P * H, 0, SK2, epoch, v[i]);
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0) {
@@ -756,7 +757,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     }
 }
 
-int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
+int launch_stream(cudaStream_t s, StreamArgs a, bool pdl) {
     static int sms[64] = {};
     static bool configured[64][5] = {};
     int dev = 0;
@@ -774,12 +775,14 @@ int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl) {
                                      : stream_kernel<1, false, 2>;
     size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
     GF_REQUIRE(smem <= ST_MAX_SMEM, "routing table too large for the window kernel");
-    // CTAs per SM.  One has shorter chains for few units (one token: 24.4 us a layer against 28.6 with two); two fill the decode
-    // pipes (16 rows: 85 against 95 us).  The lines cross at about 16 units per SM, counted with one expert per pick of this GPU's
-    // window (2,160 units: 37.8 | 38.7 us, 2,880: 44.5 | 43.6).
+    // CTAs per SM.  One has shorter chains for few units (one token: 23.8 us a layer, 28.6 with two); two fill the decode pipes (16
+    // rows: 80 against 95 us).  The lines cross at about nine units of 512 k per SM, counted with one expert per pick of this GPU's
+    // window (us with one | two; 2048 x 1536, 2 rows, 9.7 units: 34.2 | 33.2; 3 rows, 14.6: 42.1 | 38.9; 2304 x 768, 2 rows, 6.5: 26.0 |
+    // 26.4; 1024 x 2048, 3 rows, 7.8: 24.9 | 26.7).
     const long pairs = (long)a.rows * (((long)(a.slots - 1) * (a.e_hi - a.e_lo) + a.E - 1) / a.E + (a.shared ? 1 : 0));
     const long units = std::min<long>(pairs, a.umax) * (2L * ((a.H + 511) / 512) * (a.I / 128) + (long)((a.I + 511) / 512) * (a.H / 128));
-    const int per_sm = units >= 16L * sms[dev] ? 2 : 1;
+    const int per_sm = units >= 9L * sms[dev] ? 2 : 1;
+    a.two = per_sm == 2;
     const dim3 grid((unsigned)(sms[dev] * per_sm)), block(ST_THREADS);
     // One CTA per SM asks for more than half of the shared memory: next to a few CTAs of another kernel (the router of the next
     // layer) the second CTA of an emptier SM was placed before the first of a busier one (8 layers of one token with their

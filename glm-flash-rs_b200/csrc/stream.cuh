@@ -43,6 +43,7 @@ struct StreamArgs {
     StreamCut cut1, cut2;                                    // of the gate / up and the down matrix
     float limit;
     int vec;                                                 // the scale vectors are 8-byte aligned
+    int two;                                                 // two CTAs share an SM (set by launch_stream)
     int do_g, do_d;                                          // profiling aid: the phases to run
 };
 
@@ -63,6 +64,6 @@ inline size_t stream_xdl_words(const glmflash_config &c) { return (size_t)c.max_
 
 // Most rows of a chunk that the kernel takes (its tables live in shared memory and its exchange areas grow with the rows).
 constexpr int ST_MAX_ROWS = 128;
-int launch_stream(cudaStream_t s, const StreamArgs &a, bool pdl);
+int launch_stream(cudaStream_t s, StreamArgs a, bool pdl);
 
 }  // namespace gf
