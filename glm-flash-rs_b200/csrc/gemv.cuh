@@ -8,13 +8,13 @@
 //     16-byte slot of four consecutive k-tiles.
 //   * states are cut with funnel shifts in pairs (state_j << 16 | state_{j+4}), multiplied by the codebook constant, masked, and the
 //     two fp16 halves of a codeword are added by one HADD2: exactly upstream's fp16 weight (bit-exact decode).
-//   * pairs of weights are packed into the A operand of mma.m16n8k8 (rows = 16 output columns); the k slots of the instruction
-//     are whatever k the lane holds, and the B operand (members, eight per set) is read to match.  fp32 accumulation; a member's
-//     column depends on its own activations only.  An instruction adds eight products to the accumulator and rounds, which fixes the
-//     bits of a sum: m16n8k16 over every weight duplicated (a doubled K whose other half is zero) has the same ones, m16n8k16 over
-//     sixteen packed weights has not.
-// A loop of nothing else runs 19.1 weights per clock and SM with sixteen packed products an instruction, against 17.4 with every
-// weight duplicated over a doubled K; eight packed products cost the layer kernels up to 2 % of the former.
+//   * pairs of weights are packed into the A operand of mma.m16n8k8 or m16n8k16 (rows = 16 output columns); the k slots of the
+//     instruction are whatever k the lane holds, and the B operand (members, eight per set) is read to match.  fp32 accumulation; a
+//     member's column depends on its own activations only.
+// An instruction adds its products to the accumulator and rounds, so their number is part of a sum's bits.  Windows of up to 16 rows add
+// eight (m16n8k8 has the bits of m16n8k16 over every weight duplicated, a doubled K whose other half is zero, which their kernels
+// once ran); the single linear and chunks of more rows add sixteen: half as many roundings, up to 2 % faster (a chunk of 40 rows
+// 174 -> 171 us).  A loop of nothing else runs 19.1 weights per clock and SM with sixteen, 17.4 with every weight duplicated.
 #pragma once
 #include "common.cuh"
 #include "tensor_map.cuh"
@@ -74,8 +74,8 @@ inline int bank_map(CUtensorMap *map, const uint32_t *bank, int experts, int K, 
 
 // ---- decode: one stage (256 k of one matrix and 128 columns) by eight warps ------------------------------------------
 // words: the stage; x: the members' activations of its 256 k; warp = n-tile.  acc[s] += columns G, G + 8 of members 8 s + 2 T, + 1.
-// ROUNDS: 2, or 1 for a stage of 128 k.
-template <int SETS, int ROUNDS = 2>
+// ROUNDS: 2, or 1 for a stage of 128 k.  WIDE: sixteen products an instruction instead of eight.
+template <int SETS, bool WIDE, int ROUNDS = 2>
 __device__ __forceinline__ void st_decode(const unsigned char *words, const unsigned char *x, int warp, int lane, float (&acc)[SETS][4]) {
     const int G = lane >> 2, T = lane & 3;
     // row (n-tile, k-tile) of 128 bytes; its 16-byte chunk c sits at c ^ (k-tile & 7): k-tiles T and 4 + T of a pair of groups
@@ -106,16 +106,21 @@ __device__ __forceinline__ void st_decode(const unsigned char *words, const unsi
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const uint32_t pw = t == 0 ? before[q] : w[t - 1];
+                uint32_t af[4];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     uint32_t hi[2], lo[2];
                     codeword_pair(__funnelshift_r(w[t], pw, h ? 4 : 12), hi[0], lo[0]);         // k = 2t + 8h:     columns G, G + 8
                     codeword_pair(h ? w[t] : __funnelshift_r(w[t], pw, 8), hi[1], lo[1]);       // k = 2t + 8h + 1
-                    const uint32_t a0 = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410),
-                                   a1 = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
+                    af[2 * h] = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410);
+                    af[2 * h + 1] = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
+                    if (!WIDE)
 #pragma unroll
-                    for (int s = 0; s < SETS; ++s) mma1688(acc[s], a0, a1, h ? b1[s][t] : b0[s][t]);
+                        for (int s = 0; s < SETS; ++s) mma1688(acc[s], af[2 * h], af[2 * h + 1], h ? b1[s][t] : b0[s][t]);
                 }
+                if (WIDE)
+#pragma unroll
+                    for (int s = 0; s < SETS; ++s) mma16816(acc[s], af, b0[s][t], b1[s][t]);
             }
         }
     }

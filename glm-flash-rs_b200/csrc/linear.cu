@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_kernel(const __grid_consta
         for (int c = 0; c < 4; ++c) acc[s][c] = 0.f;
     for (int i = 0; i < stages; ++i)
         if (__all_sync(0xffffffffu, mbar_wait(bars + i, 0)))                                 // (bounded; a copy that never lands leaves the sum short)
-            st_decode<SETS>(words + (size_t)i * ST_WBYTES, xbuf + (size_t)i * XBYTES, warp, lane, acc);
+            st_decode<SETS, true>(words + (size_t)i * ST_WBYTES, xbuf + (size_t)i * XBYTES, warp, lane, acc);
     const int G = lane >> 2, T = lane & 3;
 #pragma unroll
     for (int s = 0; s < SETS; ++s) {

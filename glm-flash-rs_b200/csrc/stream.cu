@@ -10,7 +10,7 @@
 // (16 KB, 32,768 weights).  A CTA (512 threads) has four roles:
 //   warps 0-7   decode: warp = n-tile.  A lane reads 16 bytes (4 words of one tile: all 16 k of columns G and G + 8) with
 //               one LDS.128, cuts the states in pairs with funnel shifts, forms the weights exactly as upstream does (fp16
-//               sum of the codeword halves) and packs them into A operands of mma.m16n8k8; members are the N dimension
+//               sum of the codeword halves) and packs them into A operands of mma.m16n8k8 (chunks: k16); members are the N dimension
 //               (8 per set, two sets for 9..16 rows), fp32 accumulation over the split.
 //   warps 8-10  X: put the members' activations of a stage's k range into shared memory as soon as they are there: rotated layer
 //               inputs (gate / up) or the finished rows of the gate / up phase (down).
@@ -28,8 +28,8 @@
 // and everything that a later unit or job waits for has been drawn by a CTA that runs: the launch makes progress with any
 // number of resident CTAs, next to any other kernel (no co-residency is assumed).
 //
-// Sums have a fixed order that does not depend on the window: eight products an instruction, the k-tiles of a split in order, the
-// splits ascending.  A row has the bits of its 1-row call, and of the cluster kernels that this one replaced.  With sixteen products
+// The sums of a window of up to 16 rows have a fixed order that does not depend on it: eight products an instruction, the k-tiles of a
+// split in order, the splits ascending.  A row has the bits of its 1-row call, and of the cluster kernels that this one replaced.  With sixteen products
 // an instruction, 512 k a split and half as many partials, the sums were as far from 64-bit ones (6.3e-7 against 6.2e-7 of a down
 // row at K = 1536; 47 layers of one token 1142 us against 1101 now), but other bits: now and then a bf16 rounding behind them fell the
 // other way, and a one-row layer moved by up to 1e-3.
@@ -520,8 +520,8 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             const unsigned char *ws = words + s * SBYTES, *xs = xbuf + s * XBYTES;
             // (few experts of a window or chunk have more than eight members; with the second set's operand loads in every
             // unit, eleven rows of the 4096 x 512 layer took 115 us instead of 107 and a chunk of 40 192 instead of 180)
-            if (SETS == 1 || nmem <= 8) st_decode<1, ROUNDS>(ws, xs, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
-            else st_decode<SETS, ROUNDS>(ws, xs, warp, lane, acc);
+            if (SETS == 1 || nmem <= 8) st_decode<1, MANY, ROUNDS>(ws, xs, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
+            else st_decode<SETS, MANY, ROUNDS>(ws, xs, warp, lane, acc);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + s);
             if (!(d.x & DESC_LAST)) continue;

@@ -13,8 +13,9 @@ struct StreamCut {
     int split, splits;                                       // k-tiles of a split, number of splits
 };
 // Windows of up to 16 rows: at most eight splits, 256 k each where that suffices, else the next power of two that divides K, else the
-// largest number of equal splits of whole 128-k blocks (K = 2304: six of 384).  A K that has no such split of at most 1024 k, and
-// chunks of more than 16 rows, are cut into 512 k: half the exchange, which for chunks is what grows with the rows.
+// largest number of equal splits of whole 128-k blocks (K = 2304: six of 384).  A K that has no such split of at most 1024 k (3328) is
+// cut into 256 k.  Chunks of more than 16 rows are cut into 512 k: half the exchange, which grows with the rows, and with sixteen
+// products an instruction as many roundings a partial as 256 k have with eight.
 inline StreamCut stream_cut(int K, bool chunk) {
     const int KT = K / 16;
     StreamCut c{16, 0};
@@ -22,7 +23,8 @@ inline StreamCut stream_cut(int K, bool chunk) {
     if (KT % c.split)
         for (int n = 8; n >= 1; --n)
             if (KT % n == 0 && KT / n % 8 == 0) { c.split = KT / n; break; }
-    if (chunk || c.split > 64) c.split = 32;
+    if (c.split > 64) c.split = 16;
+    if (chunk) c.split = 32;
     c.splits = (KT + c.split - 1) / c.split;
     return c;
 }

@@ -22,7 +22,8 @@ def run(pkg, cuda, bank, x, picks, rw, H, I, E, S, rows, synth, max_rows=None, *
 
 
 @pytest.mark.parametrize("H,I,E,S,rows", [(256, 256, 3, 2, 1), (768, 256, 5, 3, 7), (512, 1280, 9, 4, 16), (2304, 768, 8, 5, 9),
-                                          (1024, 512, 40, 32, 16), (256, 768, 1, 2, 8)])
+                                          (1024, 512, 40, 32, 16), (256, 768, 1, 2, 8),
+                                          (3328, 256, 3, 2, 3), (256, 3328, 3, 2, 10)])
 def test_edges_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows):
     bank = synth.expert_bank(31 + H + I, H, I, E, svh_scale=True)
     x, (picks, rw) = synth.activations_bf16(32, rows, H), synth.route(33, rows, E, S - 1, shared_bias=rows > 1)
