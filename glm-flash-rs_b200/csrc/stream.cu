@@ -176,7 +176,7 @@ struct StTables {
     uint32_t *rows_of;                   // [E + 1][words] rows that picked the expert, a bit each
     int words;
 };
-constexpr int ST_META = 1024;            // barriers and descriptors
+constexpr int ST_META = 512;             // barriers and descriptors
 inline size_t st_smem_bytes(int sets, int umax, int rows, int P, int E) {
     const size_t tables = (size_t)(3 * umax + 1) * 4 + (size_t)umax * 32 + (size_t)P * 2 + 64 +
                           (rows > 16 ? (size_t)(E + 1) * 4 * (1 + (rows + 31) / 32) : 0);
