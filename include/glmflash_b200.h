@@ -114,7 +114,9 @@ const int32_t *glmflash_grouping_members(const glmflash_grouping *g);
 
 /* ---- ExpertGpu: decode / verify windows of 1..16 rows  (src/experts.rs:365-563) --------------------- */
 typedef struct glmflash_experts glmflash_experts;
-/* ExpertGpu::new_rows(d, native, max_rows); max_rows in 1..16 (src/experts.rs:391-394). */
+/* ExpertGpu::new_rows(d, native, max_rows); max_rows in 1..16 (src/experts.rs:391-394).  The handle holds, for each row, exchange
+ * words of 8 slots (2 n(hidden) inter + n(inter) hidden + hidden + inter / 2) bytes, n(K) the number of partial sums that K is cut
+ * into (K / 256, at most eight): 1.6 MB at hidden 2048, inter 1536, slots 5. */
 int  glmflash_experts_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_experts **out);
 void glmflash_experts_free(glmflash_experts *e);
 /* ExpertGpu::run_rows(stream, .., input, picks, ids, count, members, rows, maxm).  input: bf16
