@@ -5,32 +5,37 @@
 // fast_down_large (native/exl3_prefill.cu:402-430,657-889), which decode each 16x16 trellis tile into mma.sync
 // fragments in registers.  Here:
 //
-//   plan      members per distinct expert, chunks of at most 256 rows (as even as an expert's rows go, long ones first) and the
+//   plan      members per distinct expert, chunks of at most 320 rows (as even as an expert's rows go, long ones first) and the
 //             GROUPED row order (rows of an expert contiguous): src_pair[j] = pair index of grouped row j.
-//   rot       the input rotation writes Xs[j] = fp16(H(x[row] * suh[e]) / sqrt 128) in grouped order, so the A operand of a chunk is
+//   rot       the input rotation writes Xs[j] = fp16(H(x[row] * suh[e]) / sqrt 128) in grouped order, so the rows of a chunk are
 //             a contiguous slab that TMA tensor loads bring into shared memory in the 128-byte-swizzled K-major layout the tensor
 //             core reads.
 //   gemm      persistent PAIRS of CTAs (74 clusters of two), one CTA per SM, 28 warps.  A work item is (chunk, pair of 128-column
-//             blocks): tcgen05.mma.cta_group::2, M 256 x N 256 x K 16 -- each CTA brings half of the rows and decodes ONE of the two
-//             column blocks, and keeps its rows' accumulators for both.  Roles:
-//               warp 0       TMA producer of the row tiles (128 rows x 64 k per stage)
+//             blocks).  The decoded weights are the M operand and live in TENSOR MEMORY, the rows are N, only as many as there are
+//             (in 32): tcgen05.mma.cta_group::2, M 256 x N <= 256 x K 16 -- each CTA decodes one of the two column blocks and brings half of
+//             the rows, and holds its columns' accumulators of all rows.  Roles:
+//               warp 0       TMA producer of the rows (half of the chunk's x 128 k per stage)
 //               warp 1       first CTA: issues the MMAs of the pair, commits stages and passes to both CTAs; second CTA: relays
-//                            "my half of the stage is there" to the first
+//                            "my rows of the stage are there" to the first
 //               warp 2       allocates / frees tensor memory (512 columns)
 //               warp 3       TMA producer of the packed words, a ring of its own
-//               warps 4-11   epilogue, one accumulator row per thread (column block 0: warps 4-7, block 1: warps 8-11):
-//                            tcgen05.ld 128 fp32, the 128-point Hadamard transform in the thread's registers, scales, limited
-//                            SwiGLU, down-input rotation; fp16 Xd rows (gate/up) or fp32 Y rows (down)
-//               warps 12-27  decode the trellis tiles (bit-exact codebook) in registers and, when the slot is free, store them to
-//                            the swizzled K-major tile
-//             The gate and the up projection of an item are two PASSES over K with their own accumulators (256 columns each):
-//             while the up pass runs, the epilogue warps turn the gate accumulators into silu(gate) (kept as bf16 in shared
-//             memory), and the up pass's epilogue overlaps the next item's gate pass, so tensor memory is double-buffered by
-//             construction.  Down is one pass per item, alternating the two accumulator halves.
-//             What bounds it: with one CTA per tile pair (M 128 x N 128 instructions) the operand reads of the MMAs alone filled
-//             shared memory (128 bytes a clock); the pair halves them.  What is left is the loop from a stage's release to its
-//             next use (decode store, relay, issue, commit) and the decode itself: 4096 tokens, gate/up 407 -> 358 us, of which
-//             249 us remain without decode and epilogue arithmetic.
+//               warps 4-11   epilogue: 32 rows x 128 columns at a time from tensor memory, transposed through shared memory so that four
+//                            lanes hold a row; the 128-point Hadamard transform, scales, limited SwiGLU, down-input rotation;
+//                            fp16 Xd rows (gate/up) or fp32 Y rows (down)
+//               warps 12-27  decode the trellis tiles (bit-exact codebook) in registers and store them to tensor memory (tcgen05.st):
+//                            the places of a word's weights are those that the instruction gives a lane
+//             The gate and the up projection of an item are two PASSES over K with their own accumulators: while the up pass
+//             runs, the epilogue warps turn the gate accumulators into silu(gate) (kept as bf16 in the places of Xd), and the up pass's
+//             epilogue overlaps the next item's gate pass.  Down is one pass per item.
+//             Before, the rows were M (256 a tile, filled or not) and the weights went through shared memory: a chunk of 40 rows cost as
+//             much as one of 256, an expert of 257 rows twice as much as one of 256.  us gate/up | down, before -> now: 500 rows 197 | 101
+//             -> 143 | 73, 4096 rows 350 | 181 -> 280 | 139, eight experts of 64 at 4096 rows 81 | 39 -> 52 | 34 (2048 x 1536, 64 experts,
+//             top-4); 8192 rows of 4096 x 512, 288 experts, top-8: 587 | 697 -> 559 | 539.  What bounds it now: at 4096 rows instruction
+//             issue (0.71 of the cycles while all SMs work: decode, epilogue) and the last round of items (0.87 of the time); at 500 rows the
+//             issuing warp, about 1,000 clocks a stage of its own beside the busy decode warps; short K (512): the epilogue's stores.
+//             Tried: three epilogue warpgroups of 104 registers (309 against 280 us), the words' copies prefetched to L2 a pass ahead (no
+//             change), stages of 64 k (158 | 83 at 500 rows: the same steps for half the work), silu(gate) in shared memory (chunks of 256 rows
+//             then: 314 | 157 at 4096).
 // Arithmetic: one full-K fp32 accumulation chain per output (as upstream's prefill path, which is likewise not
 // bit-equal to its decode path: native/exl3_prefill.cu:20-23), the same transforms and rounding points as
 // upstream's epilogue (native/exl3_prefill.cu:596-622 == native/exl3.cu:260-321) with exp / divide in their fast
@@ -48,15 +53,17 @@ namespace gf {
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 int *fast_experts_status_word(glmflash_fast_experts *f);
 
-constexpr int FG_DEC = 16;                                 // trellis-decode warps: n-tile by n-tile, round robin
+constexpr int FG_DEC = 16;                                 // trellis-decode warps
 constexpr int FG_THREADS = (12 + FG_DEC) * 32;
-constexpr int FG_BM = 128, FG_BN = 128, FG_BK = 64;        // rows and columns of a CTA's operand tiles, k of a stage
-constexpr int FG_TILE_BYTES = FG_BM * FG_BK * 2;           // 16 KB: one 128 x 64 fp16 operand tile
-constexpr int FG_WORD_BYTES = 4096;                        // packed words of a stage: 4 k-tiles x 8 n-tiles
-constexpr int FG_CHUNK = 2 * FG_BM;                        // rows of a work item: 128 per CTA of the pair
+constexpr int FG_BN = 128, FG_BK = 128;                    // columns of a CTA, k of a stage
+constexpr int FG_CHUNK = 320;                              // most rows of a work item
+constexpr int FG_BOXES = 8;                                // boxes of rows that one copy takes: 16, 32, .. 128
+constexpr int FG_HALF_BYTES = FG_CHUNK / 2 * 128;          // 20 KB: a CTA's rows x 64 k of fp16, half of a stage
+constexpr int FG_TILE_BYTES = 2 * FG_HALF_BYTES;
+constexpr int FG_WORD_BYTES = 8192;                        // packed words of a stage: 8 k-tiles x 8 n-tiles
 constexpr int FG_MAXU = 1024;
 
-// plan layout (int32): [0] total 128-row tiles, [1] total grouped rows, [2] chunks
+// plan layout (int32): [0] 128-row tiles of all experts (informative), [1] total grouped rows, [2] chunks
 constexpr int PLAN_INTS = 4;
 // ---------------------------------------------------------------------------------------------- plan
 // Launched with one block per bank entry: every block recomputes the (tiny) scans, block 0 publishes the plan,
@@ -66,8 +73,8 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
                                                           int shared_exl3, int e_lo, int e_hi, int srow_lo, int srow_hi,
                                                           int *__restrict__ plan, int4 *__restrict__ chunks,
                                                           int *__restrict__ src_pair, int *__restrict__ row_expert) {
-    __shared__ int cnt_sh[FG_MAXU], row_sh[FG_MAXU], e_sh[FG_MAXU], first_sh[FG_MAXU];
-    __shared__ int wsum[4][32];
+    __shared__ int cnt_sh[FG_MAXU], row_sh[FG_MAXU], e_sh[FG_MAXU], first_sh[FG_MAXU], order_sh[FG_MAXU];
+    __shared__ int wsum[3][32];
     const int u = threadIdx.x, lane = u & 31, warp = u >> 5;
     pdl_wait();                                             // (every kernel of the chain: nothing is read or written before)
     pdl_launch_dependents();
@@ -99,31 +106,36 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
             }
         }
     }
-    // chunks of at most 256 rows, as even as they go; those of more than 128 rows come first in the list, so that the static
-    // round robin over the CTA pairs ends with the short ones
-    const int tiles = (cnt + FG_BM - 1) / FG_BM, nch = (cnt + FG_CHUNK - 1) / FG_CHUNK, size = nch ? (cnt + nch - 1) / nch : 0;
-    const int pairs = size > FG_BM ? nch : 0, single = nch - pairs;
-    // block-wide exclusive scans of long chunks, short chunks, rows (and the tile total)
-    int p_inc = pairs, s_inc = single, r_inc = cnt, t_inc = tiles;
+    // chunks of at most 320 rows, as even as they go, in the order of their length (in 32 rows, long ones first), so that the static
+    // round robin over the CTA pairs takes about equal ones in a turn and ends with the short ones
+    const int tiles = (cnt + 127) / 128, nch = (cnt + FG_CHUNK - 1) / FG_CHUNK, size = nch ? (cnt + nch - 1) / nch : 0;
+    const int key = (size + 31) >> 5;
+    // block-wide exclusive scan of rows, totals of tiles and chunks
+    int r_inc = cnt, t_inc = tiles, c_inc = nch;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, p_inc, d), b = __shfl_up_sync(0xffffffffu, s_inc, d),
-                  c = __shfl_up_sync(0xffffffffu, r_inc, d), t = __shfl_up_sync(0xffffffffu, t_inc, d);
-        if (lane >= d) { p_inc += a; s_inc += b; r_inc += c; t_inc += t; }
+        const int a = __shfl_up_sync(0xffffffffu, r_inc, d), b = __shfl_up_sync(0xffffffffu, t_inc, d), c = __shfl_up_sync(0xffffffffu, c_inc, d);
+        if (lane >= d) { r_inc += a; t_inc += b; c_inc += c; }
     }
-    if (lane == 31) { wsum[0][warp] = p_inc; wsum[1][warp] = s_inc; wsum[2][warp] = r_inc; wsum[3][warp] = t_inc; }
+    if (lane == 31) { wsum[0][warp] = r_inc; wsum[1][warp] = t_inc; wsum[2][warp] = c_inc; }
+    order_sh[u] = key << 16 | nch;
     __syncthreads();
-    int p_off = 0, s_off = 0, r_off = 0, p_all = 0, s_all = 0, r_all = 0, t_all = 0;
+    int r_off = 0, r_all = 0, t_all = 0, c_all = 0;
     for (int w = 0; w < 32; ++w) {
-        if (w < warp) { p_off += wsum[0][w]; s_off += wsum[1][w]; r_off += wsum[2][w]; }
-        p_all += wsum[0][w]; s_all += wsum[1][w]; r_all += wsum[2][w]; t_all += wsum[3][w];
+        if (w < warp) r_off += wsum[0][w];
+        r_all += wsum[0][w]; t_all += wsum[1][w]; c_all += wsum[2][w];
     }
-    const int p_ex = p_off + p_inc - pairs, s_ex = s_off + s_inc - single, r_ex = r_off + r_inc - cnt;
+    const int r_ex = r_off + r_inc - cnt;
     cnt_sh[u] = cnt; row_sh[u] = r_ex; e_sh[u] = e; first_sh[u] = first;
-    if (u == 0 && blockIdx.x == 0) { plan[0] = t_all; plan[1] = r_all; plan[2] = p_all + s_all; }
-    if (u < n && u % (int)gridDim.x == (int)blockIdx.x)
-        for (int c = 0; c < nch; ++c)
-            chunks[(pairs ? p_ex : p_all + s_ex) + c] = make_int4(e, r_ex + c * size, min(size, cnt - c * size), 0);
+    if (u == 0 && blockIdx.x == 0) { plan[0] = t_all; plan[1] = r_all; plan[2] = c_all; }
+    if (u < n && u % (int)gridDim.x == (int)blockIdx.x) {
+        int at = 0;                                         // chunks of longer ones, and of experts in front with as long ones
+        for (int w = 0; w < n; ++w) {
+            const int o = order_sh[w], k = o >> 16;
+            if (k > key || (k == key && w < u)) at += o & 0xffff;
+        }
+        for (int c = 0; c < nch; ++c) chunks[at + c] = make_int4(e, r_ex + c * size, min(size, cnt - c * size), 0);
+    }
     __syncthreads();
     for (int uu = blockIdx.x; uu < n; uu += gridDim.x) {
         const int c = cnt_sh[uu], rb = row_sh[uu], ee = e_sh[uu], f0 = first_sh[uu];
@@ -231,15 +243,24 @@ __device__ __forceinline__ void tmem_alloc(uint32_t *slot_smem, uint32_t cols) {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T over a pair of CTAs, M 256 x N 256 x K 16, fp16 operands, fp32 accumulate: each CTA
-// brings 128 rows of A and 128 rows (columns of D) of B at the same shared-memory offsets and keeps its 128 rows of D
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem desc]^T over a pair of CTAs, M 256 x N x K 16, fp16 operands, fp32 accumulate: each CTA brings 128
+// rows of A (lanes of its tensor memory, two k a column) and N / 2 rows of B, and keeps its 128 rows of D for all N columns
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// sixteen lanes x 32 columns of tensor memory: lane (G, T) of the warp holds columns 4 x + T of rows G (r[2 x]) and G + 8 (r[2 x + 1])
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // arrive on the mbarrier of both CTAs of the pair when every tcgen05.mma issued so far by this thread has completed
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
@@ -281,6 +302,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
+// the same, complete on return
+__device__ __forceinline__ void tmem_ld32_now(uint32_t taddr, float *v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart; the tile base is 1024-aligned and
@@ -294,8 +331,8 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                               // SWIZZLE_128B
     return d;
 }
-// kind::f16: D fp32, A and B fp16, both K-major, N 256, M 256 (the pair's)
-constexpr uint32_t UMMA_IDESC = (1u << 4) | ((uint32_t)(2 * FG_BN >> 3) << 17) | ((uint32_t)(2 * FG_BM >> 4) << 24);
+// kind::f16: D fp32, A and B fp16, both K-major, M 256 (the pair's columns of the matrix), N rows
+__device__ __forceinline__ uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(2 * FG_BN >> 4) << 24); }
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
     asm volatile(
@@ -321,35 +358,49 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, vo
     return false;
 }
 
-// In-register 128-point Walsh-Hadamard transform, butterflies stride 1..64, (lower + upper, lower - upper):
-// upstream's order (native/exl3.cu:208-219), so every sum associates as there.
 // Two values rounded to bf16 (nearest even) by one packed conversion, read back as fp32: per value the bits of bf16r.
 __device__ __forceinline__ float2 bf16r2(float x, float y) {
     const __nv_bfloat162 b = __float22bfloat162_rn(make_float2(x, y));
     const uint32_t w = *reinterpret_cast<const uint32_t *>(&b);
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
-// From stride 2 on, the two neighbours (i, i + 1) take the same side of their butterflies, so a pair goes through one
-// packed fp32 instruction of sm_100 (add.f32x2 / fma.f32x2; a - b as b * -1 + a, one rounding, the same bits): half
-// the issue slots of the transform, which matters because this kernel is bound by instruction issue.
-__device__ __forceinline__ void fwht128_regs(float (&v)[128]) {
+// 128-point Walsh-Hadamard transform of a row that four neighbouring lanes hold: lane t has columns 16 j + 4 t + i at v[4 j + i].  Butterflies
+// stride 1..64, (lower + upper, lower - upper): upstream's order (native/exl3.cu:208-219), so every sum associates as there.  Strides 4 and 8
+// cross lanes; from stride 2 on two neighbours take the same side and share one packed fp32 instruction of sm_100 (add.f32x2 /
+// fma.f32x2; a - b as b * -1 + a, one rounding, the same bits).
+__device__ __forceinline__ void fwht128_quad(float (&v)[32], int t) {
 #pragma unroll
-    for (int i = 0; i < 128; i += 2) {
+    for (int i = 0; i < 32; i += 2) {
         const float a = v[i], b = v[i + 1];
         v[i] = a + b;
         v[i + 1] = a - b;
     }
     const float2 neg1 = make_float2(-1.f, -1.f);
+    auto in_lane = [&](int s) {
 #pragma unroll
-    for (int s = 2; s < 128; s <<= 1)
-#pragma unroll
-        for (int i = 0; i < 128; i += 2)
+        for (int i = 0; i < 32; i += 2)
             if (!(i & s)) {
                 const float2 a = make_float2(v[i], v[i + 1]), b = make_float2(v[i | s], v[(i | s) + 1]);
                 const float2 lo = __fadd2_rn(a, b), hi = __ffma2_rn(b, neg1, a);
                 v[i] = lo.x; v[i + 1] = lo.y;
                 v[i | s] = hi.x; v[(i | s) + 1] = hi.y;
             }
+    };
+    in_lane(2);
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1) {
+        const float sg = t & d ? -1.f : 1.f;
+        const float2 s2 = make_float2(sg, sg);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, v[i], d), __shfl_xor_sync(0xffffffffu, v[i + 1], d));
+            const float2 r = __ffma2_rn(make_float2(v[i], v[i + 1]), s2, o);
+            v[i] = r.x; v[i + 1] = r.y;
+        }
+    }
+    in_lane(4);
+    in_lane(8);
+    in_lane(16);
 }
 
 struct FastGemmArgs {
@@ -363,68 +414,105 @@ struct FastGemmArgs {
     float limit;
 };
 
-// One work item of a CTA pair: a chunk of an expert's rows and a pair of 128-column blocks.  This CTA brings `cnt` of the rows
-// (starting at grouped row `row`) and decodes column block 2 * nbp + its rank.
-struct ItemInfo {
-    int e, row, cnt, nbp;
+// One work item of a CTA pair: a chunk of an expert's rows and a pair of 128-column blocks.  Each CTA decodes one of them (2 * nbp + its
+// rank) and brings half of the rows.  A role walks its pair's items with the next one's chunk already on the way.
+struct Items {
+    const int4 *chunks;
+    int total, step, NBP, item;
+    int4 next;
+    int e, row, cnt, n, nbp;                                 // n: rows of the MMAs (cnt rounded up to 32)
+    __device__ __forceinline__ Items(const int4 *c, int first, int all, int pairs, int nbps) : chunks(c), total(all), step(pairs), NBP(nbps), item(first - pairs) {
+        if (first < total) next = __ldg(chunks + first / NBP);
+    }
+    __device__ __forceinline__ bool advance() {
+        item += step;
+        if (item >= total) return false;
+        e = next.x; row = next.y; cnt = next.z; n = (next.z + 31) & ~31; nbp = item % NBP;
+        if (item + step < total) next = __ldg(chunks + (item + step) / NBP);
+        return true;
+    }
 };
-__device__ __forceinline__ ItemInfo item_info(int item, int NBP, const int4 *chunks, int rank) {
-    const int4 c = __ldg(chunks + item / NBP);
-    const int h = (c.z + 1) >> 1;                            // rows of the first CTA; both take about half
-    return ItemInfo{c.x, c.y + (rank ? h : 0), rank ? c.z - h : h, item % NBP};
-}
+
+// position in a ring of barriers and the parity of its phase
+struct Ring {
+    uint32_t slot, parity;
+    __device__ __forceinline__ void next(uint32_t depth) {
+        if (++slot == depth) { slot = 0; parity ^= 1; }
+    }
+};
+
+struct FgMaps {
+    CUtensorMap rows[2][FG_BOXES];                           // grouped rows of the gate and up (or the down) input
+    CUtensorMap bank[2];                                     // packed words
+};
+
+// Tensor memory: columns [0, 192) three stages of decoded weights (64 columns = 128 k), [192, 512) accumulators.  Even passes have theirs
+// at the lower end, odd ones at the upper, so that two of up to 160 rows have room side by side; longer ones wait until the epilogue has
+// taken out the columns that they share with the last pass, while the decode fills the stages.
+constexpr int FG_ASTAGES = 3, FG_ACOLS = FG_BK / 2, FG_DCOL = FG_ASTAGES * FG_ACOLS, FG_DCOLS = 512 - FG_DCOL;
+static_assert(FG_DCOLS >= FG_CHUNK, "accumulators of a pass");
 
 template <int MATS>
 struct FgCfg {
-    static constexpr int ASTAGES = MATS == 2 ? 4 : 6;        // rows
-    static constexpr int BSTAGES = 4;                        // decoded weights: written from registers as soon as the slot is free
-    static constexpr int WSTAGES = MATS == 2 ? 5 : 6;        // packed words
-    static constexpr int DONE = 8;                           // ring of stage-completed barriers (more than any ring above)
-    static constexpr int GBUF_BYTES = MATS == 2 ? 64 * 256 * 4 : 0;                          // silu(gate) as bf16 pairs
-    static constexpr int TABLE_BYTES = 512 + 2 * 3 * 128 * 4;                                // barriers, scale vectors
-    static constexpr int TBUF_BYTES = MATS == 1 ? 8 * 2 * 32 * 16 * 4 : 0;    // down: per epilogue warp two tiles of 32 rows x 16 floats
-    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)(ASTAGES + BSTAGES) * FG_TILE_BYTES + (size_t)WSTAGES * FG_WORD_BYTES +
-                                   GBUF_BYTES + TABLE_BYTES + TBUF_BYTES;
+    static constexpr int BSTAGES = 4;                        // rows
+    static constexpr int WSTAGES = 4;                        // packed words
+    static constexpr int DONE = 4;                           // ring of stage-completed barriers (at least as deep as any ring)
+    // Waits go by the parity of a phase: whoever waits for one has to know that the phase before it is over.  The decode warps take every
+    // second stage, so the stage in front of theirs in a slot of words has to be one of theirs as well: copies land in any order.  (The MMAs
+    // of stages complete in order.)
+    static_assert(WSTAGES % 2 == 0, "words of the decode warps");
+    static_assert(DONE >= BSTAGES && DONE >= FG_ASTAGES, "ring of completed stages");
+    static constexpr int SCALES = MATS == 2 ? 3 * 128 : 128, SCALE_BUFS = MATS == 2 ? 1 : 2;   // scale vectors of an item, of one or two items
+    static constexpr int TABLE_BYTES = 256 + SCALE_BUFS * SCALES * 4;                        // barriers, scale vectors
+    static constexpr int TBUF_BYTES = 2 * 32 * 128 * 4;                                      // per epilogue warpgroup a slab of 32 rows
+    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)BSTAGES * FG_TILE_BYTES + (size_t)WSTAGES * FG_WORD_BYTES + TABLE_BYTES + TBUF_BYTES;
 };
 
-// Registers per thread: launched with 72 x 896; the producer warpgroup and the decode warpgroups give theirs to the two epilogue
-// warpgroups (24 + 2 x 152 + 4 x 40 = 488 of 504).
+// Registers per thread: launched with 72 x 896; the producer warpgroup gives to the two epilogue warpgroups (24 + 2 x 160 + 4 x 40 = 504).
 constexpr uint32_t FG_SLEEP = 500;
-constexpr int FG_REGS_MMA = 24, FG_REGS_EPI = 152, FG_REGS_DEC = 40;
+constexpr int FG_REGS_MMA = 24, FG_REGS_EPI = 160, FG_REGS_DEC = 40;
+
+// All 128 threads of an epilogue warpgroup: whether every one of them says yes.
+__device__ __forceinline__ bool group_all(int group, bool yes) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.red.and.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)yes), "r"(2 + group) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void group_barrier(int group) { asm volatile("barrier.sync %0, 128;" ::"r"(2 + group) : "memory"); }
 
 template <int MATS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FG_THREADS, 1)
-fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1, const __grid_constant__ CUtensorMap mapT0,
-                 const __grid_constant__ CUtensorMap mapT1, const FastGemmArgs a) {
+fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
     using C = FgCfg<MATS>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // 1024-aligned operand tiles
-    unsigned char *aring = smem, *bring = aring + (size_t)C::ASTAGES * FG_TILE_BYTES;
-    unsigned char *wring = bring + (size_t)C::BSTAGES * FG_TILE_BYTES;     // [WSTAGES] packed words, 128-byte swizzle
-    uint32_t *gbuf = reinterpret_cast<uint32_t *>(wring + (size_t)C::WSTAGES * FG_WORD_BYTES);       // [64][256]
-    unsigned char *tables = wring + (size_t)C::WSTAGES * FG_WORD_BYTES + C::GBUF_BYTES;
-    uint64_t *afull = reinterpret_cast<uint64_t *>(tables);                // [ASTAGES] rows landed
-    uint64_t *bfull = afull + C::ASTAGES;                                  // [BSTAGES] decoded (+ in the first CTA: the second CTA's half)
-    uint64_t *done = bfull + C::BSTAGES;                                   // [DONE] MMAs of stage i completed: done[i % DONE]
-    uint64_t *wfull = done + C::DONE;                                   // [WSTAGES] packed words landed
+    unsigned char *bring = smem;                                           // [BSTAGES] rows
+    unsigned char *wring = bring + (size_t)C::BSTAGES * FG_TILE_BYTES;     // [WSTAGES] packed words
+    float *tbuf = reinterpret_cast<float *>(wring + (size_t)C::WSTAGES * FG_WORD_BYTES);             // [2 groups][32 rows][128]
+    unsigned char *tables = reinterpret_cast<unsigned char *>(tbuf) + C::TBUF_BYTES;
+    uint64_t *bfull = reinterpret_cast<uint64_t *>(tables);                // [BSTAGES] rows landed (first CTA: in both)
+    uint64_t *afull = bfull + C::BSTAGES;                                  // [FG_ASTAGES] (first CTA) decoded, in both
+    uint64_t *done = afull + FG_ASTAGES;                                   // [DONE] MMAs of stage i completed: done[i % DONE]
+    uint64_t *wfull = done + C::DONE;                                      // [WSTAGES] packed words landed
     uint64_t *wempty = wfull + C::WSTAGES;                                 // [WSTAGES] read by the stage's decode warps
     uint64_t *tmem_full = wempty + C::WSTAGES;                             // [2] accumulators of a pass complete
     uint64_t *tmem_empty = tmem_full + 2;                                  // [2] (first CTA) accumulators drained, both CTAs' warps
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
+    uint64_t *tmem_early = tmem_empty + 2;                                 // [2] (first CTA) what the next pass overwrites of them drained
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_early + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    float *scales = reinterpret_cast<float *>(tables + 512);               // [2 column blocks][3][128]
-    float *tbuf = reinterpret_cast<float *>(tables + C::TABLE_BYTES);      // [8 warps][2][32 rows][16] (down only)
+    float *scales = reinterpret_cast<float *>(tables + 256);               // [SCALE_BUFS][SCALES]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int KT = a.K >> 4, NBP = a.N >> 8, KS = a.K / FG_BK;
 
     if (tid == 0) {
-        for (int s = 0; s < C::ASTAGES; ++s) mbar_init(afull + s, 1);
-        for (int s = 0; s < C::BSTAGES; ++s) mbar_init(bfull + s, 8 + (rank == 0));
+        for (int s = 0; s < C::BSTAGES; ++s) mbar_init(bfull + s, 1 + (rank == 0));
+        for (int s = 0; s < FG_ASTAGES; ++s) mbar_init(afull + s, FG_DEC);
         for (int s = 0; s < C::DONE; ++s) mbar_init(done + s, 1);
-        for (int s = 0; s < C::WSTAGES; ++s) { mbar_init(wfull + s, 1); mbar_init(wempty + s, 8); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + b, 1); mbar_init(tmem_empty + b, 16); }
+        for (int s = 0; s < C::WSTAGES; ++s) { mbar_init(wfull + s, 1); mbar_init(wempty + s, FG_DEC / 2); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + b, 1); mbar_init(tmem_empty + b, 16); mbar_init(tmem_early + b, 16); }
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -443,54 +531,79 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
         return wait_or_abort<FG_SLEEP>(done + j % C::DONE, (j / C::DONE) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT);
     };
 
+    // after a give-up: the copies in flight, if any, have landed before the CTA leaves (bounded)
+    auto land = [&](uint64_t *bar, uint32_t depth, uint32_t it) {
+        for (uint32_t k = it > depth ? it - depth : 0; k < it; ++k) mbar_wait(bar + k % depth, (k / depth) & 1, nullptr, 1000u);
+    };
+
     if (warp < 4) {
         // ------------------------------------------------------------------ warpgroup 0: TMA, MMA issue, relay
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_MMA));
         if (warp == 0 && lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (int item = pair; item < total && ok && !*abort_flag; item += pairs) {
-                const ItemInfo t = item_info(item, NBP, a.chunks, rank);
+            for (Items t(a.chunks, pair, total, pairs, NBP); ok && !*abort_flag && t.advance();) {
+                // n / 2 rows of this CTA, those of the second MMA of more than 256 apart
+                const int n1 = min(t.n, 256), n2 = t.n - n1, row1 = t.row + rank * (n1 >> 1), row2 = t.row + 256 + rank * (n2 >> 1);
                 for (int pm = 0; pm < MATS && ok; ++pm) {
-                    const CUtensorMap *map = (pm == 1 && !a.shared_x) ? &mapA1 : &mapA0;
+                    const CUtensorMap *map = maps.rows[pm == 1 && !a.shared_x], *map1 = map + (n1 >> 5) - 1, *map2 = map + max((n2 >> 5) - 1, 0);
                     for (int s = 0; s < KS; ++s, ++it) {
-                        const uint32_t slot = it % C::ASTAGES;
-                        if (!slot_free(it, C::ASTAGES)) { ok = false; break; }
-                        if (t.cnt == 0) { mbar_arrive(afull + slot); continue; }       // (a chunk of one row: the peer has it)
-                        mbar_expect_tx(afull + slot, FG_TILE_BYTES);
-                        tma_load_2d(aring + (size_t)slot * FG_TILE_BYTES, map, s * FG_BK, t.row, afull + slot);
+                        const uint32_t slot = it % C::BSTAGES;
+                        if (!slot_free(it, C::BSTAGES)) { ok = false; break; }
+                        mbar_expect_tx(bfull + slot, (uint32_t)t.n * FG_BK);
+                        unsigned char *dst = bring + slot * FG_TILE_BYTES;
+                        tma_load_2d(dst, map1, s * FG_BK, row1, bfull + slot);
+                        tma_load_2d(dst + FG_HALF_BYTES, map1, s * FG_BK + 64, row1, bfull + slot);
+                        if (n2) {
+                            tma_load_2d(dst + 128 * 128, map2, s * FG_BK, row2, bfull + slot);
+                            tma_load_2d(dst + 128 * 128 + FG_HALF_BYTES, map2, s * FG_BK + 64, row2, bfull + slot);
+                        }
                     }
                 }
             }
+            if (!ok) land(bfull, C::BSTAGES, it);
         } else if (warp == 1 && rank == 0) {
             // One elected thread of this warp issues every MMA of the pair; the warp runs the loop together, so that the descriptors
-            // stay in uniform registers.  Its instruction stream is the critical path of the tensor pipe, so the
-            // shared-memory descriptors are built once (stage 0) and advanced by adding constants: the address field
-            // counts 16-byte units, a stage is a tile apart, a K step of 16 halves is 32 bytes.
-            const uint64_t desc_a0 = umma_desc_sw128(smem_u32(aring)), desc_b0 = umma_desc_sw128(smem_u32(bring));
-            uint32_t it = 0, pc = 0;
+            // stay in uniform registers.  Its instruction stream is the critical path of the tensor pipe: ring positions and parities are
+            // counted along (with modulo arithmetic a stage took 800 clocks of it beside the busy decode warps, 500 rows) and
+            // the shared-memory descriptor is built once and advanced by adding constants (the address field
+            // counts 16-byte units, a K step of 16 halves is 32 bytes; of A: eight columns).
+            const uint64_t desc_b0 = umma_desc_sw128(smem_u32(bring));
+            Ring ra{0, 0}, rb{0, 0}, rd{0, 0};
+            uint32_t pc = 0;
+            int before = 0;                                          // rows of the pass in front
             bool ok = true;
-            for (int item = pair; item < total && ok; item += pairs) {
+            for (Items t(a.chunks, pair, total, pairs, NBP); ok && t.advance();) {
+                const int n2 = t.n - min(t.n, 256);                  // (one instruction takes 256 rows)
+                const uint32_t idesc = umma_idesc(t.n - n2), idesc2 = umma_idesc(n2);
                 for (int pm = 0; pm < MATS && ok; ++pm, ++pc) {
                     const uint32_t pb = pc & 1;
-                    ok = __all_sync(0xffffffffu, wait_or_abort<0>(tmem_empty + pb, ((pc >> 1) & 1) ^ 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
+                    // the accumulators of the pass before the last one, and where they reach into these, of the last one have been drained
+                    ok = __all_sync(0xffffffffu, wait_or_abort<0>(tmem_empty + pb, ((pc >> 1) & 1) ^ 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
+                                                     (before + t.n <= FG_DCOLS || wait_or_abort<0>((t.n <= before ? tmem_early : tmem_empty) + (pb ^ 1), ((pc - 1) >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)));
                     if (!ok) break;
+                    before = t.n;
                     tc_fence_after();
-                    const uint32_t d0 = tmem_base + pb * 256;
-                    for (int s = 0; s < KS; ++s, ++it) {
-                        const uint32_t sa = it % C::ASTAGES, sb = it % C::BSTAGES;
-                        ok = __all_sync(0xffffffffu, wait_or_abort<0>(afull + sa, (it / C::ASTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
-                                                         wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
+                    const uint32_t d0 = tmem_base + FG_DCOL + (pb ? FG_DCOLS - t.n : 0);
+                    for (int s = KS; s; --s) {
+                        ok = __all_sync(0xffffffffu, wait_or_abort<0>(bfull + rb.slot, rb.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
+                                                         wait_or_abort<0>(afull + ra.slot, ra.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
                         if (!ok) break;
                         tc_fence_after();
-                        const uint64_t da = desc_a0 + (uint64_t)(sa * (FG_TILE_BYTES >> 4)), db = desc_b0 + (uint64_t)(sb * (FG_TILE_BYTES >> 4));
+                        const uint64_t db = desc_b0 + rb.slot * (FG_TILE_BYTES >> 4);
+                        const uint32_t ta = tmem_base + ra.slot * FG_ACOLS, first = s != KS;
                         if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < FG_BK / 16; ++kk) umma_f16(d0, da + 2 * kk, db + 2 * kk, UMMA_IDESC, kk > 0 || s > 0 ? 1u : 0u);
-                            umma_commit(done + it % C::DONE);       // both CTAs may overwrite the stage once these MMAs have read it
-                            if (s == KS - 1) umma_commit(tmem_full + pb);      // the accumulators of this pass are complete
+                            for (int kk = 0; kk < FG_BK / 16; ++kk) {
+                                const uint64_t dk = db + 2 * (kk & 3) + (kk >> 2) * (FG_HALF_BYTES >> 4);
+                                umma_f16(d0, ta + 8 * kk, dk, idesc, kk > 0 ? 1u : first);
+                                if (n2) umma_f16(d0 + 256, ta + 8 * kk, dk + (128 * 128 >> 4), idesc2, kk > 0 ? 1u : first);
+                            }
+                            umma_commit(done + rd.slot);            // both CTAs may overwrite the stage once these MMAs have read it
+                            if (s == 1) umma_commit(tmem_full + pb);           // the accumulators of this pass are complete
                         }
                         __syncwarp();
+                        ra.next(FG_ASTAGES); rb.next(C::BSTAGES); rd.next(C::DONE);
                     }
                 }
             }
@@ -498,197 +611,215 @@ fast_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constan
             // packed words of this CTA's column block, a ring of their own a few stages ahead of the decode
             uint32_t it = 0;
             bool ok = true;
-            for (int item = pair; item < total && ok && !*abort_flag; item += pairs) {
-                const ItemInfo t = item_info(item, NBP, a.chunks, rank);
+            for (Items t(a.chunks, pair, total, pairs, NBP); ok && !*abort_flag && t.advance();) {
                 for (int pm = 0; pm < MATS && ok; ++pm)
                     for (int s = 0; s < KS; ++s, ++it) {
                         const uint32_t ws = it % C::WSTAGES;
                         if (!wait_or_abort<FG_SLEEP>(wempty + ws, ((it / C::WSTAGES) & 1) ^ 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT)) { ok = false; break; }
                         mbar_expect_tx(wfull + ws, FG_WORD_BYTES);
-                        tma_load_3d(wring + ws * FG_WORD_BYTES, pm ? &mapT1 : &mapT0, 0, t.e * KT + 4 * s, (2 * t.nbp + rank) * 8, wfull + ws);
+                        tma_load_3d(wring + ws * FG_WORD_BYTES, &maps.bank[pm], 0, t.e * KT + 8 * s, (2 * t.nbp + rank) * 8, wfull + ws);
                     }
             }
+            if (!ok) land(wfull, C::WSTAGES, it);
         } else if (warp == 1 && lane == 0) {
-            // second CTA: tell the issuing thread that this CTA's half of a stage is there
+            // second CTA: tell the issuing thread that this CTA's rows of a stage are there (its decode warps say so themselves)
             uint32_t it = 0;
             bool ok = true;
-            for (int item = pair; item < total && ok && !*abort_flag; item += pairs)
-                for (int s = 0; s < MATS * KS && ok; ++s, ++it) {
-                    const uint32_t sa = it % C::ASTAGES, sb = it % C::BSTAGES;
-                    ok = wait_or_abort<0>(afull + sa, (it / C::ASTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
-                         wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
-                    if (ok) mbar_arrive_cluster(bfull + sb, 0);
-                }
+            for (const uint32_t stages = (uint32_t)(items * MATS * KS); it < stages && ok; ++it) {
+                const uint32_t sb = it % C::BSTAGES;
+                ok = wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
+                if (ok) mbar_arrive_cluster(bfull + sb, 0);
+            }
         }
     } else if (warp < 12) {
-        // ------------------------------------------------------------------ warpgroups 1-2: epilogue (column block 0 | 1)
+        // ------------------------------------------------------------------ warpgroups 1-2: epilogue
+        // The accumulators have the columns of the matrix as lanes and rows as columns.  A warpgroup takes every other slab of 32 rows: a
+        // thread reads its lane's 32 rows, the slab is transposed through shared memory, and four neighbouring lanes hold a row
+        // (columns 16 j + 4 t + i).
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FG_REGS_EPI));
-        const int q = warp & 3, cb = (warp - 4) >> 2;        // TMEM lane quadrant, column block of the item
-        const int m = q * 32 + lane, em = cb * 128 + m;      // row of this CTA, thread of the epilogue (0..255)
-        const float *sc = scales + cb * 384;
-        uint32_t pc = 0;
+        const int q = warp & 3, group = (warp - 4) >> 2, m = q * 32 + lane, em = tid - 128;
+        const int rr = m >> 2, t4 = (m & 3) * 4;             // row of a slab, first column of a group of 16
+        // element (row r, column c) of a slab sits at r * 128 + (c ^ 16 (r & 1)): conflict-free both ways
+        float *slab = tbuf + group * 32 * 128;
+        uint32_t pc = 0, turn = 0;
         bool ok = true;
-        // A warp whose wait gave up (or that sees the abort flag) does not leave this loop: it walks the remaining items
-        // arriving at the two barriers only, so that a sibling which passed the same wait at the last moment never
-        // stands alone at a barrier of eight warps.
-        for (int item = pair; item < total; item += pairs) {
-            const ItemInfo t = item_info(item, NBP, a.chunks, rank);
-            const int nb = 2 * t.nbp + cb;
-            // scale vectors of (expert, column block): written by the block's 128 threads, read by them
-            asm volatile("bar.sync 1, 256;");
-            if (ok && *abort_flag) ok = false;
-            if (ok) {
-                const size_t o = (size_t)t.e * a.N + nb * 128 + m;
-                // the 1 / sqrt(128) of every Hadamard transform is folded into the scale vectors here (the transform is
-                // linear), which takes one multiply per element out of each epilogue step
-                float *w = scales + cb * 384 + m;
-                w[0] = __half2float(a.sv0[o]) * HAD_SCALE;
-                if (MATS == 2) { w[128] = __half2float(a.sv1[o]) * HAD_SCALE; w[256] = __half2float(a.sd[o]) * HAD_SCALE; }
-            }
-            asm volatile("bar.sync 1, 256;");
+        // scale vectors of an item: fetched while the one before it runs, by both warpgroups (the 1 / sqrt(128) of every Hadamard transform is
+        // folded into them, the transform is linear: one multiply per element less in each epilogue step)
+        Items t(a.chunks, pair, total, pairs, NBP);
+        float sc0 = 0.f, sc1 = 0.f;
+        auto fetch = [&](int item, int e) {
+            const size_t o = (size_t)e * a.N + (2 * (item % NBP) + rank) * 128 + (em & 127);
+            if (em < 128) sc0 = __half2float(a.sv0[o]);
+            else if (MATS == 2) { sc0 = __half2float(a.sv1[o]); sc1 = __half2float(a.sd[o]); }
+        };
+        if (pair < total) fetch(pair, t.next.x);
+        // A warpgroup decides together whether a wait has given up: a warp never stands alone at a barrier.  One that has goes on through the
+        // items for the barrier of both.
+        while (t.advance()) {
+            const int nb = 2 * t.nbp + rank;
+            float *sc = scales + (C::SCALE_BUFS == 2 ? (turn++ & 1) * C::SCALES : 0);
+            if (C::SCALE_BUFS == 1) asm volatile("bar.sync 1, 256;" ::: "memory");           // (the last item's have been read)
+            if (em < 128) sc[em] = sc0 * HAD_SCALE;
+            else if (MATS == 2) { sc[em] = sc0 * HAD_SCALE; sc[em + 128] = sc1 * HAD_SCALE; }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
             if (!ok) continue;
-            float v[128];
+            if (t.item + t.step < total) fetch(t.item + t.step, t.next.x);
+            const int mine = ((t.cnt + 31) / 32 - group + 1) >> 1;       // slabs of this warpgroup: group, group + 2, ..
+            float v[3][32];
+#pragma unroll 1
             for (int pm = 0; pm < MATS; ++pm, ++pc) {
                 const uint32_t pb = pc & 1;
-                if (!wait_or_abort<FG_SLEEP>(tmem_full + pb, (pc >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT)) { ok = false; break; }
+                ok = wait_or_abort<FG_SLEEP>(tmem_full + pb, (pc >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
+                if (!(ok = group_all(group, ok))) break;
+                __syncwarp();                                            // (tcgen05.ld is for the warp as one)
                 tc_fence_after();
-                const bool has = t.cnt > q * 32;             // (uniform: rows of this warp)
-                if (has) {
-                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + pb * 256 + cb * FG_BN;
+                // Slabs in the order in which the next pass needs their columns: from the top at even passes, from the bottom at odd ones.  Three
+                // are taken out at once, which for up to 256 rows covers what a next pass of no more rows overwrites.
+                const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), col = FG_DCOL + (pb ? FG_DCOLS - t.n : 0);
+                auto slab_of = [&](int k) { return 2 * (pb ? k : max(mine - 1 - k, 0)) + group; };
+                auto at = [&](int k) { return lanes + min(col + 32 * slab_of(k), 480u); };     // (past the end: some other slab, no branches)
+                auto arrive = [&](uint64_t *bar) {                       // this warp's lanes are in registers
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(bar + pb, 0);
+                    __syncwarp();
+                };
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_ld32(taddr + c * 32, v + c * 32);
-                    tmem_ld_wait();
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(tmem_empty + pb, 0);  // this warp's rows are in registers
-                if (!has) continue;
-                fwht128_regs(v);
-                const float2 *sc2 = reinterpret_cast<const float2 *>(sc);
-                if (MATS == 2 && pm == 0) {
-                    // gate: scale, bf16 rounding, clamp, silu (rounded) -> two bf16 per word, this thread's column of gbuf
+                for (int k = 0; k < 3; ++k) tmem_ld32(at(k), v[k]);
+                tmem_ld_wait();
+                if (t.n <= 256) arrive(tmem_early);
+                if (t.n <= 192) arrive(tmem_empty);
+                auto finish = [&](float (&x)[32], int k) {
+                    group_barrier(group);                                // (the last slab has been read)
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) {
-                        const float2 sg = sc2[i];
-                        const float2 gr = bf16r2(v[2 * i] * sg.x, v[2 * i + 1] * sg.y);
-                        const float g0 = fminf(gr.x, a.limit), g1 = fminf(gr.y, a.limit);
-                        // (one packed conversion rounds both values to bf16 and packs them: .x in the low half)
-                        const __nv_bfloat162 sp = __float22bfloat162_rn(make_float2(__fdividef(g0, 1.f + __expf(-g0)),
-                                                                                   __fdividef(g1, 1.f + __expf(-g1))));
-                        gbuf[i * 256 + em] = *reinterpret_cast<const uint32_t *>(&sp);
+                    for (int r = 0; r < 32; ++r) slab[r * 128 + (m ^ (r & 1 ? 16 : 0))] = x[r];
+                    const int row = slab_of(k) * 32 + rr;                // of the chunk
+                    const bool here = row < t.cnt;
+                    __half *o = a.xd + (size_t)(t.row + row) * a.N + nb * 128 + t4;
+                    uint2 gate[8];
+                    int p = 0;
+                    if (MATS == 2 && pm == 1 && here)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) gate[j] = *reinterpret_cast<const uint2 *>(o + 16 * j);
+                    if (MATS == 1 && here) p = __ldg(a.src_pair + t.row + row);
+                    group_barrier(group);
+                    const float *src = slab + rr * 128 + t4;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 f = *reinterpret_cast<const float4 *>(src + (16 * j ^ ((rr & 1) * 16)));
+                        x[4 * j] = f.x; x[4 * j + 1] = f.y; x[4 * j + 2] = f.z; x[4 * j + 3] = f.w;
                     }
-                } else if (MATS == 2) {
+                    fwht128_quad(x, m & 3);
+                    if (MATS == 2 && pm == 0) {
+                        // gate: scale, bf16 rounding, clamp, silu (rounded).  The values wait in this thread's places of the row of Xd, which its
+                        // up pass overwrites (80 KB of shared memory otherwise)
+                        if (here)
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) {
-                        const uint32_t gp = gbuf[i * 256 + em];
-                        const float2 su = sc2[64 + i], sd2 = sc2[128 + i];
-                        const float2 ur = bf16r2(v[2 * i] * su.x, v[2 * i + 1] * su.y);
-                        const float u0 = fminf(fmaxf(ur.x, -a.limit), a.limit), u1 = fminf(fmaxf(ur.y, -a.limit), a.limit);
-                        const float2 pr = bf16r2(__uint_as_float(gp << 16) * u0, __uint_as_float(gp & 0xffff0000u) * u1);
-                        v[2 * i] = pr.x * sd2.x;
-                        v[2 * i + 1] = pr.y * sd2.y;
-                    }
-                    fwht128_regs(v);
-                    if (m < t.cnt) {
-                        uint4 *o = reinterpret_cast<uint4 *>(a.xd + (size_t)(t.row + m) * a.N + nb * 128);
+                            for (int j = 0; j < 8; ++j) {
+                                const float4 sg = *reinterpret_cast<const float4 *>(sc + 16 * j + t4);
+                                const float2 r0 = bf16r2(x[4 * j] * sg.x, x[4 * j + 1] * sg.y), r1 = bf16r2(x[4 * j + 2] * sg.z, x[4 * j + 3] * sg.w);
+                                const float g0 = fminf(r0.x, a.limit), g1 = fminf(r0.y, a.limit), g2 = fminf(r1.x, a.limit), g3 = fminf(r1.y, a.limit);
+                                // (one packed conversion rounds both values to bf16 and packs them: .x in the low half)
+                                const __nv_bfloat162 s0 = __float22bfloat162_rn(make_float2(__fdividef(g0, 1.f + __expf(-g0)), __fdividef(g1, 1.f + __expf(-g1))));
+                                const __nv_bfloat162 s1 = __float22bfloat162_rn(make_float2(__fdividef(g2, 1.f + __expf(-g2)), __fdividef(g3, 1.f + __expf(-g3))));
+                                *reinterpret_cast<uint2 *>(o + 16 * j) = make_uint2(*reinterpret_cast<const uint32_t *>(&s0), *reinterpret_cast<const uint32_t *>(&s1));
+                            }
+                    } else if (MATS == 2) {
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) {
-                            __half2 h[4];
+                        for (int j = 0; j < 8; ++j) {
+                            const float4 su = *reinterpret_cast<const float4 *>(sc + 128 + 16 * j + t4), sd = *reinterpret_cast<const float4 *>(sc + 256 + 16 * j + t4);
+                            const float2 r0 = bf16r2(x[4 * j] * su.x, x[4 * j + 1] * su.y), r1 = bf16r2(x[4 * j + 2] * su.z, x[4 * j + 3] * su.w);
+                            const float u0 = fminf(fmaxf(r0.x, -a.limit), a.limit), u1 = fminf(fmaxf(r0.y, -a.limit), a.limit);
+                            const float u2 = fminf(fmaxf(r1.x, -a.limit), a.limit), u3 = fminf(fmaxf(r1.y, -a.limit), a.limit);
+                            const float2 p0 = bf16r2(__uint_as_float(gate[j].x << 16) * u0, __uint_as_float(gate[j].x & 0xffff0000u) * u1);
+                            const float2 p1 = bf16r2(__uint_as_float(gate[j].y << 16) * u2, __uint_as_float(gate[j].y & 0xffff0000u) * u3);
+                            x[4 * j] = p0.x * sd.x; x[4 * j + 1] = p0.y * sd.y; x[4 * j + 2] = p1.x * sd.z; x[4 * j + 3] = p1.y * sd.w;
+                        }
+                        fwht128_quad(x, m & 3);
+                        if (here)
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)       // one packed conversion per pair (the same rounding per value)
-                                h[j] = __float22half2_rn(make_float2(v[8 * c + 2 * j], v[8 * c + 2 * j + 1]));
-                            o[c] = make_uint4(*reinterpret_cast<uint32_t *>(&h[0]), *reinterpret_cast<uint32_t *>(&h[1]),
-                                              *reinterpret_cast<uint32_t *>(&h[2]), *reinterpret_cast<uint32_t *>(&h[3]));
+                            for (int j = 0; j < 8; ++j)
+                                *reinterpret_cast<uint2 *>(o + 16 * j) = make_uint2(pack_half2(x[4 * j], x[4 * j + 1]), pack_half2(x[4 * j + 2], x[4 * j + 3]));
+                    } else if (here) {
+                        // down: y rows are pair rows; 64 contiguous bytes a row and instruction
+                        float *y = a.y + (size_t)p * a.N + nb * 128 + t4;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float4 s4 = *reinterpret_cast<const float4 *>(sc + 16 * j + t4);
+                            *reinterpret_cast<float4 *>(y + 16 * j) = make_float4(x[4 * j] * s4.x, x[4 * j + 1] * s4.y, x[4 * j + 2] * s4.z, x[4 * j + 3] * s4.w);
                         }
                     }
-                } else {
-                    // down: y rows are pair rows, scattered by src_pair.  A thread owns one row, so direct stores would
-                    // put 32 rows x 16 bytes into every store instruction (half-filled sectors).  The rows go through
-                    // per-warp shared-memory tiles, 16 columns at a time, and leave as 8 rows x 64 contiguous bytes per
-                    // instruction.  Chunk c of row r sits at chunk c ^ ((r >> 1) & 3): conflict-free both ways.  Two tiles in
-                    // turn, so that a block of columns is written while the one before is on its way out: with one, the 16
-                    // steps ran one after the other, 16,000 of an item's 20,000 epilogue clocks (4096 tokens: 200 -> 191 us).
-                    const int p = m < t.cnt ? a.src_pair[t.row + m] : -1;
-                    float *wbuf = tbuf + (warp - 4) * 1024;
-                    int pr[4];                               // pair rows that this lane writes
+                };
+                // One copy of the slab's code: unrolled over the three slabs it came from L2 again and again (20 clocks an instruction).
+#pragma unroll 1
+                for (int k = 0; k < mine; ++k) {
+                    finish(v[0], k);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) pr[i] = __shfl_sync(0xffffffffu, p, (lane >> 2) + 8 * i);
-                    auto put = [&](int ch) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const int col = ch * 16 + 4 * c;
-                            const float4 s4 = *reinterpret_cast<const float4 *>(sc + col);
-                            *reinterpret_cast<float4 *>(wbuf + (ch & 1) * 512 + lane * 16 + ((c ^ ((lane >> 1) & 3)) << 2)) =
-                                make_float4(v[col] * s4.x, v[col + 1] * s4.y, v[col + 2] * s4.z, v[col + 3] * s4.w);
-                        }
-                    };
-                    put(0);
-#pragma unroll
-                    for (int ch = 0; ch < 8; ++ch) {
-                        __syncwarp();
-                        float4 val[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int rr = (lane >> 2) + 8 * i;
-                            val[i] = *reinterpret_cast<const float4 *>(wbuf + (ch & 1) * 512 + rr * 16 + (((lane & 3) ^ ((rr >> 1) & 3)) << 2));
-                        }
-                        if (ch < 7) put(ch + 1);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (pr[i] >= 0)
-                                *reinterpret_cast<float4 *>(a.y + (size_t)pr[i] * a.N + nb * 128 + ch * 16 + 4 * (lane & 3)) = val[i];
+                    for (int r = 0; r < 32; ++r) { v[0][r] = v[1][r]; v[1][r] = v[2][r]; }
+                    if (k == 0 && t.n > 192) {                           // the fourth and the fifth slab, as soon as there is room
+                        tmem_ld32_now(at(3), v[2]);
+                        if (t.n <= 256) arrive(tmem_empty);
                     }
-                    __syncwarp();                            // (the next item's first tile overwrites one that is read here)
+                    if (k == 1 && t.n > 256) {
+                        tmem_ld32_now(at(4), v[2]);
+                        arrive(tmem_early);
+                        arrive(tmem_empty);
+                    }
                 }
             }
         }
+        // the arrivals of the last commits have come in before this CTA ends (the accumulators are complete: these are on their way)
+        const uint32_t stages = (uint32_t)(items * MATS * KS);
+        for (uint32_t k = stages > C::DONE ? stages - C::DONE : 0; k < stages && ok; ++k)
+            ok = wait_or_abort<FG_SLEEP>(done + k % C::DONE, (k / C::DONE) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
     } else {
-        // ------------------------------------------------------------------ warpgroups 3-6: trellis decode of B
-        // An n-tile of a stage at a time, round robin over the warps.  A lane reads 16 bytes (four words: all 16 k of columns G and
-        // G + 8) of k-tile T of the stage, decodes them in registers and, once the slot is free, stores them as four 16-byte pieces
-        // of the K-major tile, conflict-free under its swizzle: the decode is not part of the loop from a slot's release to the
-        // next MMA.
+        // ------------------------------------------------------------------ warpgroups 3-6: trellis decode
+        // A warp takes every second stage and, of it, one of the two n-tiles (16 columns) whose lanes of tensor memory it may write.  A lane
+        // reads word number `lane` of a tile and the word in front of it: those are k 2 T, 2 T + 1, 2 T + 8, 2 T + 9 of columns G and G + 8,
+        // just the places that tcgen05.st gives it.  The first half of the stage is decoded before the slot is free.
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_DEC));
-        const int G = lane >> 2, T = lane & 3;
-        // byte offsets in the n-tile of the B tile: rows G and + 8; 16-byte pieces 2 T and 2 T + 1, piece c of row r at c ^ (r & 7)
-        const uint32_t off0 = G * 128 + ((2 * T) ^ G) * 16, off1 = G * 128 + ((2 * T + 1) ^ G) * 16;
-        const uint32_t tiles_all = (uint32_t)(items * MATS * KS) * 8;
-        for (uint32_t c = warp - 12; c < tiles_all; c += FG_DEC) {
-            const uint32_t it = c >> 3, nt = c & 7, sb = it % C::BSTAGES, ws = it % C::WSTAGES;
+        const int q = warp & 3, half = (warp >> 2) & 1;
+        const uint32_t stages = (uint32_t)(items * MATS * KS);
+        const uint32_t lanes = tmem_base + ((uint32_t)(q * 32 + half * 16) << 16);
+        const unsigned char *words = wring + (2 * q + half) * 1024;
+        for (uint32_t it = (warp - 12) >> 3; it < stages; it += 2) {
+            const uint32_t ws = it % C::WSTAGES, sa = it % FG_ASTAGES;
             // (the vote also brings the lanes together again: they may have left the wait apart)
             if (!__all_sync(0xffffffffu, wait_or_abort<FG_SLEEP>(wfull + ws, (it / C::WSTAGES) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT))) break;
-            // the lane's four words and the word in front of them (circular): row (n-tile, k-tile) of 128 bytes, piece c of row r at
-            // c ^ (r & 7)
-            const uint32_t row = nt * 4 + T;
-            const unsigned char *wp = wring + ws * FG_WORD_BYTES + row * 128;
-            const uint4 wv = *reinterpret_cast<const uint4 *>(wp + ((G ^ (row & 7)) << 4));
-            const uint32_t before = *reinterpret_cast<const uint32_t *>(wp + ((((G + 7) & 7) ^ (row & 7)) << 4) + 12);
-            const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
-            uint32_t o[4][4];
+            const uint32_t *wp = reinterpret_cast<const uint32_t *>(words + ws * FG_WORD_BYTES);
+            bool ok = true;
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h, wp += 128) {
+                uint32_t o[16];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const uint32_t pw = t == 0 ? before : w[t - 1];
-                uint32_t hi[4], lo[4];
-                codeword_pair(__funnelshift_r(w[t], pw, 12), hi[0], lo[0]);                  // k = 2t:     columns G, G + 8
-                codeword_pair(__funnelshift_r(w[t], pw, 8), hi[1], lo[1]);                   // k = 2t + 1
-                codeword_pair(__funnelshift_r(w[t], pw, 4), hi[2], lo[2]);                   // k = 2t + 8
-                codeword_pair(w[t], hi[3], lo[3]);                                           // k = 2t + 9
-                o[0][t] = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410);
-                o[1][t] = __byte_perm(weight_dup(hi[2]), weight_dup(hi[3]), 0x5410);
-                o[2][t] = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
-                o[3][t] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
+                for (int kt = 0; kt < 4; ++kt) {
+                    const uint32_t w = wp[kt * 32 + lane], pw = wp[kt * 32 + ((lane + 31) & 31)];
+                    uint32_t hi[4], lo[4];
+                    codeword_pair(__funnelshift_r(w, pw, 12), hi[0], lo[0]);                 // k = 2 T:     columns G, G + 8
+                    codeword_pair(__funnelshift_r(w, pw, 8), hi[1], lo[1]);                  // k = 2 T + 1
+                    codeword_pair(__funnelshift_r(w, pw, 4), hi[2], lo[2]);                  // k = 2 T + 8
+                    codeword_pair(w, hi[3], lo[3]);                                          // k = 2 T + 9
+                    o[4 * kt] = __byte_perm(weight_dup(hi[0]), weight_dup(hi[1]), 0x5410);
+                    o[4 * kt + 1] = __byte_perm(weight_dup(lo[0]), weight_dup(lo[1]), 0x5410);
+                    o[4 * kt + 2] = __byte_perm(weight_dup(hi[2]), weight_dup(hi[3]), 0x5410);
+                    o[4 * kt + 3] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
+                }
+                if (h == 0) {
+                    ok = __all_sync(0xffffffffu, slot_free(it, FG_ASTAGES));
+                    if (!ok) break;
+                    __syncwarp();                            // (tcgen05.st is for the warp as one: the lanes may have left the wait apart)
+                    tc_fence_after();
+                }
+                tmem_st16(lanes + sa * FG_ACOLS + h * (FG_ACOLS / 2), o);
             }
+            if (!ok) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(wempty + ws);
-            if (!__all_sync(0xffffffffu, slot_free(it, C::BSTAGES))) break;
-            unsigned char *bt = bring + (size_t)sb * FG_TILE_BYTES + nt * 2048;
-            *reinterpret_cast<uint4 *>(bt + off0) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
-            *reinterpret_cast<uint4 *>(bt + off1) = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
-            *reinterpret_cast<uint4 *>(bt + off0 + 1024) = make_uint4(o[2][0], o[2][1], o[2][2], o[2][3]);
-            *reinterpret_cast<uint4 *>(bt + off1 + 1024) = make_uint4(o[3][0], o[3][1], o[3][2], o[3][3]);
-            fence_async_smem();                              // generic-proxy stores -> visible to the tensor core
             __syncwarp();
-            if (lane == 0) mbar_arrive(bfull + sb);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(afull + sa, 0);
         }
     }
 
@@ -707,11 +838,14 @@ using namespace gf;
 namespace {
 int fail_if(cudaError_t e) { return e == cudaSuccess ? 0 : gf::fail_cuda(e, "cudaFuncSetAttribute"); }
 
-// fp16 matrix [rows][K] row-major; box = 128 rows x 64 halves (128 bytes), 128-byte swizzle
-int make_map(CUtensorMap *map, void *base, uint64_t rows, uint64_t K) {
+// fp16 matrix [rows][K] row-major; boxes of 16, 32, .. 128 rows x 64 halves (128 bytes), 128-byte swizzle
+int make_maps(CUtensorMap (&map)[FG_BOXES], void *base, uint64_t rows, uint64_t K) {
     const uint64_t dims[2] = {K, rows}, strides[1] = {K * 2};
-    const uint32_t box[2] = {FG_BK, FG_BM};
-    return gf::encode_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, "grouped rows");
+    for (uint32_t i = 0; i < FG_BOXES; ++i) {
+        const uint32_t box[2] = {64, 16 * (i + 1)};
+        if (gf::encode_map(map + i, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, "grouped rows")) return -1;
+    }
+    return 0;
 }
 }  // namespace
 
@@ -722,7 +856,7 @@ struct glmflash_fast_experts {
     float *out = nullptr;                                   // pair rows
     int4 *chunks = nullptr;
     int *plan = nullptr, *src_pair = nullptr, *row_expert = nullptr, *status = nullptr;
-    CUtensorMap map_xg, map_xu, map_xd;
+    FgMaps gateup, down;                                    // (the words' maps are filled in for each run)
     int sms = 0;
     int phases = 15;                                        // profiling aid: 1 plan, 2 rotation, 4 gate/up, 8 down
 };
@@ -757,8 +891,7 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
     pool.take(&f->src_pair, P * 4);
     pool.take(&f->row_expert, P * 4);
     pool.take(&f->status, 16);
-    if (pool.alloc(&f->pool) || make_map(&f->map_xg, f->xg, P, H) ||
-        make_map(&f->map_xu, f->xu, P, H) || make_map(&f->map_xd, f->xd, P, I) ||
+    if (pool.alloc(&f->pool) || make_maps(f->gateup.rows[0], f->xg, P, H) || make_maps(f->gateup.rows[1], f->xu, P, H) || make_maps(f->down.rows[0], f->xd, P, I) ||
         fail_if(cudaFuncSetAttribute(fast_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<2>::SMEM)) ||
         fail_if(cudaFuncSetAttribute(fast_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<1>::SMEM))) {
         glmflash_fast_experts_free(f);
@@ -799,16 +932,16 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
             return -1;
     FastGemmArgs a{};
     a.plan = f->plan; a.chunks = f->chunks; a.src_pair = f->src_pair; a.status = f->status; a.limit = c.limit;
-    CUtensorMap mg, mu, md;
-    if (bank_map(&mg, w->gt, c.experts + 1, H, I, 4) || bank_map(&mu, w->ut, c.experts + 1, H, I, 4) || bank_map(&md, w->dt, c.experts + 1, I, H, 4))
+    if (bank_map(&f->gateup.bank[0], w->gt, c.experts + 1, H, I, 8, false) || bank_map(&f->gateup.bank[1], w->ut, c.experts + 1, H, I, 8, false) ||
+        bank_map(&f->down.bank[0], w->dt, c.experts + 1, I, H, 8, false))
         return -1;
     a.sv0 = (const __half *)w->svh_g; a.sv1 = (const __half *)w->svh_u; a.sd = (const __half *)w->suh_d;
     a.xd = f->xd; a.y = nullptr; a.K = H; a.N = I; a.shared_x = shared_x ? 1 : 0;
-    if ((f->phases & 4) && launch_k(fast_gemm_kernel<2>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<2>::SMEM, s, pdl, f->map_xg, f->map_xu, mg, mu, a))
+    if ((f->phases & 4) && launch_k(fast_gemm_kernel<2>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<2>::SMEM, s, pdl, f->gateup, a))
         return -1;
     a.sv0 = (const __half *)w->svh_d; a.sv1 = nullptr; a.sd = nullptr;
     a.xd = nullptr; a.y = f->out; a.K = I; a.N = H; a.shared_x = 1;
-    if ((f->phases & 8) && launch_k(fast_gemm_kernel<1>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<1>::SMEM, s, pdl, f->map_xd, f->map_xd, md, md, a))
+    if ((f->phases & 8) && launch_k(fast_gemm_kernel<1>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<1>::SMEM, s, pdl, f->down, a))
         return -1;
     return 0;
 }

@@ -65,11 +65,12 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 }
 
 // A trellis bank [experts][K / 16][N / 16][32 words] seen as (word of a tile, k-tile of any expert, n-tile): the box of a stage is
-// 32 words x `ktiles` k-tiles x 8 n-tiles, [n-tile][k-tile] rows of 128 bytes in shared memory.
-inline int bank_map(CUtensorMap *map, const uint32_t *bank, int experts, int K, int N, uint32_t ktiles = 16) {
+// 32 words x `ktiles` k-tiles x 8 n-tiles, [n-tile][k-tile] rows of 128 bytes in shared memory (swizzled for lanes that read 16 bytes of
+// four rows at a time; kernels whose warps read a row at a time take them as they are).
+inline int bank_map(CUtensorMap *map, const uint32_t *bank, int experts, int K, int N, uint32_t ktiles = 16, bool swizzle = true) {
     const uint64_t dims[3] = {32, (uint64_t)experts * (K / 16), (uint64_t)(N / 16)}, strides[2] = {(uint64_t)(N / 16) * 128, 128};
     const uint32_t box[3] = {32, ktiles, 8};
-    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint32_t *>(bank), dims, strides, box, "trellis bank");
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint32_t *>(bank), dims, strides, box, "trellis bank", swizzle);
 }
 
 // ---- decode: one stage (256 k of one matrix and 128 columns) by eight warps ------------------------------------------

@@ -183,6 +183,48 @@ def test_prefill_config4_vs_upstream(pkg, oracle, synth, cuda, bank, dbank, bank
     assert rel_err(out, want_out)[0] < 1e-5
 
 
+# rows of an expert around every edge of the GEMM: 32-row slabs and MMA sizes, the slabs taken out at once (192), two accumulators side by
+# side (160), one MMA or two (256), one chunk or more (320), chunks of one expert that differ by a slab (513 = 257 + 256)
+EDGES = (1, 2, 31, 32, 33, 64, 65, 128, 129, 159, 160, 161, 191, 192, 193, 224, 225, 255, 256, 257, 287, 288, 289, 319, 320, 321, 513, 641)
+
+
+@pytest.mark.parametrize("h,i,slots", [(256, 512, 2), (768, 256, 2), (2048, 512, 2), (512, 768, 3)])
+def test_chunk_edges(pkg, oracle, synth, cuda, h, i, slots):
+    """A row's bytes do not depend on how many rows its expert has: all experts at once against pieces of 100 rows, and a sample
+    against the oracle."""
+    import torch
+    e1 = len(EDGES)
+    wd_host = synth.expert_bank(77, h, i, e1, svh_scale=True)
+    wd = synth.to_device(wd_host, cuda)
+    rows = sum(EDGES)
+    rng = np.random.default_rng(5)
+    first = rng.permutation(np.repeat(np.arange(e1, dtype=np.int32), EDGES))
+    extra = [(first + 1 + s) % e1 for s in range(slots - 2)]                  # (more slots: other experts' counts shifted by one)
+    picks = np.stack([first] + extra + [np.full(rows, e1, np.int32)], 1).astype(np.int32)
+    x = synth.activations_bf16(6, rows, h)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+
+    def run(fe, sel):
+        n = len(sel)
+        ids, count, members = oracle.grouping(picks[sel], n, slots, e1 + 1, n)
+        fe.output.fill_(float("nan"))
+        fe.run(wd, _bf16_dev(x[sel], cuda), t(picks[sel]), t(ids), t(np.array([count], np.int32)), t(members), n, n)
+        torch.cuda.synchronize()
+        assert int(fe.status.cpu()[0]) == 0
+        return fe.output[: n * slots].cpu().numpy().reshape(n, slots, h)[:, : slots - 1].copy()
+    fe = pkg.FastExperts(pkg.make_config(h, i, e1, slots, max_rows=rows, shared_exl3=0))
+    full = run(fe, np.arange(rows))
+    assert np.isfinite(full).all()
+    order = rng.permutation(rows)
+    for lo in range(0, rows, 100):
+        sel = order[lo:lo + 100]
+        assert (run(fe, sel).view(np.uint32) == full[sel].view(np.uint32)).all(), lo
+    sample = order[:5]
+    want = oracle.experts_run_rows(wd_host, h, i, e1 + 1, slots, x[sample], picks[sample], mode=1).reshape(5, slots, h)[:, : slots - 1]
+    emax, erms = rel_err(full[sample], want)
+    assert emax < TOL and erms < TOL, (emax, erms)
+
+
 def test_shared_expert_row_window(pkg, synth, cuda, dbank):
     """Expert-parallel prefill splits the shared expert by rows: a handle with shared_rows = (lo, hi) computes the shared
     pair only for window rows in [lo, hi); every other pair is untouched.  Checked against the layer without a row
