@@ -142,90 +142,111 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
         for (int m = u; m < c; m += FG_MAXU) {
             const int code = members[(size_t)uu * maxm + f0 + m];
             src_pair[rb + m] = (code >> 5) * slots + (code & 31);
-            row_expert[rb + m] = ee;
+            row_expert[rb + m] = (code >> 5) << 10 | ee;
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------------- rotation
-// A warp takes 512 values of a grouped row: 8 lanes per 128-block, 16 values per lane, so that four of the seven butterflies run in
-// registers (from stride 2 on as packed fp32) and three across lanes.  The butterflies keep their order (stride 1..64), so the
-// sums are those of a warp per block.  With four values per lane and five butterflies across lanes the kernel issued 29
-// instructions a value and took 83 us at 4096 rows x 2048 x 5 pairs x 2 matrices (168 MB written).
-__global__ void __launch_bounds__(256) fast_rot_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride,
-                                                       const int *__restrict__ plan, const int *__restrict__ src_pair,
-                                                       const int *__restrict__ row_expert, const __half *__restrict__ suh0,
-                                                       const __half *__restrict__ suh1, __half *__restrict__ out0,
-                                                       __half *__restrict__ out1, int K, int slots, int mats, bool vec) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int KB = K >> 7, parts = (KB + 3) >> 2;
+// Four lanes hold a 128-block, 32 values each (columns 32 j + 8 t + i: 16-byte pieces, 64 contiguous bytes a block and instruction), so that five of
+// the seven butterflies run in registers, from stride 2 on as packed fp32, and two across lanes.  The butterflies keep their order (stride
+// 1..64).  A warp stays with eight blocks of one matrix and walks grouped rows: the sign / scale vector waits in registers as fp32 until the
+// expert changes, and the next row's input is on its way meanwhile.
+// What bounds it: issue slots and shuffles (about 8 instructions a value) and the trips for the next row; the writes alone take 30 and 90 us
+// (6 TB/s).  With 16 values a lane, three butterflies across lanes and the vector read and converted for every row: 67 us at 4096 rows x 2048 x
+// 5 pairs x 2 matrices (168 MB written) and 237 us at 8192 x 4096 x 8 x 1 (537 MB); now 53 and 160.  More warps with fewer registers spill
+// (71 and 225), several waves of blocks change nothing.
+constexpr int ROT_WARPS = 4;
+__global__ void __launch_bounds__(ROT_WARPS * 32, 4) fast_rot_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride, const int *__restrict__ plan,
+                                                                 const int *__restrict__ row_expert, const __half *__restrict__ suh0,
+                                                                 const __half *__restrict__ suh1, __half *__restrict__ out0,
+                                                                 __half *__restrict__ out1, int K, bool vec) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3, group = lane >> 2;
+    const int KB = K >> 7, slices = (KB + 7) >> 3, per_warp = KB < 8 ? 8 / KB : 1;         // rows of a warp (short rows: several)
+    const __half *suh = blockIdx.y ? suh1 : suh0;
+    __half *out = blockIdx.y ? out1 : out0;
+    const float2 neg1 = make_float2(-1.f, -1.f);
+    const int w = blockIdx.x * ROT_WARPS + warp, slice = w % slices, part = w / slices, parts = (int)gridDim.x * ROT_WARPS / slices;
+    const int sub = KB < 8 ? group / KB : 0, blk = KB < 8 ? group - sub * KB : slice * 8 + group, k = blk * 128 + 8 * t;
     pdl_wait();
     pdl_launch_dependents();
-    const long items = (long)plan[1] * parts;
-    const float2 neg1 = make_float2(-1.f, -1.f);
-    for (long it = (long)blockIdx.x * 8 + warp; it < items; it += (long)gridDim.x * 8) {
-        const int j = (int)(it / parts), blk = (int)(it % parts) * 4 + (lane >> 3);
-        if (blk >= KB) continue;                                           // (whole groups of eight lanes)
-        const unsigned group = 0xffu << (lane & 24);
-        const int e = row_expert[j], row = src_pair[j] / slots, k = blk * 128 + (lane & 7) * 16;
-        const __nv_bfloat16 *xp = x + (size_t)row * x_stride + k;
-        uint32_t xw[8];
-        if (vec) {
-            const uint4 a = *reinterpret_cast<const uint4 *>(xp), b = *reinterpret_cast<const uint4 *>(xp + 8);
-            xw[0] = a.x; xw[1] = a.y; xw[2] = a.z; xw[3] = a.w; xw[4] = b.x; xw[5] = b.y; xw[6] = b.z; xw[7] = b.w;
-        } else {
+    const int rows = plan[1], size = (rows + parts - 1) / parts, end = min(rows, (part + 1) * size);
+    const bool mine = blk < KB && sub < per_warp && part < parts;
+    int j = part * size + sub, code = 0, next = 0, e = -1;
+    uint4 xv[4];
+    auto fetch = [&] {                                                     // row j's input (code: row and expert)
+        if (!mine || j >= end) return;
+        code = next;
+        next = row_expert[min(j + per_warp, end - 1)];
+        const __nv_bfloat16 *p = x + (size_t)(code >> 10) * x_stride + k;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint2 a = *reinterpret_cast<const uint2 *>(xp + 4 * i);
-                xw[2 * i] = a.x; xw[2 * i + 1] = a.y;
+        for (int i = 0; i < 4; ++i) {
+            if (vec) xv[i] = *reinterpret_cast<const uint4 *>(p + 32 * i);
+            else {
+                const uint2 a = *reinterpret_cast<const uint2 *>(p + 32 * i), b = *reinterpret_cast<const uint2 *>(p + 32 * i + 4);
+                xv[i] = make_uint4(a.x, a.y, b.x, b.y);
             }
         }
-#pragma unroll 1
-        for (int mat = 0; mat < mats; ++mat) {
-            const __half *sp = (mat ? suh1 : suh0) + (size_t)e * K + k;
-            uint32_t sw[8];
-            if (vec) {
-                const uint4 a = __ldg(reinterpret_cast<const uint4 *>(sp)), b = __ldg(reinterpret_cast<const uint4 *>(sp + 8));
-                sw[0] = a.x; sw[1] = a.y; sw[2] = a.z; sw[3] = a.w; sw[4] = b.x; sw[5] = b.y; sw[6] = b.z; sw[7] = b.w;
-            } else {
+    };
+    if (mine && j < end) next = row_expert[j];
+    fetch();
+    float2 sv[16];
+    for (int first = part * size; first < end && part < parts; first += per_warp) {
+        const bool here = mine && j < end;
+        if (here && (code & 1023) != e) {
+            e = code & 1023;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint2 a = __ldg(reinterpret_cast<const uint2 *>(sp + 4 * i));
-                    sw[2 * i] = a.x; sw[2 * i + 1] = a.y;
+            for (int i = 0; i < 16; ++i) {                                 // (8-byte aligned at least)
+                const uint32_t h = __ldg(reinterpret_cast<const uint32_t *>(suh + (size_t)e * K + k + 32 * (i >> 2)) + (i & 3));
+                sv[i] = __half22float2(*reinterpret_cast<const __half2 *>(&h));
+            }
+        }
+        float2 v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {                                     // times the sign / scale vector, stride 1
+            const uint32_t b = i & 2 ? (i & 1 ? xv[i >> 2].w : xv[i >> 2].z) : (i & 1 ? xv[i >> 2].y : xv[i >> 2].x);
+            const float2 m = __fmul2_rn(make_float2(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), sv[i]);
+            v[i] = make_float2(m.x + m.y, m.x - m.y);
+        }
+        const int row = j;
+        j += per_warp;
+        fetch();
+        auto in_lane = [&](int d) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (!(i & d)) {
+                    const float2 a = v[i], b = v[i | d];
+                    v[i] = __fadd2_rn(a, b);
+                    v[i | d] = __ffma2_rn(b, neg1, a);
                 }
+        };
+        in_lane(1);
+        in_lane(2);
+#pragma unroll
+        for (int d = 1; d < 4; d <<= 1) {                                  // strides 8, 16: lower + upper | lower - upper
+            const float sg = t & d ? -1.f : 1.f;
+            const float2 s2 = make_float2(sg, sg);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, v[i].x, d), __shfl_xor_sync(0xffffffffu, v[i].y, d));
+                v[i] = __ffma2_rn(v[i], s2, o);
             }
-            float2 v[8];
+        }
+        in_lane(4);
+        in_lane(8);
+        if (here) {
+            __half *o = out + (size_t)row * K + k;
+            const float2 sc = make_float2(HAD_SCALE, HAD_SCALE);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {                                   // times the sign / scale vector, stride 1
-                const float2 s = __half22float2(*reinterpret_cast<const __half2 *>(&sw[i]));
-                const float a = __uint_as_float(xw[i] << 16) * s.x, b = __uint_as_float(xw[i] & 0xffff0000u) * s.y;
-                v[i] = make_float2(a + b, a - b);
-            }
+            for (int i = 0; i < 4; ++i) {
+                uint32_t h[4];
 #pragma unroll
-            for (int d = 1; d < 8; d <<= 1)                                // strides 2, 4, 8
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (!(i & d)) {
-                        const float2 a = v[i], b = v[i | d];
-                        v[i] = __fadd2_rn(a, b);
-                        v[i | d] = __ffma2_rn(b, neg1, a);
-                    }
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1) {                              // strides 16, 32, 64: lower + upper | lower - upper
-                const float sg = lane & d ? -1.f : 1.f;
-                const float2 s2 = make_float2(sg, sg);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 o = make_float2(__shfl_xor_sync(group, v[i].x, d), __shfl_xor_sync(group, v[i].y, d));
-                    v[i] = __ffma2_rn(v[i], s2, o);
+                for (int q = 0; q < 4; ++q) {
+                    const float2 r = __fmul2_rn(v[4 * i + q], sc);
+                    h[q] = pack_half2(r.x, r.y);
                 }
+                *reinterpret_cast<uint4 *>(o + 32 * i) = make_uint4(h[0], h[1], h[2], h[3]);
             }
-            uint32_t w[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = pack_half2(v[i].x * HAD_SCALE, v[i].y * HAD_SCALE);
-            uint4 *dst = reinterpret_cast<uint4 *>((mat ? out1 : out0) + (size_t)j * K + k);
-            dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
     }
 }
@@ -836,6 +857,13 @@ using namespace gf;
 
 // ---------------------------------------------------------------------------------------------- host side
 namespace {
+// Blocks of the rotation a matrix: what the SMs hold at once, fewer where a warp would have less than two rows, a whole number of the
+// slices of a row.
+long rot_blocks(long rows, int K, int mats, int sms) {
+    const long slices = (K / 128 + 7) / 8, warps = (rows + 1) / 2 * slices;
+    const long blocks = std::min((warps + ROT_WARPS - 1) / ROT_WARPS, 4L * sms / mats);
+    return (blocks + slices - 1) / slices * slices;
+}
 int fail_if(cudaError_t e) { return e == cudaSuccess ? 0 : gf::fail_cuda(e, "cudaFuncSetAttribute"); }
 
 // fp16 matrix [rows][K] row-major; boxes of 16, 32, .. 128 rows x 64 halves (128 bytes), 128-byte swizzle
@@ -855,7 +883,7 @@ struct glmflash_fast_experts {
     __half *xg = nullptr, *xu = nullptr, *xd = nullptr;     // grouped rows
     float *out = nullptr;                                   // pair rows
     int4 *chunks = nullptr;
-    int *plan = nullptr, *src_pair = nullptr, *row_expert = nullptr, *status = nullptr;
+    int *plan = nullptr, *src_pair = nullptr, *row_expert = nullptr /* row << 10 | expert */, *status = nullptr;
     FgMaps gateup, down;                                    // (the words' maps are filled in for each run)
     int sms = 0;
     int phases = 15;                                        // profiling aid: 1 plan, 2 rotation, 4 gate/up, 8 down
@@ -926,9 +954,9 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
             return -1;
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)
-        if (launch_k(fast_rot_kernel, dim3((unsigned)std::min<long>((P * ((H + 511) / 512) + 7) / 8, 32L * f->sms)), dim3(256), 0, s, pdl,
-            (const __nv_bfloat16 *)input, x_stride, f->plan, f->src_pair, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg,
-            f->xu, H, c.slots, mats, (((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 16 == 0 && x_stride % 8 == 0)))
+        if (launch_k(fast_rot_kernel, dim3((unsigned)rot_blocks(P, H, mats, f->sms), (unsigned)mats), dim3(ROT_WARPS * 32), 0, s, pdl, (const __nv_bfloat16 *)input, x_stride,
+                     f->plan, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg, f->xu, H,
+                     ((uintptr_t)input % 16 == 0 && x_stride % 8 == 0)))
             return -1;
     FastGemmArgs a{};
     a.plan = f->plan; a.chunks = f->chunks; a.src_pair = f->src_pair; a.status = f->status; a.limit = c.limit;

@@ -188,7 +188,7 @@ def test_prefill_config4_vs_upstream(pkg, oracle, synth, cuda, bank, dbank, bank
 EDGES = (1, 2, 31, 32, 33, 64, 65, 128, 129, 159, 160, 161, 191, 192, 193, 224, 225, 255, 256, 257, 287, 288, 289, 319, 320, 321, 513, 641)
 
 
-@pytest.mark.parametrize("h,i,slots", [(256, 512, 2), (768, 256, 2), (2048, 512, 2), (512, 768, 3)])
+@pytest.mark.parametrize("h,i,slots", [(256, 512, 2), (768, 256, 2), (2048, 512, 2), (512, 768, 3), (2304, 256, 2)])
 def test_chunk_edges(pkg, oracle, synth, cuda, h, i, slots):
     """A row's bytes do not depend on how many rows its expert has: all experts at once against pieces of 100 rows, and a sample
     against the oracle."""
@@ -223,6 +223,28 @@ def test_chunk_edges(pkg, oracle, synth, cuda, h, i, slots):
     want = oracle.experts_run_rows(wd_host, h, i, e1 + 1, slots, x[sample], picks[sample], mode=1).reshape(5, slots, h)[:, : slots - 1]
     emax, erms = rel_err(full[sample], want)
     assert emax < TOL and erms < TOL, (emax, erms)
+
+
+@pytest.mark.parametrize("h", [256, 1280])
+def test_input_rows_of_odd_strides(pkg, oracle, synth, cuda, h):
+    """Input rows that are 8-byte aligned only (a view of a wider tensor) give the bytes of densely packed ones."""
+    import torch
+    rows, e, i = 70, 5, 256
+    wd = synth.to_device(synth.expert_bank(78, h, i, e, svh_scale=True), cuda)
+    x = _bf16_dev(synth.activations_bf16(7, rows, h), cuda)
+    wide = torch.zeros((rows, h + 12), dtype=torch.bfloat16, device=cuda)
+    wide[:, 4:h + 4] = x
+    picks = np.stack([np.arange(rows, dtype=np.int32) % e, np.full(rows, e, np.int32)], 1)
+    ids, count, members = oracle.grouping(picks, rows, 2, e + 1, rows)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    fe = pkg.FastExperts(pkg.make_config(h, i, e, 2, max_rows=rows))
+    got = []
+    for view in (x, wide[:, 4:h + 4]):
+        fe.output.fill_(float("nan"))
+        fe.run(wd, view, t(picks), t(ids), t(np.array([count], np.int32)), t(members), rows, rows)
+        torch.cuda.synchronize()
+        got.append(fe.output[: rows * 2].cpu().numpy().view(np.uint32).copy())
+    assert (got[0] == got[1]).all()
 
 
 def test_shared_expert_row_window(pkg, synth, cuda, dbank):
