@@ -7,16 +7,17 @@
 //
 // Work is cut into units of one partial sum: (distinct expert, matrix, split of k, 128-column block), the gate / up units of all experts
 // first, the down units after them.  A split is 256 k at K <= 2048 (stream_cut), one or more stages of 16 k-tiles x 8 n-tiles
-// (16 KB, 32,768 weights).  A CTA (512 threads) has four roles:
+// (16 KB, 32,768 weights).  A CTA (512 threads, 768 with two teams of decode warps) has four roles:
 //   warps 0-7   decode: warp = n-tile.  A lane reads 16 bytes (4 words of one tile: all 16 k of columns G and G + 8) with
 //               one LDS.128, cuts the states in pairs with funnel shifts, forms the weights exactly as upstream does (fp16
 //               sum of the codeword halves) and packs them into A operands of mma.m16n8k8 (chunks: k16); members are the N dimension
 //               (8 per set, two sets for 9..16 rows), fp32 accumulation over the split.
-//   warps 8-10  X: put the members' activations of a stage's k range into shared memory as soon as they are there: rotated layer
+//               Two teams (one CTA an SM, units of one stage) take the stages in turn.
+//   then three  X: put the members' activations of a stage's k range into shared memory as soon as they are there: rotated layer
 //               inputs (gate / up) or the finished rows of the gate / up phase (down).
-//   warp 11     feeds a four-stage ring, ONE tensor copy per stage (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
+//   one warp    feeds a four-stage ring, ONE tensor copy per stage (box 128 B x 16 k-tiles x 8 n-tiles, 128-byte swizzle).  Sixteen
 //               bulk copies of the 1-KB rows held the issuing warp for 2,900 clocks a stage, longer than its decode takes.
-//   warps 12-15 finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of
+//   four warps  finish: rotate the layer input (fp16(H(x * suh) / sqrt 128), once per pair and matrix), then add the splits of
 //               an output block, ascending, and run the epilogue (Hadamard, scales, limited SwiGLU, down-input
 //               rotation; for the down phase Hadamard, output scale and the weighted sum over the row's slots,
 //               ascending, shared expert last).
@@ -35,8 +36,8 @@
 // other way, and a one-row layer moved by up to 1e-3.
 //
 // What bounds it: the decode instructions, about 5 a weight; a loop that does nothing else sustains 17.6 weights per clock and SM with 8
-// warps (two chunks in flight per warp) and 18.7 with 16, so 8 decode warps per CTA and one or two CTAs per SM
-// (launch_stream) are enough.  The earlier form (clusters of short-lived CTAs, three launches per layer) spent half of its time on the
+// warps (two chunks in flight per warp) and 18.7 with 16, so an SM has 16 decode warps where it can: two CTAs, or one with two teams
+// (launch_stream).  The earlier form (clusters of short-lived CTAs, three launches per layer) spent half of its time on the
 // phases around the decode.  Units of 512 k leave some SMs with twice the work of others at one row: 24.4 us a layer, 23.4 with 256 k.
 #include <algorithm>
 
@@ -46,9 +47,12 @@
 
 namespace gf {
 
-constexpr int ST_THREADS = 512, ST_STAGES = 4;
-constexpr int ST_DEC = 8, ST_XW = 3;                         // decode and X warps, then the producer, then four finish warps
-constexpr int ST_PROD = ST_DEC + ST_XW, ST_FIN = ST_PROD + 1;
+constexpr int ST_STAGES = 4, ST_XW = 3;
+// Warps of a CTA: eight decode warps a team, the X warps, the producer, four finish warps.
+template <int TEAMS>
+struct StWarps {
+    static constexpr int DEC = 8 * TEAMS, PROD = DEC + ST_XW, FIN = PROD + 1, THREADS = (FIN + 4) * 32;
+};
 constexpr size_t ST_MAX_SMEM = 227 * 1024 - 4352;            // dynamic part (4,240 bytes are static)
 constexpr size_t ST_HALF_SM = 116 * 1024;                    // two such CTAs do not fit an SM
 constexpr uint32_t ST_POLLS = 1u << 21;                      // polls of a global word before a wait gives up (about a second)
@@ -116,16 +120,17 @@ __device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long lon
     return true;
 }
 
-// v += the partials [lo, hi) of four columns of a pair, ascending, four requested at a time and polled until all carry the epoch.
-// last_only: between the attempts only the last of the four is polled; it is mostly the last to come.  With two CTAs an SM polls of all
+// v += the partials [lo, hi) of four columns of a pair, ascending, DEPTH requested at a time and polled until all carry the epoch.
+// last_only: between the attempts only the last of them is polled; it is mostly the last to come.  With two CTAs an SM polls of all
 // four cost the decode warps issue slots (8 rows 60.3 -> 59.5 us a layer); with one the extra round trip costs more (47 layers of
 // one token 1113 -> 1144 us).
+template <int DEPTH>
 __device__ __forceinline__ bool sum_splits(bool last_only, const StCta &c, const unsigned long long *z, size_t split_stride, int lo, int hi, uint32_t epoch,
                                            float (&v)[4]) {
     z += (size_t)lo * split_stride;
 #pragma unroll 1
-    for (; lo < hi; lo += 4, z += 4 * split_stride) {
-        unsigned long long w[4][4];
+    for (; lo < hi; lo += DEPTH, z += DEPTH * split_stride) {
+        unsigned long long w[DEPTH][4];
         uint32_t n = 0;
 #pragma unroll 1
         for (;;) {
@@ -133,20 +138,20 @@ __device__ __forceinline__ bool sum_splits(bool last_only, const StCta &c, const
             bool ok = true;
             const unsigned long long *zi = z;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < DEPTH; ++i) {
                 ll_load4(zi, w[i]);
                 if (lo + i + 1 < hi) zi += split_stride;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) ok = ok && ll_ready(w[i], epoch);
+            for (int i = 0; i < DEPTH; ++i) ok = ok && ll_ready(w[i], epoch);
             if (__all_sync(0xffffffffu, ok)) break;
             if (!__all_sync(0xffffffffu, c.again(n))) return false;
             __nanosleep(20);
             unsigned long long last[4];
-            if (last_only && !ll_wait4(c, z + (size_t)(min(hi - lo, 4) - 1) * split_stride, epoch, last)) return false;
+            if (last_only && !ll_wait4(c, z + (size_t)(min(hi - lo, DEPTH) - 1) * split_stride, epoch, last)) return false;
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < DEPTH; ++i)
             if (lo + i < hi)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) v[j] += __uint_as_float((uint32_t)w[i][j]);
@@ -193,6 +198,7 @@ __device__ __forceinline__ bool st_skipped(const StreamArgs &a, int row, int e, 
 // their members (one finish job per member and column block).  All threads of the CTA; the caller's barrier publishes the
 // tables.  This is the head of every layer's critical path.  `used` (32 words) and tb.mask are zero on entry; row, slot: of
 // pick number threadIdx.x.  Returns the number of experts.
+template <int TEAMS>
 __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTables &tb, uint32_t *used, int row, int slot) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (a.picks && a.rows == 1 && a.shared != 2) {
@@ -225,7 +231,7 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
         __syncwarp();
         return U;
     }
-    const int P = a.rows * a.slots;                              // <= 512 = one per thread
+    const int P = a.rows * a.slots;                              // <= 512: one per thread
     // key: the expert id (routing table) or the place in ids (grouping tables)
     int key = -1, e = -1, n_ids = 0;
     if (a.picks) {
@@ -297,7 +303,7 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
         if (u >= 0 && !dup) tb.pair[u * 16 + __popc(tb.mask[u] & ((1u << row) - 1u))] = (uint16_t)tid;
         if (tid < P) tb.state[tid] = u < 0 ? (short)-1 : dup ? (short)-2 : (short)e;
     }
-    if (warp == ST_FIN) {
+    if (warp == StWarps<TEAMS>::FIN) {
         int run = 0;
         for (int u0 = 0; u0 < U; u0 += 32) {
             const int c = u0 + lane < U ? __popc(tb.mask[u0 + lane]) : 0;
@@ -317,7 +323,9 @@ __device__ __forceinline__ int st_build_tables(const StreamArgs &a, const StTabl
 
 // The same for chunks of more than 16 rows (routing table only): an expert with more than 16 members gets an entry for every 16
 // of them, for which its weights are decoded again.  Every CTA has to come to the same tables.  tb.rows_of is zero on entry.
+template <int TEAMS>
 __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const StTables &tb) {
+    constexpr int THREADS = StWarps<TEAMS>::THREADS;
     __shared__ int total;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, P = a.rows * a.slots, W = tb.words;
     const float inv_slots = fast_inv(a.slots);
@@ -326,7 +334,7 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
         for (int w = 0; w < W; ++w) n += __popc(tb.rows_of[e * W + w]);
         return n;
     };
-    for (int i = tid; i < P; i += ST_THREADS) {
+    for (int i = tid; i < P; i += THREADS) {
         const int e = __ldcg(a.picks + i);
         tb.state[i] = e < 0 || e > a.E ? (short)-1 : (short)e;
     }
@@ -337,7 +345,7 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
         return !dup;
     };
     auto skipped = [&](int row, int e) { return st_skipped(a, row, e, a.shared); };
-    for (int i = tid; i < P; i += ST_THREADS) {
+    for (int i = tid; i < P; i += THREADS) {
         const int e = tb.state[i], row = fast_div(i, inv_slots);
         if (!skipped(row, e) && first_of_row(i, row, e)) atomicOr(&tb.rows_of[e * W + (row >> 5)], 1u << (row & 31));
     }
@@ -358,7 +366,7 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
         if (lane == 0) total = run;
     }
     __syncthreads();
-    for (int i = tid; i < P; i += ST_THREADS) {
+    for (int i = tid; i < P; i += THREADS) {
         const int e = tb.state[i], row = fast_div(i, inv_slots);
         // (marking a pick changes nothing for the row's others: the first one of an expert keeps its id)
         if (skipped(row, e)) { tb.state[i] = -1; continue; }
@@ -374,7 +382,7 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
     }
     __syncthreads();
     const int U = total;
-    if (warp == ST_FIN) {
+    if (warp == StWarps<TEAMS>::FIN) {
         int run = 0;
         for (int u0 = 0; u0 < U; u0 += 32) {
             const int c = u0 + lane < U ? __popc(tb.mask[u0 + lane]) : 0;
@@ -392,18 +400,23 @@ __device__ __forceinline__ int st_build_tables_many(const StreamArgs &a, const S
     return U;
 }
 
-// Register split over the warpgroups: decode and decode keep the 64 of the launch, X + producer give 16 to finish (64 + 64 + 48 + 80).
-// Decode at 56 registers took 60.5 us instead of 58.1 at 8 rows.
+// Register split over the warpgroups.  One team: decode and decode keep the 64 of the launch, X + producer give 16 to finish (64 + 64 + 48 +
+// 80); decode at 56 registers took 60.5 instead of 58.1 at 8 rows.  Two teams: launched with 80, all give to finish (4 x 64 + 48 + 176).
 template <bool INC, int N>
 __device__ __forceinline__ void st_regs() {
     if (INC) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-template <int SETS, bool MANY, int ROUNDS>
-__global__ void __launch_bounds__(ST_THREADS, 2)
+// TEAMS: groups of eight decode warps that take the stages in turn.  Two: one CTA an SM with all its registers, for windows whose units
+// are one stage each.
+template <int SETS, bool MANY, int ROUNDS, int TEAMS>
+__global__ void __launch_bounds__(StWarps<TEAMS>::THREADS, TEAMS == 1 ? 2 : 1)
 stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_d,
               const __grid_constant__ StreamArgs a) {
+    constexpr int ST_DEC = StWarps<TEAMS>::DEC, ST_PROD = StWarps<TEAMS>::PROD, ST_FIN = StWarps<TEAMS>::FIN, ST_THREADS = StWarps<TEAMS>::THREADS;
+    constexpr int DEPTH = TEAMS == 2 ? 8 : 4;                         // partials that a finish warp has on the way: its registers
+    static_assert(ST_STAGES % TEAMS == 0, "a team keeps its slots of the ring");
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);          // the swizzle atom is 1024 bytes
     constexpr int XBYTES = SETS * 8 * ST_XROW, SKT = 8 * ROUNDS, SBYTES = SKT * 1024;          // k-tiles and bytes of a stage
@@ -437,7 +450,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             mbar_init(ready + s, 1);
             mbar_init(wfull + s, 1);
             mbar_init(xfull + s, ST_XW);
-            mbar_init(empty + s, ST_DEC);
+            mbar_init(empty + s, 8);
         }
         abort_sh = 0;
         mbar_fence_init();
@@ -461,7 +474,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
     if (tid == ST_PROD * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
     if (tid == ST_FIN * 32) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
     const uint32_t epoch = next_epoch(__ldcg(a.ctrl + CTRL_EPOCH));   // words of earlier launches carry others
-    const int U = MANY ? st_build_tables_many(a, tb) : st_build_tables(a, tb, used_sh, row, slot);
+    const int U = MANY ? st_build_tables_many<TEAMS>(a, tb) : st_build_tables<TEAMS>(a, tb, used_sh, row, slot);
     if (tid == ST_FIN * 32) first_sh = drawn;
     __syncthreads();
     const int units_g = a.do_g ? U * 2 * SK1 * NB1 : 0, units = units_g + (a.do_d ? U * SK2 * NB2 : 0);
@@ -500,9 +513,10 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
     if (warp < ST_DEC) {
         // ---------------------------------------------------------------------------------------------- decode
-        const int G = lane >> 2, T = lane & 3;
+        if (TEAMS == 2) st_regs<false, 64>();
+        const int G = lane >> 2, T = lane & 3, tile = warp & 7;
         float acc[SETS][4];                                           // over a split
-        for (uint32_t it = 0;; ++it) {
+        for (uint32_t it = warp >> 3;; it += TEAMS) {
             const int s = it % ST_STAGES, phase = (it / ST_STAGES) & 1;
             if (!__all_sync(0xffffffffu, cta.wait(wfull + s, phase))) break;
             const int4 d = desc[s];
@@ -520,13 +534,13 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             const unsigned char *ws = words + s * SBYTES, *xs = xbuf + s * XBYTES;
             // (few experts of a window or chunk have more than eight members; with the second set's operand loads in every
             // unit, eleven rows of the 4096 x 512 layer took 115 us instead of 107 and a chunk of 40 192 instead of 180)
-            if (SETS == 1 || nmem <= 8) st_decode<1, MANY, ROUNDS>(ws, xs, warp, lane, reinterpret_cast<float (&)[1][4]>(acc));
-            else st_decode<SETS, MANY, ROUNDS>(ws, xs, warp, lane, acc);
+            if (SETS == 1 || nmem <= 8) st_decode<1, MANY, ROUNDS>(ws, xs, tile, lane, reinterpret_cast<float (&)[1][4]>(acc));
+            else st_decode<SETS, MANY, ROUNDS>(ws, xs, tile, lane, acc);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + s);
             if (!(d.x & DESC_LAST)) continue;
             const int N = kind == UNIT_G ? I : H;
-            unsigned long long *z = (kind == UNIT_G ? a.z1 : a.z2) + (unsigned)d.z + warp * 16 + 2 * G;
+            unsigned long long *z = (kind == UNIT_G ? a.z1 : a.z2) + (unsigned)d.z + tile * 16 + 2 * G;
 #pragma unroll
             for (int q = 0; q < SETS; ++q) {
                 const uint32_t pp = q ? p23 : p01;
@@ -574,17 +588,17 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             if (lane == 0) mbar_arrive(xfull + s);
         }
     } else if (warp >= ST_FIN) {
-        st_regs<true, 80>();
+        st_regs<true, TEAMS == 2 ? 176 : 80>();
         // ---------------------------------------------------------------------------------------------- finish
         const int fw = warp - ST_FIN, ft = tid - ST_FIN * 32;
         const int jobs_g = jobs_r + (a.do_g ? tb.pref[U] * NB1 : 0), jobs = jobs_g + (a.do_d ? a.rows * NB2 : 0);
         const float inv_nb1 = fast_inv(NB1), inv_nb2 = fast_inv(NB2);
         if (ft == 0 && drawn < jobs_r) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);      // the first job was a rotation: done above
         for (uint32_t it = 0;; ++it) {
-            // one thread publishes the group's job and draws the next; a group that has given up ends together here
+            // one thread publishes the group's job and draws the one behind a gate / up job; a group that has given up ends together here
             if (ft == 0) {
                 job_sh[it & 1] = abort_sh ? 0x7fffffff : drawn;
-                if (drawn < jobs) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
+                if (drawn < (a.two ? jobs_g : jobs)) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
             }
             asm volatile("bar.sync 5, 128;" ::: "memory");
             const int j = job_sh[it & 1];
@@ -611,7 +625,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                     asm volatile("bar.sync 5, 128;" ::: "memory");
                 }
                 if (!half) {
-                    sum_splits(a.two, cta, z, (size_t)P * I, 0, SK1, epoch, v);
+                    sum_splits<DEPTH>(a.two, cta, z, (size_t)P * I, 0, SK1, epoch, v);
                     z_columns(v, lane);
                     fwht128(v, lane);
                     const float2 c01 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.x)), c23 = __half22float2(*reinterpret_cast<const __half2 *>(&sv.y));
@@ -647,6 +661,8 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                 // down: the slots of a row eight at a time, two per warp, then the weighted sum, ascending slots
                 const int row = fast_div(j - jobs_g, inv_nb2), nb = j - jobs_g - row * NB2, col = nb * 128 + 4 * lane;
                 float acc = 0.f;
+                // (a routing weight a lane, on its way while the sums are: one after another behind them they were 3,000 clocks at the end of a layer)
+                const float wgt = a.out && lane < a.slots ? __ldcg(a.route_w + row * a.slots + lane) : 0.f;
                 for (int s0 = 0; s0 < a.slots; s0 += 8) {
                     int e[2];
                     float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -660,7 +676,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0)
-                            sum_splits(a.two, cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + nb * 128 + z_word(lane), (size_t)P * H, 0, SK2, epoch, v[i]);
+                            sum_splits<DEPTH>(a.two, cta, a.z2 + (size_t)(row * a.slots + s0 + 4 * i + fw) * H + nb * 128 + z_word(lane), (size_t)P * H, 0, SK2, epoch, v[i]);
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
                         if (e[i] >= 0) {
@@ -680,13 +696,19 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
                             *reinterpret_cast<float4 *>(&fin_sh[4 * i + fw][4 * lane]) = *reinterpret_cast<const float4 *>(y);
                         }
                     }
+                    // A down job's successor is drawn behind its sums: one that waited behind a waiting job was done after it, with other CTAs
+                    // idle (16 rows: 7,000 clocks at the end of a layer, 8 layers 625 -> 590 us; one row has a job for one CTA in nine, and
+                    // loses 6 us of 1,050 by the late draw).
+                    if (a.two && ft == 0 && s0 + 8 >= a.slots) drawn = (int)atomicAdd(a.ctrl + CTRL_FIN, 1u);
                     if (a.out) {
                         asm volatile("bar.sync 5, 128;" ::: "memory");
-                        for (int i = 0; i < min(8, a.slots - s0); ++i)
+                        for (int i = 0; i < min(8, a.slots - s0); ++i) {
+                            const float w = __shfl_sync(0xffffffffu, wgt, s0 + i);
                             if (tb.state[row * a.slots + s0 + i] != -1) {
                                 const float y = fin_sh[i][ft];
-                                acc = s0 + i == a.slots - 1 ? acc + y : acc + __ldcg(a.route_w + row * a.slots + s0 + i) * y;
+                                acc = s0 + i == a.slots - 1 ? acc + y : fmaf(w, y, acc);       // (one rounding, however the branch is compiled)
                             }
+                        }
                         asm volatile("bar.sync 5, 128;" ::: "memory");
                     }
                 }
@@ -710,10 +732,18 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             if (it && lane == 0) drawn = (int)atomicAdd(a.ctrl + CTRL_UNIT, 1u);
             int t = __shfl_sync(0xffffffffu, drawn, 0);
             if (t >= units) {
-                if (lane == 0) {
-                    desc[s] = make_int4(UNIT_END, 0, 0, 0);
-                    mbar_arrive(ready + s);
-                    mbar_arrive(wfull + s);
+                for (int team = 0; team < TEAMS && ok; ++team) {      // one end for each
+                    if (team) {
+                        s = ++it % ST_STAGES;
+                        ok = __all_sync(0xffffffffu, cta.wait(empty + s, ((it / ST_STAGES) & 1) ^ 1));
+                        if (!ok) break;
+                    }
+                    if (lane == 0) {
+                        desc[s] = make_int4(UNIT_END, 0, 0, 0);
+                        mbar_arrive(ready + s);
+                        mbar_arrive(wfull + s);
+                    }
+                    __syncwarp();
                 }
                 break;
             }
@@ -759,20 +789,14 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 
 int launch_stream(cudaStream_t s, StreamArgs a, bool pdl) {
     static int sms[64] = {};
-    static bool configured[64][5] = {};
+    static bool configured[64][7] = {};
     int dev = 0;
     GF_CUDA(cudaGetDevice(&dev));
     GF_REQUIRE(dev >= 0 && dev < 64, "device ordinal out of range");
     if (!sms[dev]) GF_CUDA(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
     // Stages of 128 k where a split is not a whole number of 256 k (K = 2304): the stage is a constant of the kernel.
     const bool fine = a.cut1.split % 16 || a.cut2.split % 16;
-    const int sets = a.rows > 8 ? 2 : 1, which = a.rows > 16 ? 4 : sets - 1 + 2 * fine;
-    // (chunks have a kernel of their own: with their tables as a branch, windows of 11 rows were 1 % slower)
-    const auto kernel = which == 4   ? stream_kernel<2, true, 2>
-                        : which == 3 ? stream_kernel<2, false, 1>
-                        : which == 2 ? stream_kernel<1, false, 1>
-                        : which      ? stream_kernel<2, false, 2>
-                                     : stream_kernel<1, false, 2>;
+    const int sets = a.rows > 8 ? 2 : 1;
     size_t smem = st_smem_bytes(sets, a.umax, a.rows, a.rows * a.slots, a.E);
     GF_REQUIRE(smem <= ST_MAX_SMEM, "routing table too large for the window kernel");
     // CTAs per SM.  One has shorter chains for few units (one token: 23.8 us a layer, 28.6 with two); two fill the decode pipes (16
@@ -783,7 +807,20 @@ int launch_stream(cudaStream_t s, StreamArgs a, bool pdl) {
     const long units = std::min<long>(pairs, a.umax) * (2L * ((a.H + 511) / 512) * (a.I / 128) + (long)((a.I + 511) / 512) * (a.H / 128));
     const int per_sm = units >= 9L * sms[dev] ? 2 : 1;
     a.two = per_sm == 2;
-    const dim3 grid((unsigned)(sms[dev] * per_sm)), block(ST_THREADS);
+    // Two teams of decode warps (sixteen) where one CTA has an SM and every unit is one stage of 256 k (a unit of more would have to stay
+    // with its team): eight warps form 15 weights a clock beside the other roles, sixteen 18 (47 layers of one row 1105 -> 1050 us, 8 with
+    // their router 257 -> 245).
+    const bool teams = per_sm == 1 && a.rows <= 16 && a.cut1.split == 16 && a.cut2.split == 16;
+    // (chunks have a kernel of their own: with their tables as a branch, windows of 11 rows were 1 % slower)
+    const int which = a.rows > 16 ? 4 : teams ? 4 + sets : sets - 1 + 2 * fine;
+    const auto kernel = which == 0   ? stream_kernel<1, false, 2, 1>
+                        : which == 1 ? stream_kernel<2, false, 2, 1>
+                        : which == 2 ? stream_kernel<1, false, 1, 1>
+                        : which == 3 ? stream_kernel<2, false, 1, 1>
+                        : which == 4 ? stream_kernel<2, true, 2, 1>
+                        : which == 5 ? stream_kernel<1, false, 2, 2>
+                                     : stream_kernel<2, false, 2, 2>;
+    const dim3 grid((unsigned)(sms[dev] * per_sm)), block(teams ? StWarps<2>::THREADS : StWarps<1>::THREADS);
     // One CTA per SM asks for more than half of the shared memory: next to a few CTAs of another kernel (the router of the next
     // layer) the second CTA of an emptier SM was placed before the first of a busier one (8 layers of one token with their
     // router 293 -> 266 us; 47 without 1140 -> 1144, whose next layer now sets up after this one).
