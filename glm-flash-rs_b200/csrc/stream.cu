@@ -106,7 +106,33 @@ struct StCta {
         give_up(GF_STATUS_TMA_TIMEOUT);
         return false;
     }
+    // The same for a whole warp, by the barrier's shared-memory address; the lanes go on together, or not at all.
+    __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity) const {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (__all_sync(0xffffffffu, ok != 0)) return true;
+        for (uint32_t i = 0;; ++i) {
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+            if (__all_sync(0xffffffffu, ok != 0)) return true;
+            bool end = *abort_flag != 0;
+            if (!end && (i & 255u) == 255u && *reinterpret_cast<volatile int *>(status) != 0) {
+                *abort_flag = 1;
+                end = true;
+            }
+            if (!end && i >= 4000000u) {
+                give_up(GF_STATUS_TMA_TIMEOUT);
+                end = true;
+            }
+            if (__any_sync(0xffffffffu, end)) return false;
+        }
+    }
 };
+// Arrival of a warp's first lane on a barrier of this CTA, predicated (no branch for the warp).
+__device__ __forceinline__ void arrive_lane0(uint32_t bar, int lane) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+}
 
 // Four words of this lane, polled until they carry the epoch (uniform result for the warp).
 __device__ __forceinline__ bool ll_wait4(const StCta &c, const unsigned long long *p, uint32_t epoch, unsigned long long (&w)[4]) {
@@ -515,17 +541,18 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         // ---------------------------------------------------------------------------------------------- decode
         if (TEAMS == 2) st_regs<false, 64>();
         const int G = lane >> 2, T = lane & 3, tile = warp & 7;
+        const uint32_t wfull0 = smem_u32(wfull), xfull0 = smem_u32(xfull), empty0 = smem_u32(empty);
         float acc[SETS][4];                                           // over a split
         for (uint32_t it = warp >> 3;; it += TEAMS) {
             const int s = it % ST_STAGES, phase = (it / ST_STAGES) & 1;
-            if (!__all_sync(0xffffffffu, cta.wait(wfull + s, phase))) break;
+            if (!cta.wait_warp(wfull0 + 8 * s, phase)) break;
             const int4 d = desc[s];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
             const int nmem = __popc(tb.mask[d.y]);
             const uint32_t p01 = *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 2 * T);
             const uint32_t p23 = SETS == 2 ? *reinterpret_cast<const uint32_t *>(tb.pair + d.y * 16 + 8 + 2 * T) : 0u;
-            if (!__all_sync(0xffffffffu, cta.wait(xfull + s, phase))) break;
+            if (!cta.wait_warp(xfull0 + 8 * s, phase)) break;
             if (!(d.x & DESC_CONT))
 #pragma unroll
                 for (int q = 0; q < SETS; ++q)
@@ -537,7 +564,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             if (SETS == 1 || nmem <= 8) st_decode<1, MANY, ROUNDS>(ws, xs, tile, lane, reinterpret_cast<float (&)[1][4]>(acc));
             else st_decode<SETS, MANY, ROUNDS>(ws, xs, tile, lane, acc);
             __syncwarp();
-            if (lane == 0) mbar_arrive(empty + s);
+            arrive_lane0(empty0 + 8 * s, lane);
             if (!(d.x & DESC_LAST)) continue;
             const int N = kind == UNIT_G ? I : H;
             unsigned long long *z = (kind == UNIT_G ? a.z1 : a.z2) + (unsigned)d.z + tile * 16 + 2 * G;
@@ -554,9 +581,10 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
         st_regs<false, 48>();
         // ---------------------------------------------------------------------------------------------- activations
         const int xw = warp - ST_DEC;
+        const uint32_t ready0 = smem_u32(ready), xfull0 = smem_u32(xfull);
         for (uint32_t it = 0;; ++it) {
             const int s = it % ST_STAGES;
-            if (!__all_sync(0xffffffffu, cta.wait(ready + s, (it / ST_STAGES) & 1))) break;
+            if (!cta.wait_warp(ready0 + 8 * s, (it / ST_STAGES) & 1)) break;
             const int4 d = desc[s];
             const int kind = d.x & 0xff;
             if (kind == UNIT_END) break;
@@ -585,7 +613,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             }
             __syncwarp();
             if (!ok) break;
-            if (lane == 0) mbar_arrive(xfull + s);
+            arrive_lane0(xfull0 + 8 * s, lane);
         }
     } else if (warp >= ST_FIN) {
         st_regs<true, TEAMS == 2 ? 176 : 80>();
