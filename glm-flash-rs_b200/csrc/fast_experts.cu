@@ -15,8 +15,8 @@
 //             (in 32): tcgen05.mma.cta_group::2, M 256 x N <= 256 x K 16 -- each CTA decodes one of the two column blocks and brings half of
 //             the rows, and holds its columns' accumulators of all rows.  Roles:
 //               warp 0       TMA producer of the rows (half of the chunk's x 128 k per stage)
-//               warp 1       first CTA: issues the MMAs of the pair, commits stages and passes to both CTAs; second CTA: relays
-//                            "my rows of the stage are there" to the first
+//               warp 1       first CTA: issues the MMAs of the pair, commits stages and passes to both CTAs.  It waits for one barrier a
+//                            stage, on which the rows' bytes and the decode warps of both CTAs count
 //               warp 2       allocates / frees tensor memory (512 columns)
 //               warp 3       TMA producer of the packed words, a ring of its own
 //               warps 4-11   epilogue: 32 rows x 128 columns at a time from tensor memory, transposed through shared memory so that four
@@ -29,13 +29,15 @@
 //             epilogue overlaps the next item's gate pass.  Down is one pass per item.
 //             Before, the rows were M (256 a tile, filled or not) and the weights went through shared memory: a chunk of 40 rows cost as
 //             much as one of 256, an expert of 257 rows twice as much as one of 256.  us gate/up | down, before -> now: 500 rows 197 | 101
-//             -> 143 | 73, 4096 rows 350 | 181 -> 280 | 139, eight experts of 64 at 4096 rows 81 | 39 -> 52 | 34 (2048 x 1536, 64 experts,
-//             top-4); 8192 rows of 4096 x 512, 288 experts, top-8: 587 | 697 -> 559 | 539.  What bounds it now: at 4096 rows instruction
-//             issue (0.71 of the cycles while all SMs work: decode, epilogue) and the last round of items (0.87 of the time); at 500 rows the
-//             issuing warp, about 1,000 clocks a stage of its own beside the busy decode warps; short K (512): the epilogue's stores.
-//             Tried: three epilogue warpgroups of 104 registers (309 against 280 us), the words' copies prefetched to L2 a pass ahead (no
-//             change), stages of 64 k (158 | 83 at 500 rows: the same steps for half the work), silu(gate) in shared memory (chunks of 256 rows
-//             then: 314 | 157 at 4096).
+//             -> 132 | 68, 4096 rows 350 | 181 -> 274 | 136, eight experts of 64 at 4096 rows 81 | 39 -> 49 | 33 (2048 x 1536, 64 experts,
+//             top-4); 8192 rows of 4096 x 512, 288 experts, top-8: 587 | 697 -> 540 | 505.  What bounds it now: instruction issue (0.70 to 0.80 of the
+//             cycles while all SMs work: decode, epilogue) and the last round of items (0.82 to 0.87 of the time); short K (512): the
+//             epilogue, which a pass of four stages does not cover.
+//             Tried: more epilogue warps (three warpgroups of 104 registers 309 against 280 us at 4096 rows; four and eight decode warps for
+//             down 157 against 139, 8192 rows 687 against 530), the words' copies prefetched to L2 a pass ahead and deeper rings of rows
+//             or words (no change; two stages of words: 190 against 143 at 500 rows), stages of 64 k (158 | 83 at 500 rows: the same steps
+//             for half the work), silu(gate) in shared memory (chunks of 256 rows then: 314 | 157 at 4096), down's rows out by bulk copies (640
+//             against 530 at 8192 rows).
 // Arithmetic: one full-K fp32 accumulation chain per output (as upstream's prefill path, which is likewise not
 // bit-equal to its decode path: native/exl3_prefill.cu:20-23), the same transforms and rounding points as
 // upstream's epilogue (native/exl3_prefill.cu:596-622 == native/exl3.cu:260-321) with exp / divide in their fast
@@ -355,15 +357,22 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 // kind::f16: D fp32, A and B fp16, both K-major, M 256 (the pair's columns of the matrix), N rows
 __device__ __forceinline__ uint32_t umma_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(2 * FG_BN >> 4) << 24); }
 
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+// Tensor copy of one CTA of a pair whose bytes count on a barrier of either of them (its address in the cluster).
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
         : "memory");
+}
+// address in the cluster of the barrier at the same offset in CTA `cta`
+__device__ __forceinline__ uint32_t mbar_of_cluster(uint64_t *bar, uint32_t cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(bar)), "r"(cta));
+    return r;
 }
 
 // Wait on an mbarrier phase, giving up when the abort flag is up or after a bounded number of polls.  SLEEP: nanoseconds a poll may
-// sleep; every role but the two on the critical path (MMA issue, relay) sleeps, because two dozen polling warps delay those two
+// sleep; every role but the one on the critical path (MMA issue) sleeps, because two dozen polling warps delay it
 // by some 200 clocks per wait.
 template <uint32_t SLEEP>
 __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
@@ -424,6 +433,40 @@ __device__ __forceinline__ void fwht128_quad(float (&v)[32], int t) {
     in_lane(16);
 }
 
+// The same for a whole warp, by the barrier's shared-memory address; the lanes go on together, or not at all.
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
+    for (uint32_t i = 0;; ++i) {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity), "r"(500u) : "memory");
+        if (__all_sync(0xffffffffu, ok != 0)) return true;
+        bool end = *abort_flag != 0;
+        if (!end && (i & 15u) == 15u) end = *reinterpret_cast<volatile int *>(status) != 0;
+        if (!end && i >= 4000000u) {
+            atomicExch(status, code);
+            end = true;
+        }
+        if (__any_sync(0xffffffffu, end)) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+// Arrival of a warp's first lane, predicated (no branch for the warp): on a barrier of this CTA, or by its address in the cluster.
+template <bool CLUSTER>
+__device__ __forceinline__ void mbar_arrive_lane0(uint32_t bar, int lane) {
+    if (CLUSTER) asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+    else asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+}
+
 struct FastGemmArgs {
     const int *plan, *src_pair;
     const int4 *chunks;            // {expert, first grouped row, rows, -}
@@ -460,6 +503,11 @@ struct Ring {
     __device__ __forceinline__ void next(uint32_t depth) {
         if (++slot == depth) { slot = 0; parity ^= 1; }
     }
+    template <uint32_t N>
+    __device__ __forceinline__ void skip(uint32_t depth) {                  // N < depth
+        slot += N;
+        if (slot >= depth) { slot -= depth; parity ^= 1; }
+    }
 };
 
 struct FgMaps {
@@ -470,23 +518,21 @@ struct FgMaps {
 // Tensor memory: columns [0, 192) three stages of decoded weights (64 columns = 128 k), [192, 512) accumulators.  Even passes have theirs
 // at the lower end, odd ones at the upper, so that two of up to 160 rows have room side by side; longer ones wait until the epilogue has
 // taken out the columns that they share with the last pass, while the decode fills the stages.
-constexpr int FG_ASTAGES = 3, FG_ACOLS = FG_BK / 2, FG_DCOL = FG_ASTAGES * FG_ACOLS, FG_DCOLS = 512 - FG_DCOL;
+constexpr int FG_STAGES = 3, FG_ACOLS = FG_BK / 2, FG_DCOL = FG_STAGES * FG_ACOLS, FG_DCOLS = 512 - FG_DCOL;
 static_assert(FG_DCOLS >= FG_CHUNK, "accumulators of a pass");
 
 template <int MATS>
 struct FgCfg {
-    static constexpr int BSTAGES = 4;                        // rows
     static constexpr int WSTAGES = 4;                        // packed words
-    static constexpr int DONE = 4;                           // ring of stage-completed barriers (at least as deep as any ring)
     // Waits go by the parity of a phase: whoever waits for one has to know that the phase before it is over.  The decode warps take every
     // second stage, so the stage in front of theirs in a slot of words has to be one of theirs as well: copies land in any order.  (The MMAs
     // of stages complete in order.)
     static_assert(WSTAGES % 2 == 0, "words of the decode warps");
-    static_assert(DONE >= BSTAGES && DONE >= FG_ASTAGES, "ring of completed stages");
     static constexpr int SCALES = MATS == 2 ? 3 * 128 : 128, SCALE_BUFS = MATS == 2 ? 1 : 2;   // scale vectors of an item, of one or two items
     static constexpr int TABLE_BYTES = 256 + SCALE_BUFS * SCALES * 4;                        // barriers, scale vectors
+    static_assert((2 * FG_STAGES + 2 * WSTAGES + 6 + 1) * 8 <= 256, "barriers");
     static constexpr int TBUF_BYTES = 2 * 32 * 128 * 4;                                      // per epilogue warpgroup a slab of 32 rows
-    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)BSTAGES * FG_TILE_BYTES + (size_t)WSTAGES * FG_WORD_BYTES + TABLE_BYTES + TBUF_BYTES;
+    static constexpr size_t SMEM = 1024 /*align*/ + (size_t)FG_STAGES * FG_TILE_BYTES + (size_t)WSTAGES * FG_WORD_BYTES + TABLE_BYTES + TBUF_BYTES;
 };
 
 // Registers per thread: launched with 72 x 896; the producer warpgroup gives to the two epilogue warpgroups (24 + 2 x 160 + 4 x 40 = 504).
@@ -508,14 +554,13 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
     using C = FgCfg<MATS>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // 1024-aligned operand tiles
-    unsigned char *bring = smem;                                           // [BSTAGES] rows
-    unsigned char *wring = bring + (size_t)C::BSTAGES * FG_TILE_BYTES;     // [WSTAGES] packed words
+    unsigned char *bring = smem;                                           // [FG_STAGES] rows
+    unsigned char *wring = bring + (size_t)FG_STAGES * FG_TILE_BYTES;      // [WSTAGES] packed words
     float *tbuf = reinterpret_cast<float *>(wring + (size_t)C::WSTAGES * FG_WORD_BYTES);             // [2 groups][32 rows][128]
     unsigned char *tables = reinterpret_cast<unsigned char *>(tbuf) + C::TBUF_BYTES;
-    uint64_t *bfull = reinterpret_cast<uint64_t *>(tables);                // [BSTAGES] rows landed (first CTA: in both)
-    uint64_t *afull = bfull + C::BSTAGES;                                  // [FG_ASTAGES] (first CTA) decoded, in both
-    uint64_t *done = afull + FG_ASTAGES;                                   // [DONE] MMAs of stage i completed: done[i % DONE]
-    uint64_t *wfull = done + C::DONE;                                      // [WSTAGES] packed words landed
+    uint64_t *full = reinterpret_cast<uint64_t *>(tables);                 // [FG_STAGES] (first CTA) rows landed and weights decoded, in both
+    uint64_t *done = full + FG_STAGES;                                     // [FG_STAGES] MMAs of the stage completed
+    uint64_t *wfull = done + FG_STAGES;                                    // [WSTAGES] packed words landed
     uint64_t *wempty = wfull + C::WSTAGES;                                 // [WSTAGES] read by the stage's decode warps
     uint64_t *tmem_full = wempty + C::WSTAGES;                             // [2] accumulators of a pass complete
     uint64_t *tmem_empty = tmem_full + 2;                                  // [2] (first CTA) accumulators drained, both CTAs' warps
@@ -529,9 +574,7 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
     const int KT = a.K >> 4, NBP = a.N >> 8, KS = a.K / FG_BK;
 
     if (tid == 0) {
-        for (int s = 0; s < C::BSTAGES; ++s) mbar_init(bfull + s, 1 + (rank == 0));
-        for (int s = 0; s < FG_ASTAGES; ++s) mbar_init(afull + s, FG_DEC);
-        for (int s = 0; s < C::DONE; ++s) mbar_init(done + s, 1);
+        for (int s = 0; s < FG_STAGES; ++s) { mbar_init(full + s, 1 + FG_DEC); mbar_init(done + s, 1); }
         for (int s = 0; s < C::WSTAGES; ++s) { mbar_init(wfull + s, 1); mbar_init(wempty + s, FG_DEC / 2); }
         for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + b, 1); mbar_init(tmem_empty + b, 16); mbar_init(tmem_early + b, 16); }
         *abort_flag = 0;
@@ -545,22 +588,21 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
     pdl_wait();
     pdl_launch_dependents();
     const int total = a.plan[2] * NBP, items = total > pair ? (total - pair + pairs - 1) / pairs : 0;
-    // the slot that stage `it` of a ring of `depth` stages takes is free: stage it - depth has been consumed
-    auto slot_free = [&](uint32_t it, uint32_t depth) {
-        if (it < depth) return true;
-        const uint32_t j = it - depth;
-        return wait_or_abort<FG_SLEEP>(done + j % C::DONE, (j / C::DONE) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT);
+    // the slot that stage `it` takes is free: stage it - FG_STAGES has been consumed
+    auto slot_free = [&](uint32_t it) {
+        return it < FG_STAGES || wait_or_abort<FG_SLEEP>(done + it % FG_STAGES, (it / FG_STAGES - 1) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT);
     };
-
     // after a give-up: the copies in flight, if any, have landed before the CTA leaves (bounded)
     auto land = [&](uint64_t *bar, uint32_t depth, uint32_t it) {
         for (uint32_t k = it > depth ? it - depth : 0; k < it; ++k) mbar_wait(bar + k % depth, (k / depth) & 1, nullptr, 1000u);
     };
 
     if (warp < 4) {
-        // ------------------------------------------------------------------ warpgroup 0: TMA, MMA issue, relay
+        // ------------------------------------------------------------------ warpgroup 0: TMA, MMA issue
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_MMA));
         if (warp == 0 && lane == 0) {
+            // (the copies of both CTAs count on the first one's barrier)
+            const uint32_t full0 = mbar_of_cluster(full, 0);
             uint32_t it = 0;
             bool ok = true;
             for (Items t(a.chunks, pair, total, pairs, NBP); ok && !*abort_flag && t.advance();) {
@@ -569,20 +611,20 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                 for (int pm = 0; pm < MATS && ok; ++pm) {
                     const CUtensorMap *map = maps.rows[pm == 1 && !a.shared_x], *map1 = map + (n1 >> 5) - 1, *map2 = map + max((n2 >> 5) - 1, 0);
                     for (int s = 0; s < KS; ++s, ++it) {
-                        const uint32_t slot = it % C::BSTAGES;
-                        if (!slot_free(it, C::BSTAGES)) { ok = false; break; }
-                        mbar_expect_tx(bfull + slot, (uint32_t)t.n * FG_BK);
+                        const uint32_t slot = it % FG_STAGES, bar = full0 + 8 * slot;
+                        if (!slot_free(it)) { ok = false; break; }
+                        if (rank == 0) mbar_expect_tx(full + slot, (uint32_t)t.n * FG_BK * 2);        // (of both CTAs)
                         unsigned char *dst = bring + slot * FG_TILE_BYTES;
-                        tma_load_2d(dst, map1, s * FG_BK, row1, bfull + slot);
-                        tma_load_2d(dst + FG_HALF_BYTES, map1, s * FG_BK + 64, row1, bfull + slot);
+                        tma_load_2d_pair(dst, map1, s * FG_BK, row1, bar);
+                        tma_load_2d_pair(dst + FG_HALF_BYTES, map1, s * FG_BK + 64, row1, bar);
                         if (n2) {
-                            tma_load_2d(dst + 128 * 128, map2, s * FG_BK, row2, bfull + slot);
-                            tma_load_2d(dst + 128 * 128 + FG_HALF_BYTES, map2, s * FG_BK + 64, row2, bfull + slot);
+                            tma_load_2d_pair(dst + 128 * 128, map2, s * FG_BK, row2, bar);
+                            tma_load_2d_pair(dst + 128 * 128 + FG_HALF_BYTES, map2, s * FG_BK + 64, row2, bar);
                         }
                     }
                 }
             }
-            if (!ok) land(bfull, C::BSTAGES, it);
+            if (!ok || *abort_flag) land(rank ? done : full, FG_STAGES, it);      // (the second CTA's copies count elsewhere: it stays that long)
         } else if (warp == 1 && rank == 0) {
             // One elected thread of this warp issues every MMA of the pair; the warp runs the loop together, so that the descriptors
             // stay in uniform registers.  Its instruction stream is the critical path of the tensor pipe: ring positions and parities are
@@ -590,7 +632,7 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
             // the shared-memory descriptor is built once and advanced by adding constants (the address field
             // counts 16-byte units, a K step of 16 halves is 32 bytes; of A: eight columns).
             const uint64_t desc_b0 = umma_desc_sw128(smem_u32(bring));
-            Ring ra{0, 0}, rb{0, 0}, rd{0, 0};
+            Ring ring{0, 0};
             uint32_t pc = 0;
             int before = 0;                                          // rows of the pass in front
             bool ok = true;
@@ -607,12 +649,11 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                     tc_fence_after();
                     const uint32_t d0 = tmem_base + FG_DCOL + (pb ? FG_DCOLS - t.n : 0);
                     for (int s = KS; s; --s) {
-                        ok = __all_sync(0xffffffffu, wait_or_abort<0>(bfull + rb.slot, rb.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
-                                                         wait_or_abort<0>(afull + ra.slot, ra.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
+                        ok = __all_sync(0xffffffffu, wait_or_abort<0>(full + ring.slot, ring.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
                         if (!ok) break;
                         tc_fence_after();
-                        const uint64_t db = desc_b0 + rb.slot * (FG_TILE_BYTES >> 4);
-                        const uint32_t ta = tmem_base + ra.slot * FG_ACOLS, first = s != KS;
+                        const uint64_t db = desc_b0 + ring.slot * (FG_TILE_BYTES >> 4);
+                        const uint32_t ta = tmem_base + ring.slot * FG_ACOLS, first = s != KS;
                         if (elect_one()) {
 #pragma unroll
                             for (int kk = 0; kk < FG_BK / 16; ++kk) {
@@ -620,11 +661,11 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                                 umma_f16(d0, ta + 8 * kk, dk, idesc, kk > 0 ? 1u : first);
                                 if (n2) umma_f16(d0 + 256, ta + 8 * kk, dk + (128 * 128 >> 4), idesc2, kk > 0 ? 1u : first);
                             }
-                            umma_commit(done + rd.slot);            // both CTAs may overwrite the stage once these MMAs have read it
+                            umma_commit(done + ring.slot);          // both CTAs may overwrite the stage once these MMAs have read it
                             if (s == 1) umma_commit(tmem_full + pb);           // the accumulators of this pass are complete
                         }
                         __syncwarp();
-                        ra.next(FG_ASTAGES); rb.next(C::BSTAGES); rd.next(C::DONE);
+                        ring.next(FG_STAGES);
                     }
                 }
             }
@@ -641,16 +682,7 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                         tma_load_3d(wring + ws * FG_WORD_BYTES, &maps.bank[pm], 0, t.e * KT + 8 * s, (2 * t.nbp + rank) * 8, wfull + ws);
                     }
             }
-            if (!ok) land(wfull, C::WSTAGES, it);
-        } else if (warp == 1 && lane == 0) {
-            // second CTA: tell the issuing thread that this CTA's rows of a stage are there (its decode warps say so themselves)
-            uint32_t it = 0;
-            bool ok = true;
-            for (const uint32_t stages = (uint32_t)(items * MATS * KS); it < stages && ok; ++it) {
-                const uint32_t sb = it % C::BSTAGES;
-                ok = wait_or_abort<0>(bfull + sb, (it / C::BSTAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
-                if (ok) mbar_arrive_cluster(bfull + sb, 0);
-            }
+            if (!ok || *abort_flag) land(wfull, C::WSTAGES, it);
         }
     } else if (warp < 12) {
         // ------------------------------------------------------------------ warpgroups 1-2: epilogue
@@ -667,11 +699,11 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
         // scale vectors of an item: fetched while the one before it runs, by both warpgroups (the 1 / sqrt(128) of every Hadamard transform is
         // folded into them, the transform is linear: one multiply per element less in each epilogue step)
         Items t(a.chunks, pair, total, pairs, NBP);
-        float sc0 = 0.f, sc1 = 0.f;
+        __half sc0, sc1;                                     // (converted when they are used: the loads are not waited for)
         auto fetch = [&](int item, int e) {
             const size_t o = (size_t)e * a.N + (2 * (item % NBP) + rank) * 128 + (em & 127);
-            if (em < 128) sc0 = __half2float(a.sv0[o]);
-            else if (MATS == 2) { sc0 = __half2float(a.sv1[o]); sc1 = __half2float(a.sd[o]); }
+            if (em < 128) sc0 = a.sv0[o];
+            else if (MATS == 2) { sc0 = a.sv1[o]; sc1 = a.sd[o]; }
         };
         if (pair < total) fetch(pair, t.next.x);
         // A warpgroup decides together whether a wait has given up: a warp never stands alone at a barrier.  One that has goes on through the
@@ -680,8 +712,8 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
             const int nb = 2 * t.nbp + rank;
             float *sc = scales + (C::SCALE_BUFS == 2 ? (turn++ & 1) * C::SCALES : 0);
             if (C::SCALE_BUFS == 1) asm volatile("bar.sync 1, 256;" ::: "memory");           // (the last item's have been read)
-            if (em < 128) sc[em] = sc0 * HAD_SCALE;
-            else if (MATS == 2) { sc[em] = sc0 * HAD_SCALE; sc[em + 128] = sc1 * HAD_SCALE; }
+            if (em < 128) sc[em] = __half2float(sc0) * HAD_SCALE;
+            else if (MATS == 2) { sc[em] = __half2float(sc0) * HAD_SCALE; sc[em + 128] = __half2float(sc1) * HAD_SCALE; }
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (!ok) continue;
             if (t.item + t.step < total) fetch(t.item + t.step, t.next.x);
@@ -724,10 +756,10 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                         for (int j = 0; j < 8; ++j) gate[j] = *reinterpret_cast<const uint2 *>(o + 16 * j);
                     if (MATS == 1 && here) p = __ldg(a.src_pair + t.row + row);
                     group_barrier(group);
-                    const float *src = slab + rr * 128 + t4;
+                    const float *even = slab + rr * 128 + t4 + (rr & 1) * 16, *odd = slab + rr * 128 + t4 - (rr & 1) * 16;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float4 f = *reinterpret_cast<const float4 *>(src + (16 * j ^ ((rr & 1) * 16)));
+                        const float4 f = *reinterpret_cast<const float4 *>((j & 1 ? odd : even) + 16 * j);
                         x[4 * j] = f.x; x[4 * j + 1] = f.y; x[4 * j + 2] = f.z; x[4 * j + 3] = f.w;
                     }
                     fwht128_quad(x, m & 3);
@@ -791,30 +823,34 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
         }
         // the arrivals of the last commits have come in before this CTA ends (the accumulators are complete: these are on their way)
         const uint32_t stages = (uint32_t)(items * MATS * KS);
-        for (uint32_t k = stages > C::DONE ? stages - C::DONE : 0; k < stages && ok; ++k)
-            ok = wait_or_abort<FG_SLEEP>(done + k % C::DONE, (k / C::DONE) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
+        for (uint32_t k = stages > FG_STAGES ? stages - FG_STAGES : 0; k < stages && ok; ++k)
+            ok = wait_or_abort<FG_SLEEP>(done + k % FG_STAGES, (k / FG_STAGES) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
     } else {
         // ------------------------------------------------------------------ warpgroups 3-6: trellis decode
         // A warp takes every second stage and, of it, one of the two n-tiles (16 columns) whose lanes of tensor memory it may write.  A lane
         // reads word number `lane` of a tile and the word in front of it: those are k 2 T, 2 T + 1, 2 T + 8, 2 T + 9 of columns G and G + 8,
         // just the places that tcgen05.st gives it.  The first half of the stage is decoded before the slot is free.
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FG_REGS_DEC));
+        // Beside the 320 instructions of a warp's share of a stage (64 weights a lane) the loop had 125 of its own with modulo arithmetic, generic
+        // addresses and branches around single arrivals, and this kernel is bound by instruction issue (500 rows: 0.80 of the active
+        // cycles): addresses and parities are counted along, arrivals are predicated.
         const int q = warp & 3, half = (warp >> 2) & 1;
         const uint32_t stages = (uint32_t)(items * MATS * KS);
         const uint32_t lanes = tmem_base + ((uint32_t)(q * 32 + half * 16) << 16);
-        const unsigned char *words = wring + (2 * q + half) * 1024;
-        for (uint32_t it = (warp - 12) >> 3; it < stages; it += 2) {
-            const uint32_t ws = it % C::WSTAGES, sa = it % FG_ASTAGES;
-            // (the vote also brings the lanes together again: they may have left the wait apart)
-            if (!__all_sync(0xffffffffu, wait_or_abort<FG_SLEEP>(wfull + ws, (it / C::WSTAGES) & 1, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT))) break;
-            const uint32_t *wp = reinterpret_cast<const uint32_t *>(words + ws * FG_WORD_BYTES);
+        const uint32_t words0 = smem_u32(wring) + (2 * q + half) * 1024, word = words0 + lane * 4, before = words0 + ((lane + 31) & 31) * 4;
+        const uint32_t wfull0 = smem_u32(wfull), wempty0 = smem_u32(wempty), done0 = smem_u32(done), full0 = mbar_of_cluster(full, 0);
+        const uint32_t first = (warp - 12) >> 3;
+        Ring rw{first, 0}, rs{first, 1};                     // (the first turn of a stage's slot waits for nothing: the phase before the first is over)
+        for (uint32_t it = first; it < stages; it += 2) {
+            if (!wait_warp(wfull0 + 8 * rw.slot, rw.parity, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT)) break;
+            const uint32_t at = rw.slot * FG_WORD_BYTES;
             bool ok = true;
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h, wp += 128) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
                 uint32_t o[16];
 #pragma unroll
                 for (int kt = 0; kt < 4; ++kt) {
-                    const uint32_t w = wp[kt * 32 + lane], pw = wp[kt * 32 + ((lane + 31) & 31)];
+                    const uint32_t w = lds32(word + at + h * 512 + kt * 128), pw = lds32(before + at + h * 512 + kt * 128);
                     uint32_t hi[4], lo[4];
                     codeword_pair(__funnelshift_r(w, pw, 12), hi[0], lo[0]);                 // k = 2 T:     columns G, G + 8
                     codeword_pair(__funnelshift_r(w, pw, 8), hi[1], lo[1]);                  // k = 2 T + 1
@@ -826,21 +862,21 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                     o[4 * kt + 3] = __byte_perm(weight_dup(lo[2]), weight_dup(lo[3]), 0x5410);
                 }
                 if (h == 0) {
-                    ok = __all_sync(0xffffffffu, slot_free(it, FG_ASTAGES));
+                    ok = wait_warp(done0 + 8 * rs.slot, rs.parity, abort_flag, a.status, GF_STATUS_TMA_TIMEOUT);
                     if (!ok) break;
-                    __syncwarp();                            // (tcgen05.st is for the warp as one: the lanes may have left the wait apart)
                     tc_fence_after();
                 }
-                tmem_st16(lanes + sa * FG_ACOLS + h * (FG_ACOLS / 2), o);
+                tmem_st16(lanes + rs.slot * FG_ACOLS + h * (FG_ACOLS / 2), o);
             }
             if (!ok) break;
             __syncwarp();
-            if (lane == 0) mbar_arrive(wempty + ws);
-            __syncwarp();
+            mbar_arrive_lane0<false>(wempty0 + 8 * rw.slot, lane);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(afull + sa, 0);
+            mbar_arrive_lane0<true>(full0 + 8 * rs.slot, lane);
+            rw.skip<2>(C::WSTAGES);
+            rs.skip<2>(FG_STAGES);
         }
     }
 
