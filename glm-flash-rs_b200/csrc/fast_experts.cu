@@ -5,7 +5,7 @@
 // fast_down_large (native/exl3_prefill.cu:402-430,657-889), which decode each 16x16 trellis tile into mma.sync
 // fragments in registers.  Here:
 //
-//   plan      members per distinct expert, chunks of at most 320 rows (as even as an expert's rows go, long ones first) and the
+//   plan      members per distinct expert, chunks of at most 320 or 160 rows (as even as an expert's rows go, long ones first) and the
 //             GROUPED row order (rows of an expert contiguous): src_pair[j] = pair index of grouped row j.
 //   rot       the input rotation writes Xs[j] = fp16(H(x[row] * suh[e]) / sqrt 128) in grouped order, so the rows of a chunk are
 //             a contiguous slab that TMA tensor loads bring into shared memory in the 128-byte-swizzled K-major layout the tensor
@@ -74,10 +74,11 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
                                                           const int *__restrict__ members, int maxm, int slots, int E,
                                                           int shared_exl3, int e_lo, int e_hi, int srow_lo, int srow_hi,
                                                           int *__restrict__ plan, int4 *__restrict__ chunks,
-                                                          int *__restrict__ src_pair, int *__restrict__ row_expert) {
+                                                          int *__restrict__ src_pair, int *__restrict__ row_expert, int nbp, int workers) {
     __shared__ int cnt_sh[FG_MAXU], row_sh[FG_MAXU], e_sh[FG_MAXU], first_sh[FG_MAXU], order_sh[FG_MAXU];
-    __shared__ int wsum[3][32];
+    __shared__ int wsum[3][32], at_sh, classes_sh[2][12], cost_sh[2];
     const int u = threadIdx.x, lane = u & 31, warp = u >> 5;
+    if (u < 24) classes_sh[u / 12][u % 12] = 0;
     pdl_wait();                                             // (every kernel of the chain: nothing is read or written before)
     pdl_launch_dependents();
     const int n = min(count[0], FG_MAXU);
@@ -86,31 +87,61 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
         e = ids[u];
         if (!expert_skipped(e, E, shared_exl3, e_lo, e_hi)) {
             const int *m = members + (size_t)u * maxm;
-            int lo = 0, hi = maxm;                          // members come first: the count is the first -1
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (m[mid] >= 0) lo = mid + 1; else hi = mid;
-            }
-            cnt = lo;
+            // the first place in [0, end) whose member is past something that the list does not come back from, else end.  Seven probes a
+            // step: a list of 8192 takes five trips through L2 instead of thirteen
+            auto first_past = [&](int end, auto past) {
+                int lo = 0, hi = end;
+                while (lo < hi) {
+                    const int step = (hi - lo + 7) >> 3;    // probes at the ends of the first seven of eight parts
+                    int below = 0;
+#pragma unroll
+                    for (int i = 1; i < 8; ++i) below += lo + i * step <= hi && !past(m[min(lo + i * step, hi) - 1]);
+                    hi = below < 7 ? min(hi, lo + (below + 1) * step - 1) : hi;
+                    lo = lo + below * step;
+                }
+                return lo;
+            };
+            cnt = first_past(maxm, [](int code) { return code < 0; });       // members come first, then -1
             if (e == E && srow_hi > srow_lo) {
                 // the shared expert is computed here for a window of rows only: members ascend by row (code = row * 32
                 // + slot), so the window is a contiguous run of the list
-                auto lower = [&](int row) {                 // first member whose row is >= `row`
-                    int a = 0, b = cnt;
-                    while (a < b) {
-                        const int mid = (a + b) >> 1;
-                        if ((m[mid] >> 5) < row) a = mid + 1; else b = mid;
-                    }
-                    return a;
-                };
-                first = lower(srow_lo);
-                cnt = lower(srow_hi) - first;
+                first = first_past(cnt, [=](int code) { return (code >> 5) >= srow_lo; });
+                cnt = first_past(cnt, [=](int code) { return (code >> 5) >= srow_hi; }) - first;
             }
         }
     }
-    // chunks of at most 320 rows, as even as they go, in the order of their length (in 32 rows, long ones first), so that the static
-    // round robin over the CTA pairs takes about equal ones in a turn and ends with the short ones
-    const int tiles = (cnt + 127) / 128, nch = (cnt + FG_CHUNK - 1) / FG_CHUNK, size = nch ? (cnt + nch - 1) / nch : 0;
+    // Chunks of at most 320 rows, or of 160: twice as many decode the weights twice, but a few long ones (the shared expert's, at 500 rows)
+    // hold up their pairs: 135 against 128 us (gate / up), at 4096 rows 284 against 344.  What the gate / up items cost the pairs that
+    // have the longest of every turn, in clocks a stage: 1,000 for the decode or 4.4 a row for the MMAs.
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int cap = FG_CHUNK >> i, n_i = (cnt + cap - 1) / cap;
+        if (n_i) atomicAdd(&classes_sh[i][((cnt + n_i - 1) / n_i + 31) >> 5], n_i);
+    }
+    __syncthreads();
+    if (warp < 2) {
+        const int *classes = classes_sh[warp];
+        int all = 0, cost = 0;
+        for (int k = 1; k <= FG_CHUNK / 32; ++k) all += classes[k];
+        const int turns = (all * nbp + workers - 1) / workers;
+        for (int t = lane; t < turns; t += 32) {
+            const int place = t * workers / nbp;            // the turn's first chunk, and its class
+            int k = FG_CHUNK / 32 + 1, longer = 0;
+#pragma unroll
+            for (int c = FG_CHUNK / 32; c >= 1; --c)
+                if (longer <= place) { k = c; longer += classes[c]; }
+            cost += max(1000, 141 * k);
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) cost += __shfl_xor_sync(0xffffffffu, cost, d);
+        if (lane == 0) cost_sh[warp] = cost;
+    }
+    __syncthreads();
+    const int cap = cost_sh[1] < cost_sh[0] ? FG_CHUNK / 2 : FG_CHUNK;
+    // as even as they go, in the order of their length (in 32 rows, long ones first), so that the static round robin over the CTA pairs takes
+    // about equal ones in a turn and ends with the short ones
+    const int tiles = (cnt + 127) / 128, nch = (cnt + cap - 1) / cap, size = nch ? (cnt + nch - 1) / nch : 0;
     const int key = (size + 31) >> 5;
     // block-wide exclusive scan of rows, totals of tiles and chunks
     int r_inc = cnt, t_inc = tiles, c_inc = nch;
@@ -121,6 +152,7 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
     }
     if (lane == 31) { wsum[0][warp] = r_inc; wsum[1][warp] = t_inc; wsum[2][warp] = c_inc; }
     order_sh[u] = key << 16 | nch;
+    if (u == 0) at_sh = 0;
     __syncthreads();
     int r_off = 0, r_all = 0, t_all = 0, c_all = 0;
     for (int w = 0; w < 32; ++w) {
@@ -130,15 +162,19 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
     const int r_ex = r_off + r_inc - cnt;
     cnt_sh[u] = cnt; row_sh[u] = r_ex; e_sh[u] = e; first_sh[u] = first;
     if (u == 0 && blockIdx.x == 0) { plan[0] = t_all; plan[1] = r_all; plan[2] = c_all; }
-    if (u < n && u % (int)gridDim.x == (int)blockIdx.x) {
-        int at = 0;                                         // chunks of longer ones, and of experts in front with as long ones
-        for (int w = 0; w < n; ++w) {
-            const int o = order_sh[w], k = o >> 16;
-            if (k > key || (k == key && w < u)) at += o & 0xffff;
-        }
-        for (int c = 0; c < nch; ++c) chunks[at + c] = make_int4(e, r_ex + c * size, min(size, cnt - c * size), 0);
+    // chunks of this block's expert (there are at least as many blocks as experts): behind those of longer ones and of experts in front with as
+    // long ones, counted by all threads
+    const int b = blockIdx.x;
+    if (b < n) {
+        const int mine = order_sh[b] >> 16;
+        int at = key > mine || (key == mine && u < b) ? nch : 0;
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) at += __shfl_xor_sync(0xffffffffu, at, d);
+        if (lane == 0 && at) atomicAdd(&at_sh, at);
     }
     __syncthreads();
+    if (u == b && u < n)
+        for (int c = 0; c < nch; ++c) chunks[at_sh + c] = make_int4(e, r_ex + c * size, min(size, cnt - c * size), 0);
     for (int uu = blockIdx.x; uu < n; uu += gridDim.x) {
         const int c = cnt_sh[uu], rb = row_sh[uu], ee = e_sh[uu], f0 = first_sh[uu];
         for (int m = u; m < c; m += FG_MAXU) {
@@ -951,7 +987,7 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
     pool.take(&f->xd, P * I * 2);
     pool.take(&f->out, P * H * 4);
     pool.take(&f->plan, PLAN_INTS * 4);
-    pool.take(&f->chunks, (P / FG_CHUNK + cfg->experts + 1) * sizeof(int4));
+    pool.take(&f->chunks, (P / (FG_CHUNK / 2) + cfg->experts + 1) * sizeof(int4));
     pool.take(&f->src_pair, P * 4);
     pool.take(&f->row_expert, P * 4);
     pool.take(&f->status, 16);
@@ -986,7 +1022,7 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
     const bool pdl = c.pdl != 0;                            // a kernel's launch and set-up overlap the tail of the one in front
     if (f->phases & 1)
         if (launch_k(fast_plan_kernel, dim3((unsigned)c.experts + 1), dim3(FG_MAXU), 0, s, pdl, ids, count, members, maxm, c.slots, c.experts,
-                     c.shared_exl3, c.expert_lo, c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->chunks, f->src_pair, f->row_expert))
+                     c.shared_exl3, c.expert_lo, c.expert_hi, c.shared_row_lo, c.shared_row_hi, f->plan, f->chunks, f->src_pair, f->row_expert, I / 256, f->sms / 2))
             return -1;
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)

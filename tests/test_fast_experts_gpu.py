@@ -247,6 +247,36 @@ def test_input_rows_of_odd_strides(pkg, oracle, synth, cuda, h):
     assert (got[0] == got[1]).all()
 
 
+@pytest.mark.parametrize("rows,e", [(500, 64), (900, 64), (3000, 16), (40, 3)])
+def test_chunk_length(pkg, oracle, synth, cuda, rows, e):
+    """The plan cuts chunks of 160 rows where a few long experts would hold up the rest, else of 320: the rows are all there once, and their
+    bytes are those of the other cut (a call of fewer experts' rows at a time)."""
+    import torch
+    h, i, s = 512, 512, 3
+    wd = synth.to_device(synth.expert_bank(79, h, i, e, svh_scale=True), cuda)
+    x = synth.activations_bf16(8, rows, h)
+    picks, _ = synth.route(9, rows, e, s - 1, uniform=True)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    fe = pkg.FastExperts(pkg.make_config(h, i, e, s, max_rows=rows))
+
+    def run(sel):
+        n = len(sel)
+        ids, count, members = oracle.grouping(picks[sel], n, s, e + 1, n)
+        fe.output.fill_(float("nan"))
+        fe.run(wd, _bf16_dev(x[sel], cuda), t(picks[sel]), t(ids), t(np.array([count], np.int32)), t(members), n, n)
+        torch.cuda.synchronize()
+        assert int(fe.status.cpu()[0]) == 0
+        return fe.output[: n * s].cpu().numpy().reshape(n, s, h).copy()
+    full = run(np.arange(rows))
+    assert np.isfinite(full).all()
+    counts = np.bincount(picks.ravel(), minlength=e + 1)
+    plan = fe.plan.cpu().numpy()
+    assert plan[1] == counts.sum() and plan[0] == (-(-counts // 128)).sum()
+    for lo in range(0, rows, 150):
+        sel = np.arange(lo, min(rows, lo + 150))
+        assert (run(sel).view(np.uint32) == full[sel].view(np.uint32)).all()
+
+
 def test_shared_expert_row_window(pkg, synth, cuda, dbank):
     """Expert-parallel prefill splits the shared expert by rows: a handle with shared_rows = (lo, hi) computes the shared
     pair only for window rows in [lo, hi); every other pair is untouched.  Checked against the layer without a row
