@@ -81,3 +81,26 @@ def test_router_feeds_the_layer(pkg, oracle, synth, cuda):
     torch.cuda.synchronize()
     ref = moe2.output[:rows]
     assert torch.allclose(got, ref, rtol=1e-5, atol=1e-6 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("rows,experts,k", [(1, 64, 4), (33, 64, 8), (4096, 64, 4), (40, 5, 5), (20, 65, 3), (600, 128, 16), (17, 100, 4), (3000, 8, 1),
+                                            (2400, 127, 7), (9, 64, 9), (5, 129, 8)])
+def test_route_selects_as_topk(pkg, cuda, rows, experts, k):
+    """The selection inside the router (several rows of a warp side by side) has the bytes of the stand-alone kernel on the same logits:
+    ties, zero rows, infinities and NaN among them."""
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(rows)
+    h = 256
+    x = torch.randn((rows, h), generator=g, device=cuda).to(torch.bfloat16)
+    wr = torch.randn((experts, h), generator=g, device=cuda).to(torch.bfloat16)
+    x[::5] = 0                                           # all tied
+    wr[experts // 2] = wr[0]                             # a tie between two experts in every row
+    if rows > 3:
+        x[1, 0], x[2, 0], x[3, 3] = float("inf"), float("nan"), -float("inf")
+    out = [torch.full((rows, experts), 9.0, device=cuda), torch.full((rows, k + 1), -7, dtype=torch.int32, device=cuda), torch.zeros((rows, k + 1), device=cuda)]
+    pkg.route(x, wr, *out)
+    picks, weights = torch.full_like(out[1], -7), torch.zeros_like(out[2])
+    pkg.topk(out[0], picks, weights, pdl=0)
+    torch.cuda.synchronize()
+    assert torch.equal(out[1], picks)
+    assert torch.equal(out[2].view(torch.int32), weights.view(torch.int32))
