@@ -99,13 +99,10 @@ static int run_stream(const glmflash_experts *e, cudaStream_t s, StreamArgs a, c
     if (!a.status) a.status = e->status;
     a.H = c.hidden; a.I = c.inter; a.rows = rows; a.slots = c.slots; a.E = c.experts;
     a.e_lo = c.expert_lo; a.e_hi = c.expert_hi; a.shared = c.shared_exl3; a.limit = c.limit;
-    // distinct experts that THIS GPU computes: at most one per pick, and at most its expert window (+ the shared expert)
     a.srow_lo = c.shared_row_lo; a.srow_hi = c.shared_row_hi;
     a.cut1 = stream_cut(c.hidden, rows > 16);
     a.cut2 = stream_cut(c.inter, rows > 16);
-    a.umax = std::max(1, std::min(rows * c.slots, (c.expert_hi - c.expert_lo) + (c.shared_exl3 ? 1 : 0)));
-    if (!a.picks) a.umax = std::max(1, std::min(rows * c.slots, c.experts + 1));   // (places in ids, skipped experts included)
-    if (rows > 16) a.umax += rows * c.slots / 16;                  // (an entry for every 16 members)
+    a.umax = stream_umax(c, rows, a.picks == nullptr);
     a.do_g = (e->phases & 2) != 0;
     a.do_d = (e->phases & 4) != 0;
     return launch_stream(s, a, c.pdl != 0);

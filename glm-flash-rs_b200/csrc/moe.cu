@@ -100,14 +100,16 @@ bool gf::one_launch_selected() {
     return env && env[0] == '1';
 }
 
-// Chunks up to this many rows go to the streamed kernel, which decodes an expert's weights once per 16 of its rows (the GEMMs:
-// once per 256).  It wins while the decoding bounds both: us a layer, streamed | GEMMs, 2048 x 1536, 64 experts, top-4: 17 rows
-// 144 | 221, 40: 195 | 289, 128: 263 | 323, 192: 321 | 323, 256: 577 | 327; 4096 x 512, 288 experts, top-8: 17: 230 | 380, 128:
-// 814 | 974, 256: 1153 | 1009; eight experts of 64: 17: 45 | 83, 128: 83 | 94, 192: 110 | 96.  Hence 128 rows, fewer where the
-// routed experts have more than 16 rows on average (1024 x 2048, 24 experts, top-3, 128 rows: 141 | 145), and none where the
-// exchange areas, which grow with the rows, would pass 256 MB.
+// Chunks up to this many rows go to the streamed kernel, which decodes an expert's weights once per 16 of its rows and adds partial sums
+// for every row (the GEMMs: once per 320, for a fixed 35 us of kernels in front and behind).  us a layer, streamed | GEMMs: 2048 x 1536,
+// 64 experts, top-4: 17 rows 120 | 144, 64: 186 | 197, 80: 205 | 206, 128: 251 | 210; eight experts of 64: 80: 59 | 60; 1024 x 2048, 24
+// experts, top-3: 48: 75 | 80, 64: 86 | 81; 1536 x 768, 100, top-5: 112: 142 | 147, 128: 151 | 146; 3072 x 1024, 16, top-2: 48: 75 | 75.  The
+// lines cross at five to seven rows per routed expert: 5.5 here, at most 128 rows, and none where the exchange areas, which grow with
+// the rows, would pass 256 MB.  With many experts the window's tables leave no room for the second CTA of an SM, and the GEMMs win earlier
+// (4096 x 512, 288 experts, top-8: 17 rows 190 | 222, 24: 298 | 280, 40: 416 | 385, 128: 717 | 522; 18 rows are the last of two CTAs).
 static int short_chunk_rows(const glmflash_config &c) {
-    const size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)16 * c.experts / (c.slots - 1), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
+    size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)11 * c.experts / (2 * (c.slots - 1)), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
+    while (rows > 16 && !stream_chunk_pairs(c, (int)rows)) --rows;
     return rows > 16 ? (int)rows : 0;
 }
 

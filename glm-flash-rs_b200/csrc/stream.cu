@@ -55,6 +55,7 @@ struct StWarps {
 };
 constexpr size_t ST_MAX_SMEM = 227 * 1024 - 4352;            // dynamic part (4,240 bytes are static)
 constexpr size_t ST_HALF_SM = 116 * 1024;                    // two such CTAs do not fit an SM
+constexpr size_t ST_TWO_SMEM = 228 * 1024 / 2 - 1024 - 4352; // dynamic part of one of two (each has 1 KB of the system's as well)
 constexpr uint32_t ST_POLLS = 1u << 21;                      // polls of a global word before a wait gives up (about a second)
 
 enum : int { UNIT_G = 0, UNIT_D = 1, UNIT_END = 2 };       // low byte of a descriptor, matrix in bit 8
@@ -813,6 +814,11 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
             a.ctrl[CTRL_EPOCH] = epoch;
         }
     }
+}
+
+// Whether two CTAs of a chunk of these rows share an SM: with many experts the tables of the window take the room.
+bool stream_chunk_pairs(const glmflash_config &c, int rows) {
+    return st_smem_bytes(2, stream_umax(c, rows, false), rows, rows * c.slots, c.experts) <= ST_TWO_SMEM;
 }
 
 int launch_stream(cudaStream_t s, StreamArgs a, bool pdl) {

@@ -66,6 +66,14 @@ inline size_t stream_xdl_words(const glmflash_config &c) { return (size_t)c.max_
 
 // Most rows of a chunk that the kernel takes (its tables live in shared memory and its exchange areas grow with the rows).
 constexpr int ST_MAX_ROWS = 128;
+// Most entries of the tables: distinct experts that this GPU computes (at most one per pick, and at most its window and the shared
+// one; with the grouping's tables the places in ids, skipped ones included), and for chunks one more for every 16 members.
+inline int stream_umax(const glmflash_config &c, int rows, bool tables) {
+    const int here = tables ? c.experts + 1 : (c.expert_hi - c.expert_lo) + (c.shared_exl3 ? 1 : 0), picks = rows * c.slots;
+    const int distinct = picks < here ? picks : here;
+    return (distinct > 1 ? distinct : 1) + (rows > 16 ? picks / 16 : 0);
+}
+bool stream_chunk_pairs(const glmflash_config &c, int rows);
 int launch_stream(cudaStream_t s, StreamArgs a, bool pdl);
 
 }  // namespace gf

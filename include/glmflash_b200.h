@@ -153,9 +153,9 @@ int  glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream, const glm
                                const int32_t *count, const int32_t *members, int rows, int maxm, int shared_x);
 float *glmflash_fast_experts_output(const glmflash_fast_experts *f);       /* fp32 [rows*slots][H], pair order */
 /* Down-projection inputs of the last run, fp16 [grouped rows][I].  The prefill path keeps its intermediate rows
- * GROUPED (the rows of an expert are contiguous, experts in ascending id order, so that an M tile is one TMA
- * tensor load); grouped row j belongs to pair glmflash_fast_experts_row_pairs()[j]; the number of grouped rows
- * is plan[1], the number of 128-row M tiles plan[0]. */
+ * GROUPED (the rows of an expert are contiguous, experts in ascending id order, so that the rows of a work item are one
+ * TMA tensor load); grouped row j belongs to pair glmflash_fast_experts_row_pairs()[j]; the number of grouped rows
+ * is plan[1], the number of 128-row tiles of all experts plan[0]. */
 const uint16_t *glmflash_fast_experts_xd(const glmflash_fast_experts *f);
 const int32_t *glmflash_fast_experts_row_pairs(const glmflash_fast_experts *f);
 const int32_t *glmflash_fast_experts_plan(const glmflash_fast_experts *f);
@@ -173,11 +173,12 @@ typedef struct glmflash_moe glmflash_moe;
  * router-to-combine sequence src/moe.rs:101-181 takes eight kernels).  The environment variable GLMFLASH_LAYER_KERNELS=1
  * (read when an owner is created) selects an alternative one-launch kernel, which also carries the cross-GPU exchange of
  * glmflash_moe_run_ep; on one GPU it is slower.
- * Calls of up to min(max_rows, 128, 16 experts / (slots - 1)) rows take that launch on a handle for more rows as well.  For them such
- * a handle holds, beside the prefill scratch, exchange words of
+ * Calls of up to min(max_rows, 128, 5.5 experts / (slots - 1)) rows take that launch on a handle for more rows as well (with several
+ * hundred experts fewer: the launch's tables grow with them; 18 rows of 288 experts, slots 9).  For them such a handle holds, beside
+ * the prefill scratch, exchange words of
  *   8 slots (2 ceil(hidden / 512) inter + ceil(inter / 512) hidden + hidden + inter / 2) bytes
- * for each of these rows (and never less than sixteen rows of a window take), at most about 256 MB: 850 KB a row, 109 MB a handle
- * at hidden 2048, inter 1536, slots 5. */
+ * for each of these rows (and never less than sixteen rows of a window take), at most about 256 MB: 850 KB a row, 75 MB a handle
+ * at hidden 2048, inter 1536, 64 experts, slots 5. */
 int  glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_moe **out);
 void glmflash_moe_free(glmflash_moe *m);
 /* group -> routed and shared experts -> combine:

@@ -52,6 +52,27 @@ def test_short_chunks_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows, kw):
     assert emax < TOL and erms < TOL, (emax, erms)
 
 
+@pytest.mark.parametrize("H,I,E,S,rows,kw", [(512, 512, 40, 3, 96, {}), (768, 256, 30, 2, 128, {}), (256, 512, 24, 4, 17, {}),
+                                             (512, 512, 24, 4, 40, dict(expert_lo=1, expert_hi=19, shared_rows=(10, 30))),
+                                             (256, 256, 300, 9, 18, {}), (256, 256, 300, 9, 40, {})])
+def test_chunks_on_both_sides_of_the_line(pkg, oracle, synth, cuda, H, I, E, S, rows, kw):
+    # few rows per expert: streamed, unless the tables of many experts take a CTA's room (the last one).  A row is held against both orders of
+    # the oracle's sums: in row 88 of (768, 256, 30) they round a 16-bit product of 32..64 to neighbours, and differ by 2.03e-3 themselves.
+    bank = synth.expert_bank(51 + H + rows, H, I, E, svh_scale=True)
+    x, (picks, rw) = synth.activations_bf16(52, rows, H), synth.route(53, rows, E, S - 1)
+    got = run(pkg, cuda, synth.to_device(bank, cuda), x, picks, rw, H, I, E, S, rows, synth, **kw)
+    lo, hi = kw.get("expert_lo", 0), kw.get("expert_hi", E)
+    r0, r1 = kw.get("shared_rows", (0, rows))
+    here = (picks >= lo) & (picks < hi) | (picks == E) & (np.arange(rows)[:, None] >= r0) & (np.arange(rows)[:, None] < r1)
+    scale, off = 0, []
+    for mode in (0, 1):
+        Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=mode).reshape(rows, S, H)
+        want = np.where(here[..., None], np.where((np.arange(S) == S - 1)[None, :, None], 1, rw[..., None]) * Y, 0).sum(1)
+        scale = max(scale, np.abs(want).max())
+        off.append(np.abs(got - want).max(1))
+    assert np.min(off, axis=0).max() < TOL * scale
+
+
 @pytest.mark.parametrize("rows", [1, 8, 16])
 @pytest.mark.parametrize("shared_rows", [(512, 1024), (3, 6), (0, 1), (5, 64), (0, 64)])
 @pytest.mark.parametrize("share", [{}, dict(expert_lo=2, expert_hi=7)])
