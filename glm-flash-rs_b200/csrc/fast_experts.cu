@@ -202,12 +202,12 @@ __global__ void __launch_bounds__(ROT_WARPS * 32, 4) fast_rot_kernel(const __nv_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3, group = lane >> 2;
     const int KB = K >> 7, slices = (KB + 7) >> 3, per_warp = KB < 8 ? 8 / KB : 1;         // rows of a warp (short rows: several)
     const __half *suh = blockIdx.y ? suh1 : suh0;
-    __half *out = blockIdx.y ? out1 : out0;
     const float2 neg1 = make_float2(-1.f, -1.f);
     const int w = blockIdx.x * ROT_WARPS + warp, slice = w % slices, part = w / slices, parts = (int)gridDim.x * ROT_WARPS / slices;
     const int sub = KB < 8 ? group / KB : 0, blk = KB < 8 ? group - sub * KB : slice * 8 + group, k = blk * 128 + 8 * t;
     pdl_wait();
     pdl_launch_dependents();
+    __half *out = blockIdx.y ? out1 : out0;
     const int rows = plan[1], size = (rows + parts - 1) / parts, end = min(rows, (part + 1) * size);
     const bool mine = blk < KB && sub < per_warp && part < parts;
     int j = part * size + sub, code = 0, next = 0, e = -1;
