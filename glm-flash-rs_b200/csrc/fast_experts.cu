@@ -29,7 +29,7 @@
 //             epilogue overlaps the next item's gate pass.  Down is one pass per item.
 //             Before, the rows were M (256 a tile, filled or not) and the weights went through shared memory: a chunk of 40 rows cost as
 //             much as one of 256, an expert of 257 rows twice as much as one of 256.  us gate/up | down, before -> now: 500 rows 197 | 101
-//             -> 132 | 68, 4096 rows 350 | 181 -> 274 | 136, eight experts of 64 at 4096 rows 81 | 39 -> 49 | 33 (2048 x 1536, 64 experts,
+//             -> 127 | 66, 4096 rows 350 | 181 -> 277 | 137, eight experts of 64 at 4096 rows 81 | 39 -> 49 | 33 (2048 x 1536, 64 experts,
 //             top-4); 8192 rows of 4096 x 512, 288 experts, top-8: 587 | 697 -> 540 | 505.  What bounds it now: instruction issue (0.70 to 0.80 of the
 //             cycles while all SMs work: decode, epilogue) and the last round of items (0.82 to 0.87 of the time); short K (512): the
 //             epilogue, which a pass of four stages does not cover.
