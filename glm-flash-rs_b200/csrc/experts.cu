@@ -59,7 +59,7 @@ int gf::experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_l
     pool.take(&e->ll_xr, stream_xr_words(*cfg) * 8);
     pool.take(&e->ll_xd, stream_xdl_words(*cfg) * 8);
     pool.take(&e->ctrl, CTRL_WORDS * 4);
-    if (cfg->max_rows <= 16 && one_launch_selected()) {                          // scratch of the alternative layer kernel (window.cu)
+    if (max_rows_limit <= 16 && one_launch_selected()) {                         // scratch of the alternative layer kernel (window.cu)
         e->sync_words = experts_window_sync_words(*cfg);
         pool.take(&e->z1, (size_t)2 * (H / 128) * P * I * 4);
         pool.take(&e->z2, (size_t)(I / 128) * P * H * 4);

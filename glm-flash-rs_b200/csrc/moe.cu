@@ -100,17 +100,21 @@ bool gf::one_launch_selected() {
     return env && env[0] == '1';
 }
 
-// Chunks up to this many rows go to the streamed kernel, which decodes an expert's weights once per 16 of its rows and adds partial sums
-// for every row (the GEMMs: once per 320, for a fixed 35 us of kernels in front and behind).  us a layer, streamed | GEMMs: 2048 x 1536,
+// Calls up to this many rows go to the streamed kernel on a handle for more than 16.  Windows of up to 16 always do, as on a handle of their
+// own: one launch, and the bytes do not depend on the handle (16 experts of 2048 x 1536, top-6: 1 row 26 us a layer against 56 by the GEMMs,
+// 16 rows 61 | 83; 384 of 1024 x 1024, top-8: 21 | 56 and 105 | 152; 8 of 2048 x 768, top-8: 25 | 52 and 42 | 53; behind the
+// GEMMs where a row takes all of 16 experts: 1024 x 1024, 30 | 48 and 66 | 49).  Longer ones: the kernel
+// decodes an expert's weights once per 16 of its rows and adds partial sums for every row (the GEMMs: once per 320, for a fixed 35 us of
+// kernels in front and behind).  us a layer, streamed | GEMMs: 2048 x 1536,
 // 64 experts, top-4: 17 rows 120 | 144, 64: 186 | 197, 80: 205 | 206, 128: 251 | 210; eight experts of 64: 80: 59 | 60; 1024 x 2048, 24
 // experts, top-3: 48: 75 | 80, 64: 86 | 81; 1536 x 768, 100, top-5: 112: 142 | 147, 128: 151 | 146; 3072 x 1024, 16, top-2: 48: 75 | 75.  The
-// lines cross at five to seven rows per routed expert: 5.5 here, at most 128 rows, and none where the exchange areas, which grow with
-// the rows, would pass 256 MB.  With many experts the window's tables leave no room for the second CTA of an SM, and the GEMMs win earlier
+// lines cross at five to seven rows per routed expert: 5.5 here, at most 128 rows, and none above 16 where the exchange areas, which grow with
+// the rows, would pass 256 MB.  With many experts the chunk's tables leave no room for the second CTA of an SM, and the GEMMs win earlier
 // (4096 x 512, 288 experts, top-8: 17 rows 190 | 222, 24: 298 | 280, 40: 416 | 385, 128: 717 | 522; 18 rows are the last of two CTAs).
 static int short_chunk_rows(const glmflash_config &c) {
     size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)11 * c.experts / (2 * (c.slots - 1)), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
     while (rows > 16 && !stream_chunk_pairs(c, (int)rows)) --rows;
-    return rows > 16 ? (int)rows : 0;
+    return (int)std::max<size_t>(rows, 16);
 }
 
 struct glmflash_moe {
@@ -118,7 +122,7 @@ struct glmflash_moe {
     glmflash_grouping *grouping = nullptr;
     glmflash_experts *experts = nullptr;            // windows of <= 16 rows
     glmflash_fast_experts *fast = nullptr;          // chunks of > 16 rows
-    glmflash_experts *chunk = nullptr;              // the streamed kernel's buffers for chunks of up to chunk_rows rows
+    glmflash_experts *chunk = nullptr;              // beside them: the streamed kernel's buffers for calls of up to chunk_rows rows
     int chunk_rows = 0;
     void *pool = nullptr;                           // the one allocation behind the buffers below
     float *out = nullptr;
@@ -140,14 +144,12 @@ extern "C" int glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, gl
     if (cfg->max_rows <= 16) rc = glmflash_experts_new(cfg, cfg_bytes, &m->experts);
     else if (!(rc = glmflash_grouping_new(cfg, cfg_bytes, &m->grouping)) && !(rc = glmflash_fast_experts_new(cfg, cfg_bytes, &m->fast))) {
         m->chunk_rows = short_chunk_rows(*cfg);
-        if (m->chunk_rows > 0) {
-            glmflash_config cc = *cfg;
-            cc.max_rows = m->chunk_rows;
-            cc.shared_row_lo = cc.shared_row_hi = 0;
-            rc = experts_new(&cc, sizeof(cc), ST_MAX_ROWS, &m->chunk);
-            if (!rc)                                // (the row window counts rows of the chunk, whatever the owner holds)
-                m->chunk->cfg.shared_row_lo = cfg->shared_row_lo, m->chunk->cfg.shared_row_hi = cfg->shared_row_hi;
-        }
+        glmflash_config cc = *cfg;
+        cc.max_rows = m->chunk_rows;
+        cc.shared_row_lo = cc.shared_row_hi = 0;
+        rc = experts_new(&cc, sizeof(cc), ST_MAX_ROWS, &m->chunk);
+        if (!rc)                                    // (the row window counts rows of the chunk, whatever the owner holds)
+            m->chunk->cfg.shared_row_lo = cfg->shared_row_lo, m->chunk->cfg.shared_row_hi = cfg->shared_row_hi;
     }
     const size_t rows = cfg->max_rows;
     Pool pool;
@@ -186,8 +188,9 @@ extern "C" int glmflash_moe_run(glmflash_moe *m, void *stream, const glmflash_we
         // one streamed launch: grouping, input rotation, both projections, epilogues and the combine
         return experts_run_fused(m->experts, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows,
                                  nullptr, nullptr);
-    } else if (m->chunk && rows <= m->chunk_rows && (m->phases | 16) == 31) {
-        // a short chunk: the streamed kernel as well, its pair rows and status word those of the chunk owner
+    } else if (rows <= m->chunk_rows && (m->phases | 16) == 31) {
+        // a window or a short chunk on a handle for more rows: the streamed kernel as well, its pair rows and status word those of
+        // the chunk owner
         return experts_run_fused(m->chunk, (cudaStream_t)stream, w, input, x_stride, picks, route_w, m->phases & 16 ? m->out : nullptr, nullptr, rows,
                                  glmflash_fast_experts_output(m->fast), fast_experts_status_word(m->fast));
     } else {

@@ -173,11 +173,11 @@ typedef struct glmflash_moe glmflash_moe;
  * router-to-combine sequence src/moe.rs:101-181 takes eight kernels).  The environment variable GLMFLASH_LAYER_KERNELS=1
  * (read when an owner is created) selects an alternative one-launch kernel, which also carries the cross-GPU exchange of
  * glmflash_moe_run_ep; on one GPU it is slower.
- * Calls of up to min(max_rows, 128, 5.5 experts / (slots - 1)) rows take that launch on a handle for more rows as well (with several
- * hundred experts fewer: the launch's tables grow with them; 18 rows of 288 experts, slots 9).  For them such a handle holds, beside
- * the prefill scratch, exchange words of
+ * A handle for more rows serves calls of up to 16 rows by that launch as well, whatever its experts and slots, and with the bytes of
+ * a handle for 16; and longer ones of up to min(128, 5.5 experts / (slots - 1)) rows (with several hundred experts fewer: the launch's
+ * tables grow with them; 18 rows of 288 experts, slots 9).  For them such a handle holds, beside the prefill scratch, exchange words of
  *   8 slots (2 ceil(hidden / 512) inter + ceil(inter / 512) hidden + hidden + inter / 2) bytes
- * for each of these rows (and never less than sixteen rows of a window take), at most about 256 MB: 850 KB a row, 75 MB a handle
+ * for each of these rows, at most about 256 MB, and never less than a handle for 16 rows: 850 KB a row, 75 MB a handle
  * at hidden 2048, inter 1536, 64 experts, slots 5. */
 int  glmflash_moe_new(const glmflash_config *cfg, size_t cfg_bytes, glmflash_moe **out);
 void glmflash_moe_free(glmflash_moe *m);

@@ -73,6 +73,41 @@ def test_chunks_on_both_sides_of_the_line(pkg, oracle, synth, cuda, H, I, E, S, 
     assert np.min(off, axis=0).max() < TOL * scale
 
 
+def launches(pkg, moe, *args):
+    """Kernels of one call, counted as the nodes of its graph."""
+    import torch
+    cache, side = pkg.GraphCache(bounded=True), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    cache.run(1, lambda: moe.run(*args), stream=side)
+    side.synchronize()
+    return cache.stats()["retained_nodes"]
+
+
+@pytest.mark.parametrize("H,I,E,S", [(512, 512, 16, 7), (256, 256, 384, 9), (256, 256, 4, 3), (512, 256, 2, 2), (256, 512, 16, 17), (256, 256, 200, 11)])
+def test_windows_of_large_handles(pkg, synth, cuda, H, I, E, S):
+    # calls of up to 16 rows are one launch with the bytes of a handle for 16, also where the line for longer chunks is at 16 rows or fewer
+    # (few experts for the slots, tables of many experts); a call of 17 rows in between
+    import torch
+    dbank = synth.to_device(synth.expert_bank(61 + H, H, I, E, svh_scale=True), cuda)
+    x, (picks, rw) = synth.activations_bf16(62, 17, H), synth.route(63, 17, E, S - 1)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd, pd, wd = t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw)
+    small, large = (pkg.Moe(pkg.make_config(H, I, E, S, max_rows=n)) for n in (16, 8192))
+    for rows in (1, 2, 17, 9, 16):
+        args = (dbank, xd[:rows], pd[:rows], wd[:rows], rows)
+        large.run(*args)
+        torch.cuda.synchronize()
+        assert int(large.status.cpu()[0]) == 0
+        if rows > 16:
+            continue
+        small.run(*args)
+        torch.cuda.synchronize()
+        assert torch.equal(large.output[:rows].view(torch.int32), small.output[:rows].view(torch.int32))
+        pairs = [pkg._view(m.pairs_ptr.value, (rows * S, H), torch.int32) for m in (large, small)]
+        assert torch.equal(*pairs)
+        assert launches(pkg, large, *args) == launches(pkg, small, *args) == 1
+
+
 @pytest.mark.parametrize("rows", [1, 8, 16])
 @pytest.mark.parametrize("shared_rows", [(512, 1024), (3, 6), (0, 1), (5, 64), (0, 64)])
 @pytest.mark.parametrize("share", [{}, dict(expert_lo=2, expert_hi=7)])
