@@ -136,6 +136,9 @@ __device__ __forceinline__ void codeword_pair(uint32_t u, uint32_t &x_hi, uint32
 
 // ---- rounding helpers (the rounding points of upstream's epilogues, native/exl3.cu:243) ------------------
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+// silu, in every layer kernel with the full exponential and divide.  The fast forms (2 ulp each, the exponential 1.4 |g| of 2^-24 more) put
+// more of the bf16 roundings behind them on the other side.
+__device__ __forceinline__ float silu(float g) { return g / (1.f + expf(-g)); }
 
 // ---- Hadamard ------------------------------------------------------------------------------------------
 // 128 values held 4 per lane (lane L: values 4L..4L+3), natural order; butterflies stride 1, 2 in

@@ -41,7 +41,8 @@
 // Arithmetic: one full-K fp32 accumulation chain per output (as upstream's prefill path, which is likewise not
 // bit-equal to its decode path: native/exl3_prefill.cu:20-23), the same transforms and rounding points as
 // upstream's epilogue (native/exl3_prefill.cu:596-622 == native/exl3.cu:260-321) with exp / divide in their fast
-// forms.  Deterministic: static work assignment, no atomics; every pair's result depends only on its own row.
+// forms; short calls of the layer in finer steps (FINE).  Deterministic: static work assignment, no atomics; every pair's result depends only
+// on its own row.
 // Every wait is bounded; a wait that gives up raises the abort flag, every role leaves its loops, tensor memory
 // is freed and the status word reports the failure.
 #include <cuda.h>
@@ -54,11 +55,15 @@
 namespace gf {
 int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit);
 int *fast_experts_status_word(glmflash_fast_experts *f);
+int fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_weights *w, const void *input, int x_stride, const int32_t *picks,
+                     const int32_t *ids, const int32_t *count, const int32_t *members, int rows, int maxm, int shared_x, bool fine);
 
 constexpr int FG_DEC = 16;                                 // trellis-decode warps
 constexpr int FG_THREADS = (12 + FG_DEC) * 32;
 constexpr int FG_BN = 128, FG_BK = 128;                    // columns of a CTA, k of a stage
 constexpr int FG_CHUNK = 320;                              // most rows of a work item
+constexpr int FG_FINE_ROWS = 128;                          // most rows of a call with partial sums (FINE)
+constexpr int FG_CHAIN = 512 / FG_BK;                      // stages of one of them
 constexpr int FG_BOXES = 8;                                // boxes of rows that one copy takes: 16, 32, .. 128
 constexpr int FG_HALF_BYTES = FG_CHUNK / 2 * 128;          // 20 KB: a CTA's rows x 64 k of fp16, half of a stage
 constexpr int FG_TILE_BYTES = 2 * FG_HALF_BYTES;
@@ -557,6 +562,11 @@ struct FgMaps {
 constexpr int FG_STAGES = 3, FG_ACOLS = FG_BK / 2, FG_DCOL = FG_STAGES * FG_ACOLS, FG_DCOLS = 512 - FG_DCOL;
 static_assert(FG_DCOLS >= FG_CHUNK, "accumulators of a pass");
 
+// FINE: chains of FG_CHAIN stages with accumulators of their own, as many a pass as have room in half of the columns: the stages of a pass
+// of n <= 128 rows.
+__device__ __forceinline__ int fine_stages(int n) { return (n <= 32 ? 5 : n <= 64 ? 2 : 1) * FG_CHAIN; }
+static_assert(5 * 32 <= FG_DCOLS / 2 && FG_FINE_ROWS <= FG_DCOLS / 2, "accumulators of a pass with partial sums");
+
 template <int MATS>
 struct FgCfg {
     static constexpr int WSTAGES = 4;                        // packed words
@@ -584,7 +594,14 @@ __device__ __forceinline__ bool group_all(int group, bool yes) {
 }
 __device__ __forceinline__ void group_barrier(int group) { asm volatile("barrier.sync %0, 128;" ::"r"(2 + group) : "memory"); }
 
-template <int MATS>
+// FINE: the layer's calls of up to FG_FINE_ROWS rows, whose neighbours the streamed kernel serves, are as exact as there.  A sum is made of
+// chains of at most 512 k, added in ascending order, and silu takes the full exponential and divide.  Mean distance of a layer's rows from
+// sums in 64 bits with all rounding points in place, one chain and fast forms | FINE | streamed kernel: 2048 x 1536, 64 experts, top-4, 112
+// rows 1.34e-4 | 5.6e-5 | 5.5e-5; 1024 x 2048, 24, top-3, 96 rows 9.6e-5 | 6.3e-5 | 6.1e-5; 3072 x 1024, 16, top-2, 112 rows 1.55e-4 | 4.2e-5
+// | 4.2e-5; 4096 x 512, 288, top-8, 64 rows 1.73e-4 | 5.2e-5 | 5.1e-5 (600 rows each, standard error 3e-6 to 2e-5).  The chains make the difference:
+// they cost up to 2 % (with a wait of the MMAs for the epilogue at each of them 10 %), the silu 2 to 6 % (128 rows of the first shape 206 | 212 us);
+// for all calls it would cost 5 % at 4096 rows (590 | 618 us).
+template <int MATS, bool FINE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(FG_THREADS, 1)
 fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
     using C = FgCfg<MATS>;
@@ -675,7 +692,11 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
             for (Items t(a.chunks, pair, total, pairs, NBP); ok && t.advance();) {
                 const int n2 = t.n - min(t.n, 256);                  // (one instruction takes 256 rows)
                 const uint32_t idesc = umma_idesc(t.n - n2), idesc2 = umma_idesc(n2);
-                for (int pm = 0; pm < MATS && ok; ++pm, ++pc) {
+                const int most = FINE ? fine_stages(t.n) : KS, passes = FINE ? MATS * ((KS + most - 1) / most) : MATS;
+                int left = KS;                                       // (FINE) stages of the matrix that are left
+                for (int pm = 0; pm < passes && ok; ++pm, ++pc) {
+                    const int steps = FINE ? min(left, most) : KS;
+                    if (FINE && (left -= steps) == 0) left = KS;
                     const uint32_t pb = pc & 1;
                     // the accumulators of the pass before the last one, and where they reach into these, of the last one have been drained
                     ok = __all_sync(0xffffffffu, wait_or_abort<0>(tmem_empty + pb, ((pc >> 1) & 1) ^ 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT) &&
@@ -683,19 +704,20 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                     if (!ok) break;
                     before = t.n;
                     tc_fence_after();
-                    const uint32_t d0 = tmem_base + FG_DCOL + (pb ? FG_DCOLS - t.n : 0);
-                    for (int s = KS; s; --s) {
+                    uint32_t d0 = tmem_base + FG_DCOL + (pb ? FINE ? FG_DCOLS / 2 : FG_DCOLS - t.n : 0);
+                    for (int s = steps; s; --s) {
                         ok = __all_sync(0xffffffffu, wait_or_abort<0>(full + ring.slot, ring.parity, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT));
                         if (!ok) break;
                         tc_fence_after();
                         const uint64_t db = desc_b0 + ring.slot * (FG_TILE_BYTES >> 4);
-                        const uint32_t ta = tmem_base + ring.slot * FG_ACOLS, first = s != KS;
+                        const uint32_t ta = tmem_base + ring.slot * FG_ACOLS, first = FINE ? (steps - s) % FG_CHAIN : s != steps;
+                        if (FINE && !first && s != steps) d0 += t.n;
                         if (elect_one()) {
 #pragma unroll
                             for (int kk = 0; kk < FG_BK / 16; ++kk) {
                                 const uint64_t dk = db + 2 * (kk & 3) + (kk >> 2) * (FG_HALF_BYTES >> 4);
                                 umma_f16(d0, ta + 8 * kk, dk, idesc, kk > 0 ? 1u : first);
-                                if (n2) umma_f16(d0 + 256, ta + 8 * kk, dk + (128 * 128 >> 4), idesc2, kk > 0 ? 1u : first);
+                                if (!FINE && n2) umma_f16(d0 + 256, ta + 8 * kk, dk + (128 * 128 >> 4), idesc2, kk > 0 ? 1u : first);
                             }
                             umma_commit(done + ring.slot);          // both CTAs may overwrite the stage once these MMAs have read it
                             if (s == 1) umma_commit(tmem_full + pb);           // the accumulators of this pass are complete
@@ -742,6 +764,7 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
             else if (MATS == 2) { sc0 = a.sv1[o]; sc1 = a.sd[o]; }
         };
         if (pair < total) fetch(pair, t.next.x);
+        auto act = [](float g) { return FINE ? silu(g) : __fdividef(g, 1.f + __expf(-g)); };
         // A warpgroup decides together whether a wait has given up: a warp never stands alone at a barrier.  One that has goes on through the
         // items for the barrier of both.
         while (t.advance()) {
@@ -756,7 +779,7 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
             const int mine = ((t.cnt + 31) / 32 - group + 1) >> 1;       // slabs of this warpgroup: group, group + 2, ..
             float v[3][32];
 #pragma unroll 1
-            for (int pm = 0; pm < MATS; ++pm, ++pc) {
+            for (int pm = 0, left = KS; pm < MATS; ++pm, ++pc) {
                 const uint32_t pb = pc & 1;
                 ok = wait_or_abort<FG_SLEEP>(tmem_full + pb, (pc >> 1) & 1, abort_flag, a.status, GF_STATUS_MMA_TIMEOUT);
                 if (!(ok = group_all(group, ok))) break;
@@ -764,8 +787,8 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                 tc_fence_after();
                 // Slabs in the order in which the next pass needs their columns: from the top at even passes, from the bottom at odd ones.  Three
                 // are taken out at once, which for up to 256 rows covers what a next pass of no more rows overwrites.
-                const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), col = FG_DCOL + (pb ? FG_DCOLS - t.n : 0);
-                auto slab_of = [&](int k) { return 2 * (pb ? k : max(mine - 1 - k, 0)) + group; };
+                const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), col = FG_DCOL + (pb ? FINE ? FG_DCOLS / 2 : FG_DCOLS - t.n : 0);
+                auto slab_of = [&](int k) { return 2 * (pb || FINE ? k : max(mine - 1 - k, 0)) + group; };
                 auto at = [&](int k) { return lanes + min(col + 32 * slab_of(k), 480u); };     // (past the end: some other slab, no branches)
                 auto arrive = [&](uint64_t *bar) {                       // this warp's lanes are in registers
                     tc_fence_before();
@@ -773,11 +796,41 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                     if (lane == 0) mbar_arrive_cluster(bar + pb, 0);
                     __syncwarp();
                 };
+                if (FINE) {
+                    // the next chains of the sums (v[0], v[1]: no more than two slabs); behind the matrix's last ones it goes on below
+                    const int chains = (min(left, fine_stages(t.n)) + FG_CHAIN - 1) / FG_CHAIN;
+                    int c = 0;
+                    if (left == KS) {
+                        tmem_ld32(at(0), v[0]);
+                        tmem_ld32(at(1), v[1]);
+                        tmem_ld_wait();
+                        c = 1;
+                    }
+                    auto add = [&](int k, int c) {
+                        tmem_ld32_now(at(k) + c * t.n, v[2]);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) tmem_ld32(at(k), v[k]);
-                tmem_ld_wait();
-                if (t.n <= 256) arrive(tmem_early);
-                if (t.n <= 192) arrive(tmem_empty);
+                        for (int r = 0; r < 32; r += 2) {
+                            const float2 sum = __fadd2_rn(make_float2(v[k][r], v[k][r + 1]), make_float2(v[2][r], v[2][r + 1]));
+                            v[k][r] = sum.x; v[k][r + 1] = sum.y;
+                        }
+                    };
+#pragma unroll 1
+                    for (; c < chains && mine; ++c) {
+                        add(0, c);
+                        if (mine > 1) add(1, c);
+                    }
+                    arrive(tmem_early);
+                    arrive(tmem_empty);
+                    left -= chains * FG_CHAIN;
+                    if (left > 0) { --pm; continue; }
+                    left = KS;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) tmem_ld32(at(k), v[k]);
+                    tmem_ld_wait();
+                    if (t.n <= 256) arrive(tmem_early);
+                    if (t.n <= 192) arrive(tmem_empty);
+                }
                 auto finish = [&](float (&x)[32], int k) {
                     group_barrier(group);                                // (the last slab has been read)
 #pragma unroll
@@ -809,8 +862,8 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                                 const float2 r0 = bf16r2(x[4 * j] * sg.x, x[4 * j + 1] * sg.y), r1 = bf16r2(x[4 * j + 2] * sg.z, x[4 * j + 3] * sg.w);
                                 const float g0 = fminf(r0.x, a.limit), g1 = fminf(r0.y, a.limit), g2 = fminf(r1.x, a.limit), g3 = fminf(r1.y, a.limit);
                                 // (one packed conversion rounds both values to bf16 and packs them: .x in the low half)
-                                const __nv_bfloat162 s0 = __float22bfloat162_rn(make_float2(__fdividef(g0, 1.f + __expf(-g0)), __fdividef(g1, 1.f + __expf(-g1))));
-                                const __nv_bfloat162 s1 = __float22bfloat162_rn(make_float2(__fdividef(g2, 1.f + __expf(-g2)), __fdividef(g3, 1.f + __expf(-g3))));
+                                const __nv_bfloat162 s0 = __float22bfloat162_rn(make_float2(act(g0), act(g1)));
+                                const __nv_bfloat162 s1 = __float22bfloat162_rn(make_float2(act(g2), act(g3)));
                                 *reinterpret_cast<uint2 *>(o + 16 * j) = make_uint2(*reinterpret_cast<const uint32_t *>(&s0), *reinterpret_cast<const uint32_t *>(&s1));
                             }
                     } else if (MATS == 2) {
@@ -845,11 +898,11 @@ fast_gemm_kernel(const __grid_constant__ FgMaps maps, const FastGemmArgs a) {
                     finish(v[0], k);
 #pragma unroll
                     for (int r = 0; r < 32; ++r) { v[0][r] = v[1][r]; v[1][r] = v[2][r]; }
-                    if (k == 0 && t.n > 192) {                           // the fourth and the fifth slab, as soon as there is room
+                    if (!FINE && k == 0 && t.n > 192) {                           // the fourth and the fifth slab, as soon as there is room
                         tmem_ld32_now(at(3), v[2]);
                         if (t.n <= 256) arrive(tmem_empty);
                     }
-                    if (k == 1 && t.n > 256) {
+                    if (!FINE && k == 1 && t.n > 256) {
                         tmem_ld32_now(at(4), v[2]);
                         arrive(tmem_early);
                         arrive(tmem_empty);
@@ -992,8 +1045,10 @@ extern "C" int glmflash_fast_experts_new(const glmflash_config *cfg, size_t cfg_
     pool.take(&f->row_expert, P * 4);
     pool.take(&f->status, 16);
     if (pool.alloc(&f->pool) || make_maps(f->gateup.rows[0], f->xg, P, H) || make_maps(f->gateup.rows[1], f->xu, P, H) || make_maps(f->down.rows[0], f->xd, P, I) ||
-        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<2>::SMEM)) ||
-        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<1>::SMEM))) {
+        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<2>::SMEM)) ||
+        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<1>::SMEM)) ||
+        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<2>::SMEM)) ||
+        fail_if(cudaFuncSetAttribute(fast_gemm_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FgCfg<1>::SMEM))) {
         glmflash_fast_experts_free(f);
         return -1;
     }
@@ -1007,13 +1062,14 @@ extern "C" void glmflash_fast_experts_free(glmflash_fast_experts *f) {
     delete f;
 }
 
-extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_weights *w, const void *input,
-                                         int x_stride, const int32_t *picks, const int32_t *ids, const int32_t *count,
-                                         const int32_t *members, int rows, int maxm, int shared_x) {
+// fine: a call of up to FG_FINE_ROWS rows takes partial sums; no expert may have more members than the call has rows
+int gf::fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_weights *w, const void *input, int x_stride, const int32_t *picks,
+                         const int32_t *ids, const int32_t *count, const int32_t *members, int rows, int maxm, int shared_x, bool fine) {
     GF_REQUIRE(f && w && input && picks && ids && count && members, "null argument");
     const glmflash_config &c = f->cfg;
     GF_REQUIRE(rows > 0 && rows <= c.max_rows && maxm >= rows && maxm <= c.max_rows, "expert rows/member stride outside scratch");
     GF_REQUIRE(x_stride >= c.hidden && x_stride % 4 == 0, "x_stride must be >= hidden and a multiple of 4");
+    fine = fine && rows <= FG_FINE_ROWS;
     GF_REQUIRE(((uintptr_t)w->gt | (uintptr_t)w->ut | (uintptr_t)w->dt) % 16 == 0, "trellis tensors must be 16-byte aligned");
     GF_REQUIRE(((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 8 == 0, "input and scale vectors must be 8-byte aligned");
     cudaStream_t s = (cudaStream_t)stream;
@@ -1037,13 +1093,19 @@ extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream,
         return -1;
     a.sv0 = (const __half *)w->svh_g; a.sv1 = (const __half *)w->svh_u; a.sd = (const __half *)w->suh_d;
     a.xd = f->xd; a.y = nullptr; a.K = H; a.N = I; a.shared_x = shared_x ? 1 : 0;
-    if ((f->phases & 4) && launch_k(fast_gemm_kernel<2>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<2>::SMEM, s, pdl, f->gateup, a))
+    if ((f->phases & 4) && launch_k(fine ? fast_gemm_kernel<2, true> : fast_gemm_kernel<2, false>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<2>::SMEM, s, pdl, f->gateup, a))
         return -1;
     a.sv0 = (const __half *)w->svh_d; a.sv1 = nullptr; a.sd = nullptr;
     a.xd = nullptr; a.y = f->out; a.K = I; a.N = H; a.shared_x = 1;
-    if ((f->phases & 8) && launch_k(fast_gemm_kernel<1>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<1>::SMEM, s, pdl, f->down, a))
+    if ((f->phases & 8) && launch_k(fine ? fast_gemm_kernel<1, true> : fast_gemm_kernel<1, false>, dim3((unsigned)f->sms & ~1u), dim3(FG_THREADS), FgCfg<1>::SMEM, s, pdl, f->down, a))
         return -1;
     return 0;
+}
+
+extern "C" int glmflash_fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_weights *w, const void *input,
+                                         int x_stride, const int32_t *picks, const int32_t *ids, const int32_t *count,
+                                         const int32_t *members, int rows, int maxm, int shared_x) {
+    return fast_experts_run(f, stream, w, input, x_stride, picks, ids, count, members, rows, maxm, shared_x, false);
 }
 
 int *gf::fast_experts_status_word(glmflash_fast_experts *f) { return f->status; }

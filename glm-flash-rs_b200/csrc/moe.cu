@@ -15,6 +15,8 @@ namespace gf {
 int experts_run_fused(glmflash_experts *e, cudaStream_t s, const glmflash_weights *w, const void *input, int x_stride,
                       const int32_t *picks, const float *route_w, float *out, float *out2, int rows, float *y, int *status);
 int *fast_experts_status_word(glmflash_fast_experts *f);
+int fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_weights *w, const void *input, int x_stride, const int32_t *picks,
+                     const int32_t *ids, const int32_t *count, const int32_t *members, int rows, int maxm, int shared_x, bool fine);
 
 // out[r][d] = sum_{s < slots-1, expert computed here} w[r][s] * Y[r*slots+s][d]  (+ Y[shared pair] if computed here)
 // fp32, ascending slot order, shared last: the order of the oracle's combine.
@@ -197,8 +199,10 @@ extern "C" int glmflash_moe_run(glmflash_moe *m, void *stream, const glmflash_we
         if ((m->phases & 1) && glmflash_grouping_run(m->grouping, stream, picks, rows)) return -1;
         const int32_t *ids = glmflash_grouping_ids(m->grouping), *count = glmflash_grouping_count(m->grouping),
                       *members = glmflash_grouping_members(m->grouping);
-        if (glmflash_fast_experts_run(m->fast, stream, w, input, x_stride, picks, ids, count, members, rows,
-                                      m->cfg.max_rows, w->suh_g == w->suh_u))
+        // calls as short as some that the streamed kernel serves are as exact as there (the tables are of this call: no expert has more members
+        // than it has rows)
+        if (fast_experts_run(m->fast, stream, w, input, x_stride, picks, ids, count, members, rows, m->cfg.max_rows, w->suh_g == w->suh_u,
+                             (m->phases & 1) != 0))
             return -1;
         Y = glmflash_fast_experts_output(m->fast);
     }

@@ -670,7 +670,7 @@ stream_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float g = fminf(r[i], a.limit);
-                            sg[i] = bf16r(g / (1.f + expf(-g)));
+                            sg[i] = bf16r(silu(g));
                         }
                         pair_barrier(2);
                         const float4 uu = *reinterpret_cast<const float4 *>(&fin_sh[2][4 * lane]);

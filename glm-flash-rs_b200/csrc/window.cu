@@ -466,7 +466,7 @@ __device__ __noinline__ void win_stage_swiglu(const WinArgs &a, WinShared &sh, u
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float gg = fminf(bf16r(v[q] * HAD_SCALE * sc[q]), a.limit);
-                    sg[q] = bf16r(gg / (1.f + expf(-gg)));
+                    sg[q] = bf16r(silu(gg));
                 }
             }
         }

@@ -108,6 +108,43 @@ def test_windows_of_large_handles(pkg, synth, cuda, H, I, E, S):
         assert launches(pkg, large, *args) == launches(pkg, small, *args) == 1
 
 
+# members of the experts: one, and around the MMAs' and slabs' sizes of the GEMMs, of which 32, 64 and more rows have different numbers of
+# partial sums on the way at once; the shared expert has all 128 rows
+FINE_COUNTS = (1, 31, 32, 33, 64, 65, 96, 97, 93)
+
+
+@pytest.mark.parametrize("H,I", [(256, 256), (512, 768), (768, 512), (1024, 2304), (2048, 512), (2304, 256), (3072, 256), (4096, 256), (256, 4096)])
+def test_chunks_are_as_exact_as_windows(pkg, oracle, synth, cuda, H, I):
+    # beyond the line a chunk of up to 128 rows goes to the GEMMs, whose sums are then chains of at most 512 k like the streamed kernel's: as near
+    # to sums in 64 bits (oracle mode 1) as the same rows in windows of 16.  What separates either from those are bf16 roundings that fall the
+    # other way, some hundred of a run, so the two distances agree to a tenth or so; one chain over K = 2048 is 2 to 4 times as far.
+    import torch
+    rows, S, E = 128, 5, len(FINE_COUNTS)
+    bank = synth.expert_bank(81 + H + I, H, I, E, svh_scale=True)
+    dbank = synth.to_device(bank, cuda)
+    order = np.repeat(np.arange(E, dtype=np.int32), FINE_COUNTS)         # (no expert twice in a row: none has more than 128 members)
+    picks = np.concatenate([order.reshape(S - 1, rows).T, np.full((rows, 1), E, np.int32)], 1).astype(np.int32)
+    x, rw = synth.activations_bf16(82, rows, H), np.full((rows, S), 0.25, np.float32)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd, pd, wd = t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw)
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=rows))
+    Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1).reshape(rows, S, H)
+
+    def run(lo, n):
+        moe.run(dbank, xd[lo:], pd[lo:], wd[lo:], n)
+        torch.cuda.synchronize()
+        assert int(moe.status.cpu()[0]) == 0
+        return pkg._view(moe.pairs_ptr.value, (n, S, H), torch.float32).cpu().numpy().copy()
+    assert launches(pkg, moe, dbank, xd, pd, wd, rows) > 1
+    chunk, windows = run(0, rows), np.concatenate([run(lo, 16) for lo in range(0, rows, 16)])
+    # (one flipped rounding moves a product of up to 8 times the rms by 2^-8, and with weights of up to 3.5 times theirs an element of a sum of
+    # I >= 256 products by 2^-8 * 8 * 3.5 / (4 sqrt(256)) = 1.7e-3 of the largest; a lost or doubled chain by much more)
+    emax, erms = rel_err(chunk, Y)
+    assert emax < 4e-3 and erms < TOL, (emax, erms)
+    off = [(np.linalg.norm(y - Y, axis=2) / np.linalg.norm(Y, axis=2)).mean() for y in (chunk, windows)]
+    assert off[0] < 1.5 * off[1], off
+
+
 @pytest.mark.parametrize("rows", [1, 8, 16])
 @pytest.mark.parametrize("shared_rows", [(512, 1024), (3, 6), (0, 1), (5, 64), (0, 64)])
 @pytest.mark.parametrize("share", [{}, dict(expert_lo=2, expert_hi=7)])
