@@ -199,7 +199,9 @@ __global__ void __launch_bounds__(FG_MAXU) fast_plan_kernel(const int *__restric
 // (6 TB/s).  With 16 values a lane, three butterflies across lanes and the vector read and converted for every row: 67 us at 4096 rows x 2048 x
 // 5 pairs x 2 matrices (168 MB written) and 237 us at 8192 x 4096 x 8 x 1 (537 MB); now 53 and 160.  More warps with fewer registers spill
 // (71 and 225), several waves of blocks change nothing.
+// HALVES: the sign / scale vectors are 2-byte aligned only (the streamed kernel takes such vectors, and so do short calls here).
 constexpr int ROT_WARPS = 4;
+template <bool HALVES>
 __global__ void __launch_bounds__(ROT_WARPS * 32, 4) fast_rot_kernel(const __nv_bfloat16 *__restrict__ x, int x_stride, const int *__restrict__ plan,
                                                                  const int *__restrict__ row_expert, const __half *__restrict__ suh0,
                                                                  const __half *__restrict__ suh1, __half *__restrict__ out0,
@@ -239,8 +241,9 @@ __global__ void __launch_bounds__(ROT_WARPS * 32, 4) fast_rot_kernel(const __nv_
         if (here && (code & 1023) != e) {
             e = code & 1023;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {                                 // (8-byte aligned at least)
-                const uint32_t h = __ldg(reinterpret_cast<const uint32_t *>(suh + (size_t)e * K + k + 32 * (i >> 2)) + (i & 3));
+            for (int i = 0; i < 16; ++i) {
+                const __half *q = suh + (size_t)e * K + k + 32 * (i >> 2) + 2 * (i & 3);
+                const uint32_t h = HALVES ? __half_as_ushort(__ldg(q)) | (uint32_t)__half_as_ushort(__ldg(q + 1)) << 16 : __ldg(reinterpret_cast<const uint32_t *>(q));
                 sv[i] = __half22float2(*reinterpret_cast<const __half2 *>(&h));
             }
         }
@@ -1071,7 +1074,8 @@ int gf::fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_
     GF_REQUIRE(x_stride >= c.hidden && x_stride % 4 == 0, "x_stride must be >= hidden and a multiple of 4");
     fine = fine && rows <= FG_FINE_ROWS;
     GF_REQUIRE(((uintptr_t)w->gt | (uintptr_t)w->ut | (uintptr_t)w->dt) % 16 == 0, "trellis tensors must be 16-byte aligned");
-    GF_REQUIRE(((uintptr_t)input | (uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 8 == 0, "input and scale vectors must be 8-byte aligned");
+    const bool aligned = ((uintptr_t)w->suh_g | (uintptr_t)w->suh_u) % 8 == 0;
+    GF_REQUIRE((uintptr_t)input % 8 == 0 && (aligned || fine), "input and scale vectors must be 8-byte aligned");
     cudaStream_t s = (cudaStream_t)stream;
     const int H = c.hidden, I = c.inter;
     const long P = (long)rows * c.slots;
@@ -1082,7 +1086,7 @@ int gf::fast_experts_run(glmflash_fast_experts *f, void *stream, const glmflash_
             return -1;
     const int mats = shared_x ? 1 : 2;
     if (f->phases & 2)
-        if (launch_k(fast_rot_kernel, dim3((unsigned)rot_blocks(P, H, mats, f->sms), (unsigned)mats), dim3(ROT_WARPS * 32), 0, s, pdl, (const __nv_bfloat16 *)input, x_stride,
+        if (launch_k(aligned ? fast_rot_kernel<false> : fast_rot_kernel<true>, dim3((unsigned)rot_blocks(P, H, mats, f->sms), (unsigned)mats), dim3(ROT_WARPS * 32), 0, s, pdl, (const __nv_bfloat16 *)input, x_stride,
                      f->plan, f->row_expert, (const __half *)w->suh_g, (const __half *)w->suh_u, f->xg, f->xu, H,
                      ((uintptr_t)input % 16 == 0 && x_stride % 8 == 0)))
             return -1;

@@ -145,6 +145,32 @@ def test_chunks_are_as_exact_as_windows(pkg, oracle, synth, cuda, H, I):
     assert off[0] < 1.5 * off[1], off
 
 
+@pytest.mark.parametrize("rows", [1, 16, 17, 18, 100, 128])
+def test_scale_vectors_at_any_address(pkg, synth, cuda, rows):
+    # the layer's calls of up to 128 rows take scale vectors that are 2-byte aligned only, on either side of the line: the bytes of
+    # aligned ones
+    import torch
+    H, I, E, S = 512, 256, 11, 6
+    dbank = synth.to_device(synth.expert_bank(91, H, I, E, svh_scale=True), cuda)
+    odd = dict(dbank)
+    for i, name in enumerate(n for n in dbank if n[:3] in ("suh", "svh")):
+        wide = torch.zeros(dbank[name].numel() + 8, dtype=dbank[name].dtype, device=cuda)
+        at = 1 + i % 3                                           # 2, 4 and 6 bytes
+        odd[name] = wide[at:at + dbank[name].numel()].view_as(dbank[name]).copy_(dbank[name])
+        assert odd[name].data_ptr() % 8 == 2 * at
+    x, (picks, rw) = synth.activations_bf16(92, rows, H), synth.route(93, rows, E, S - 1)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd, pd, wd = t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw)
+    moe, out = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=128)), []
+    for b in (dbank, odd):
+        moe.output.fill_(float("nan"))
+        moe.run(b, xd, pd, wd, rows)
+        torch.cuda.synchronize()
+        assert int(moe.status.cpu()[0]) == 0
+        out.append(moe.output[:rows].clone().view(torch.int32))
+    assert torch.equal(*out)
+
+
 @pytest.mark.parametrize("rows", [1, 8, 16])
 @pytest.mark.parametrize("shared_rows", [(512, 1024), (3, 6), (0, 1), (5, 64), (0, 64)])
 @pytest.mark.parametrize("share", [{}, dict(expert_lo=2, expert_hi=7)])
