@@ -103,18 +103,23 @@ bool gf::one_launch_selected() {
 }
 
 // Calls up to this many rows go to the streamed kernel on a handle for more than 16.  Windows of up to 16 always do, as on a handle of their
-// own: one launch, and the bytes do not depend on the handle (16 experts of 2048 x 1536, top-6: 1 row 26 us a layer against 56 by the GEMMs,
-// 16 rows 61 | 83; 384 of 1024 x 1024, top-8: 21 | 56 and 105 | 152; 8 of 2048 x 768, top-8: 25 | 52 and 42 | 53; behind the
-// GEMMs where a row takes all of 16 experts: 1024 x 1024, 30 | 48 and 66 | 49).  Longer ones: the kernel
-// decodes an expert's weights once per 16 of its rows and adds partial sums for every row (the GEMMs: once per 320, for a fixed 35 us of
-// kernels in front and behind).  us a layer, streamed | GEMMs: 2048 x 1536,
-// 64 experts, top-4: 17 rows 120 | 144, 64: 186 | 197, 80: 205 | 206, 128: 251 | 210; eight experts of 64: 80: 59 | 60; 1024 x 2048, 24
-// experts, top-3: 48: 75 | 80, 64: 86 | 81; 1536 x 768, 100, top-5: 112: 142 | 147, 128: 151 | 146; 3072 x 1024, 16, top-2: 48: 75 | 75.  The
-// lines cross at five to seven rows per routed expert: 5.5 here, at most 128 rows, and none above 16 where the exchange areas, which grow with
-// the rows, would pass 256 MB.  With many experts the chunk's tables leave no room for the second CTA of an SM, and the GEMMs win earlier
-// (4096 x 512, 288 experts, top-8: 17 rows 190 | 222, 24: 298 | 280, 40: 416 | 385, 128: 717 | 522; 18 rows are the last of two CTAs).
+// own: one launch, and the bytes do not depend on the handle (us a layer, streamed | GEMMs: 16 experts of 2048 x 1536, top-6: 1 row 26 | 56, 16
+// rows 61 | 83; 384 of 1024 x 1024, top-8: 21 | 56 and 105 | 152; 8 of 2048 x 768, top-8: 25 | 52 and 42 | 53; behind the GEMMs where a row
+// takes all of 16 experts: 1024 x 1024, 30 | 48 and 66 | 49).  For longer ones the kernel decodes an expert's weights once per 16 of its rows
+// and adds partial sums for every row (the GEMMs: once per 320, for a fixed 35 us of kernels in front and behind, which weigh the more rows
+// the smaller an expert is).  us a layer, streamed | GEMMs, and the rows per routed expert where the lines cross:
+//   2048 x 1536, 64 experts, top-4: 64 rows 190 | 195, 80: 204 | 204, 128: 253 | 210     5.0     512 x 1024, 16, top-6: 24: 39 | 40, 32: 45 | 40     9.7
+//   2304 x 2048, 32, top-4: 44: 160 | 161, 52: 171 | 161     5.6                           1024 x 512, 48, top-5: 100: 65 | 70, 128: 75 | 70     12
+//   3072 x 1024, 16, top-2: 40: 71 | 73, 48: 74 | 74     5.8                               1536 x 256, 30, top-2: 96: 42 | 57, 128: 50 | 60     > 8.5
+//   1024 x 2048, 24, top-3: 54: 79 | 82, 64: 86 | 82     7.3                               512 x 512, 32, top-3: 60: 34 | 38, 90: 43 | 42     8.2
+//   1536 x 768, 100, top-5: 112: 140 | 149, 128: 150 | 150     6.4                         512 x 256, 64, top-8: 40: 34 | 40, 60: 42 | 41     7.2
+// Hence 4.5 + 3 * 2^20 / (hidden * inter) rows per routed expert, 8 at most; at most 128 rows, and none above 16 where the exchange areas, which
+// grow with the rows, would pass 256 MB.  With many experts the chunk's tables leave no room for the second CTA of an SM, and the GEMMs win earlier
+// (4096 x 512, 288 experts, top-8: 18 rows, the last of two CTAs, 200 | 263, 19: 259 | 266, 24: 307 | 292, 40: 417 | 388; 1024 x 1024, 128,
+// top-8: 60: 132 | 147, 80: 200 | 152).
 static int short_chunk_rows(const glmflash_config &c) {
-    size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)11 * c.experts / (2 * (c.slots - 1)), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
+    const double per_expert = std::min(8., 4.5 + (3 << 20) / ((double)c.hidden * c.inter));
+    size_t rows = std::min<size_t>({(size_t)c.max_rows, ST_MAX_ROWS, (size_t)(per_expert * c.experts / (c.slots - 1)), ((size_t)256 << 20) / stream_chunk_row_bytes(c)});
     while (rows > 16 && !stream_chunk_pairs(c, (int)rows)) --rows;
     return (int)std::max<size_t>(rows, 16);
 }

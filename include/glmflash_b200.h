@@ -174,8 +174,9 @@ typedef struct glmflash_moe glmflash_moe;
  * (read when an owner is created) selects an alternative one-launch kernel, which also carries the cross-GPU exchange of
  * glmflash_moe_run_ep; on one GPU it is slower.
  * A handle for more rows serves calls of up to 16 rows by that launch as well, whatever its experts and slots, and with the bytes of
- * a handle for 16; and longer ones of up to min(128, 5.5 experts / (slots - 1)) rows (with several hundred experts fewer: the launch's
- * tables grow with them; 18 rows of 288 experts, slots 9).  For them such a handle holds, beside the prefill scratch, exchange words of
+ * a handle for 16; and longer ones of up to min(128, r experts / (slots - 1)) rows, r = min(8, 4.5 + 3 * 2^20 / (hidden inter)) rows per
+ * routed expert (with several hundred experts fewer: the launch's tables grow with them; 18 rows of 288 experts, slots 9).  For them
+ * such a handle holds, beside the prefill scratch, exchange words of
  *   8 slots (2 ceil(hidden / 512) inter + ceil(inter / 512) hidden + hidden + inter / 2) bytes
  * for each of these rows, at most about 256 MB, and never less than a handle for 16 rows: 850 KB a row, 75 MB a handle
  * at hidden 2048, inter 1536, 64 experts, slots 5. */

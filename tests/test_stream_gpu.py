@@ -108,6 +108,19 @@ def test_windows_of_large_handles(pkg, synth, cuda, H, I, E, S):
         assert launches(pkg, large, *args) == launches(pkg, small, *args) == 1
 
 
+@pytest.mark.parametrize("H,I,E,S,last", [(1536, 256, 30, 3, 120), (1024, 1024, 20, 5, 37), (1024, 2048, 12, 4, 24), (512, 512, 64, 3, 128)])
+def test_line_between_the_kernels(pkg, synth, cuda, H, I, E, S, last):
+    # one launch up to 4.5 + 3 * 2^20 / (H I) rows per routed expert, at most 8 (128 rows): small experts have the line later
+    import torch
+    dbank = synth.to_device(synth.expert_bank(64 + H, H, I, E, svh_scale=True), cuda)
+    x, (picks, rw) = synth.activations_bf16(65, last + 1, H), synth.route(66, last + 1, E, S - 1)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    xd, pd, wd = t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw)
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=512))
+    assert launches(pkg, moe, dbank, xd, pd, wd, last) == 1
+    assert launches(pkg, moe, dbank, xd, pd, wd, last + 1) > 1
+
+
 # members of the experts: one, and around the MMAs' and slabs' sizes of the GEMMs, of which 32, 64 and more rows have different numbers of
 # partial sums on the way at once; the shared expert has all 128 rows
 FINE_COUNTS = (1, 31, 32, 33, 64, 65, 96, 97, 93)
