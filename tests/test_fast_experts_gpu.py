@@ -188,7 +188,25 @@ def test_prefill_config4_vs_upstream(pkg, oracle, synth, cuda, bank, dbank, bank
 EDGES = (1, 2, 31, 32, 33, 64, 65, 128, 129, 159, 160, 161, 191, 192, 193, 224, 225, 255, 256, 257, 287, 288, 289, 319, 320, 321, 513, 641)
 
 
-@pytest.mark.parametrize("h,i,slots", [(256, 512, 2), (768, 256, 2), (2048, 512, 2), (512, 768, 3), (2304, 256, 2)])
+def plan_cap(counts, inter):
+    """Most rows of a chunk by the plan's rule: what the gate / up items cost the CTA pairs that have the longest of every turn, 1,000 clocks a
+    stage for the decode or 141 per 32 rows for the MMAs, with chunks of 320 and of 160 rows."""
+    import torch
+    workers, nbp, cost = torch.cuda.get_device_properties(0).multi_processor_count // 2, inter // 256, []
+    for cap in (320, 160):
+        pieces = [(c, -(-c // cap)) for c in counts if c]
+        items = sorted((-(-(-(-c // n)) // 32) for c, n in pieces for _ in range(n * nbp)), reverse=True)
+        cost.append(sum(max(1000, 141 * k) for k in items[::workers]))
+    return 160 if cost[1] < cost[0] else 320
+
+
+def chunks_of(pkg, fe):
+    import torch
+    return int(pkg._view(fe.plan.data_ptr(), (3,), torch.int32).cpu()[2])
+
+
+# (inter 256: 160 rows a chunk by the plan's rule, the others 320)
+@pytest.mark.parametrize("h,i,slots", [(256, 512, 2), (768, 256, 2), (2048, 512, 2), (512, 768, 3), (2304, 256, 2), (768, 1024, 2), (2304, 768, 2)])
 def test_chunk_edges(pkg, oracle, synth, cuda, h, i, slots):
     """A row's bytes do not depend on how many rows its expert has: all experts at once against pieces of 100 rows, and a sample
     against the oracle."""
@@ -215,6 +233,8 @@ def test_chunk_edges(pkg, oracle, synth, cuda, h, i, slots):
     fe = pkg.FastExperts(pkg.make_config(h, i, e1, slots, max_rows=rows, shared_exl3=0))
     full = run(fe, np.arange(rows))
     assert np.isfinite(full).all()
+    counts = np.bincount(picks[:, :-1].ravel(), minlength=e1)
+    assert plan_cap(counts, i) == (160 if i == 256 else 320) and chunks_of(pkg, fe) == sum(-(-c // plan_cap(counts, i)) for c in counts)
     order = rng.permutation(rows)
     for lo in range(0, rows, 100):
         sel = order[lo:lo + 100]
@@ -247,12 +267,12 @@ def test_input_rows_of_odd_strides(pkg, oracle, synth, cuda, h):
     assert (got[0] == got[1]).all()
 
 
-@pytest.mark.parametrize("rows,e", [(500, 64), (900, 64), (3000, 16), (40, 3)])
-def test_chunk_length(pkg, oracle, synth, cuda, rows, e):
+@pytest.mark.parametrize("rows,e,i,cap", [(500, 64, 512, 160), (900, 64, 512, 160), (3000, 16, 512, 160), (40, 3, 512, 320), (2500, 16, 768, 320), (2500, 24, 1536, 320)])
+def test_chunk_length(pkg, oracle, synth, cuda, rows, e, i, cap):
     """The plan cuts chunks of 160 rows where a few long experts would hold up the rest, else of 320: the rows are all there once, and their
     bytes are those of the other cut (a call of fewer experts' rows at a time)."""
     import torch
-    h, i, s = 512, 512, 3
+    h, s = 512, 3
     wd = synth.to_device(synth.expert_bank(79, h, i, e, svh_scale=True), cuda)
     x = synth.activations_bf16(8, rows, h)
     picks, _ = synth.route(9, rows, e, s - 1, uniform=True)
@@ -272,6 +292,8 @@ def test_chunk_length(pkg, oracle, synth, cuda, rows, e):
     counts = np.bincount(picks.ravel(), minlength=e + 1)
     plan = fe.plan.cpu().numpy()
     assert plan[1] == counts.sum() and plan[0] == (-(-counts // 128)).sum()
+    # (at 148 SMs; the sets that take 320 have an expert longer than 160 rows, but for the smallest, whose cut is the same)
+    assert plan_cap(counts, i) == cap and chunks_of(pkg, fe) == (-(-counts // cap)).sum()
     for lo in range(0, rows, 150):
         sel = np.arange(lo, min(rows, lo + 150))
         assert (run(sel).view(np.uint32) == full[sel].view(np.uint32)).all()

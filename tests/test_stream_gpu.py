@@ -36,13 +36,52 @@ def test_edges_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows):
 @pytest.mark.parametrize("H,I,E,S,rows,kw", [(256, 512, 3, 3, 17, {}), (512, 512, 40, 9, 40, {}), (768, 512, 8, 2, 128, {}),
                                              (512, 512, 12, 4, 64, dict(expert_lo=1, expert_hi=9, shared_rows=(10, 50)))])
 def test_short_chunks_vs_oracle(pkg, oracle, synth, cuda, H, I, E, S, rows, kw):
-    # more than 16 rows: experts with one member, with a whole number of sixteens and with a remainder; a rank's share
+    # chunks of many rows an expert: the GEMMs in fine steps (40 experts: at the line, streamed); a repeated pick, a rank's share
     bank = synth.expert_bank(51 + H + rows, H, I, E, svh_scale=True)
     x, (picks, rw) = synth.activations_bf16(52, rows, H), synth.route(53, rows, E, S - 1)
     if S > 2:
         picks[3, 1] = picks[3, 0]                        # a repeated pick is not computed again
         rw[3, 1] = 0
     got = run(pkg, cuda, synth.to_device(bank, cuda), x, picks, rw, H, I, E, S, rows, synth, **kw)
+    Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1).reshape(rows, S, H)
+    lo, hi = kw.get("expert_lo", 0), kw.get("expert_hi", E)
+    r0, r1 = kw.get("shared_rows", (0, rows))
+    here = (picks >= lo) & (picks < hi) | (picks == E) & (np.arange(rows)[:, None] >= r0) & (np.arange(rows)[:, None] < r1)
+    want = np.where(here[..., None], np.where((np.arange(S) == S - 1)[None, :, None], 1, rw[..., None]) * Y, 0).sum(1)
+    emax, erms = rel_err(got, want)
+    assert emax < TOL and erms < TOL, (emax, erms)
+
+
+def launches(pkg, moe, *args):
+    """Kernels of one call, counted as the nodes of its graph."""
+    import torch
+    cache, side = pkg.GraphCache(bounded=True), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    cache.run(1, lambda: moe.run(*args), stream=side)
+    side.synchronize()
+    return cache.stats()["retained_nodes"]
+
+
+@pytest.mark.parametrize("H,I,E,rows,kw", [(256, 512, 24, 17, {}), (512, 512, 24, 40, {}), (768, 256, 48, 101, {}), (512, 768, 48, 128, {}),
+                                           (512, 512, 24, 40, dict(expert_lo=1, expert_hi=19, shared_rows=(10, 30)))])
+def test_streamed_chunks_with_popular_experts(pkg, oracle, synth, cuda, H, I, E, rows, kw):
+    # few rows an expert on average, so that the chunk is streamed, but three that most rows pick: whole sixteens of members, a remainder, one more
+    # than a sixteen; and a repeated pick, which is not computed again
+    import torch
+    S = 4
+    bank = synth.expert_bank(54 + H + rows, H, I, E, svh_scale=True)
+    x, (_, rw) = synth.activations_bf16(52, rows, H), synth.route(53, rows, E, S - 1)
+    rng = np.random.default_rng(55)
+    picks = np.stack([np.append(8 + rng.permutation(E - 8)[:S - 1], E) for _ in range(rows)]).astype(np.int32)
+    picks[:rows - 3, 0] = 5
+    picks[:max(16, (rows - 4) // 16 * 16), 1] = 6
+    picks[rows - 17:, 2] = 7
+    picks[3, 1], rw[3, 1] = picks[3, 0], 0
+    dbank = synth.to_device(bank, cuda)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    moe = pkg.Moe(pkg.make_config(H, I, E, S, max_rows=rows, **kw))
+    assert launches(pkg, moe, dbank, t(x.view(np.int16)).view(torch.bfloat16), t(picks), t(rw), rows) == 1
+    got = run(pkg, cuda, dbank, x, picks, rw, H, I, E, S, rows, synth, **kw)
     Y = oracle.experts_run_rows(bank, H, I, E + 1, S, x, picks, mode=1).reshape(rows, S, H)
     lo, hi = kw.get("expert_lo", 0), kw.get("expert_hi", E)
     r0, r1 = kw.get("shared_rows", (0, rows))
@@ -71,16 +110,6 @@ def test_chunks_on_both_sides_of_the_line(pkg, oracle, synth, cuda, H, I, E, S, 
         scale = max(scale, np.abs(want).max())
         off.append(np.abs(got - want).max(1))
     assert np.min(off, axis=0).max() < TOL * scale
-
-
-def launches(pkg, moe, *args):
-    """Kernels of one call, counted as the nodes of its graph."""
-    import torch
-    cache, side = pkg.GraphCache(bounded=True), torch.cuda.Stream()
-    torch.cuda.synchronize()
-    cache.run(1, lambda: moe.run(*args), stream=side)
-    side.synchronize()
-    return cache.stats()["retained_nodes"]
 
 
 @pytest.mark.parametrize("H,I,E,S", [(512, 512, 16, 7), (256, 256, 384, 9), (256, 256, 4, 3), (512, 256, 2, 2), (256, 512, 16, 17), (256, 256, 200, 11)])
