@@ -347,7 +347,7 @@ def exl3_linear(x, words, suh, svh, K, N, stream=None):
     rows = x.shape[0]
     if K <= 0 or N <= 0 or K % 256 or N % 128:
         raise GlmFlashError("unsupported linear shape")
-    y = x.new_empty((rows, N), dtype=torch.float16)             # (0.6 us less than torch.empty with a device argument)
+    y = x.new_empty((rows, N), dtype=torch.float16)             # (0.5 us less than torch.empty with a device argument)
     # the kernel keeps nothing in the scratch argument: any 256-byte aligned device address serves, and y outlives the call
     _check(lib().glmflash_exl3_linear(_stream_ptr(stream), x.data_ptr(), rows, words.data_ptr(), suh.data_ptr(),
                                       svh.data_ptr(), K, N, y.data_ptr(), y.data_ptr()))

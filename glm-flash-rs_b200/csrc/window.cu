@@ -74,7 +74,6 @@ constexpr int WIN_TEAM_BYTES = WIN_NBUF * WIN_WBUF + WIN_ACT + WIN_SCR;
 constexpr int WIN_BARS = WIN_NBUF * (WIN_NG + 1);             // per team: copy barriers and one "consumed" barrier per buffer
 constexpr int WIN_UMAX = 160;                                 // distinct experts of a window the tables hold
 constexpr int WIN_QMAX = 32;                                  // deferred exchange blocks a team can hold (its F items)
-constexpr int WIN_MAXSPLIT = 32;                              // splits per projection the split-sum scratch handles (K <= 4096)
 constexpr size_t WIN_SMEM = (size_t)WIN_TEAMS * WIN_TEAM_BYTES + WIN_TEAMS * WIN_BARS * 8;
 constexpr uint32_t WIN_POLLS = 2000000u;                      // bound of every spin in the kernel (a fraction of a second)
 
@@ -860,7 +859,6 @@ __global__ void __launch_bounds__(WIN_THREADS, 1) window_kernel(const __grid_con
 
     const int tid = threadIdx.x, team = win_team(), warp = win_warp(), lane = tid & 31;
     const bool service = warp == WIN_CW;
-    unsigned char *tbase = smem + (size_t)team * WIN_TEAM_BYTES;
     // per team: full[buffer][group] count copied bytes; done[buffer] counts the compute warps that are through with it
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)WIN_TEAMS * WIN_TEAM_BYTES) + team * WIN_BARS;
     uint64_t *done = full + WIN_NBUF * WIN_NG;
