@@ -38,7 +38,7 @@ int check_config(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limi
 
 using namespace gf;
 
-// max_rows_limit: 16 for the public owner.  Chunk owners keep one for their short chunks, whose pair rows are the chunk owner's and
+// max_rows_limit: 16 for the public owner.  Chunk owners keep one for their windows and short chunks, whose pair rows are the chunk owner's and
 // whose down inputs nobody reads afterwards.
 int gf::experts_new(const glmflash_config *cfg, size_t cfg_bytes, int max_rows_limit, glmflash_experts **out) {
     GF_REQUIRE(out != nullptr, "out is null");
